@@ -8,9 +8,11 @@
 //   linear_tc       more rows: tcgen05 GEMM. Weights are the MMA's A operand (128 rows), activations its B operand
 //                   (32–256 rows), both loaded by TMA into 128-byte-swizzled stages; accumulator in tensor memory.
 //                   Grids that would leave SMs idle are cut along k; `linear_reduce` adds the pieces in order.
-//   linear_simt     f32 (true 32-bit), and bf16 shapes whose rows are not 16-byte aligned.
+//   linear_rows_f32 f32 (true 32-bit), up to 32 rows: warps stream whole weight rows.
+//   linear_f32      f32, more rows: register-blocked tiles.
+//   linear_simt     f32 and bf16 shapes whose rows are not 16-byte aligned.
 //
-// linear_tc and linear_simt also run grouped: activation rows sorted by group, one weight matrix per group, the groups'
+// linear_tc, linear_f32 and linear_simt also run grouped: activation rows sorted by group, one weight matrix per group, the groups'
 // row counts known on the device only. A CTA finds its group from the counts; the grid covers the most tiles
 // that any counts can give.
 //
@@ -623,7 +625,7 @@ template <int EPI> __global__ void __launch_bounds__(kTcThreads) linear_tc(const
 
 // Adds the pieces of a product that was cut along k, in piece order, with bias and gating. blockIdx.y is the activation
 // row; V consecutive weight rows per thread (V = 4: out is a multiple of 4).
-template <int V> __global__ void __launch_bounds__(256) linear_reduce(const __grid_constant__ LinP p) {
+template <int V, typename T = bf16> __global__ void __launch_bounds__(256) linear_reduce(const __grid_constant__ LinP p) {
     pdl_enter();
     const long long row = blockIdx.y, o = ((long long)blockIdx.x * 256 + threadIdx.x) * V;
     if (o >= p.out) return;
@@ -650,7 +652,7 @@ template <int V> __global__ void __launch_bounds__(256) linear_reduce(const __gr
         for (int e = 0; e < V; e++) s[e] += p.bias[o + e];
     if (!p.glu)
 #pragma unroll
-        for (int e = 0; e < V; e++) s[e] = activate(p, o + e, s[e]) * factor<bf16>(p, row, o + e);
+        for (int e = 0; e < V; e++) s[e] = activate(p, o + e, s[e]) * factor<T>(p, row, o + e);
     if (p.glu) {  // out is even, and so are o and V
 #pragma unroll
         for (int e = 0; e < V; e += 2) put(p, row, p.out / 2, (o + e) / 2, glu_value(p, s[e], s[e + 1]));
@@ -660,6 +662,191 @@ template <int V> __global__ void __launch_bounds__(256) linear_reduce(const __gr
 #pragma unroll
         for (int e = 0; e < V; e++)
             if (o + e < p.out) put(p, row, p.out, o + e, s[e]);
+    }
+}
+
+// ───────────────────────────── 32-bit ───────────────────────────────────
+__device__ __forceinline__ float4 ld4_f32(const float* p, bool wide) {
+    return wide ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+__device__ __forceinline__ float4 ld4_stream(const float* p) {
+    float4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
+// Up to eight activation rows per blockIdx.y (M of them formed): bound by the weights' bytes. A warp owns R weight rows and takes 128
+// consecutive k of each (512 bytes) per step, the next step's weights ahead of this step's sums; `nb` warps of a CTA share the same
+// rows and take the steps in turn where there are few rows. Lanes keep sums of their own (chains 32 times shorter than one thread's),
+// which fold over lanes at the end: value m · R + r ends up in lane m · R + r. Activations come through L1.
+// 3 rows, k 1152, 13 824 weight rows (64 MB): 25 µs, 2.6 TB/s; k 6912, 1152 weight rows: 12 µs. One 64 × 64 tile per CTA (linear_simt), a
+// grid of out / 64 CTAs that each walk all of k: 250 and 1175 µs.
+template <int M, int R> __global__ void __launch_bounds__(kThreads, 2) linear_rows_f32(const __grid_constant__ LinP p) {
+    constexpr int N = M * R;
+    __shared__ float red[kStreamWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, share = p.nb, slice = warp % share;
+    const int block_units = (int)((p.out + R - 1) / R);
+    const long long unit = (long long)blockIdx.x * (kStreamWarps / share) + warp / share;
+    const int block = p.blocks > 1 ? (int)(unit / block_units) : 0;
+    const bool live = unit < (long long)block_units * p.blocks;
+    const long long o0 = (unit - (long long)block * block_units) * R, w_at = block * p.out, x0 = p.x_off + block * p.x_step, row0 = (long long)blockIdx.y * 8;
+    const int rows = (int)min((long long)M, p.rows - row0);
+    const int c0 = (int)((p.k[0] + 127) / 128), chunks = live ? c0 + (int)((p.k[1] + 127) / 128) : 0;
+    const bool wide = ((reinterpret_cast<uintptr_t>(p.x[0]) | reinterpret_cast<uintptr_t>(p.x[1])) & 15) == 0;
+    float4 w[R];
+    auto fetch = [&](int c) {
+        const int op = c >= c0;
+        const long long k = (long long)(op ? c - c0 : c) * 128 + lane * 4;
+        const float* from = (const float*)p.w[op] + (w_at + o0) * p.k[op] + k;
+#pragma unroll
+        for (int r = 0; r < R; r++) w[r] = c < chunks && k < p.k[op] && o0 + r < p.out ? ld4_stream(from + r * p.k[op]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    pdl_trigger();
+    fetch(slice);  // constants: before the launches in front of this one are done
+    pdl_wait();
+    float acc[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) acc[i] = 0.f;
+    for (int c = slice; c < chunks; c += share) {
+        const int op = c >= c0;
+        const long long k = (long long)(op ? c - c0 : c) * 128 + lane * 4, ldx = p.ldx ? p.ldx : p.k[op];
+        const float* from = (const float*)p.x[op] + row0 * ldx + x0 + k;
+        float4 x[M], now[R];
+#pragma unroll
+        for (int m = 0; m < M; m++) x[m] = m < rows && k < p.k[op] ? ld4_f32(from + m * ldx, wide) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int r = 0; r < R; r++) now[r] = w[r];
+        fetch(c + share);
+#pragma unroll
+        for (int m = 0; m < M; m++)
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                float& a = acc[m * R + r];
+                a = fmaf(x[m].x, now[r].x, a);
+                a = fmaf(x[m].y, now[r].y, a);
+                a = fmaf(x[m].z, now[r].z, a);
+                a = fmaf(x[m].w, now[r].w, a);
+            }
+    }
+    // every step sends half of the values to the lanes that keep them; what is left of 32 / N lanes per value is added up
+#pragma unroll
+    for (int half = N / 2, o = N / 2; half >= 1; half /= 2, o /= 2)
+#pragma unroll
+        for (int i = 0; i < half; i++) {
+            const bool up = lane & o;
+            const float give = up ? acc[i] : acc[i + half], keep = up ? acc[i + half] : acc[i];
+            acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    float sum = acc[0];
+#pragma unroll
+    for (int o = 16; o >= N; o /= 2) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (share > 1) {
+        red[warp][lane] = sum;
+        __syncthreads();
+        if (slice) return;
+        sum = 0.f;
+        for (int i = 0; i < share; i++) sum += red[warp + i][lane];
+    }
+    const int m = lane / R, r = lane % R;
+    const long long o = o0 + r, row = row0 + m;
+    const bool mine = live && lane < N && m < rows && o < p.out;
+    if (p.bias && mine) sum += p.bias[w_at + o];
+    if (p.glu) {
+        const float up = __shfl_down_sync(0xffffffffu, sum, 1);
+        if (mine && !(r & 1) && o + 1 < p.out) put(p, row, p.out / 2, o >> 1, glu_value(p, sum, up));
+    } else if (mine) {
+        put(p, row, p.ldy, w_at + o, activate(p, w_at + o, sum) * factor<float>(p, row, w_at + o));
+    }
+}
+
+// More rows: 64 weight rows × 64 activation rows per CTA, 8 × 4 of them per thread, 16 k per step, the next step's operands in registers
+// while this one's are multiplied; bound by the FMA pipe (12 shared-memory words per 32 FMAs). Small grids are cut along k (blockIdx.z),
+// `linear_reduce` adds the pieces in order. k, ldx and x_off are multiples of 4. 303 rows: 31 – 33 TFLOP/s, 313 and 146 µs for the two sizes
+// above (linear_simt, one scalar shared-memory read per two FMAs and no cut along k: 569 and 1046 µs).
+constexpr int kF32Threads = 128;
+__global__ void __launch_bounds__(kF32Threads) linear_f32(const __grid_constant__ LinP p) {
+    __shared__ __align__(16) float ws[2][16][68], xs[2][16][68];
+    const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
+    const int block_tiles = (int)((p.out + 63) / 64), block = p.blocks > 1 ? (int)blockIdx.x / block_tiles : 0;
+    const long long m0 = (long long)((int)blockIdx.x - block * block_tiles) * 64, x0 = p.x_off + block * p.x_step, col0 = block * p.out;
+    long long n0 = (long long)blockIdx.y * 64, rows = p.rows, w_at = col0;  // w_at: first row of the group's or block's weights
+    pdl_enter();
+    if (p.groups) {
+        int group, row, live;
+        if (!locate_group(p, (int)blockIdx.y, 64, &group, &row, &live)) return;
+        n0 = row;
+        rows = row + live;
+        w_at = group * p.out;
+    }
+    const bool wide = ((reinterpret_cast<uintptr_t>(p.x[0]) | reinterpret_cast<uintptr_t>(p.x[1])) & 15) == 0;
+    const int s0 = (int)((p.k[0] + 15) / 16), all = s0 + (int)((p.k[1] + 15) / 16);
+    const int lo = (int)((long long)all * blockIdx.z / p.splits), hi = (int)((long long)all * (blockIdx.z + 1) / p.splits);
+    const int lr = tid >> 2, lk = (tid & 3) * 4;  // this thread loads rows lr and lr + 32, four k
+    float4 wv[2], xv[2];
+    auto fetch = [&](int s) {
+        const int op = s >= s0;
+        const long long k = (long long)(op ? s - s0 : s) * 16 + lk, ldx = p.ldx ? p.ldx : p.k[op];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int r = lr + j * 32;
+            const bool kl = s < hi && k < p.k[op];
+            wv[j] = kl && m0 + r < p.out ? *reinterpret_cast<const float4*>((const float*)p.w[op] + (w_at + m0 + r) * p.k[op] + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+            xv[j] = kl && n0 + r < rows ? ld4_f32((const float*)p.x[op] + (n0 + r) * ldx + x0 + k, wide) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    auto keep = [&](int b) {
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int r = lr + j * 32;
+            ws[b][lk][r] = wv[j].x;
+            ws[b][lk + 1][r] = wv[j].y;
+            ws[b][lk + 2][r] = wv[j].z;
+            ws[b][lk + 3][r] = wv[j].w;
+            xs[b][lk][r] = xv[j].x;
+            xs[b][lk + 1][r] = xv[j].y;
+            xs[b][lk + 2][r] = xv[j].z;
+            xs[b][lk + 3][r] = xv[j].w;
+        }
+    };
+    float acc[4][8] = {};  // [row][weight row: 4 tx …, 32 + 4 tx …]
+    fetch(lo);
+    keep(0);
+    __syncthreads();
+    for (int s = lo; s < hi; s++) {
+        const int b = (s - lo) & 1;
+        fetch(s + 1);
+#pragma unroll
+        for (int kk = 0; kk < 16; kk++) {
+            const float4 a = *reinterpret_cast<const float4*>(&xs[b][kk][ty * 4]), u = *reinterpret_cast<const float4*>(&ws[b][kk][tx * 4]),
+                         v = *reinterpret_cast<const float4*>(&ws[b][kk][32 + tx * 4]);
+            const float av[4] = {a.x, a.y, a.z, a.w}, bv[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        }
+        keep(b ^ 1);
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const long long row = n0 + ty * 4 + i;
+        if (row >= rows) continue;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const long long o = m0 + (j >> 2) * 32 + tx * 4 + (j & 3);
+            if (o >= p.out) continue;
+            if (p.splits > 1) {
+                p.partial[((size_t)blockIdx.z * p.rows + row) * p.ldy + col0 + o] = acc[i][j];
+                continue;
+            }
+            const float v = acc[i][j] + (p.bias ? p.bias[col0 + o] : 0.f);
+            if (p.glu) {
+                if (!(j & 1) && o + 1 < p.out) put(p, row, p.out / 2, o >> 1, glu_value(p, v, acc[i][(j + 1) & 7] + (p.bias ? p.bias[col0 + o + 1] : 0.f)));
+            } else {
+                put(p, row, p.ldy, col0 + o, activate(p, col0 + o, v) * factor<float>(p, row, col0 + o));
+            }
+        }
     }
 }
 
@@ -1067,6 +1254,46 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
     p.node = em.node;
     p.splits = 1;
     const Buf bx0 = fuse_norm ? kNull : x0->buf, bx1 = buf_of(x1), bw1 = buf_of(w1), bb = buf_of(bias);
+    const auto reduce = [&](const Buf& partial) {  // of a product that was cut along k
+        const bool wide = p.ldy % 4 == 0 && y.buf.off % 16 == 0;
+        const int v = wide ? 4 : p.ldy % 2 == 0 ? 2 : 1;  // gating needs pairs; out is even then
+        p.out = p.ldy;                                    // all blocks' columns
+        const auto k = tc_type ? (wide ? linear_reduce<4> : v == 2 ? linear_reduce<2> : linear_reduce<1>)
+                               : (wide ? linear_reduce<4, float> : v == 2 ? linear_reduce<2, float> : linear_reduce<1, float>);
+        em.launch(k, dim3((unsigned)((p.out + 256 * v - 1) / (256 * v)), (unsigned)d.rows), dim3(256), 0, p,
+                  {{&p.bias, bb}, {&p.y, y.buf}, {&p.mul, mul}, {&p.partial, partial}}, "linear_reduce", /*pdl=*/true);
+    };
+    const bool quads = d.k[0] % 4 == 0 && d.k[1] % 4 == 0 && p.ldx % 4 == 0 && d.x_off % 4 == 0 && d.x_step % 4 == 0 && w0.buf.off % 16 == 0 &&
+                       (!w1 || w1->buf.off % 16 == 0);
+    if (!tc_type && quads && d.rows <= 32) {
+        // Eight rows per pass over the weights. 32 rows (four passes) take the 83 µs of linear_f32's one tile of 64.
+        const int m = d.rows == 1 ? 1 : d.rows == 2 ? 2 : d.rows <= 4 ? 4 : 8;
+        auto units = [&](int r) { return (d.out + r - 1) / r * d.blocks; };
+        const bool eight = m < 8 && units(8) * kStreamWarps >= 16LL * sm_count();  // enough warps with eight weight rows each
+        const int r = eight ? 8 : 4;
+        const long long chunks = (d.k[0] + 127) / 128 + (d.k[1] + 127) / 128;
+        // warps per unit: until there are 16 per SM, with at least two steps for each
+        p.nb = 1;
+        while (p.nb < kStreamWarps && units(r) * p.nb < 16LL * sm_count() && chunks >= 4 * p.nb) p.nb *= 2;
+        const int per_cta = kStreamWarps / p.nb;
+        const auto k = m == 1 ? (eight ? linear_rows_f32<1, 8> : linear_rows_f32<1, 4>) : m == 2 ? (eight ? linear_rows_f32<2, 8> : linear_rows_f32<2, 4>)
+                     : m == 4 ? (eight ? linear_rows_f32<4, 8> : linear_rows_f32<4, 4>) : linear_rows_f32<8, 4>;
+        em.launch(k, dim3((unsigned)((units(r) + per_cta - 1) / per_cta), (unsigned)((d.rows + 7) / 8)), dim3(kThreads), 0, p,
+                  {{&p.mul, mul}, {&p.x[0], bx0}, {&p.x[1], bx1}, {&p.w[0], w0.buf}, {&p.w[1], bw1}, {&p.bias, bb}, {&p.y, y.buf}}, "linear_rows_f32", /*pdl=*/true);
+        return;
+    }
+    if (!tc_type && quads) {
+        const dim3 tiles((unsigned)((d.out + 63) / 64 * d.blocks), (unsigned)((d.rows + 63) / 64));
+        const long long steps = (d.k[0] + 15) / 16 + (d.k[1] + 15) / 16, ctas = (long long)tiles.x * tiles.y;
+        // five CTAs fit an SM; pieces of at least 16 steps until three per SM are there
+        while (p.splits < 8 && ctas * p.splits < 3LL * sm_count() && steps >= 32LL * p.splits && d.rows < 65536) p.splits *= 2;
+        const Buf partial = p.splits > 1 ? em.scratch((size_t)p.splits * d.rows * p.ldy * 4) : kNull;
+        em.launch(linear_f32, dim3(tiles.x, tiles.y, (unsigned)p.splits), dim3(kF32Threads), 0, p,
+                  {{&p.mul, mul}, {&p.x[0], bx0}, {&p.x[1], bx1}, {&p.w[0], w0.buf}, {&p.w[1], bw1}, {&p.bias, bb}, {&p.y, y.buf}, {&p.partial, partial}},
+                  "linear_f32", /*pdl=*/true);
+        if (p.splits > 1) reduce(partial);
+        return;
+    }
     if (!tc_type || !aligned) {
         const dim3 grid((unsigned)((d.out + 63) / 64 * d.blocks), (unsigned)((d.rows + 63) / 64));
         const auto k = tc_type ? linear_simt<bf16> : linear_simt<float>;
@@ -1154,14 +1381,7 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
         add_map(2, bx1, d.k[1], d.rows, (uint32_t)p.nb);
         add_map(3, bw1, d.k[1], d.out, 128u);
     }
-    if (p.splits > 1) {
-        const bool wide = p.ldy % 4 == 0 && y.buf.off % 16 == 0;
-        const int v = wide ? 4 : p.ldy % 2 == 0 ? 2 : 1;  // gating needs pairs; out is even then
-        p.out = p.ldy;                                    // all blocks' columns
-        em.launch(wide ? linear_reduce<4> : v == 2 ? linear_reduce<2> : linear_reduce<1>,
-                  dim3((unsigned)((p.out + 256 * v - 1) / (256 * v)), (unsigned)d.rows), dim3(256), 0, p,
-                  {{&p.bias, bb}, {&p.y, y.buf}, {&p.mul, mul}, {&p.partial, partial}}, "linear_reduce", /*pdl=*/true);
-    }
+    if (p.splits > 1) reduce(partial);
 }
 
 // One product per group of sorted rows.
@@ -1184,8 +1404,9 @@ void emit_grouped_linear(Emitter& em, const GroupedLinearDesc& d, const TRef& x,
     auto tiles_of = [&](int64_t size) { return std::min<int64_t>(d.rows / size + std::min(d.groups, d.rows), d.rows); };
     const bool tc_type = w.dtype == DT_BF16;
     if (!tc_type || d.k % 8 != 0) {
-        const auto k = tc_type ? linear_simt<bf16> : linear_simt<float>;
-        em.launch(k, dim3((unsigned)((d.out + 63) / 64), (unsigned)tiles_of(64)), dim3(256), 0, p,
+        const bool quads = !tc_type && d.k % 4 == 0 && w.buf.off % 16 == 0;
+        const auto k = quads ? linear_f32 : tc_type ? linear_simt<bf16> : linear_simt<float>;
+        em.launch(k, dim3((unsigned)((d.out + 63) / 64), (unsigned)tiles_of(64)), dim3(quads ? kF32Threads : 256), 0, p,
                   {{&p.x[0], x.buf}, {&p.x[1], kNull}, {&p.w[0], w.buf}, {&p.w[1], kNull}, {&p.bias, kNull}, {&p.y, y.buf}, {&p.counts, counts.buf}},
                   "grouped_simt", /*pdl=*/true);
         return;
