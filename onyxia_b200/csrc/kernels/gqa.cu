@@ -15,14 +15,15 @@
 //
 // Three launches, the key range split over CTAs in the last two:
 //   gqa_prepare  rotates q into scratch and writes the new K (rotated) / V rows
-//                into the present cache (copying the valid past unless the
-//                present buffer *is* the past buffer)
+//                into the present cache
 //   gqa_scores   one warp per key: q·k for the heads of one KV group, scaled,
 //                biased, stored as f32 rows of scratch; the last CTA of a query
 //                to finish reduces the row to (max, Σ exp)
 //   gqa_pv       one warp per key again: p = exp(s − max)/Σ, acc += p·v; the
 //                last CTA to finish adds the partial accumulators in split order
 //                and stores the output row
+// When the present buffer is not the past buffer, gqa_copy_past fills it first; what follows appends in place, with the decode kernels
+// where they take the shape.
 // "Last CTA" is decided by an arrival counter per query; nothing ever waits.
 //
 // KV tensors are [B, KV, T, D] views of buffers that hold `cap ≥ T` rows per
@@ -51,8 +52,6 @@ struct GqaPrepP {
     const void* q;
     const void* k;
     const void* v;
-    const void* past_k;
-    const void* past_v;
     const int* seqlens;
     const void* cos;
     const void* sin;
@@ -61,10 +60,10 @@ struct GqaPrepP {
     void* present_v;
     ErrWord* err;
     const long long* dyn_t;  // when set, the present length T is read from here
-    long long B, S, H, KV, D, P, T, past_cap, pres_cap, half, cache_rows;
+    long long B, S, H, KV, D, T, pres_cap, half, cache_rows;
     long long nq;    // threads that rotate q (0 without rotary)
-    long long nkv;   // threads that build the present caches
-    int in_place, node;
+    long long nkv;   // threads that write the new rows
+    int clear, node;  // clear: what lies beyond a ragged row's tokens is zeroed here (2: in front of them too)
 };
 
 template <int DT>
@@ -96,48 +95,77 @@ template <int DT> __global__ void gqa_prepare(const GqaPrepP p) {
             continue;
         }
         long long r = i - p.nq;
-        long long rows = p.in_place ? p.S : T;  // rows visited per (b, kv head)
-        long long e = r % p.D, t0 = (r / p.D) % rows, kvh = (r / (p.D * rows)) % p.KV, b = r / (p.D * rows * p.KV);
+        long long e = r % p.D, j = (r / p.D) % p.S, kvh = (r / (p.D * p.S)) % p.KV, b = r / (p.D * p.S * p.KV);
         long long tot = (long long)p.seqlens[b] + 1, past_b = tot - p.S > 0 ? tot - p.S : 0;
-        long long pres_base = (b * p.KV + kvh) * p.pres_cap * p.D, past_base = (b * p.KV + kvh) * p.past_cap * p.D;
-        auto new_k = [&](long long j) -> float {
-            long long base = ((b * p.S + j) * p.KV + kvh) * p.D;
-            if (p.half == 0) return ld<DT>(p.k, base + e);
-            long long row = past_b + j;
-            if (row >= p.cache_rows) {
-                report(p.err, ERR_GATHER_OOB, p.node, row, p.cache_rows);
-                row = 0;
-            }
-            return rope_elem<DT>(p.k, base, e, p.half, p.cos, p.sin, row);
-        };
-        auto new_v = [&](long long j) -> float { return ld<DT>(p.v, ((b * p.S + j) * p.KV + kvh) * p.D + e); };
-        if (p.in_place) {
-            // the buffer already holds the valid past; write the new rows ...
-            long long j = t0, t = past_b + j;
-            if (t < T) {
-                st<DT>(p.present_k, pres_base + t * p.D + e, new_k(j));
-                st<DT>(p.present_v, pres_base + t * p.D + e, new_v(j));
-            }
-            // ... and, for a ragged row, clear what lies beyond them
-            if (j == p.S - 1)
-                for (long long z = past_b + p.S; z < T; z++) {
-                    st<DT>(p.present_k, pres_base + z * p.D + e, 0.f);
-                    st<DT>(p.present_v, pres_base + z * p.D + e, 0.f);
+        long long pres_base = (b * p.KV + kvh) * p.pres_cap * p.D;
+        // the buffer already holds the valid past; write the new rows ...
+        const long long t = past_b + j;
+        if (t < T) {
+            const long long base = ((b * p.S + j) * p.KV + kvh) * p.D;
+            float k;
+            if (p.half == 0) {
+                k = ld<DT>(p.k, base + e);
+            } else {
+                long long row = t;
+                if (row >= p.cache_rows) {
+                    report(p.err, ERR_GATHER_OOB, p.node, row, p.cache_rows);
+                    row = 0;
                 }
-        } else {
-            long long t = t0;
-            float kv = 0.f, vv = 0.f;
-            if (t < p.P && t < past_b) {
-                kv = ld<DT>(p.past_k, past_base + t * p.D + e);
-                vv = ld<DT>(p.past_v, past_base + t * p.D + e);
-            } else if (t >= past_b && t < past_b + p.S) {
-                kv = new_k(t - past_b);
-                vv = new_v(t - past_b);
+                k = rope_elem<DT>(p.k, base, e, p.half, p.cos, p.sin, row);
             }
-            st<DT>(p.present_k, pres_base + t * p.D + e, kv);
-            st<DT>(p.present_v, pres_base + t * p.D + e, vv);
+            st<DT>(p.present_k, pres_base + t * p.D + e, k);
+            st<DT>(p.present_v, pres_base + t * p.D + e, ld<DT>(p.v, base + e));
+        }
+        // ... and, for a ragged row, clear what lies beyond them (and, in a new buffer without a past, in front of them)
+        if (p.clear && j == p.S - 1)
+            for (long long z = p.clear > 1 ? 0 : past_b + p.S; z < T; z++) {
+                if (z == past_b) z += p.S;
+                if (z >= T) break;
+                st<DT>(p.present_k, pres_base + z * p.D + e, 0.f);
+                st<DT>(p.present_v, pres_base + z * p.D + e, 0.f);
+            }
+    }
+}
+
+struct GqaCopyP {
+    const void* past[2];
+    void* present[2];
+    const int* seqlens;
+    long long S, P, T, past_cap, pres_cap, row_bytes;
+    int KV, parts, element;
+};
+
+// The valid past into a new buffer, zeros behind the rows that this step writes. blockIdx.y: keys or values; a (batch row, KV head) is
+// cut into `parts` CTAs; a thread has four 16-byte pieces in flight (rows that are no whole number of them go element by element).
+// Bound by HBM: 64 × 16 heads × 2048 rows of 128 f16, keys and values (1.07 GB read and written): 338 µs, 6.3 TB/s. One element per thread with 64-bit
+// divisions, as part of gqa_prepare, took 2230 µs.
+template <typename T> __device__ __forceinline__ void copy_past(const GqaCopyP& p, long long first, long long step, const char* src, char* dst, long long past_b) {
+    const long long per_row = p.row_bytes / (long long)sizeof(T), total = p.T * per_row, held = min(p.P, past_b) * per_row;
+    const long long fresh = past_b * per_row, after = (past_b + p.S) * per_row;  // the rows in between are this step's own
+    for (long long i = first; i < total; i += 4 * step) {
+        T v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const long long at = i + j * step;
+            v[j] = T{};
+            if (at < held) v[j] = reinterpret_cast<const T*>(src)[at];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const long long at = i + j * step;
+            if (at < total && (at < fresh || at >= after)) reinterpret_cast<T*>(dst)[at] = v[j];
         }
     }
+}
+__global__ void __launch_bounds__(256) gqa_copy_past(const GqaCopyP p) {
+    pdl_wait();  // (nothing behind this launch may read the new buffer ahead of its end: no early trigger)
+    const long long pair = blockIdx.x / p.parts, part = blockIdx.x % p.parts, b = pair / p.KV;
+    const char* src = (const char*)p.past[blockIdx.y] + pair * p.past_cap * p.row_bytes;
+    char* dst = (char*)p.present[blockIdx.y] + pair * p.pres_cap * p.row_bytes;
+    const long long past_b = max((long long)p.seqlens[b] + 1 - p.S, 0ll), first = part * 256 + threadIdx.x, step = p.parts * 256;
+    if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst) | (uintptr_t)p.row_bytes) & 15) == 0) copy_past<uint4>(p, first, step, src, dst, past_b);
+    else if (p.element == 2) copy_past<unsigned short>(p, first, step, src, dst, past_b);
+    else copy_past<unsigned>(p, first, step, src, dst, past_b);
 }
 
 struct GqaAttnP {
@@ -336,25 +364,52 @@ template <int DT> static void emit_gqa_t(Emitter& em, const GqaDesc& d, const TR
     const int esz = DT == DT_F16 ? 2 : 4;
     Buf null{kSlotNull, 0};
 
-    GqaPrepP pp{};
-    pp.B = B; pp.S = S; pp.H = H; pp.KV = KV; pp.D = D; pp.P = P; pp.T = T;
-    pp.past_cap = past_k.cap ? past_k.cap : P;
-    pp.pres_cap = present_k.cap ? present_k.cap : T;
-    // With a bucket the true length travels through the plan's per-run scalars.
+    const long long pres_cap = present_k.cap ? present_k.cap : T;
+    if (!d.in_place && P > 0) {
+        GqaCopyP cp{};
+        cp.S = S; cp.P = P; cp.T = T;
+        cp.past_cap = past_k.cap ? past_k.cap : P;
+        cp.pres_cap = pres_cap;
+        cp.row_bytes = D * esz;
+        cp.KV = (int)KV;
+        cp.element = esz;
+        // eight CTAs per SM, at least a thread's four pieces for each
+        const long long pieces = (T * D * esz + 16383) / 16384;
+        cp.parts = (int)std::max<long long>(1, std::min<long long>(pieces, (sm_count() * 8LL + 2 * B * KV - 1) / (2 * B * KV)));
+        em.launch(gqa_copy_past, dim3((unsigned)(B * KV * cp.parts), 2), dim3(256), 0, cp,
+                  {{&cp.past[0], past_k.buf}, {&cp.past[1], past_v.buf}, {&cp.present[0], present_k.buf}, {&cp.present[1], present_v.buf},
+                   {&cp.seqlens, seqlens.buf}},
+                  "gqa_copy_past", /*pdl=*/true);
+    }
+    // With a bucket the true length travels through the plan's per-run scalars. A step that has copied its cache goes on like one that
+    // appends in place; its decode launch may not start ahead of the copy.
     const bool dyn = d.t_bucket > 0 && d.in_place && !bias;
     const long long Tsz = dyn ? d.t_bucket : T;
-    Buf dyn_t = dyn ? em.dyn(T) : null;
+    Buf dyn_t = dyn || (!d.in_place && S == 1 && P > 0 && !bias) ? em.dyn(T) : null;
+    if (S == 1 && P > 0 && !bias && !d.in_place) {
+        GqaDesc now = d;
+        now.in_place = true;
+        if (emit_gqa_decode(em, now, q, k, v, seqlens, cos, sin, out, present_k, present_v, dyn_t, T)) {
+            em.recs.back().pdl = false;
+            em.recs.back().pop = nullptr;
+            return;
+        }
+    }
     if (dyn && S == 1 && emit_gqa_decode(em, d, q, k, v, seqlens, cos, sin, out, present_k, present_v, dyn_t, Tsz)) return;
-    if (dyn) pp.P = pp.T = 0;
+    GqaPrepP pp{};
+    pp.B = B; pp.S = S; pp.H = H; pp.KV = KV; pp.D = D; pp.T = T;
+    pp.pres_cap = pres_cap;
+    if (dyn) pp.T = 0;
+    else dyn_t = null;
     pp.half = d.rot_half;
     pp.cache_rows = d.cache_rows;
-    pp.in_place = d.in_place ? 1 : 0;
+    pp.clear = d.in_place ? 1 : P > 0 ? 0 : 2;
     pp.node = em.node;
     pp.nq = d.rot_half ? B * S * H * D : 0;
-    pp.nkv = B * KV * (d.in_place ? S : T) * D;
+    pp.nkv = B * KV * S * D;
     Buf qrot = d.rot_half ? em.scratch((size_t)(B * S * H * D * esz)) : null;
     em.launch(gqa_prepare<DT>, dim3(grid_for(pp.nq + pp.nkv, 256)), dim3(256), 0, pp,
-              {{&pp.q, q.buf}, {&pp.k, k.buf}, {&pp.v, v.buf}, {&pp.past_k, past_k.buf}, {&pp.past_v, past_v.buf},
+              {{&pp.q, q.buf}, {&pp.k, k.buf}, {&pp.v, v.buf},
                {&pp.seqlens, seqlens.buf}, {&pp.cos, cos ? cos->buf : null}, {&pp.sin, sin ? sin->buf : null},
                {&pp.q_rot, qrot}, {&pp.present_k, present_k.buf}, {&pp.present_v, present_v.buf}, {&pp.err, Buf{kSlotErr, 0}},
                {&pp.dyn_t, dyn_t}},

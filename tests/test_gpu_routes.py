@@ -3,9 +3,9 @@ import numpy as np
 import pytest
 
 from onyxia_b200 import backend as be
-from onyxia_b200 import ir
+from onyxia_b200 import ir, models
 from onyxia_b200.ir import HostTensor
-from gpu_util import cuda_backend
+from gpu_util import cuda_backend, differential
 from test_gpu_lovuzen import rel_err, run_linear
 
 pytestmark = pytest.mark.gpu
@@ -24,3 +24,60 @@ def test_f32_products_with_long_sums(rows):
             want = want + more["x1"].astype(np.float64) @ more["w1"].T.astype(np.float64)
         bias = r.standard_normal(n).astype(np.float32)
         assert rel_err(run_linear(ir.F32, x, w, bias=bias, **more), want + bias) < 2e-6, (k, n)
+
+
+@pytest.mark.parametrize("dtype,d,seq", [(ir.F16, 64, 1), (ir.F16, 128, 1), (ir.F16, 256, 1), (ir.F32, 64, 1), (ir.F16, 64, 3), (ir.F32, 32, 5), (ir.F16, 128, 20)])
+def test_caches_are_copied_into_a_new_buffer(dtype, d, seq):
+    """A step on caches that it cannot append to: the past arrives bit for bit (several CTAs per head, the last one short), what lies behind a
+    ragged row is zero, and the results are those of the decomposition within the tests' tolerances for these types."""
+    batch, past = 3, 517
+    module, feed = models.build_gqa(batch, 4, 2, d, past, seq, dtype, -1, True, seed=d + seq)
+    valid = [past, 130, 0]
+    feed["seqlens_k"] = HostTensor.from_numpy(np.array([v + seq - 1 for v in valid], np.int32))
+    tol = dict(atol=4e-3, rtol=4e-3) if dtype == ir.F16 else dict(atol=2e-4, rtol=1e-3)
+    got = {n: t.numpy() for n, t in differential(module, feed, **tol)[0]}
+    for name in ("key", "value"):
+        for b, v in enumerate(valid):
+            assert np.array_equal(got["present_" + name][b, :, :v], feed["past_" + name].numpy()[b, :, :v])
+            assert not got["present_" + name][b, :, v + seq:].any()
+
+
+def widened(packed, scales, n, nb, zero=8.0):
+    """The weights as the decomposition rounds them: (q − zero) · scale in the scales' type."""
+    q = np.stack([packed & 15, packed >> 4], 1).reshape(n, nb, 32).astype(np.float64)
+    return ((q - zero) * scales.astype(np.float64).reshape(n, nb, 1)).astype(scales.dtype).astype(np.float64).reshape(n, nb * 32)
+
+
+@pytest.mark.parametrize("m,k,n", [(257, 1152, 1536), (300, 1000, 200), (513, 136, 4104), (384, 6912, 4760)])
+def test_many_rows_against_weights_widened_once(m, k, n):
+    """Tiles that end inside a tile, k that ends inside a block and inside a step, one and two panels of weights, whole k and pieces of it.
+    After one rounding to f16 nearly all outputs equal the f64 sum's (the bound of the other kernel's test), none is further than an ulp of
+    the largest away."""
+    module, act = models.build_matmul_nbits(m, k, n, act_dtype=ir.F16, seed=m)
+    cfg = models.DecoderConfig("nbits", 0, 0, 0, 0, 0, 0, 0)
+    packed, scales, _ = models.nbits_arrays(cfg, m, f"w{k}x{n}", k, n)
+    want = (act.numpy().astype(np.float64) @ widened(packed, scales, n, (k + 31) // 32)[:, :k].T).astype(np.float16)
+    got = be.run_once(cuda_backend(), module, {"a": act})[0][1].numpy()
+    assert (got != want).mean() <= 0.01
+    assert np.abs(got.astype(np.float32) - want.astype(np.float32)).max() <= 2.0 ** -10 * np.abs(want.astype(np.float32)).max()
+
+
+@pytest.mark.parametrize("act_dtype", [ir.F32, ir.F16])
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 9, 17])
+def test_generic_int4_products(act_dtype, m):
+    """Every number of activation rows per pass; 1, 2, 4 and 8 warps per unit of weight rows; k that ends inside a lane's eight. f32: sums of k
+    products in 32 chains per warp are off by less than (k / 256 + 8) · 2^-24 of the sum of magnitudes."""
+    r = np.random.default_rng(m)
+    for k, n in ((512, 10), (2048, 515), (50, 7), (6912, 36), (1000, 2500)):
+        nb = (k + 31) // 32
+        packed, scales = r.integers(0, 256, n * nb * 16, dtype=np.uint8), r.uniform(0.005, 0.02, n * nb).astype(np.float32)
+        a = r.standard_normal((m, k)).astype(np.float32 if act_dtype == ir.F32 else np.float16)
+        b = ir.GraphBuilder()
+        x = b.input("a", act_dtype, [m, k])
+        ins = [x, b.constant(HostTensor(ir.U4, [n, nb, 32], packed)), b.constant(HostTensor.from_numpy(scales))]
+        b.output("y", b.composite("com.microsoft.MatMulNBits", {"K": k, "N": n, "bits": 4, "block_size": 32}, ins, [(act_dtype, [m, n])])[0])
+        got = be.run_once(cuda_backend(), b.finish(), {"a": HostTensor.from_numpy(a)})[0][1].numpy()
+        w = widened(packed, scales, n, nb)[:, :k]
+        if act_dtype == ir.F16:
+            w = w.astype(np.float16).astype(np.float64)
+        assert rel_err(got.astype(np.float64), a.astype(np.float64) @ w.T) < (1e-6 if act_dtype == ir.F32 else 4e-4), (k, n)
