@@ -392,6 +392,278 @@ __global__ void __launch_bounds__(256) nbits_gemm_reduce(const TcReduceP p) {
         if (row + e < p.seg_n[seg]) y[row + e] = __double2half(acc[e]);
 }
 
+// ───────────────────────────── many activation rows ─────────────────────────────
+// nbits_gemm_tc widens a weight again for every 256 activation rows, which is what sets its pace (1.3 µs per 128 k and CTA). Above that
+// the weights are widened once into scratch, as f16 rows that a plain tcgen05 GEMM takes by TMA.
+struct WidenP {
+    const unsigned char* tiles;  // of this panel
+    __half* w;                   // [row tiles · 16][k_tiles · 128]
+    int k_tiles, records, tile_bytes, has_zp;
+};
+// A warp widens one record: lane (g, t) rows g and g + 8 of block t, four 16-byte stores each.
+__global__ void __launch_bounds__(256) nbits_widen(const WidenP p) {
+    pdl_trigger();
+    const int i = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    if (i >= p.records) {
+        pdl_wait();
+        return;
+    }
+    const unsigned char* q = p.tiles + (size_t)i * p.tile_bytes;
+    const uint4 wl = __ldg(reinterpret_cast<const uint4*>(q) + lane), wh = __ldg(reinterpret_cast<const uint4*>(q) + 32 + lane);
+    const __half2 s2 = *reinterpret_cast<const __half2*>(q + kTileWt + lane * 4);
+    const uchar2 z = p.has_zp ? *reinterpret_cast<const uchar2*>(q + kTileWt + kTileSt + lane * 2) : make_uchar2(8, 8);
+    const __half2 s2l = __low2half2(s2), s2h = __high2half2(s2);
+    const float zl = (float)z.x, zh = (float)z.y;
+    const __half2 subl = __float2half2_rn(1024.f + zl), subh = __float2half2_rn(1024.f + zh);
+    const __half2 addl = __float2half2_rn(-64.f - zl), addh = __float2half2_rn(-64.f - zh);
+    const unsigned wls[4] = {wl.x, wl.y, wl.z, wl.w}, whs[4] = {wh.x, wh.y, wh.z, wh.w};
+    const int rt = i / p.k_tiles, kt = i - rt * p.k_tiles;
+    const long long ld = (long long)p.k_tiles * 128;
+    __half* to = p.w + ((long long)rt * 16 + g) * ld + kt * 128 + t * 32;
+    pdl_wait();  // the panel before this one may still be read
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+        *reinterpret_cast<uint4*>(to + m * 8) = widen_tc(wls[m], subl, addl, s2l);
+        *reinterpret_cast<uint4*>(to + 8 * ld + m * 8) = widen_tc(whs[m], subh, addh, s2h);
+    }
+}
+
+constexpr int kWideRows = 128, kWideThreads = 192, kWideStage = 2 * kPanelA, kWideStages = 3;  // stage: 128 weight rows and 128 activation rows × 64 k
+struct WideP {
+    alignas(64) unsigned char maps[2][128];  // weights of the panel, activations
+    __half* y[3];
+    float* partial;              // [splits][m][n_pad] with splits > 1
+    ErrWord* err;
+    long long m, n_pad;
+    long long seg_n[3];
+    int seg_rt0[4];
+    int n_seg, interleave2, row_tiles, rt_first;  // rt_first: the panel's first row tile
+    int steps, chunk, m_tiles, o_tiles, splits, node;
+};
+// Persistent CTAs, 128 weight rows × 128 activation rows per tile. The tensor core adds without rounding to nearest, so `chunk` steps of 64 k
+// go into one of two accumulators in turn and the epilogue warps add what an accumulator holds to their own f32 sums, one column per register,
+// while the next chunk runs: chains no longer than the ones of nbits_gemm_tc.
+// 300 / 512 / 1024 rows, widening included: k 1152, 13 824 weight rows 35 / 36 / 46 µs (nbits_gemm_tc 49 / 55 / 109), k 6912, 1152 weight rows
+// 27 / 29 / 38 µs (40 / 42 / 83). One pass of nbits_gemm_tc (256 rows) is the shorter way, two are not: the line lies there.
+__global__ void __launch_bounds__(kWideThreads, 2) nbits_gemm_wide(const __grid_constant__ WideP p) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + kWideStages * kWideStage);  // full, empty, finished[2], read[2]
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * kWideStages + 4);
+    const unsigned full = s_addr(bars), empty = full + kWideStages * 8, finished = empty + kWideStages * 8, read = finished + 16;
+    pdl_trigger();
+    if (tid == 0) {
+        for (int s = 0; s < 2 * kWideStages + 2; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + s * 8) : "memory");
+        for (int s = 0; s < 2; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(read + s * 8) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 5) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(s_addr(tmem_slot)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned tmem = *tmem_slot;
+    pdl_wait();
+    const int total = p.m_tiles * p.o_tiles * p.splits;
+    auto range = [&](int t, int& lo, int& n) {
+        const int piece = t / p.m_tiles / p.o_tiles;
+        lo = (int)((long long)p.steps * piece / p.splits);
+        n = (int)((long long)p.steps * (piece + 1) / p.splits) - lo;
+    };
+    bool ok = true;
+    if (warp == 4) {
+        if (lane == 0) {
+            int done = 0;
+            for (int t = (int)blockIdx.x; t < total && ok; t += (int)gridDim.x) {
+                int lo, n;
+                range(t, lo, n);
+                const int m0 = t % p.m_tiles * kWideRows, o0 = t / p.m_tiles % p.o_tiles * 128;
+                for (int i = 0; i < n; i++, done++) {
+                    const int s = done % kWideStages;
+                    if (done >= kWideStages && !bar_wait_tc(empty + s * 8, ((done / kWideStages) - 1) & 1)) {
+                        ok = false;
+                        break;
+                    }
+                    const unsigned bar = full + s * 8, dst = s_addr(smem + s * kWideStage);
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((unsigned)kWideStage) : "memory");
+#pragma unroll
+                    for (int op = 0; op < 2; op++)
+                        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                                         dst + op * kPanelA),
+                                     "l"(reinterpret_cast<unsigned long long>(&p.maps[op])), "r"((lo + i) * 64), "r"(op ? m0 : o0), "r"(bar)
+                                     : "memory");
+                }
+            }
+            // every copy has landed before this CTA's shared memory can be given away
+            for (int n = max(0, done - kWideStages); n < done; n++)
+                if (!bar_wait_tc(full + n % kWideStages * 8, (n / kWideStages) & 1)) ok = false;
+        }
+    } else if (warp == 5) {
+        const unsigned idesc = (1u << 4) | ((kWideRows >> 3) << 17) | (8u << 24);  // f16 × f16 → f32, M 128 × N 128
+        int done = 0, j = 0;
+        for (int t = (int)blockIdx.x; t < total; t += (int)gridDim.x) {
+            int lo, n;
+            range(t, lo, n);
+            for (int c = 0; c < n; c += p.chunk, j++) {
+                const unsigned d = tmem + (unsigned)((j & 1) * kWideRows);
+                if (j >= 2 && ok && !bar_wait_tc(read + (j & 1) * 8, ((j >> 1) - 1) & 1)) ok = false;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int i = c; i < min(n, c + p.chunk); i++, done++) {
+                    const int s = done % kWideStages;
+                    if (ok && !bar_wait_tc(full + s * 8, (done / kWideStages) & 1)) ok = false;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (lane == 0 && ok) {
+                        const unsigned a0 = s_addr(smem + s * kWideStage), b0 = a0 + kPanelA;
+#pragma unroll
+                        for (int e = 0; e < 4; e++)
+                            asm volatile(
+                                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                                " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n" ::"r"(d),
+                                "l"(umma_desc(a0 + e * 32)), "l"(umma_desc(b0 + e * 32)), "r"(idesc), "r"(i > c || e > 0 ? 1u : 0u), "r"(0u)
+                                : "memory");
+                        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(empty + s * 8) : "memory");
+                    }
+                    __syncwarp();
+                }
+                if (lane == 0) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(finished + (j & 1) * 8) : "memory");
+                __syncwarp();
+            }
+        }
+    } else {
+        int j = 0;
+        for (int t = (int)blockIdx.x; t < total; t += (int)gridDim.x) {
+            int lo, n;
+            range(t, lo, n);
+            float sum[kWideRows];
+#pragma unroll
+            for (int e = 0; e < kWideRows; e++) sum[e] = 0.f;
+            for (int c = 0; c < n; c += p.chunk, j++) {
+                if (ok && !bar_wait_tc(finished + (j & 1) * 8, (j >> 1) & 1)) ok = false;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const unsigned d = tmem + (unsigned)((j & 1) * kWideRows) + ((unsigned)(warp * 32) << 16);
+#pragma unroll
+                for (int e = 0; e < kWideRows; e += 16) {
+                    unsigned v[16];
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+                          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                        : "r"(d + (unsigned)e));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int q = 0; q < 16; q++) sum[e + q] += __uint_as_float(v[q]);
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) bar_arrive(read + (j & 1) * 8);
+            }
+            const long long m0 = (long long)(t % p.m_tiles) * kWideRows;
+            const int row_in_panel = t / p.m_tiles % p.o_tiles * 128 + warp * 32 + lane, rtg = p.rt_first + (row_in_panel >> 4);
+            if (p.splits > 1) {
+                float* part = p.partial + ((size_t)(t / p.m_tiles / p.o_tiles) * p.m + m0) * p.n_pad + row_in_panel;
+#pragma unroll
+                for (int e = 0; e < kWideRows; e++)
+                    if (ok && m0 + e < p.m) part[(size_t)e * p.n_pad] = sum[e];
+            } else {
+                int seg = 0;
+                long long row;
+                if (p.interleave2) {
+                    seg = rtg & 1;
+                    row = (long long)(rtg >> 1) * 16 + (row_in_panel & 15);
+                } else {
+                    if (p.n_seg > 1 && rtg >= p.seg_rt0[1]) seg = 1;
+                    if (p.n_seg > 2 && rtg >= p.seg_rt0[2]) seg = 2;
+                    row = (long long)(rtg - p.seg_rt0[seg]) * 16 + (row_in_panel & 15);
+                }
+                const long long width = p.seg_n[seg];
+                __half* y = p.y[seg] + m0 * width + row;
+                const bool row_ok = ok && rtg < p.row_tiles && row < width;
+#pragma unroll
+                for (int e = 0; e < kWideRows; e++)
+                    if (row_ok && m0 + e < p.m) y[e * width] = __float2half_rn(sum[e]);
+            }
+        }
+    }
+    if (!ok && lane == 0) report(p.err, ERR_WAIT_TIMEOUT, p.node, (long long)blockIdx.x, (long long)warp);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem) : "memory");
+}
+
+void emit_wide(Emitter& em, const NBitsGroup& gr, const TRef& x, const TRef& tiles, const TcP& t) {
+    const Buf null{kSlotNull, 0};
+    // panels of at most 64 MB of widened weights: they stay in L2 until the product reads them
+    const long long ld = (long long)t.k_tiles * 128;
+    const int per_panel = (int)std::max<long long>(8, (64LL << 20) / (ld * 32) / 8 * 8);
+    const Buf wide = em.scratch((size_t)std::min(per_panel, (t.row_tiles + 7) / 8 * 8) * 16 * ld * 2);
+    for (int first = 0; first < t.row_tiles; first += per_panel) {
+        const int count = std::min(per_panel, t.row_tiles - first);
+        WidenP a{};
+        a.k_tiles = t.k_tiles;
+        a.records = count * t.k_tiles;
+        a.tile_bytes = t.tile_bytes;
+        a.has_zp = t.has_zp;
+        em.launch(nbits_widen, dim3((unsigned)((a.records + 7) / 8)), dim3(256), 0, a,
+                  {{&a.tiles, tiles.buf.at((int64_t)first * t.k_tiles * t.tile_bytes)}, {&a.w, wide}}, "nbits_widen", /*pdl=*/true);
+        WideP p{};
+        p.m = gr.m;
+        p.steps = t.k_tiles * 2;
+        p.n_seg = t.n_seg;
+        p.interleave2 = t.interleave2;
+        p.row_tiles = t.row_tiles;
+        p.rt_first = first;
+        p.node = em.node;
+        for (int i = 0; i < 3; i++) p.seg_n[i] = t.seg_n[i];
+        for (int i = 0; i < 4; i++) p.seg_rt0[i] = t.seg_rt0[i];
+        p.m_tiles = (int)((gr.m + kWideRows - 1) / kWideRows);
+        p.o_tiles = (count + 7) / 8;
+        p.n_pad = (long long)p.o_tiles * 128;
+        // Pieces along k: waves × (steps of a piece + six steps of fill and drain) plus the partial sums' trip and a second launch
+        const long long slots = 2LL * sm_count(), ctas = (long long)p.m_tiles * p.o_tiles;
+        double best = 1e300;
+        for (int sp = 1; sp <= 8 && sp * 4 <= std::max(p.steps, 4); sp++) {
+            const double waves = (double)((ctas * sp + slots - 1) / slots);
+            double us = waves * ((double)p.steps / sp + 6.0) * 0.42;
+            if (sp > 1) us += 3.0 + (double)sp * gr.m * p.n_pad * 8.0 / 5e6;
+            if (us < best * 0.97) {
+                best = us;
+                p.splits = sp;
+            }
+        }
+        const int piece = (p.steps + p.splits - 1) / p.splits;
+        p.chunk = (piece + (piece + 7) / 8 - 1) / ((piece + 7) / 8);  // equal chunks of at most eight steps
+        const Buf partial = p.splits > 1 ? em.scratch((size_t)p.splits * gr.m * p.n_pad * 4) : null;
+        const size_t smem = kWideStages * kWideStage + 1024 + (2 * kWideStages + 4) * 8 + 16;
+        ensure_max_dynamic_smem((const void*)nbits_gemm_wide, 110 * 1024);
+        LaunchRec& rec = em.launch(nbits_gemm_wide, dim3((unsigned)std::min<long long>(slots, ctas * p.splits)), dim3(kWideThreads), (unsigned)smem, p,
+                                   {{&p.err, Buf{kSlotErr, 0}}, {&p.partial, partial}, {&p.y[0], gr.y[0].buf}, {&p.y[1], gr.n_seg > 1 ? gr.y[1].buf : null},
+                                    {&p.y[2], gr.n_seg > 2 ? gr.y[2].buf : null}},
+                                   "nbits_gemm_wide", /*pdl=*/true);
+        rec.tmaps.push_back(TmapReloc{(uint32_t)offsetof(WideP, maps), wide, (uint64_t)ld, (uint64_t)count * 16, (uint64_t)ld * 2, 64u, 128u});
+        rec.tmaps.push_back(TmapReloc{(uint32_t)offsetof(WideP, maps) + 128, x.buf, (uint64_t)gr.k, (uint64_t)gr.m, (uint64_t)gr.k * 2, 64u, (uint32_t)kWideRows});
+        if (p.splits > 1) {
+            TcReduceP q{};
+            q.m_total = gr.m;
+            q.n_pad = p.n_pad;
+            q.n_seg = p.n_seg;
+            q.interleave2 = p.interleave2;
+            q.row_tiles = first + count;
+            q.mb = (int)gr.m;
+            q.splits = p.splits;
+            q.row0 = (long long)first * 16;
+            for (int i = 0; i < 3; i++) q.seg_n[i] = p.seg_n[i];
+            for (int i = 0; i < 4; i++) q.seg_rt0[i] = p.seg_rt0[i];
+            em.launch(nbits_gemm_reduce, dim3((unsigned)((count * 4 + 255) / 256), (unsigned)gr.m), dim3(256), 0, q,
+                      {{&q.partial, partial}, {&q.y[0], gr.y[0].buf}, {&q.y[1], gr.n_seg > 1 ? gr.y[1].buf : null},
+                       {&q.y[2], gr.n_seg > 2 ? gr.y[2].buf : null}},
+                      "nbits_gemm_reduce", /*pdl=*/true);
+        }
+    }
+}
+
 }  // namespace
 
 // The GEMM form of a MatMulNBits group (no prologue, no epilogue: the caller runs those as
@@ -415,6 +687,12 @@ void emit_nbits_gemm_tc(Emitter& em, const NBitsGroup& gr, const TRef& x, const 
     p.has_zp = gr.has_zp ? 1 : 0;
     p.tile_bytes = kTileWt + kTileSt + (gr.has_zp ? kTileZt : 0);
     p.node = em.node;
+    // two passes and more: measured on both sides beside nbits_gemm_wide
+    static const long long wide_from = [] {
+        const char* e = std::getenv("ONYXIA_GEMM_WIDE_FROM");  // diagnostics: activation rows from which the weights are widened into scratch
+        return e ? std::atoll(e) : 257LL;
+    }();
+    if (gr.m >= wide_from && gr.m < 65536 && gr.k % 8 == 0 && x.buf.off % 16 == 0) return emit_wide(em, gr, x, tiles, p);
     // activation rows per pass: the smallest MMA N that holds them all, at most 256
     int mb = 16;
     while (mb < gr.m && mb < 256) mb <<= 1;
