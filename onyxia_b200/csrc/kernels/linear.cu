@@ -57,6 +57,7 @@ struct LinP {
     int act[2];           // functions of the columns before and from act_split on; none from act_end on
     long long act_split, act_end;
     int nb, stages, splits, node;  // linear_tc
+    int row_tiles, out_tiles, one;  // tiles of activation rows (not grouped) and of weight rows; one: a CTA per tile (and piece), in the grid's axes
     const int* counts;    // grouped: rows of every group
     int groups;
 };
@@ -90,6 +91,13 @@ __device__ __forceinline__ bool locate_group(const LinP& p, int tile, int size, 
         rows += __shfl_sync(0xffffffffu, r_inc, 31);
     }
     return false;
+}
+
+// Grouped: tiles of `size` rows over all groups. Called by whole warps.
+__device__ __forceinline__ int count_tiles(const LinP& p, int size) {
+    int tiles = 0;
+    for (int g = threadIdx.x & 31; g < p.groups; g += 32) tiles += (p.counts[g] + size - 1) / size;
+    return __reduce_add_sync(0xffffffffu, tiles);
 }
 
 __device__ __forceinline__ float glu_value(const LinP& p, float gate, float up) {
@@ -458,6 +466,11 @@ template <int NT, int NORM, bool BLOCKS> __global__ void __launch_bounds__(kStre
 constexpr int kTcThreads = 192;      // warps 0-3 epilogue, 4 TMA, 5 MMA
 constexpr int kTcPanelA = 128 * 128; // bytes: 128 weight rows × 64 k
 
+// A persistent CTA works through tiles (piece of k slowest, activation tiles fastest: they share a weight tile while it is in L2); loads and
+// MMAs run on into the next tile while the epilogue of the last one empties the other of two accumulators.
+// Rows × k × weight rows: 4096 × 1152 × 13 824 gated 217 → 136 µs (959 TFLOP/s), 2048 × 2560 × 20 480 gated 246 → 201, 2048 × 5376 × 16 896
+// 353 → 347 against a CTA per tile, whose fill and drain stood beside 18, 40 and 84 steps.
+//
 // What the epilogue does: EPI_PLAIN bias only, EPI_GLU the gated unit, EPI_ACT functions of columns and factors. Kernels of their own: the
 // paths of one are short enough to stay in the instruction cache.
 enum : int { EPI_PLAIN, EPI_GLU, EPI_ACT };
@@ -467,20 +480,23 @@ template <int EPI> __global__ void __launch_bounds__(kTcThreads) linear_tc(const
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nb = p.nb, S = p.stages;
     const int stage_bytes = kTcPanelA + nb * 128;
-    int group = 0, n0 = (int)blockIdx.x * nb, n_live = nb;
-    unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + (size_t)S * stage_bytes);  // full[S], empty[S], done
-    unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * S + 1);
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + (size_t)S * stage_bytes);  // full[S], empty[S], finished[2], read[2]
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * S + 4);
+    const unsigned finished = smem_u32(bars + 2 * S), read = finished + 16;
     pdl_trigger();
+    int row_tiles = p.row_tiles;
     if (p.groups) {  // the counts come from an earlier launch
         pdl_wait();
-        if (!locate_group(p, (int)blockIdx.x, nb, &group, &n0, &n_live)) return;
+        row_tiles = count_tiles(p, nb);
     }
+    const int first = p.one ? 0 : (int)blockIdx.x, total = p.one ? 1 : row_tiles * p.out_tiles * p.splits;
     if (tid == 0) {
-        for (int s = 0; s < 2 * S + 1; s++) mbar_init(smem_u32(bars + s), 1);
+        for (int s = 0; s < 2 * S + 2; s++) mbar_init(smem_u32(bars + s), 1);
+        for (int s = 0; s < 2; s++) mbar_init(read + s * 8, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     int cols = 32;
-    while (cols < nb) cols <<= 1;
+    while (cols < (p.one ? nb : 2 * nb)) cols <<= 1;
     if (warp == 5) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -491,130 +507,178 @@ template <int EPI> __global__ void __launch_bounds__(kTcThreads) linear_tc(const
     const unsigned tmem = *tmem_slot;
 
     const int s0 = (int)((p.k[0] + 63) / 64), all = s0 + (int)((p.k[1] + 63) / 64);
-    const int lo = (int)((long long)all * blockIdx.z / p.splits), steps = (int)((long long)all * (blockIdx.z + 1) / p.splits) - lo;
-    // activation tiles first: they share a weight tile while it is in L2
-    const int block_tiles = (int)((p.out + 127) / 128), block = p.blocks > 1 ? (int)blockIdx.y / block_tiles : 0;
-    const int m0 = ((int)blockIdx.y - block * block_tiles) * 128, w0 = (group + block) * (int)p.out + m0;
-    const int x0 = (int)(p.x_off + block * p.x_step);
+    const int block_tiles = (int)((p.out + 127) / 128);
+    struct Tile {
+        int group = 0, n0, live, block, m0, piece, lo, steps;
+    };
+    auto tile_of = [&](int t) {  // by whole warps
+        Tile q;
+        int x = (int)blockIdx.x, y = (int)blockIdx.y;
+        q.piece = (int)blockIdx.z;
+        if (!p.one) {
+            const int rest = t / row_tiles;
+            x = t % row_tiles;
+            y = rest % p.out_tiles;
+            q.piece = rest / p.out_tiles;
+        }
+        q.n0 = x * nb;
+        q.live = (int)min((long long)nb, p.rows - q.n0);
+        if (p.groups) locate_group(p, x, nb, &q.group, &q.n0, &q.live);
+        q.block = p.blocks > 1 ? y / block_tiles : 0;
+        q.m0 = (y - q.block * block_tiles) * 128;
+        q.lo = (int)((long long)all * q.piece / p.splits);
+        q.steps = (int)((long long)all * (q.piece + 1) / p.splits) - q.lo;
+        return q;
+    };
     bool ok = true;
 
     if (warp == 4) {
-        if (lane == 0) {
-            auto load_w = [&](int i) {
-                const int s = i % S, c = lo + i, op = c >= s0;
-                mbar_expect_tx(smem_u32(bars + s), (unsigned)stage_bytes);
-                tma_load_2d(smem_u32(smem + (size_t)s * stage_bytes), p.maps[op * 2 + 1], (op ? c - s0 : c) * 64, w0, smem_u32(bars + s));
-            };
-            auto load_x = [&](int i) {
-                const int s = i % S, c = lo + i, op = c >= s0;
-                tma_load_2d(smem_u32(smem + (size_t)s * stage_bytes + kTcPanelA), p.maps[op * 2], (op ? c - s0 : c) * 64 + x0, n0, smem_u32(bars + s));
-            };
-            const int head = min(S, steps);
-            for (int i = 0; i < head; i++) load_w(i);  // constants: may overlap the launches before this one
-            pdl_wait();
-            for (int i = 0; i < head; i++) load_x(i);
-            int issued = head;
-            for (; issued < steps; issued++) {
-                if (!mbar_wait(smem_u32(bars + S + issued % S), ((issued / S) - 1) & 1)) {
-                    ok = false;
-                    break;
+        int done = 0;  // steps so far
+        bool waited = p.groups != 0;
+        for (int t = first; t < total; t += (int)gridDim.x) {
+            const Tile q = tile_of(t);
+            if (lane == 0) {
+                const int w0 = (q.group + q.block) * (int)p.out + q.m0, x0 = (int)(p.x_off + q.block * p.x_step);
+                auto load_w = [&](int i) {
+                    const int s = (done + i) % S, c = q.lo + i, op = c >= s0;
+                    mbar_expect_tx(smem_u32(bars + s), (unsigned)stage_bytes);
+                    tma_load_2d(smem_u32(smem + (size_t)s * stage_bytes), p.maps[op * 2 + 1], (op ? c - s0 : c) * 64, w0, smem_u32(bars + s));
+                };
+                auto load_x = [&](int i) {
+                    const int s = (done + i) % S, c = q.lo + i, op = c >= s0;
+                    tma_load_2d(smem_u32(smem + (size_t)s * stage_bytes + kTcPanelA), p.maps[op * 2], (op ? c - s0 : c) * 64 + x0, q.n0, smem_u32(bars + s));
+                };
+                int i = 0;
+                if (!waited) {
+                    const int head = min(S, q.steps);
+                    for (; i < head; i++) load_w(i);  // constants: may overlap the launches before this one
+                    pdl_wait();
+                    for (i = 0; i < head; i++) load_x(i);
                 }
-                load_w(issued);
-                load_x(issued);
+                for (; ok && i < q.steps; i++) {
+                    const int n = done + i;
+                    if (n >= S && !mbar_wait(smem_u32(bars + S + n % S), ((n / S) - 1) & 1)) {
+                        ok = false;
+                        break;
+                    }
+                    load_w(i);
+                    load_x(i);
+                }
+                done += i;
+            } else if (!waited) {
+                pdl_wait();
             }
-            // every copy has landed before this CTA's shared memory can be given away
-            for (int s = 0; s < head; s++)
-                if (!mbar_wait(smem_u32(bars + s), ((issued - 1 - s) / S) & 1)) ok = false;
-        } else {
-            pdl_wait();
+            waited = true;
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (!ok) break;
         }
+        // every copy has landed before this CTA's shared memory can be given away
+        if (lane == 0)
+            for (int n = max(0, done - S); n < done; n++)
+                if (!mbar_wait(smem_u32(bars + n % S), (n / S) & 1)) ok = false;
     } else if (warp == 5) {
         pdl_wait();
         const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(nb >> 3) << 17) | (8u << 24);  // bf16 × bf16 → f32, M 128 × N nb
-        for (int i = 0; i < steps; i++) {
-            const int s = i % S;
-            if (ok && !mbar_wait(smem_u32(bars + s), (i / S) & 1)) ok = false;
+        int n = 0, j = 0;
+        for (int t = first; t < total; t += (int)gridDim.x, j++) {
+            const int piece = p.one ? (int)blockIdx.z : t / row_tiles / p.out_tiles, steps = (int)((long long)all * (piece + 1) / p.splits) - (int)((long long)all * piece / p.splits);
+            const unsigned d = tmem + (unsigned)((j & 1) * nb);
+            if (j >= 2 && ok && !mbar_wait(read + (j & 1) * 8, ((j >> 1) - 1) & 1)) ok = false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (lane == 0 && ok) {
-                const unsigned a0 = smem_u32(smem + (size_t)s * stage_bytes), b0 = a0 + kTcPanelA;
+            for (int i = 0; i < steps; i++, n++) {
+                const int s = n % S;
+                if (ok && !mbar_wait(smem_u32(bars + s), (n / S) & 1)) ok = false;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (lane == 0 && ok) {
+                    const unsigned a0 = smem_u32(smem + (size_t)s * stage_bytes), b0 = a0 + kTcPanelA;
 #pragma unroll
-                for (int j = 0; j < 4; j++) umma_bf16(tmem, umma_kmajor_desc(a0 + j * 32), umma_kmajor_desc(b0 + j * 32), idesc, i > 0 || j > 0);
-                umma_commit(smem_u32(bars + S + s));
+                    for (int e = 0; e < 4; e++) umma_bf16(d, umma_kmajor_desc(a0 + e * 32), umma_kmajor_desc(b0 + e * 32), idesc, i > 0 || e > 0);
+                    umma_commit(smem_u32(bars + S + s));
+                }
+                __syncwarp();
             }
+            if (lane == 0) umma_commit(finished + (j & 1) * 8);
             __syncwarp();
         }
-        if (lane == 0) umma_commit(smem_u32(bars + 2 * S));
-        __syncwarp();
     } else {
         pdl_wait();
-        if (!mbar_wait(smem_u32(bars + 2 * S), 0)) ok = false;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const long long o = (long long)m0 + warp * 32 + lane;  // weight row = accumulator lane
-        const long long col0 = block * p.out;
-        const float bias = p.bias && p.splits == 1 && o < p.out ? p.bias[col0 + o] : 0.f;
-        const long long live = min((long long)n_live, p.rows - n0);
-        const int f = EPI == EPI_ACT && col0 + o < p.act_end ? p.act[col0 + o >= p.act_split] : ACT_NONE;
-        for (int c = 0; c < nb && c < live; c += 16) {
-            unsigned v[16];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                  "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                : "r"(tmem + ((unsigned)(warp * 32) << 16) + (unsigned)c));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (p.splits > 1) {
-                float* part = p.partial + ((size_t)blockIdx.z * p.rows + n0 + c) * p.ldy + col0 + o;
+        int j = 0;
+        for (int t = first; t < total; t += (int)gridDim.x, j++) {
+            const Tile q = tile_of(t);
+            if (ok && !mbar_wait(finished + (j & 1) * 8, (j >> 1) & 1)) ok = false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const long long o = (long long)q.m0 + warp * 32 + lane;  // weight row = accumulator lane
+            const long long n0 = q.n0, col0 = q.block * p.out;
+            const float bias = p.bias && p.splits == 1 && o < p.out ? p.bias[col0 + o] : 0.f;
+            const int live = q.live;
+            const int f = EPI == EPI_ACT && col0 + o < p.act_end ? p.act[col0 + o >= p.act_split] : ACT_NONE;
+            const unsigned d = tmem + (unsigned)((j & 1) * nb) + ((unsigned)(warp * 32) << 16);
+            for (int c = 0; c < nb && c < live; c += 16) {
+                unsigned v[16];
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                      "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                    : "r"(d + (unsigned)c));
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (p.splits > 1) {
+                    float* part = p.partial + ((size_t)q.piece * p.rows + n0 + c) * p.ldy + col0 + o;
 #pragma unroll
-                for (int j = 0; j < 16; j++)
-                    if (ok && o < p.out && c + j < live) part[(size_t)j * p.ldy] = __uint_as_float(v[j]);
-            } else if constexpr (EPI == EPI_GLU) {
-                // lanes 2i and 2i + 1 hold gate and up; of two activation rows the even lane finishes the first, the odd one
-                // the second
-                const int odd = lane & 1;
-                const long long width = p.out / 2, at = (n0 + c + odd) * width + (o >> 1);
-                const bool mine = ok && (o | 1) < p.out;
+                    for (int e = 0; e < 16; e++)
+                        if (ok && o < p.out && c + e < live) part[(size_t)e * p.ldy] = __uint_as_float(v[e]);
+                } else if constexpr (EPI == EPI_GLU) {
+                    // lanes 2i and 2i + 1 hold gate and up; of two activation rows the even lane finishes the first, the odd one
+                    // the second
+                    const int odd = lane & 1;
+                    const long long width = p.out / 2, at = (n0 + c + odd) * width + (o >> 1);
+                    const bool mine = ok && (o | 1) < p.out;
 #pragma unroll
-                for (int j = 0; j < 16; j += 2) {
-                    const float lo = __uint_as_float(v[j]) + bias, hi = __uint_as_float(v[j + 1]) + bias;
-                    const float got = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1);
-                    const float y = glu_value(p, odd ? got : lo, odd ? hi : got);
-                    if (!mine || c + j + odd >= live) continue;
-                    if (p.y_bf16) ((bf16*)p.y)[at + j * width] = __float2bfloat16_rn(y);
-                    else ((float*)p.y)[at + j * width] = y;
-                }
-            } else if (ok && o < p.out) {
-                float y[16];
-#pragma unroll
-                for (int j = 0; j < 16; j++) y[j] = __uint_as_float(v[j]) + bias;
-                if constexpr (EPI == EPI_ACT) {
-                    if (f == ACT_SOFTPLUS) {
-#pragma unroll
-                        for (int j = 0; j < 16; j++) y[j] = softplus_fast(y[j]);
-                    } else if (f != ACT_NONE && p.y_bf16) {
-#pragma unroll
-                        for (int j = 0; j < 16; j++) y[j] = sigmoid_fast(y[j]) * (f == ACT_SILU ? y[j] : 1.f);
-                    } else if (f != ACT_NONE) {
-#pragma unroll
-                        for (int j = 0; j < 16; j++) y[j] = sigmoid_f(y[j]) * (f == ACT_SILU ? y[j] : 1.f);
+                    for (int e = 0; e < 16; e += 2) {
+                        const float lo = __uint_as_float(v[e]) + bias, hi = __uint_as_float(v[e + 1]) + bias;
+                        const float got = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1);
+                        const float y = glu_value(p, odd ? got : lo, odd ? hi : got);
+                        if (!mine || c + e + odd >= live) continue;
+                        if (p.y_bf16) ((bf16*)p.y)[at + e * width] = __float2bfloat16_rn(y);
+                        else ((float*)p.y)[at + e * width] = y;
                     }
-                    if (p.mul)
+                } else if (ok && o < p.out) {
+                    float y[16];
 #pragma unroll
-                        for (int j = 0; j < 16; j++)
-                            if (c + j < live) y[j] *= factor<bf16>(p, n0 + c + j, col0 + o);
+                    for (int e = 0; e < 16; e++) y[e] = __uint_as_float(v[e]) + bias;
+                    if constexpr (EPI == EPI_ACT) {
+                        if (f == ACT_SOFTPLUS) {
+#pragma unroll
+                            for (int e = 0; e < 16; e++) y[e] = softplus_fast(y[e]);
+                        } else if (f != ACT_NONE && p.y_bf16) {
+#pragma unroll
+                            for (int e = 0; e < 16; e++) y[e] = sigmoid_fast(y[e]) * (f == ACT_SILU ? y[e] : 1.f);
+                        } else if (f != ACT_NONE) {
+#pragma unroll
+                            for (int e = 0; e < 16; e++) y[e] = sigmoid_f(y[e]) * (f == ACT_SILU ? y[e] : 1.f);
+                        }
+                        if (p.mul)
+#pragma unroll
+                            for (int e = 0; e < 16; e++)
+                                if (c + e < live) y[e] *= factor<bf16>(p, n0 + c + e, col0 + o);
+                    }
+                    const long long at = (n0 + c) * p.ldy + col0 + o;
+                    if (p.y_bf16) {
+                        bf16* to = (bf16*)p.y + at;
+#pragma unroll
+                        for (int e = 0; e < 16; e++)
+                            if (c + e < live) to[e * p.ldy] = __float2bfloat16_rn(y[e]);
+                    } else {
+                        float* to = (float*)p.y + at;
+#pragma unroll
+                        for (int e = 0; e < 16; e++)
+                            if (c + e < live) to[e * p.ldy] = y[e];
+                    }
                 }
-                const long long at = (n0 + c) * p.ldy + col0 + o;
-                if (p.y_bf16) {
-                    bf16* to = (bf16*)p.y + at;
-#pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (c + j < live) to[j * p.ldy] = __float2bfloat16_rn(y[j]);
-                } else {
-                    float* to = (float*)p.y + at;
-#pragma unroll
-                    for (int j = 0; j < 16; j++)
-                        if (c + j < live) to[j * p.ldy] = y[j];
-                }
+                __syncwarp();
             }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(read + (j & 1) * 8) : "memory");
         }
     }
     if (!ok && lane == 0) report(p.err, ERR_WAIT_TIMEOUT, p.node, (long long)blockIdx.x, (long long)warp);
@@ -1265,8 +1329,9 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
     };
     const bool quads = d.k[0] % 4 == 0 && d.k[1] % 4 == 0 && p.ldx % 4 == 0 && d.x_off % 4 == 0 && d.x_step % 4 == 0 && w0.buf.off % 16 == 0 &&
                        (!w1 || w1->buf.off % 16 == 0);
-    if (!tc_type && quads && d.rows <= 32) {
-        // Eight rows per pass over the weights. 32 rows (four passes) take the 83 µs of linear_f32's one tile of 64.
+    if (!tc_type && quads && d.rows <= 32 && d.k[0] + d.k[1] >= 512) {
+        // Eight rows per pass over the weights. 32 rows (four passes) take the 83 µs of linear_f32's one tile of 64; a short k is few steps
+        // of such a tile, and its sums are added in order.
         const int m = d.rows == 1 ? 1 : d.rows == 2 ? 2 : d.rows <= 4 ? 4 : 8;
         auto units = [&](int r) { return (d.out + r - 1) / r * d.blocks; };
         const bool eight = m < 8 && units(8) * kStreamWarps >= 16LL * sm_count();  // enough warps with eight weight rows each
@@ -1364,13 +1429,19 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
         }
     }
     const size_t stage = kTcPanelA + (size_t)p.nb * 128;
-    const bool alone = mt * ((d.rows + p.nb - 1) / p.nb) * p.splits <= sm_count();  // one CTA per SM: all of its shared memory
+    p.row_tiles = (int)((d.rows + p.nb - 1) / p.nb);
+    p.out_tiles = (int)mt;
+    const long long tiles = mt * p.row_tiles * p.splits;
+    if (tiles >= INT32_MAX) throw std::runtime_error("onyxia.Linear: too many tiles");
+    const bool alone = tiles <= sm_count();  // one CTA per SM: all of its shared memory
     p.stages = (int)std::min<size_t>(8, (p.nb <= 128 && !alone ? 108 * 1024 : 208 * 1024) / stage);
-    const size_t smem = stage * p.stages + 1024 + (2 * p.stages + 1) * 8 + 16;
+    const size_t smem = stage * p.stages + 1024 + (2 * p.stages + 4) * 8 + 16;
     const auto kernel = d.glu ? linear_tc<EPI_GLU> : d.act[0] || d.act[1] || d.mul ? linear_tc<EPI_ACT> : linear_tc<EPI_PLAIN>;
     ensure_max_dynamic_smem((const void*)kernel, 220 * 1024);
     const Buf partial = p.splits > 1 ? em.scratch((size_t)p.splits * d.rows * p.ldy * 4) : kNull;
-    LaunchRec& rec = em.launch(kernel, dim3((unsigned)((d.rows + p.nb - 1) / p.nb), (unsigned)mt, (unsigned)p.splits), dim3(kTcThreads), (unsigned)smem, p,
+    const long long slots = (long long)sm_count() * (p.nb <= 128 ? 2 : 1);
+    p.one = tiles <= slots;
+    LaunchRec& rec = em.launch(kernel, p.one ? dim3((unsigned)p.row_tiles, (unsigned)mt, (unsigned)p.splits) : dim3((unsigned)slots), dim3(kTcThreads), (unsigned)smem, p,
                                {{&p.bias, bb}, {&p.y, y.buf}, {&p.mul, mul}, {&p.partial, partial}, {&p.err, Buf{kSlotErr, 0}}}, "linear_tc", /*pdl=*/true);
     auto add_map = [&](int i, const Buf& b, int64_t k, int64_t rows, uint32_t box) {
         rec.tmaps.push_back(TmapReloc{(uint32_t)(offsetof(LinP, maps) + 128 * i), b, (uint64_t)k, (uint64_t)rows, (uint64_t)k * 2, 64u, box});
@@ -1430,11 +1501,14 @@ void emit_grouped_linear(Emitter& em, const GroupedLinearDesc& d, const TRef& x,
         if (nb == 32 || nb == 64 || nb == 128 || nb == 256) p.nb = nb;
     }
     const size_t stage = kTcPanelA + (size_t)p.nb * 128;
+    p.out_tiles = (int)mt;
+    const long long tiles = tiles_of(p.nb) * mt;  // at most
+    if (tiles >= INT32_MAX) throw std::runtime_error("grouped product: too many tiles");
     p.stages = (int)std::min<size_t>(8, (p.nb <= 128 ? 108 * 1024 : 208 * 1024) / stage);
-    const size_t smem = stage * p.stages + 1024 + (2 * p.stages + 1) * 8 + 16;
+    const size_t smem = stage * p.stages + 1024 + (2 * p.stages + 4) * 8 + 16;
     const auto kernel = d.glu ? linear_tc<EPI_GLU> : linear_tc<EPI_PLAIN>;
     ensure_max_dynamic_smem((const void*)kernel, 220 * 1024);
-    LaunchRec& rec = em.launch(kernel, dim3((unsigned)tiles_of(p.nb), (unsigned)mt, 1), dim3(kTcThreads), (unsigned)smem, p,
+    LaunchRec& rec = em.launch(kernel, dim3((unsigned)std::min<long long>(tiles, (long long)sm_count() * (p.nb <= 128 ? 2 : 1))), dim3(kTcThreads), (unsigned)smem, p,
                                {{&p.bias, kNull}, {&p.y, y.buf}, {&p.partial, kNull}, {&p.err, Buf{kSlotErr, 0}}, {&p.counts, counts.buf}}, "grouped_tc",
                                /*pdl=*/true);
     auto add_map = [&](int i, const Buf& b, int64_t rows, uint32_t box) {
