@@ -340,6 +340,8 @@ ox_status ox_llm_create(ox_session*, int64_t max_seq_len, ox_llm** out);
 void ox_llm_free(ox_llm*);
 int64_t ox_llm_sequence_length(const ox_llm*);
 int32_t ox_llm_logits_dtype(const ox_llm*); /* ox_dtype code of the logits `ox_llm_step` copies out */
+/* Widens `n` IEEE half-precision values in host memory (such logits) exactly. */
+void ox_f16_to_f32(const void* src, float* dst, size_t n);
 void ox_llm_reset(ox_llm*);
 ox_status ox_llm_step(ox_llm*, const int64_t* ids, int32_t n_ids, int64_t* token_out, void* logits_out, size_t logits_cap,
                       size_t* logits_written);

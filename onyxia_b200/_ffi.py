@@ -6,6 +6,7 @@ device path.
 """
 from __future__ import annotations
 
+import array
 import ctypes as C
 import os
 
@@ -138,6 +139,7 @@ SIGNATURES = {
     "ox_llm_sequence_length": (C.c_int64, [_P]),
     "ox_llm_logits_dtype": (C.c_int32, [_P]),
     "ox_llm_reset": (None, [_P]),
+    "ox_f16_to_f32": (None, [C.c_void_p, C.POINTER(C.c_float), C.c_size_t]),
     "ox_llm_step": (C.c_int32, [_P, C.POINTER(C.c_int64), C.c_int32, C.POINTER(C.c_int64), C.c_void_p, C.c_size_t,
                                 C.POINTER(C.c_size_t)]),
     "ox_llm_generate": (C.c_int32, [_P, C.POINTER(C.c_int64), C.c_int32, C.c_int32, C.POINTER(C.c_int64)]),
@@ -212,6 +214,23 @@ class OnyxiaError(RuntimeError):
         super().__init__(message)
         self.status = status
         self.kind = self.KINDS.get(status, "Unknown")
+
+
+def whole_words(code: str, values) -> array.array:
+    """The values in one buffer of type "q" (int64) or "i" (int32). As with ctypes' integers, too large ones keep their low bits."""
+    try:
+        return array.array(code, values)
+    except OverflowError:
+        kind = C.c_int64 if code == "q" else C.c_int32
+        return array.array(code, [kind(v).value for v in values])
+
+
+def int_words(code: str, values) -> array.array:
+    """The same for anything that int() makes a whole number of."""
+    try:
+        return whole_words(code, values)
+    except TypeError:
+        return whole_words(code, [int(v) for v in values])
 
 
 def check(status: int) -> None:

@@ -1,6 +1,7 @@
 """Batched serving over a prepared module with paged caches and per-sequence state (``ox_engine_*``)."""
 from __future__ import annotations
 
+import array
 import ctypes as C
 
 import numpy as np
@@ -29,17 +30,22 @@ class Engine:
     def forward(self, entries, logits: bool = True):
         """One batch: `entries` are (id, next tokens, places among them whose logits are wanted). Returns the wanted
         rows in entry order as f32 [wanted, vocab], or None (and does not wait) with ``logits=False``."""
-        arr = (_ffi.EngineEntry * max(len(entries), 1))()
-        keep, wanted = [], 0
-        for i, (seq, tokens, want) in enumerate(entries):
-            t = (C.c_int64 * max(len(tokens), 1))(*[int(v) for v in tokens])
-            w = (C.c_int32 * max(len(want), 1))(*[int(v) for v in want])
-            keep += [t, w]
-            arr[i] = _ffi.EngineEntry(int(seq), t, len(tokens), w, len(want))
-            wanted += len(want)
+        # all tokens in one buffer, all places in another, and the entries (ox_engine_entry: 40 bytes) as words that point into them
+        flat, places, ids, spans = array.array("q"), array.array("i"), [], []
+        for seq, tokens, want in entries:
+            words, wanted = _ffi.int_words("q", tokens), _ffi.int_words("i", want)
+            ids.append(int(seq))
+            spans.append((len(flat), len(words), len(places), len(wanted)))
+            flat += words
+            places += wanted
+        at, where, words = flat.buffer_info()[0], places.buffer_info()[0], array.array("q")
+        for seq, (first, n, place, m) in zip(_ffi.whole_words("q", ids), spans):
+            words.extend((seq, at + 8 * first, n, where + 4 * place, m))
+        wanted = len(places)
         out = np.empty((wanted, self.vocab), dtype=np.float32) if logits else None
         ptr = out.ctypes.data_as(C.POINTER(C.c_float)) if logits else None
-        check(self._lib.ox_engine_forward(self._h, arr, len(entries), ptr, out.size if logits else 0))
+        arr = C.cast(words.buffer_info()[0] if spans else C.byref(_ffi.EngineEntry()), C.POINTER(_ffi.EngineEntry))
+        check(self._lib.ox_engine_forward(self._h, arr, len(spans), ptr, out.size if logits else 0))
         return out
 
     def release(self, seq: int) -> None:
@@ -47,10 +53,10 @@ class Engine:
 
     def submit(self, prompt, max_new: int, *, eos: int = -1, temperature: float = 0.0, top_k: int = 0, top_p: float = 1.0,
                seed: int = 0) -> int:
-        arr = (C.c_int64 * max(len(prompt), 1))(*[int(v) for v in prompt])
+        words = _ffi.int_words("q", prompt)
         out = C.c_int64()
-        check(self._lib.ox_engine_submit(self._h, arr, len(prompt), int(max_new), int(eos), float(temperature), int(top_k), float(top_p),
-                                         int(seed) & (2 ** 64 - 1), C.byref(out)))
+        check(self._lib.ox_engine_submit(self._h, C.cast(words.buffer_info()[0], C.POINTER(C.c_int64)), len(words), int(max_new), int(eos),
+                                         float(temperature), int(top_k), float(top_p), int(seed) & (2 ** 64 - 1), C.byref(out)))
         return out.value
 
     def step(self, token_budget: int = 2048) -> list:

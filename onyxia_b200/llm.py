@@ -138,6 +138,7 @@ class NativeLlmSession:
         h = C.c_void_p()
         _ffi.check(self._lib.ox_llm_create(self.session._h, max_seq_len, C.byref(h)))
         self._h = h
+        self._raw = np.empty(1 << 20, dtype=np.uint8)  # a step's logits as they are stored
 
     def step_greedy(self, ids) -> int:
         C = self._C
@@ -170,13 +171,16 @@ class NativeLlmSession:
     def step_logits(self, ids) -> np.ndarray:
         C = self._C
         from . import _ffi
-        arr = (C.c_int64 * len(ids))(*ids)
-        buf = np.empty(1 << 20, dtype=np.uint8)
+        arr = _ffi.whole_words("q", ids)
+        buf = self._raw
         written = C.c_size_t()
-        _ffi.check(self._lib.ox_llm_step(self._h, arr, len(ids), None, buf.ctypes.data_as(C.c_void_p), buf.size, C.byref(written)))
-        raw = buf[:written.value]
-        np_dt = np.float16 if self._lib.ox_llm_logits_dtype(self._h) == ir.F16 else np.float32
-        return raw.view(np_dt).astype(np.float32)
+        _ffi.check(self._lib.ox_llm_step(self._h, C.cast(arr.buffer_info()[0], C.POINTER(C.c_int64)), len(arr), None,
+                                         buf.ctypes.data_as(C.c_void_p), buf.size, C.byref(written)))
+        if self._lib.ox_llm_logits_dtype(self._h) != ir.F16:
+            return buf[:written.value].view(np.float32).copy()
+        out = np.empty(written.value // 2, dtype=np.float32)
+        self._lib.ox_f16_to_f32(buf.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.POINTER(C.c_float)), out.size)
+        return out
 
     def sequence_length(self) -> int:
         return self._lib.ox_llm_sequence_length(self._h)

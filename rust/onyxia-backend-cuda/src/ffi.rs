@@ -211,6 +211,7 @@ unsafe extern "C" {
     pub fn ox_llm_free(l: *mut ox_llm);
     pub fn ox_llm_sequence_length(l: *const ox_llm) -> i64;
     pub fn ox_llm_logits_dtype(l: *const ox_llm) -> i32;
+    pub fn ox_f16_to_f32(src: *const c_void, dst: *mut f32, n: usize);
     pub fn ox_llm_reset(l: *mut ox_llm);
     pub fn ox_llm_step(l: *mut ox_llm, ids: *const i64, n_ids: i32, token_out: *mut i64, logits_out: *mut c_void, logits_cap: usize,
                        logits_written: *mut usize) -> i32;

@@ -186,3 +186,19 @@ def test_byte_accounting_matches_the_roofline_figures():
     assert [cfg.layer_window(l) for l in range(6)] == [512, 512, 512, 512, 512, -1]
     c27 = models.config_gemma3_27b()
     assert c27.weight_bytes_per_token() == 15_191_801_856
+
+
+def test_words_keep_what_ctypes_took():
+    assert list(_ffi.int_words("q", [1, 2.9, True, np.int32(4)])) == [1, 2, 1, 4]
+    assert list(_ffi.int_words("q", range(3))) == [0, 1, 2] and len(_ffi.int_words("i", [])) == 0
+    assert list(_ffi.whole_words("q", [2 ** 64 - 1, 7])) == [-1, 7] and list(_ffi.int_words("i", np.array([2 ** 32 + 5]))) == [5]
+    with pytest.raises(TypeError):
+        _ffi.whole_words("q", [1.5])
+
+
+def test_half_precision_widens_exactly():
+    bits = np.arange(65536, dtype=np.uint16)[1:]  # an odd count: a tail behind the eights
+    want, got = bits.view(np.float16).astype(np.float32), np.empty(65535, np.float32)
+    _ffi.cuda_lib().ox_f16_to_f32(bits.ctypes.data_as(C.c_void_p), got.ctypes.data_as(C.POINTER(C.c_float)), got.size)
+    assert np.array_equal(got, want, equal_nan=True)
+    assert np.array_equal(np.signbit(got)[~np.isnan(want)], np.signbit(want)[~np.isnan(want)])
