@@ -6,6 +6,8 @@ from onyxia_b200 import backend as be
 from onyxia_b200 import ir, models
 from onyxia_b200.ir import HostTensor
 from gpu_util import cuda_backend, differential
+from lovuzen_util import to_bf16
+from test_gpu_kipizen import Experts
 from test_gpu_lovuzen import rel_err, run_linear
 
 pytestmark = pytest.mark.gpu
@@ -81,3 +83,88 @@ def test_generic_int4_products(act_dtype, m):
         if act_dtype == ir.F16:
             w = w.astype(np.float16).astype(np.float64)
         assert rel_err(got.astype(np.float64), a.astype(np.float64) @ w.T) < (1e-6 if act_dtype == ir.F32 else 4e-4), (k, n)
+
+
+@pytest.mark.parametrize("rows", [1, 3, 8, 9, 17, 32])
+def test_bf16_products_of_few_rows(rows):
+    """One, two and four CTAs per row tile; several tiles per CTA; k that ends inside a chunk, a second operand that begins inside a CTA's share;
+    a ring that wraps. Inputs are on the bf16 grid and products exact: f32 sums of k products are off by less than 2e-6 of the result's rms."""
+    r = np.random.default_rng(rows)
+    for k, k1, n in ((4608, 0, 1152), (2056, 136, 24), (1152, 0, 15000), (1096, 0, 2400)):
+        x, w, more = to_bf16(r.standard_normal((rows, k))), to_bf16(r.standard_normal((n, k))), {}
+        want = x.astype(np.float64) @ w.T.astype(np.float64)
+        if k1:
+            more = {"x1": to_bf16(r.standard_normal((rows, k1))), "w1": to_bf16(r.standard_normal((n, k1)))}
+            want = want + more["x1"].astype(np.float64) @ more["w1"].T.astype(np.float64)
+        assert rel_err(run_linear(ir.BF16, x, w, **more), want) < 2e-6, (k, n)
+    x, w = to_bf16(r.standard_normal((rows, 2304))), to_bf16(r.standard_normal((130, 2304)) / 48)
+    z = x.astype(np.float64) @ w.T.astype(np.float64)
+    g, u = np.minimum(z[:, ::2], 1.5), np.clip(z[:, 1::2], -1.5, 1.5)
+    assert rel_err(run_linear(ir.BF16, x, w, glu=(1.7, 1.5, 1.0)), g / (1 + np.exp(-1.7 * g)) * (u + 1)) < 3e-6
+
+
+@pytest.mark.parametrize("rows", [40, 300, 1100])
+def test_bf16_products_in_persistent_tiles(rows):
+    """More tiles than resident CTAs, the last round short; tiles that end inside a tile in both directions; plain, gated, with a function."""
+    r = np.random.default_rng(rows)
+    for k, n in ((136, 20010), (520, 9000)):
+        x, w = to_bf16(r.standard_normal((rows, k))), to_bf16(r.standard_normal((n, k)) / np.sqrt(k))
+        z = x.astype(np.float64) @ w.T.astype(np.float64)
+        assert rel_err(run_linear(ir.BF16, x, w), z) < 2e-6
+        g, u = np.minimum(z[:, ::2], 2.0), np.clip(z[:, 1::2], -2.0, 2.0)
+        assert rel_err(run_linear(ir.BF16, x, w, glu=(1.7, 2.0, 1.0)), g / (1 + np.exp(-1.7 * g)) * (u + 1)) < 3e-6
+
+
+@pytest.mark.parametrize("n", [1, 8, 9, 32, 70, 600])
+def test_experts_with_long_products(n):
+    """Weights that go through the rings several times, pieces of the second product over clusters; grouped tiles of many experts. `check` compares with
+    the plain implementation at the tolerance of its own tests."""
+    m = Experts("bf16", 1160, 12, 3, 840)
+    m.check(m.rows(n))
+
+
+def test_gelu_of_every_half():
+    """All 65 536 values, many times over, alone and times another: the table's bits are those of the element-wise kernel that small tensors take."""
+    bits = np.arange(65536, dtype=np.uint16).view(np.float16)
+    for form in ("tanh", "none"):
+        outs = []
+        for copies in (1, 17):
+            x = np.tile(bits, copies)
+            m = (0.5 + np.arange(x.size) % 7).astype(np.float16)
+            b = ir.GraphBuilder()
+            xi, mi = b.input("x", ir.F16, [x.size]), b.input("m", ir.F16, [x.size])
+            g = b.composite("Gelu", {"approximate": form}, [xi], [(ir.F16, [x.size])])[0]
+            h = b.composite("Gelu", {"approximate": form}, [xi], [(ir.F16, [x.size])])[0]
+            b.output("g", g)
+            b.output("p", b.mul(h, mi))
+            got = be.run_once(cuda_backend(), b.finish(), {"x": HostTensor.from_numpy(x), "m": HostTensor.from_numpy(m)})
+            outs.append([v.numpy()[:65536] for _, v in got])
+        assert np.array_equal(outs[0][0], outs[1][0], equal_nan=True) and np.array_equal(outs[0][1], outs[1][1], equal_nan=True)
+
+
+@pytest.mark.parametrize("heads,kv,d,past,seq,window", [(4, 1, 256, 0, 100, -1), (8, 2, 64, 300, 40, 70), (3, 3, 128, 50, 33, -1), (6, 2, 128, 0, 700, 129),
+                                                        (2, 1, 64, 1, 16, 0)])
+def test_prefill_attention_with_kept_scores(heads, kv, d, past, seq, window):
+    """Pairs of heads and single ones, windows shorter and longer than a block, ranges that end inside a block, a query tile that is not full;
+    the bounds are those of the kernel's own tests (every rounding of the decomposition is repeated, sums differ in the last bits)."""
+    module, feed = models.build_gqa(2, heads, kv, d, past, seq, ir.F16, window, True, seed=seq)
+    got, want = differential(module, feed, atol=4e-3, rtol=4e-3)
+    g, w = got[0][1].numpy(), want[0][1].numpy()
+    assert (g != w).mean() <= 0.15
+
+
+@pytest.mark.parametrize("rows,k,k1,n", [(1100, 2056, 0, 9000), (700, 1032, 1032, 12000), (2048, 1152, 0, 4610)])
+def test_bf16_products_of_pairs_of_ctas(rows, k, k1, n):
+    """Enough tiles for pairs; tiles that end inside either CTA's half in both directions, several rounds per pair, rings that wrap."""
+    r = np.random.default_rng(rows)
+    x, w, more = to_bf16(r.standard_normal((rows, k))), to_bf16(r.standard_normal((n, k)) / np.sqrt(k)), {}
+    z = x.astype(np.float64) @ w.T.astype(np.float64)
+    if k1:
+        more = {"x1": to_bf16(r.standard_normal((rows, k1))), "w1": to_bf16(r.standard_normal((n, k1)) / np.sqrt(k1))}
+        z = z + more["x1"].astype(np.float64) @ more["w1"].T.astype(np.float64)
+    bias = to_bf16(r.standard_normal(n))
+    assert rel_err(run_linear(ir.BF16, x, w, bias=bias, **more), z + bias) < 2e-6
+    if not k1:
+        z = z + bias
+        g, u = np.minimum(z[:, ::2], 2.0), np.clip(z[:, 1::2], -2.0, 2.0)
+        assert rel_err(run_linear(ir.BF16, x, w, bias=bias, glu=(1.7, 2.0, 1.0)), g / (1 + np.exp(-1.7 * g)) * (u + 1)) < 3e-6
