@@ -428,24 +428,26 @@ __global__ void __launch_bounds__(256) nbits_widen(const WidenP p) {
     }
 }
 
-constexpr int kWideRows = 128, kWideThreads = 192, kWideStage = 2 * kPanelA, kWideStages = 3;  // stage: 128 weight rows and 128 activation rows × 64 k
+constexpr int kWideRows = 128, kWideWarps = 10, kWideThreads = kWideWarps * 32;  // warps 0-7 epilogue, 8 TMA, 9 MMA
+constexpr int kWideStage = 2 * kPanelA, kWideStages = 6;                          // stage: 128 weight rows and 128 activation rows × 64 k
 struct WideP {
     alignas(64) unsigned char maps[2][128];  // weights of the panel, activations
     __half* y[3];
-    float* partial;              // [splits][m][n_pad] with splits > 1
+    float* partial;              // apart: [pieces][m][n_pad]
     ErrWord* err;
     long long m, n_pad;
     long long seg_n[3];
     int seg_rt0[4];
     int n_seg, interleave2, row_tiles, rt_first;  // rt_first: the panel's first row tile
-    int steps, chunk, m_tiles, o_tiles, splits, node;
+    int k_tiles, n_full, splits; // as in nbits_gemm_tc: row blocks before n_full take all of k, the others that many pieces
+    int apart;                   // pieces are CTAs' work of their own; nbits_gemm_reduce adds them up
+    int m_tiles, o_tiles, node;
 };
-// Persistent CTAs, 128 weight rows × 128 activation rows per tile. The tensor core adds without rounding to nearest, so `chunk` steps of 64 k
-// go into one of two accumulators in turn and the epilogue warps add what an accumulator holds to their own f32 sums, one column per register,
-// while the next chunk runs: chains no longer than the ones of nbits_gemm_tc.
-// 300 / 512 / 1024 rows, widening included: k 1152, 13 824 weight rows 35 / 36 / 46 µs (nbits_gemm_tc 49 / 55 / 109), k 6912, 1152 weight rows
-// 27 / 29 / 38 µs (40 / 42 / 83). One pass of nbits_gemm_tc (256 rows) is the shorter way, two are not: the line lies there.
-__global__ void __launch_bounds__(kWideThreads, 2) nbits_gemm_wide(const __grid_constant__ WideP p) {
+// Persistent CTAs, 128 weight rows × 128 activation rows per tile. Every sum is formed as nbits_gemm_tc forms it, bit for bit: 128-k steps go in
+// turn into two accumulators, which are added in f32 (the tensor core adds without rounding to nearest: shorter chains), and the pieces
+// of k are added in f64. A piece's accumulators are read, half of the columns per group of four warps, while the next piece runs in the other two.
+// 2047 rows through six layers of the 1B architecture (24 products): 1.06 ms and 0.13 ms of widening; nbits_gemm_tc and its reductions took 3.75.
+__global__ void __launch_bounds__(kWideThreads, 1) nbits_gemm_wide(const __grid_constant__ WideP p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -455,11 +457,11 @@ __global__ void __launch_bounds__(kWideThreads, 2) nbits_gemm_wide(const __grid_
     pdl_trigger();
     if (tid == 0) {
         for (int s = 0; s < 2 * kWideStages + 2; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + s * 8) : "memory");
-        for (int s = 0; s < 2; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(read + s * 8) : "memory");
+        for (int s = 0; s < 2; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(read + s * 8) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 5) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(s_addr(tmem_slot)) : "memory");
+    if (warp == 9) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(s_addr(tmem_slot)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -467,21 +469,30 @@ __global__ void __launch_bounds__(kWideThreads, 2) nbits_gemm_wide(const __grid_
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned tmem = *tmem_slot;
     pdl_wait();
-    const int total = p.m_tiles * p.o_tiles * p.splits;
-    auto range = [&](int t, int& lo, int& n) {
-        const int piece = t / p.m_tiles / p.o_tiles;
-        lo = (int)((long long)p.steps * piece / p.splits);
-        n = (int)((long long)p.steps * (piece + 1) / p.splits) - lo;
+    const int units = p.m_tiles * p.o_tiles * (p.apart ? p.splits : 1);  // activation tiles fastest, pieces slowest
+    // a unit's tile and pieces; a piece's 128-k steps
+    struct Unit {
+        int m0, o0, pieces, from, to;
     };
+    auto unit_of = [&](int u) {
+        Unit q;
+        const int rest = u / p.m_tiles, o = rest % p.o_tiles;
+        q.m0 = u % p.m_tiles * kWideRows;
+        q.o0 = o * 128;
+        q.pieces = (p.rt_first >> 3) + o < p.n_full ? 1 : p.splits;
+        q.from = p.apart ? rest / p.o_tiles : 0;
+        q.to = p.apart ? q.from + 1 : q.pieces;
+        return q;
+    };
+    auto first_step = [&](const Unit& q, int piece) { return (int)((long long)p.k_tiles * piece / q.pieces); };
     bool ok = true;
-    if (warp == 4) {
+    if (warp == 8) {
         if (lane == 0) {
             int done = 0;
-            for (int t = (int)blockIdx.x; t < total && ok; t += (int)gridDim.x) {
-                int lo, n;
-                range(t, lo, n);
-                const int m0 = t % p.m_tiles * kWideRows, o0 = t / p.m_tiles % p.o_tiles * 128;
-                for (int i = 0; i < n; i++, done++) {
+            for (int u = (int)blockIdx.x; u < units && ok; u += (int)gridDim.x) {
+                const Unit q = unit_of(u);
+                const int lo = first_step(q, q.from) * 2, hi = first_step(q, q.to) * 2;  // 64-k steps; pieces follow one another
+                for (int i = lo; i < hi; i++, done++) {
                     const int s = done % kWideStages;
                     if (done >= kWideStages && !bar_wait_tc(empty + s * 8, ((done / kWideStages) - 1) & 1)) {
                         ok = false;
@@ -493,7 +504,7 @@ __global__ void __launch_bounds__(kWideThreads, 2) nbits_gemm_wide(const __grid_
                     for (int op = 0; op < 2; op++)
                         asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
                                          dst + op * kPanelA),
-                                     "l"(reinterpret_cast<unsigned long long>(&p.maps[op])), "r"((lo + i) * 64), "r"(op ? m0 : o0), "r"(bar)
+                                     "l"(reinterpret_cast<unsigned long long>(&p.maps[op])), "r"(i * 64), "r"(op ? q.m0 : q.o0), "r"(bar)
                                      : "memory");
                 }
             }
@@ -501,17 +512,17 @@ __global__ void __launch_bounds__(kWideThreads, 2) nbits_gemm_wide(const __grid_
             for (int n = max(0, done - kWideStages); n < done; n++)
                 if (!bar_wait_tc(full + n % kWideStages * 8, (n / kWideStages) & 1)) ok = false;
         }
-    } else if (warp == 5) {
+    } else if (warp == 9) {
         const unsigned idesc = (1u << 4) | ((kWideRows >> 3) << 17) | (8u << 24);  // f16 × f16 → f32, M 128 × N 128
         int done = 0, j = 0;
-        for (int t = (int)blockIdx.x; t < total; t += (int)gridDim.x) {
-            int lo, n;
-            range(t, lo, n);
-            for (int c = 0; c < n; c += p.chunk, j++) {
-                const unsigned d = tmem + (unsigned)((j & 1) * kWideRows);
+        for (int u = (int)blockIdx.x; u < units; u += (int)gridDim.x) {
+            const Unit q = unit_of(u);
+            for (int piece = q.from; piece < q.to; piece++, j++) {
+                const int n = first_step(q, piece + 1) - first_step(q, piece);
+                const unsigned d = tmem + (unsigned)((j & 1) * 2 * kWideRows);
                 if (j >= 2 && ok && !bar_wait_tc(read + (j & 1) * 8, ((j >> 1) - 1) & 1)) ok = false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int i = c; i < min(n, c + p.chunk); i++, done++) {
+                for (int i = 0; i < 2 * n; i++, done++) {
                     const int s = done % kWideStages;
                     if (ok && !bar_wait_tc(full + s * 8, (done / kWideStages) & 1)) ok = false;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -521,8 +532,8 @@ __global__ void __launch_bounds__(kWideThreads, 2) nbits_gemm_wide(const __grid_
                         for (int e = 0; e < 4; e++)
                             asm volatile(
                                 "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                                " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n" ::"r"(d),
-                                "l"(umma_desc(a0 + e * 32)), "l"(umma_desc(b0 + e * 32)), "r"(idesc), "r"(i > c || e > 0 ? 1u : 0u), "r"(0u)
+                                " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n" ::"r"(d + (unsigned)((i >> 1 & 1) * kWideRows)),
+                                "l"(umma_desc(a0 + e * 32)), "l"(umma_desc(b0 + e * 32)), "r"(idesc), "r"(i >= 4 || (i & 1) || e > 0 ? 1u : 0u), "r"(0u)
                                 : "memory");
                         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(empty + s * 8) : "memory");
                     }
@@ -533,66 +544,76 @@ __global__ void __launch_bounds__(kWideThreads, 2) nbits_gemm_wide(const __grid_
             }
         }
     } else {
+        constexpr int kCols = kWideRows / 2;
+        const int lanes = (warp & 3) * 32, col0 = (warp >> 2) * kCols;
         int j = 0;
-        for (int t = (int)blockIdx.x; t < total; t += (int)gridDim.x) {
-            int lo, n;
-            range(t, lo, n);
-            float sum[kWideRows];
+        for (int u = (int)blockIdx.x; u < units; u += (int)gridDim.x) {
+            const Unit q = unit_of(u);
+            const long long m0 = q.m0 + col0;
+            const int row_in_panel = q.o0 + lanes + lane, rtg = p.rt_first + (row_in_panel >> 4);
+            double sum[kCols];
 #pragma unroll
-            for (int e = 0; e < kWideRows; e++) sum[e] = 0.f;
-            for (int c = 0; c < n; c += p.chunk, j++) {
+            for (int e = 0; e < kCols; e++) sum[e] = 0.0;
+            for (int piece = q.from; piece < q.to; piece++, j++) {
+                const int accs = min(2, first_step(q, piece + 1) - first_step(q, piece));
                 if (ok && !bar_wait_tc(finished + (j & 1) * 8, (j >> 1) & 1)) ok = false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const unsigned d = tmem + (unsigned)((j & 1) * kWideRows) + ((unsigned)(warp * 32) << 16);
+                const unsigned d = tmem + (unsigned)((j & 1) * 2 * kWideRows + col0) + ((unsigned)lanes << 16);
 #pragma unroll
-                for (int e = 0; e < kWideRows; e += 16) {
-                    unsigned v[16];
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                        : "r"(d + (unsigned)e));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                for (int c = 0; c < kCols; c += 16) {
+                    float part[16];
 #pragma unroll
-                    for (int q = 0; q < 16; q++) sum[e + q] += __uint_as_float(v[q]);
+                    for (int e = 0; e < 16; e++) part[e] = 0.f;
+                    for (int a = 0; a < accs; a++) {
+                        unsigned v[16];
+                        asm volatile(
+                            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+                            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+                              "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                            : "r"(d + (unsigned)(a * kWideRows + c)));
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int e = 0; e < 16; e++) part[e] += __uint_as_float(v[e]);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 16; e++) sum[c + e] += (double)part[e];
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) bar_arrive(read + (j & 1) * 8);
             }
-            const long long m0 = (long long)(t % p.m_tiles) * kWideRows;
-            const int row_in_panel = t / p.m_tiles % p.o_tiles * 128 + warp * 32 + lane, rtg = p.rt_first + (row_in_panel >> 4);
-            if (p.splits > 1) {
-                float* part = p.partial + ((size_t)(t / p.m_tiles / p.o_tiles) * p.m + m0) * p.n_pad + row_in_panel;
+            if (p.apart) {
+                float* part = p.partial + ((size_t)q.from * p.m + m0) * p.n_pad + row_in_panel;
 #pragma unroll
-                for (int e = 0; e < kWideRows; e++)
-                    if (ok && m0 + e < p.m) part[(size_t)e * p.n_pad] = sum[e];
-            } else {
-                int seg = 0;
-                long long row;
-                if (p.interleave2) {
-                    seg = rtg & 1;
-                    row = (long long)(rtg >> 1) * 16 + (row_in_panel & 15);
-                } else {
-                    if (p.n_seg > 1 && rtg >= p.seg_rt0[1]) seg = 1;
-                    if (p.n_seg > 2 && rtg >= p.seg_rt0[2]) seg = 2;
-                    row = (long long)(rtg - p.seg_rt0[seg]) * 16 + (row_in_panel & 15);
-                }
-                const long long width = p.seg_n[seg];
-                __half* y = p.y[seg] + m0 * width + row;
-                const bool row_ok = ok && rtg < p.row_tiles && row < width;
-#pragma unroll
-                for (int e = 0; e < kWideRows; e++)
-                    if (row_ok && m0 + e < p.m) y[e * width] = __float2half_rn(sum[e]);
+                for (int e = 0; e < kCols; e++)
+                    if (ok && m0 + e < p.m) part[(size_t)e * p.n_pad] = (float)sum[e];  // one piece: an f32 value
+                continue;
             }
+            int seg = 0;
+            long long row;
+            if (p.interleave2) {
+                seg = rtg & 1;
+                row = (long long)(rtg >> 1) * 16 + (row_in_panel & 15);
+            } else {
+                if (p.n_seg > 1 && rtg >= p.seg_rt0[1]) seg = 1;
+                if (p.n_seg > 2 && rtg >= p.seg_rt0[2]) seg = 2;
+                row = (long long)(rtg - p.seg_rt0[seg]) * 16 + (row_in_panel & 15);
+            }
+            const long long width = p.seg_n[seg];
+            __half* y = p.y[seg] + m0 * width + row;
+            const bool row_ok = ok && rtg < p.row_tiles && row < width;
+#pragma unroll
+            for (int e = 0; e < kCols; e++)
+                if (row_ok && m0 + e < p.m) y[e * width] = __double2half(sum[e]);
         }
     }
     if (!ok && lane == 0) report(p.err, ERR_WAIT_TIMEOUT, p.node, (long long)blockIdx.x, (long long)warp);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem) : "memory");
+    if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
+// `t`: the launch of nbits_gemm_tc for these rows (its pieces of k are kept).
 void emit_wide(Emitter& em, const NBitsGroup& gr, const TRef& x, const TRef& tiles, const TcP& t) {
     const Buf null{kSlotNull, 0};
     // panels of at most 64 MB of widened weights: they stay in L2 until the product reads them
@@ -610,7 +631,9 @@ void emit_wide(Emitter& em, const NBitsGroup& gr, const TRef& x, const TRef& til
                   {{&a.tiles, tiles.buf.at((int64_t)first * t.k_tiles * t.tile_bytes)}, {&a.w, wide}}, "nbits_widen", /*pdl=*/true);
         WideP p{};
         p.m = gr.m;
-        p.steps = t.k_tiles * 2;
+        p.k_tiles = t.k_tiles;
+        p.n_full = t.n_full;
+        p.splits = t.splits;
         p.n_seg = t.n_seg;
         p.interleave2 = t.interleave2;
         p.row_tiles = t.row_tiles;
@@ -621,30 +644,23 @@ void emit_wide(Emitter& em, const NBitsGroup& gr, const TRef& x, const TRef& til
         p.m_tiles = (int)((gr.m + kWideRows - 1) / kWideRows);
         p.o_tiles = (count + 7) / 8;
         p.n_pad = (long long)p.o_tiles * 128;
-        // Pieces along k: waves × (steps of a piece + six steps of fill and drain) plus the partial sums' trip and a second launch
-        const long long slots = 2LL * sm_count(), ctas = (long long)p.m_tiles * p.o_tiles;
-        double best = 1e300;
-        for (int sp = 1; sp <= 8 && sp * 4 <= std::max(p.steps, 4); sp++) {
-            const double waves = (double)((ctas * sp + slots - 1) / slots);
-            double us = waves * ((double)p.steps / sp + 6.0) * 0.42;
-            if (sp > 1) us += 3.0 + (double)sp * gr.m * p.n_pad * 8.0 / 5e6;
-            if (us < best * 0.97) {
-                best = us;
-                p.splits = sp;
-            }
-        }
-        const int piece = (p.steps + p.splits - 1) / p.splits;
-        p.chunk = (piece + (piece + 7) / 8 - 1) / ((piece + 7) / 8);  // equal chunks of at most eight steps
-        const Buf partial = p.splits > 1 ? em.scratch((size_t)p.splits * gr.m * p.n_pad * 4) : null;
+        // Few tiles: the pieces of k go to CTAs of their own where that, with the partial sums' trip (5 TB/s) and a second launch, is shorter
+        const long long slots = sm_count(), ctas = (long long)p.m_tiles * p.o_tiles;
+        const double step_us = 0.45;  // 128 k of a tile
+        const double joined = (double)((ctas + slots - 1) / slots) * t.k_tiles * step_us;
+        const double apart = (double)((ctas * t.splits + slots - 1) / slots) * ((double)t.k_tiles / t.splits * step_us + 1.0) + 3.0 +
+                             (double)t.splits * gr.m * p.n_pad * 8.0 / 5e6;
+        p.apart = t.splits > 1 && t.n_full == 0 && apart < joined;
+        const Buf partial = p.apart ? em.scratch((size_t)p.splits * gr.m * p.n_pad * 4) : null;
         const size_t smem = kWideStages * kWideStage + 1024 + (2 * kWideStages + 4) * 8 + 16;
-        ensure_max_dynamic_smem((const void*)nbits_gemm_wide, 110 * 1024);
-        LaunchRec& rec = em.launch(nbits_gemm_wide, dim3((unsigned)std::min<long long>(slots, ctas * p.splits)), dim3(kWideThreads), (unsigned)smem, p,
+        ensure_max_dynamic_smem((const void*)nbits_gemm_wide, 220 * 1024);
+        LaunchRec& rec = em.launch(nbits_gemm_wide, dim3((unsigned)std::min<long long>(slots, ctas * (p.apart ? p.splits : 1))), dim3(kWideThreads), (unsigned)smem, p,
                                    {{&p.err, Buf{kSlotErr, 0}}, {&p.partial, partial}, {&p.y[0], gr.y[0].buf}, {&p.y[1], gr.n_seg > 1 ? gr.y[1].buf : null},
                                     {&p.y[2], gr.n_seg > 2 ? gr.y[2].buf : null}},
                                    "nbits_gemm_wide", /*pdl=*/true);
         rec.tmaps.push_back(TmapReloc{(uint32_t)offsetof(WideP, maps), wide, (uint64_t)ld, (uint64_t)count * 16, (uint64_t)ld * 2, 64u, 128u});
         rec.tmaps.push_back(TmapReloc{(uint32_t)offsetof(WideP, maps) + 128, x.buf, (uint64_t)gr.k, (uint64_t)gr.m, (uint64_t)gr.k * 2, 64u, (uint32_t)kWideRows});
-        if (p.splits > 1) {
+        if (p.apart) {
             TcReduceP q{};
             q.m_total = gr.m;
             q.n_pad = p.n_pad;
@@ -687,12 +703,6 @@ void emit_nbits_gemm_tc(Emitter& em, const NBitsGroup& gr, const TRef& x, const 
     p.has_zp = gr.has_zp ? 1 : 0;
     p.tile_bytes = kTileWt + kTileSt + (gr.has_zp ? kTileZt : 0);
     p.node = em.node;
-    // two passes and more: measured on both sides beside nbits_gemm_wide
-    static const long long wide_from = [] {
-        const char* e = std::getenv("ONYXIA_GEMM_WIDE_FROM");  // diagnostics: activation rows from which the weights are widened into scratch
-        return e ? std::atoll(e) : 257LL;
-    }();
-    if (gr.m >= wide_from && gr.m < 65536 && gr.k % 8 == 0 && x.buf.off % 16 == 0) return emit_wide(em, gr, x, tiles, p);
     // activation rows per pass: the smallest MMA N that holds them all, at most 256
     int mb = 16;
     while (mb < gr.m && mb < 256) mb <<= 1;
@@ -744,6 +754,12 @@ void emit_nbits_gemm_tc(Emitter& em, const NBitsGroup& gr, const TRef& x, const 
     if (debug) std::fprintf(stderr, "nbits_gemm_tc: m %lld k_tiles %d grid %u mb %d: %d pieces over %lld of the row blocks\n", gr.m, p.k_tiles, grid, mb, splits, tail);
     p.n_full = (int)n_full;
     p.splits = splits;
+    // two passes and more: measured on both sides beside nbits_gemm_wide
+    static const long long wide_from = [] {
+        const char* e = std::getenv("ONYXIA_GEMM_WIDE_FROM");  // diagnostics: activation rows from which the weights are widened into scratch
+        return e ? std::atoll(e) : 257LL;
+    }();
+    if (gr.m >= wide_from && gr.m < 65536 && gr.k % 8 == 0 && x.buf.off % 16 == 0) return emit_wide(em, gr, x, tiles, p);
     p.n_pad = tail * 128;
     const Buf partial = splits > 1 ? em.scratch((size_t)splits * mb * p.n_pad * sizeof(float)) : null;
     for (long long m0 = 0; m0 < gr.m; m0 += mb) {
