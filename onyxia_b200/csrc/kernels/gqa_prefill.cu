@@ -16,6 +16,7 @@
 //   pass 3  p = round16(e / Σ) becomes the A operand of the P·V product straight from the score
 //           tile's accumulator registers; V rows are the B operand through ldmatrix.trans; the four
 //           key groups' f32 partial outputs are added in group order through shared memory
+// Where the scores of two heads' rows fit in shared memory they are kept there instead (gqa_prefill_scores).
 // K (and V in pass 3) blocks of 64 keys are staged by cp.async into padded shared-memory rows, two
 // stages deep. Products are exact f16 × f16 and are added in f32 by the tensor core (the interpreter
 // adds in f64): results differ from it by an f16 spacing on a small share of the elements, like the
@@ -53,6 +54,7 @@ struct PrefillP {
     const long long* dyn_t;  // when set, the present length T is read from here
     long long B, S, H, KV, T, cap, window;
     float scale;        // rounded to f16
+    int score_stride;   // gqa_prefill_scores: elements between two rows of scores
 };
 
 __device__ __forceinline__ void ldsm_x4(unsigned (&r)[4], unsigned addr) {
@@ -305,9 +307,218 @@ template <int D> __global__ void __launch_bounds__(kNT) gqa_prefill_tc(const Pre
     }
 }
 
+// The same where the scores of 32 rows (16 query positions of two heads that share their keys) fit in shared memory: they are formed once, turned
+// into probabilities in place and read back as the A operand. Scores, sums and outputs are formed in the order of the kernel above, bit
+// for bit. A staged block of 64 keys or values serves both heads, the warps' query fragments stay in registers, one barrier per block.
+// 2047 positions, 4 heads of 256 over one key head, windows of 512 in five layers of six: 74 µs a layer, 212 with three walks over the keys.
+constexpr int kSWarps = 16, kSThreads = kSWarps * 32, kSRows = 2 * kBM;
+template <int D> __global__ void __launch_bounds__(kSThreads, 1) gqa_prefill_scores(const PrefillP p) {
+    constexpr int RS = D + kPad, CPR = D / 8, KS = D / 16;
+    constexpr int DQ = D / 4, NDT = DQ / 8;  // this warp's output columns, in tiles of 8
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __half* Ks = reinterpret_cast<__half*>(smem_raw);  // [2][kKB][RS] keys, then values; the queries pass through it first
+    __half* Sc = Ks + 2 * kKB * RS;                    // [32][ss]
+    const int ss = p.score_stride;
+    pdl_enter();
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gq = lane >> 2, t = lane & 3;
+    const long long b = blockIdx.z, G = p.H / p.KV, head0 = blockIdx.y * 2, kvh = head0 / G;
+    const long long s0 = (long long)blockIdx.x * kBM;
+    const long long T = p.T;
+    const long long tot = (long long)p.seqlens[b] + 1, past_b = tot - p.S > 0 ? tot - p.S : 0;
+    const long long s_last = (s0 + kBM < p.S ? s0 + kBM : p.S) - 1;
+    const long long hi_blk = past_b + s_last < T - 1 ? past_b + s_last : T - 1;
+    const long long lo_blk = (p.window >= 0 && past_b + s0 - p.window > 0) ? past_b + s0 - p.window : 0;
+    const long long n_blk = hi_blk >= lo_blk ? hi_blk - lo_blk + 1 : 0;
+    const int nkb = (int)((n_blk + kKB - 1) / kKB);
+    auto out_of = [&](int row) { return p.out + ((b * p.S + s0 + (row & 15)) * p.H + head0 + (row >> 4)) * D; };
+
+    if (nkb == 0) {  // nothing visible: the rows are zero
+        for (int i = tid; i < kSRows * D; i += kSThreads)
+            if (s0 + (i / D & 15) < p.S) out_of(i / D)[i % D] = __float2half(0.f);
+        return;
+    }
+    const __half* kbase = p.pk + (b * p.KV + kvh) * p.cap * D;
+    const __half* vbase = p.pv + (b * p.KV + kvh) * p.cap * D;
+    auto load_block = [&](const __half* base, int kb) {
+        if (kb >= nkb) return;
+        __half* to = Ks + (kb & 1) * kKB * RS;
+        for (int i = tid; i < kKB * CPR; i += kSThreads) {
+            const int r = i / CPR, c = i - r * CPR;
+            long long tk = lo_blk + (long long)kb * kKB + r;
+            if (tk > hi_blk) tk = hi_blk;  // rows past the range are masked; any valid row will do
+            cp16(smem_addr(to + r * RS + c * 8), base + tk * D + c * 8);
+        }
+    };
+    auto landed = [&]() {  // this thread's copies; then everybody's
+        asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+    };
+
+    // ── scores: warp = (16 rows mt, key tile n of a block) ──
+    const int mt = warp >> 3, n = warp & 7;
+    for (int i = tid; i < kSRows * CPR; i += kSThreads) {
+        const int r = i / CPR, c = i - r * CPR;
+        const long long s = min(s0 + (r & 15), p.S - 1);  // rows past S repeat the last one; they are never stored
+        cp16(smem_addr(Ks + r * RS + c * 8), p.q + ((b * p.S + s) * p.H + head0 + (r >> 4)) * D + c * 8);
+    }
+    landed();
+    unsigned qf[KS][4];
+    {
+        const unsigned q_addr = smem_addr(Ks + (mt * 16 + (lane & 15)) * RS + (lane >> 4) * 8);
+#pragma unroll
+        for (int j = 0; j < KS; j++) ldsm_x4(qf[j], q_addr + j * 32);
+    }
+    __syncthreads();
+    int lo[2], hi[2];  // the keys that this thread's two rows may see, as offsets from lo_blk
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        const long long s = s0 + gq + r * 8, qpos = past_b + s;
+        const long long l_ = (p.window >= 0 && qpos - p.window > 0) ? qpos - p.window : 0;
+        lo[r] = (int)(l_ - lo_blk);
+        hi[r] = s < p.S ? (int)((qpos < T - 1 ? qpos : T - 1) - lo_blk) : -1;
+    }
+    load_block(kbase, 0);
+    for (int kb = 0; kb < nkb; kb++) {
+        landed();
+        load_block(kbase, kb + 1);  // into the stage that everybody has left
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        const unsigned k_addr = smem_addr(Ks + ((kb & 1) * kKB + n * 8 + (lane & 7)) * RS + (lane >> 3) * 8);
+#pragma unroll
+        for (int j = 0; j < KS; j += 2) {
+            unsigned bf[4];
+            ldsm_x4(bf, k_addr + j * 32);
+            mma16816(acc, qf[j][0], qf[j][1], qf[j][2], qf[j][3], bf[0], bf[1]);
+            mma16816(acc, qf[j + 1][0], qf[j + 1][1], qf[j + 1][2], qf[j + 1][3], bf[2], bf[3]);
+        }
+        const int col = kb * kKB + n * 8 + 2 * t;
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            __half v[2];
+#pragma unroll
+            for (int e = 0; e < 2; e++)
+                v[e] = col + e >= lo[r] && col + e <= hi[r] ? __float2half_rn(r16(acc[r * 2 + e]) * p.scale) : __ushort_as_half(0xFC00);
+            *reinterpret_cast<__half2*>(Sc + (mt * 16 + gq + r * 8) * ss + col) = __halves2half2(v[0], v[1]);
+        }
+    }
+    __syncthreads();
+    load_block(vbase, 0);  // on their way while the rows are normalised
+
+    // ── probabilities: two rows per warp, eight scores per lane and step ──
+    const int eights = nkb * kKB / 8;
+    for (int i = 0; i < kSRows / kSWarps; i++) {
+        uint4* row = reinterpret_cast<uint4*>(Sc + (warp * (kSRows / kSWarps) + i) * ss);
+        __half2 most = __halves2half2(__ushort_as_half(0xFC00), __ushort_as_half(0xFC00));
+        for (int c = lane; c < eights; c += 32) {
+            const uint4 v = row[c];
+            most = __hmax2(__hmax2(most, __hmax2(uh(v.x), uh(v.y))), __hmax2(uh(v.z), uh(v.w)));
+        }
+        float m = fmaxf(__low2float(most), __high2float(most));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const __half hmax = __float2half_rn(m);  // an f16 value already
+        if (m == -INFINITY) {                    // a row that sees nothing
+            for (int c = lane; c < eights; c += 32) row[c] = make_uint4(0, 0, 0, 0);
+            continue;
+        }
+        unsigned long long sum = 0;  // every term is a multiple of 2^-24 not above 1: added as integers
+        for (int c = lane; c < eights; c += 32) {
+            const uint4 v = row[c];
+            const unsigned in[4] = {v.x, v.y, v.z, v.w};
+            unsigned out[4], part = 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const __half2 s2 = uh(in[k]);
+                const __half lo_e = g_pf_exp_lut[__half_as_ushort(__hsub(__low2half(s2), hmax)) & 0x7FFF];
+                const __half hi_e = g_pf_exp_lut[__half_as_ushort(__hsub(__high2half(s2), hmax)) & 0x7FFF];
+                part += (unsigned)(__half2float(lo_e) * 16777216.f) + (unsigned)(__half2float(hi_e) * 16777216.f);
+                out[k] = hu(__halves2half2(lo_e, hi_e));
+            }
+            sum += part;
+            row[c] = make_uint4(out[0], out[1], out[2], out[3]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        const float total = r16d((double)sum * 5.9604644775390625e-08);
+        for (int c = lane; c < eights; c += 32) {  // (a lane's own words)
+            const uint4 v = row[c];
+            const unsigned in[4] = {v.x, v.y, v.z, v.w};
+            unsigned out[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {  // e and Σ are f16 values: their f32 quotient rounds to the same f16 as the exact one
+                const float2 e = __half22float2(uh(in[k]));
+                out[k] = hu(__floats2half2_rn(e.x / total, e.y / total));
+            }
+            row[c] = make_uint4(out[0], out[1], out[2], out[3]);
+        }
+    }
+
+    // ── probabilities × V: 16 keys of each block, all 32 rows, a quarter of the head dimension ──
+    const int kg = warp >> 2, wq = warp & 3;
+    float o[2][NDT][4];
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+        for (int v = 0; v < NDT; v++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) o[r][v][e] = 0.f;
+    for (int kb = 0; kb < nkb; kb++) {
+        landed();  // (and the rows' probabilities with the first block)
+        load_block(vbase, kb + 1);
+        unsigned a[2][4];
+#pragma unroll
+        for (int r = 0; r < 2; r++) ldsm_x4(a[r], smem_addr(Sc + (r * 16 + (lane & 15)) * ss + kb * kKB + kg * 16 + (lane >> 4) * 8));
+        const unsigned v_addr = smem_addr(Ks + ((kb & 1) * kKB + kg * 16 + (lane & 15)) * RS + wq * DQ + (lane >> 4) * 8);
+#pragma unroll
+        for (int v = 0; v < NDT; v += 2) {
+            unsigned bf[4];
+            ldsm_x4_t(bf, v_addr + v * 16);
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                mma16816(o[r][v], a[r][0], a[r][1], a[r][2], a[r][3], bf[0], bf[1]);
+                mma16816(o[r][v + 1], a[r][0], a[r][1], a[r][2], a[r][3], bf[2], bf[3]);
+            }
+        }
+    }
+    // the four key groups' partial outputs are added in group order, one head after the other in the staging area
+    float* part = reinterpret_cast<float*>(Ks);  // [4][16][D]
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        __syncthreads();
+#pragma unroll
+        for (int v = 0; v < NDT; v++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) part[(kg * kBM + gq + (e >> 1) * 8) * D + wq * DQ + v * 8 + 2 * t + (e & 1)] = o[r][v][e];
+        __syncthreads();
+        for (int i = tid; i < kBM * D / 2; i += kSThreads) {
+            const int row = i / (D / 2), col = (i - row * (D / 2)) * 2;
+            if (s0 + row >= p.S) continue;
+            float v0 = 0.f, v1 = 0.f;
+#pragma unroll
+            for (int g4 = 0; g4 < 4; g4++) {
+                const float2 f = *reinterpret_cast<const float2*>(part + (g4 * kBM + row) * D + col);
+                v0 += f.x;
+                v1 += f.y;
+            }
+            *reinterpret_cast<__half2*>(out_of(r * 16 + row) + col) = __halves2half2(__float2half_rn(v0), __float2half_rn(v1));
+        }
+    }
+}
+
 template <int D> void launch_prefill(Emitter& em, PrefillP& p, long long B, long long S, long long H, Buf q, Buf pk, Buf pv, Buf seqlens,
                                      Buf out, Buf dyn_t) {
     constexpr int RS = D + kPad;
+    // Two heads per key head and scores that fit beside the stages (200 KB: 2047 positions at a head size of 256, all visible) take the kernel
+    // that forms them once; longer ranges walk the keys three times.
+    const long long seen = p.window >= 0 ? std::min(p.T, p.window + kBM) : p.T;  // keys that a CTA's rows see, at most
+    p.score_stride = (int)((std::min<long long>(seen, 1 << 20) + kKB - 1) / kKB * kKB) + 8;  // 16 bytes off a multiple of 128: conflict-free
+    const size_t kept = ((size_t)2 * kKB * RS + (size_t)kSRows * p.score_stride) * 2;
+    if (H / p.KV % 2 == 0 && dyn_t.slot == kSlotNull && kept <= 200 * 1024) {
+        ensure_max_dynamic_smem((const void*)gqa_prefill_scores<D>, 200 * 1024);
+        em.launch(gqa_prefill_scores<D>, dim3((unsigned)((S + kBM - 1) / kBM), (unsigned)(H / 2), (unsigned)B), dim3(kSThreads), (unsigned)kept, p,
+                  {{&p.q, q}, {&p.pk, pk}, {&p.pv, pv}, {&p.seqlens, seqlens}, {&p.out, out}, {&p.dyn_t, dyn_t}}, "gqa_prefill_tc", /*pdl=*/true);
+        return;
+    }
     const size_t smem = (size_t)(kBM + 4 * kKB) * RS * 2;
     static_assert((size_t)4 * kBM * D * 4 <= (size_t)2 * kKB * (D + kPad) * 2, "the partial outputs must fit the K staging area");
     auto fn = gqa_prefill_tc<D>;
