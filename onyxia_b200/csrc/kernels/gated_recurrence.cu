@@ -433,11 +433,7 @@ template <typename T> __global__ void __launch_bounds__(128) recurrence_gates_si
         float e = 0.f, b = 0.f;
         if (token) {
             const T *wr = (const T*)p.ra + (long long)c * n, *wi = (const T*)p.ri + (long long)c * n;
-            float zr = 0.f, zi = 0.f;
-            for (int j = 0; j < n; j++) {
-                zr = fmaf(uf[j], to_f(wr[j]), zr);
-                zi = fmaf(uf[j], to_f(wi[j]), zi);
-            }
+            const float zr = dot_in_order(uf, wr, n, 0.f), zi = dot_in_order(uf, wi, n, 0.f);
             gate_values(-p.decay * softplus_f(p.lam[c]), zr + p.rab[c], zi + p.rib[c], uf[k], &e, &b);
             if (row == s.start) enter(p, s, slot, c, &e, &b);
         }

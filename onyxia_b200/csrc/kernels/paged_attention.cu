@@ -114,8 +114,7 @@ template <typename T> __global__ void __launch_bounds__(128) paged_attn_simt(con
         if (j <= pos) {
             const long long pg = page_of(p, s, j);
             const T* k = (const T*)p.pool + key_row(p, pg, g, j) * p.dim;
-            float d = 0.f;
-            for (int i = 0; i < p.dim; i++) d = fmaf(q[i], to_f(k[i]), d);
+            const float d = dot_in_order(q, k, p.dim, 0.f);
             sc = d * p.kscale[scale_at(p, pg, j)];
             if (p.bias) sc += p.bias[(long long)h * p.nd + min(pos - j, p.nd - 1)];
         }
@@ -125,15 +124,7 @@ template <typename T> __global__ void __launch_bounds__(128) paged_attn_simt(con
         l = l * keep + block_sum(e, red);  // (its barriers order the stores to w)
         m = m2;
         const int live = min(128, pos + 1 - j0);
-        for (int i = tid; i < p.dim; i += 128) {
-            float a = acc[i] * keep;
-            long long pg = 0;
-            for (int jj = 0; jj < live; jj++) {
-                if (jj == 0 || ((j0 + jj) & ((1 << p.shift) - 1)) == 0) pg = page_of(p, s, j0 + jj);
-                a = fmaf(w[jj], to_f(((const T*)p.pool)[key_row(p, pg, g, j0 + jj) * p.dim + i]), a);
-            }
-            acc[i] = a;
-        }
+        for (int i = tid; i < p.dim; i += 128) acc[i] = weigh_in_order(p, (const T*)p.pool, s, g, j0, live, p.dim, i, w, acc[i] * keep);
         __syncthreads();
     }
     for (int i = tid; i < p.dim; i += 128) ((T*)p.out)[((long long)row * p.heads + h) * p.dim + i] = from_f<T>(acc[i] / l * p.out_scale);

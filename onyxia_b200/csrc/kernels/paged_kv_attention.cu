@@ -117,9 +117,7 @@ template <typename T> __global__ void __launch_bounds__(128) paged_kv_simt(const
         float sc = -INFINITY;
         if (j <= pos) {
             const T* k = (const T*)p.keys + key_row(p, page_of(p, s, j), g, j) * p.dim;
-            float d = 0.f;
-            for (int i = 0; i < p.dim; i++) d = fmaf(q[i], to_f(k[i]), d);
-            sc = d * p.scale * temp_of(p, h);
+            sc = dot_in_order(q, k, p.dim, 0.f) * p.scale * temp_of(p, h);
             if (p.cap > 0.f) sc = p.cap * tanhf(sc / p.cap);
         }
         const float m2 = fmaxf(m, block_max(sc, red));
@@ -128,15 +126,7 @@ template <typename T> __global__ void __launch_bounds__(128) paged_kv_simt(const
         l = l * keep + block_sum(e, red);  // (its barriers order the stores to w)
         m = m2;
         const int live = min(128, pos + 1 - j0);
-        for (int i = tid; i < p.vdim; i += 128) {
-            float a = acc[i] * keep;
-            long long pg = 0;
-            for (int jj = 0; jj < live; jj++) {
-                if (jj == 0 || ((j0 + jj) & ((1 << p.shift) - 1)) == 0) pg = page_of(p, s, j0 + jj);
-                a = fmaf(w[jj], to_f(((const T*)p.values)[key_row(p, pg, g, j0 + jj) * p.ldv + i]), a);
-            }
-            acc[i] = a;
-        }
+        for (int i = tid; i < p.vdim; i += 128) acc[i] = weigh_in_order(p, (const T*)p.values, s, g, j0, live, p.ldv, i, w, acc[i] * keep);
         __syncthreads();
     }
     const float f = gate_of<T>(p, row, h) / l;

@@ -20,6 +20,17 @@ template <class P> __device__ __forceinline__ long long page_of(const P& p, int 
 template <class P> __device__ __forceinline__ long long key_row(const P& p, long long pg, int g, int pos) {
     return ((pg * p.kv_heads + g) << p.shift) + (pos & ((1 << p.shift) - 1));
 }
+// a + Σ w[jj] · (element i of the rows of positions j0 + jj), one after the other; `ld` elements per row. Several loads of a page in flight.
+template <typename T, class P>
+__device__ __forceinline__ float weigh_in_order(const P& p, const T* pool, int seq, int g, int j0, int live, long long ld, int i, const float* w, float a) {
+    for (int jj = 0; jj < live;) {
+        const int end = min(live, ((j0 + jj) | ((1 << p.shift) - 1)) + 1 - j0);
+        const T* v = pool + key_row(p, page_of(p, seq, j0 + jj), g, j0 + jj) * ld + i;
+#pragma unroll 8
+        for (; jj < end; jj++, v += ld) a = fmaf(w[jj], to_f(*v), a);
+    }
+    return a;
+}
 // Sine and cosine of every pair at a position, by `threads` threads. `turns` [2, half]: turns per position, high and low part.
 __device__ __forceinline__ void angles(const float* turns, int half, int pos, float* cs, float* sn, int tid, int threads) {
     for (int i = tid; i < half; i += threads) {

@@ -42,9 +42,7 @@ struct TalkP {
 constexpr int kSimtThreads = 256, kSimtKeys = 32;
 template <typename T> __device__ __forceinline__ float dot_key(const KvP& p, const float* q, int seq, int g, int j) {
     const T* k = (const T*)p.keys + key_row(p, page_of(p, seq, j), g, j) * p.dim;
-    float d = 0.f;
-    for (int i = 0; i < p.dim; i++) d = fmaf(q[i], to_f(k[i]), d);
-    return d;
+    return dot_in_order(q, k, p.dim, 0.f);
 }
 // One CTA per (row, head): the natural logarithm of the softmax's sum.
 template <typename T> __global__ void __launch_bounds__(kSimtThreads) talk_simt_lse(const TalkP tp) {
@@ -99,13 +97,7 @@ template <typename T> __global__ void __launch_bounds__(kSimtThreads) talk_simt(
         const int live = min(kSimtKeys, pos + 1 - j0);
         for (int i = tid; i < H * p.vdim; i += kSimtThreads) {
             const int h = i / p.vdim;
-            float a = acc[i];
-            long long pg = 0;
-            for (int jj = 0; jj < live; jj++) {
-                if (jj == 0 || ((j0 + jj) & ((1 << p.shift) - 1)) == 0) pg = page_of(p, s, j0 + jj);
-                a = fmaf(mixed[h * kSimtKeys + jj], to_f(((const T*)p.values)[key_row(p, pg, h / rep, j0 + jj) * p.ldv + i % p.vdim]), a);
-            }
-            acc[i] = a;
+            acc[i] = weigh_in_order(p, (const T*)p.values, s, h / rep, j0, live, p.ldv, i % p.vdim, mixed + h * kSimtKeys, acc[i]);
         }
         __syncthreads();
     }

@@ -95,6 +95,21 @@ template <typename T> __device__ __forceinline__ T from_f(float v);
 template <> __device__ __forceinline__ float from_f<float>(float v) { return v; }
 template <> __device__ __forceinline__ bf16 from_f<bf16>(float v) { return __float2bfloat16_rn(v); }
 
+// a + Σ x[i] · w[i], one after the other in index order; rows of f32 come four at a time where they are 16-byte aligned.
+template <typename T> __device__ __forceinline__ float dot_in_order(const float* x, const T* w, int n, float a) {
+    int i = 0;
+    if constexpr (sizeof(T) == 4) {
+        if ((reinterpret_cast<uintptr_t>(w) & 15) == 0)
+#pragma unroll 8
+            for (; i + 4 <= n; i += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(w + i);
+                a = fmaf(x[i + 3], v.w, fmaf(x[i + 2], v.z, fmaf(x[i + 1], v.y, fmaf(x[i], v.x, a))));
+            }
+    }
+    for (; i < n; i++) a = fmaf(x[i], to_f(w[i]), a);
+    return a;
+}
+
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
 __device__ __forceinline__ float gelu_tanh_f(float z) {
     return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
