@@ -188,7 +188,7 @@ def gemv_sweep(backend, shapes, ms, peak, reps=10):
                 return us, fused
 
             us, fused = time_on(backend)
-            entry_kernel = "persist_step" if fused else ("nbits_stream" if m <= 8 else "nbits_gemm_tc")
+            entry_kernel = "persist_step" if fused else ("nbits_stream" if m <= 8 else "nbits_gemm_tc" if m <= 256 else "nbits_gemm_wide")
             other = None
             if fused:  # the same products, one launch each
                 us2, _ = time_on(plain)
@@ -439,6 +439,7 @@ def lovuzen_costs(cfg, rows, seqs, past, wanted):
 _FAMILY = {"linear_stream": "linear", "linear_tc": "linear", "linear_reduce": "linear", "linear_simt": "linear",
            "paged_attn_prefill": "attn", "paged_attn_decode": "attn", "paged_attn_simt": "attn", "recurrence_step": "gates",
            "recurrence_gates": "gates", "recurrence_scan": "scan", "residual_norm": "norm",
+           "linear_rows_f32": "linear", "linear_f32": "linear", "nbits_widen": "linear", "nbits_gemm_wide": "linear",
            "nbits_stream": "linear", "nbits_gemm_tc": "linear", "nbits_gemm_reduce": "linear", "persist_step": "persist_step"}
 
 
