@@ -57,7 +57,7 @@ struct LinP {
     int act[2];           // functions of the columns before and from act_split on; none from act_end on
     long long act_split, act_end;
     int nb, stages, splits, node;  // linear_tc
-    int row_tiles, out_tiles, one;  // tiles of activation rows (not grouped) and of weight rows; one: a CTA per tile (and piece), in the grid's axes
+    int row_tiles, out_tiles;      // tiles of activation rows (not grouped) and of weight rows
     const int* counts;    // grouped: rows of every group
     int groups;
 };
@@ -469,12 +469,13 @@ constexpr int kTcPanelA = 128 * 128; // bytes: 128 weight rows × 64 k
 // A persistent CTA works through tiles (piece of k slowest, activation tiles fastest: they share a weight tile while it is in L2); loads and
 // MMAs run on into the next tile while the epilogue of the last one empties the other of two accumulators.
 // Rows × k × weight rows: 4096 × 1152 × 13 824 gated 217 → 136 µs (959 TFLOP/s), 2048 × 2560 × 20 480 gated 246 → 201, 2048 × 5376 × 16 896
-// 353 → 347 against a CTA per tile, whose fill and drain stood beside 18, 40 and 84 steps.
+// 353 → 347 against a CTA per tile, whose fill and drain stood beside 18, 40 and 84 steps. ONE: as many CTAs as tiles and pieces, which the grid's
+// axes count; the loop's code is not there. 64 rows × 2560 × 5120 cut along k: 14.1 → 13.2 µs against the kernel that had no loop, either.
 //
 // What the epilogue does: EPI_PLAIN bias only, EPI_GLU the gated unit, EPI_ACT functions of columns and factors. Kernels of their own: the
 // paths of one are short enough to stay in the instruction cache.
 enum : int { EPI_PLAIN, EPI_GLU, EPI_ACT };
-template <int EPI> __global__ void __launch_bounds__(kTcThreads) linear_tc(const __grid_constant__ LinP p) {
+template <int EPI, bool ONE> __global__ void __launch_bounds__(kTcThreads) linear_tc(const __grid_constant__ LinP p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -489,14 +490,14 @@ template <int EPI> __global__ void __launch_bounds__(kTcThreads) linear_tc(const
         pdl_wait();
         row_tiles = count_tiles(p, nb);
     }
-    const int first = p.one ? 0 : (int)blockIdx.x, total = p.one ? 1 : row_tiles * p.out_tiles * p.splits;
+    const int first = ONE ? 0 : (int)blockIdx.x, total = ONE ? 1 : row_tiles * p.out_tiles * p.splits;
     if (tid == 0) {
         for (int s = 0; s < 2 * S + 2; s++) mbar_init(smem_u32(bars + s), 1);
         for (int s = 0; s < 2; s++) mbar_init(read + s * 8, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     int cols = 32;
-    while (cols < (p.one ? nb : 2 * nb)) cols <<= 1;
+    while (cols < (ONE ? nb : 2 * nb)) cols <<= 1;
     if (warp == 5) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -515,7 +516,7 @@ template <int EPI> __global__ void __launch_bounds__(kTcThreads) linear_tc(const
         Tile q;
         int x = (int)blockIdx.x, y = (int)blockIdx.y;
         q.piece = (int)blockIdx.z;
-        if (!p.one) {
+        if (!ONE) {
             const int rest = t / row_tiles;
             x = t % row_tiles;
             y = rest % p.out_tiles;
@@ -526,8 +527,8 @@ template <int EPI> __global__ void __launch_bounds__(kTcThreads) linear_tc(const
         if (p.groups) locate_group(p, x, nb, &q.group, &q.n0, &q.live);
         q.block = p.blocks > 1 ? y / block_tiles : 0;
         q.m0 = (y - q.block * block_tiles) * 128;
-        q.lo = (int)((long long)all * q.piece / p.splits);
-        q.steps = (int)((long long)all * (q.piece + 1) / p.splits) - q.lo;
+        q.lo = (int)((unsigned)(all * q.piece) / (unsigned)p.splits);
+        q.steps = (int)((unsigned)(all * (q.piece + 1)) / (unsigned)p.splits) - q.lo;
         return q;
     };
     bool ok = true;
@@ -581,9 +582,9 @@ template <int EPI> __global__ void __launch_bounds__(kTcThreads) linear_tc(const
         const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(nb >> 3) << 17) | (8u << 24);  // bf16 × bf16 → f32, M 128 × N nb
         int n = 0, j = 0;
         for (int t = first; t < total; t += (int)gridDim.x, j++) {
-            const int piece = p.one ? (int)blockIdx.z : t / row_tiles / p.out_tiles, steps = (int)((long long)all * (piece + 1) / p.splits) - (int)((long long)all * piece / p.splits);
+            const int piece = ONE ? (int)blockIdx.z : t / row_tiles / p.out_tiles, steps = (int)((unsigned)(all * (piece + 1)) / (unsigned)p.splits) - (int)((unsigned)(all * piece) / (unsigned)p.splits);
             const unsigned d = tmem + (unsigned)((j & 1) * nb);
-            if (j >= 2 && ok && !mbar_wait(read + (j & 1) * 8, ((j >> 1) - 1) & 1)) ok = false;
+            if (!ONE && j >= 2 && ok && !mbar_wait(read + (j & 1) * 8, ((j >> 1) - 1) & 1)) ok = false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int i = 0; i < steps; i++, n++) {
                 const int s = n % S;
@@ -676,6 +677,7 @@ template <int EPI> __global__ void __launch_bounds__(kTcThreads) linear_tc(const
                 }
                 __syncwarp();
             }
+            if (ONE) break;
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(read + (j & 1) * 8) : "memory");
@@ -1436,12 +1438,14 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
     const bool alone = tiles <= sm_count();  // one CTA per SM: all of its shared memory
     p.stages = (int)std::min<size_t>(8, (p.nb <= 128 && !alone ? 108 * 1024 : 208 * 1024) / stage);
     const size_t smem = stage * p.stages + 1024 + (2 * p.stages + 4) * 8 + 16;
-    const auto kernel = d.glu ? linear_tc<EPI_GLU> : d.act[0] || d.act[1] || d.mul ? linear_tc<EPI_ACT> : linear_tc<EPI_PLAIN>;
+    const long long slots = (long long)sm_count() * (p.nb <= 128 ? 2 : 1);
+    const bool one = tiles <= slots;
+    const bool act = d.act[0] || d.act[1] || d.mul;
+    const auto kernel = one ? (d.glu ? linear_tc<EPI_GLU, true> : act ? linear_tc<EPI_ACT, true> : linear_tc<EPI_PLAIN, true>)
+                            : (d.glu ? linear_tc<EPI_GLU, false> : act ? linear_tc<EPI_ACT, false> : linear_tc<EPI_PLAIN, false>);
     ensure_max_dynamic_smem((const void*)kernel, 220 * 1024);
     const Buf partial = p.splits > 1 ? em.scratch((size_t)p.splits * d.rows * p.ldy * 4) : kNull;
-    const long long slots = (long long)sm_count() * (p.nb <= 128 ? 2 : 1);
-    p.one = tiles <= slots;
-    LaunchRec& rec = em.launch(kernel, p.one ? dim3((unsigned)p.row_tiles, (unsigned)mt, (unsigned)p.splits) : dim3((unsigned)slots), dim3(kTcThreads), (unsigned)smem, p,
+    LaunchRec& rec = em.launch(kernel, one ? dim3((unsigned)p.row_tiles, (unsigned)mt, (unsigned)p.splits) : dim3((unsigned)slots), dim3(kTcThreads), (unsigned)smem, p,
                                {{&p.bias, bb}, {&p.y, y.buf}, {&p.mul, mul}, {&p.partial, partial}, {&p.err, Buf{kSlotErr, 0}}}, "linear_tc", /*pdl=*/true);
     auto add_map = [&](int i, const Buf& b, int64_t k, int64_t rows, uint32_t box) {
         rec.tmaps.push_back(TmapReloc{(uint32_t)(offsetof(LinP, maps) + 128 * i), b, (uint64_t)k, (uint64_t)rows, (uint64_t)k * 2, 64u, box});
@@ -1506,7 +1510,7 @@ void emit_grouped_linear(Emitter& em, const GroupedLinearDesc& d, const TRef& x,
     if (tiles >= INT32_MAX) throw std::runtime_error("grouped product: too many tiles");
     p.stages = (int)std::min<size_t>(8, (p.nb <= 128 ? 108 * 1024 : 208 * 1024) / stage);
     const size_t smem = stage * p.stages + 1024 + (2 * p.stages + 4) * 8 + 16;
-    const auto kernel = d.glu ? linear_tc<EPI_GLU> : linear_tc<EPI_PLAIN>;
+    const auto kernel = d.glu ? linear_tc<EPI_GLU, false> : linear_tc<EPI_PLAIN, false>;
     ensure_max_dynamic_smem((const void*)kernel, 220 * 1024);
     LaunchRec& rec = em.launch(kernel, dim3((unsigned)std::min<long long>(tiles, (long long)sm_count() * (p.nb <= 128 ? 2 : 1))), dim3(kTcThreads), (unsigned)smem, p,
                                {{&p.bias, kNull}, {&p.y, y.buf}, {&p.partial, kNull}, {&p.err, Buf{kSlotErr, 0}}, {&p.counts, counts.buf}}, "grouped_tc",
