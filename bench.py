@@ -436,7 +436,7 @@ def lovuzen_costs(cfg, rows, seqs, past, wanted):
     return {"linear": (lin_b, lin_f), "attn": (att_b, att_f), "gates": (gate_b, gate_f), "scan": (scan_b, 0), "norm": (norm_b, 0)}
 
 
-_FAMILY = {"linear_stream": "linear", "linear_tc": "linear", "linear_reduce": "linear", "linear_simt": "linear",
+_FAMILY = {"linear_stream": "linear", "linear_flow": "linear", "linear_tc": "linear", "linear_reduce": "linear", "linear_simt": "linear",
            "paged_attn_prefill": "attn", "paged_attn_decode": "attn", "paged_attn_simt": "attn", "recurrence_step": "gates",
            "recurrence_gates": "gates", "recurrence_scan": "scan", "residual_norm": "norm",
            "linear_rows_f32": "linear", "linear_f32": "linear", "nbits_widen": "linear", "nbits_gemm_wide": "linear",

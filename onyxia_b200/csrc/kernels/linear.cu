@@ -5,6 +5,7 @@
 //                   a row), eight warps share a row tile's k. Weight loads run one batch ahead and start before the
 //                   grid dependency resolves. For up to eight rows the residual norm that makes x runs as the
 //                   prologue, in every CTA.
+//   linear_flow     the same for large matrices: more of their weights in flight, through shared memory.
 //   linear_tc       more rows: tcgen05 GEMM. Weights are the MMA's A operand (128 rows), activations its B operand
 //                   (32–256 rows), both loaded by TMA into 128-byte-swizzled stages; accumulator in tensor memory.
 //                   Grids that would leave SMs idle are cut along k; `linear_reduce` adds the pieces in order.
@@ -458,6 +459,137 @@ template <int NT, int NORM, bool BLOCKS> __global__ void __launch_bounds__(kStre
                 }
             }
             __syncthreads();
+        }
+    }
+}
+
+// The same for matrices of more bytes than all rings hold (2 CTAs per SM × 64 KB): a warp's chunks pass through a ring in shared memory by
+// 16-byte asynchronous copies, eight of them in flight instead of one batch of four between two waits. Every lane copies, and reads back, only
+// the two pieces of a chunk that are its own MMA fragment, so nothing but the lane's own copies has to be waited for. The ring is filled
+// ahead of the grid dependency and runs on across row tiles.
+// 1 row: 5376 × 43 008 gated 123 → 89 µs (5.2 TB/s), 5376 × 32 768 92 → 68, 21 504 × 5376 90 → 80; 8 rows: 1152 × 32 768 31 → 22. Below that
+// size the products are faster alone, too, but not behind one another: decode steps of small models took 3 % longer with it (13.8 against
+// 13.4 ms for 48 steps of the 1b size).
+constexpr int kRing = 8;  // 32-k chunks (1 KB) that a warp has in flight
+template <int NT, int NORM> __global__ void __launch_bounds__(kStreamWarps * 32, 2) linear_flow(const __grid_constant__ LinP p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ float red[2][kStreamWarps][16][NT * 8 + 1];
+    __shared__ float norm_red[kStreamWarps];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int c0 = (int)((p.k[0] + 31) / 32), chunks = c0 + (int)((p.k[1] + 31) / 32);
+    const int tiles = (int)((p.out + 15) / 16), per_tile = (chunks + kStreamWarps - 1) / kStreamWarps;  // chunks of a warp per row tile
+    const int my_tiles = (int)blockIdx.x < tiles ? (tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+
+    // the chunk that is asked for next: its number in the tile, and the row tile
+    unsigned char* slots = smem + warp * kRing * 1024 + lane * 16;
+    const unsigned ring = smem_u32(slots);
+    int f_at = warp, f_tile = (int)blockIdx.x, f_slot = 0, f_left = my_tiles * per_tile;
+    auto fetch = [&]() {
+        if (f_left-- > 0) {
+            const long long r0 = (long long)f_tile * 16 + g;
+            const int op = f_at >= c0;
+            const long long k = (long long)(op ? f_at - c0 : f_at) * 32 + t * 8, K = p.k[op];
+            const bf16* w = (const bf16*)p.w[op] + r0 * K + k;
+            const bool live = f_at < chunks && k < K;
+            const unsigned to = ring + (unsigned)f_slot * 1024;
+            cp_async16(to, live && r0 < p.out ? w : (const bf16*)p.w[0], live && r0 < p.out);
+            cp_async16(to + 512, live && r0 + 8 < p.out ? w + 8 * K : (const bf16*)p.w[0], live && r0 + 8 < p.out);
+            f_slot = f_slot + 1 == kRing ? 0 : f_slot + 1;
+            f_at += kStreamWarps;
+            if (f_at >= per_tile * kStreamWarps) {
+                f_at = warp;
+                f_tile += (int)gridDim.x;
+            }
+        }
+        cp_async_commit();
+    };
+    pdl_trigger();
+#pragma unroll
+    for (int i = 0; i < kRing; i++) fetch();  // constants: ahead of the launches in front of this one
+    pdl_wait();
+    bf16* xs = reinterpret_cast<bf16*>(smem + kStreamWarps * kRing * 1024);
+    const int stride = ((int)p.k[0] + 63) / 64 * 64 + 32;  // 64 bytes off a multiple of 128: conflict-free fragment loads
+    if constexpr (NORM == PRO_NORM) {
+        if (p.ny_bf16) norm_prologue<true>(p, xs, stride, norm_red);
+        else norm_prologue<false>(p, xs, stride, norm_red);
+    } else if constexpr (NORM == PRO_STREAMS) {
+        if (p.ny_bf16) streams_prologue<true>(p, xs, stride, norm_red);
+        else streams_prologue<false>(p, xs, stride, norm_red);
+    } else if constexpr (NORM == PRO_GROUPS) {
+        if (p.ny_bf16) groups_prologue<true>(p, xs, stride);
+        else groups_prologue<false>(p, xs, stride);
+    }
+    uint4 xv[NT];  // activations of a chunk, fetched one chunk ahead when they come from memory
+    auto load_x = [&](int at) {
+        const int op = at >= c0;
+        const long long k = (long long)(op ? at - c0 : at) * 32 + t * 8;
+        const bool live = at < chunks && k < p.k[op];
+#pragma unroll
+        for (int n = 0; n < NT; n++) {
+            const long long row = n * 8 + g;
+            xv[n] = make_uint4(0, 0, 0, 0);
+            if (live && row < p.rows) {
+                if constexpr (NORM != PRO_NONE) xv[n] = *reinterpret_cast<const uint4*>(xs + row * stride + k);
+                else xv[n] = *reinterpret_cast<const uint4*>((const bf16*)p.x[op] + row * p.k[op] + k);
+            }
+        }
+    };
+    int slot = 0;
+    if (NORM == PRO_NONE && my_tiles > 0) load_x(warp);
+    for (int done = 0; done < my_tiles; done++) {
+        float acc[NT][4];
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[n][e] = 0.f;
+        for (int i = 0; i < per_tile; i++) {
+            cp_async_wait<kRing - 1>();
+            const uint4 a = *reinterpret_cast<const uint4*>(slots + slot * 1024), b = *reinterpret_cast<const uint4*>(slots + slot * 1024 + 512);
+            slot = slot + 1 == kRing ? 0 : slot + 1;
+            if (NORM != PRO_NONE) load_x(i * kStreamWarps + warp);
+            uint4 x[NT];
+#pragma unroll
+            for (int n = 0; n < NT; n++) x[n] = xv[n];
+            if (NORM == PRO_NONE) {
+                if (i + 1 < per_tile) load_x((i + 1) * kStreamWarps + warp);
+                else if (done + 1 < my_tiles) load_x(warp);
+            }
+#pragma unroll
+            for (int n = 0; n < NT; n++) {
+                mma_bf16(acc[n], a.x, b.x, a.y, b.y, x[n].x, x[n].y);
+                mma_bf16(acc[n], a.z, b.z, a.w, b.w, x[n].z, x[n].w);
+            }
+            fetch();  // into the slot that has just been read
+        }
+        const int half = done & 1;  // the other half is written before the next tile's meeting, which everybody comes to behind this tile's sums
+#pragma unroll
+        for (int n = 0; n < NT; n++) {
+            red[half][warp][g][n * 8 + t * 2] = acc[n][0];
+            red[half][warp][g][n * 8 + t * 2 + 1] = acc[n][1];
+            red[half][warp][g + 8][n * 8 + t * 2] = acc[n][2];
+            red[half][warp][g + 8][n * 8 + t * 2 + 1] = acc[n][3];
+        }
+        __syncthreads();
+        const long long tile = (long long)blockIdx.x + done * (long long)gridDim.x;
+        auto total_of = [&](int r, int m) {
+            float s = 0.f;
+#pragma unroll
+            for (int w = 0; w < kStreamWarps; w++) s += red[half][w][r][m];
+            const long long o = tile * 16 + r;
+            return s + (p.bias && o < p.out ? p.bias[o] : 0.f);
+        };
+        if (p.glu) {
+            for (int i = tid; i < 8 * NT * 8; i += kThreads) {
+                const int r = i & 7, m = i >> 3;
+                const long long o = tile * 8 + r;
+                if (m < p.rows && o < p.out / 2) put(p, m, p.out / 2, o, glu_value(p, total_of(2 * r, m), total_of(2 * r + 1, m)));
+            }
+        } else {
+            for (int i = tid; i < 16 * NT * 8; i += kThreads) {
+                const int r = i & 15, m = i >> 4;
+                const long long o = tile * 16 + r;
+                if (m < p.rows && o < p.out) put(p, m, p.out, o, activate(p, o, total_of(r, m)));
+            }
         }
     }
 }
@@ -1371,16 +1503,18 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
     if (d.rows <= 32) {
         const long long tiles = (d.out + 15) / 16 * d.blocks;
         const dim3 grid((unsigned)std::min<long long>(tiles, 2 * sm_count()));
+        const bool flow = !blocks && d.out * (d.k[0] + d.k[1]) * 2 > 2LL * sm_count() * kStreamWarps * kRing * 1024;
         const int nt = d.rows <= 8 ? 1 : d.rows <= 16 ? 2 : 4;
         auto k = nt == 1 ? linear_stream<1, PRO_NONE, false> : nt == 2 ? linear_stream<2, PRO_NONE, false> : linear_stream<4, PRO_NONE, false>;
         if (blocks) k = nt == 1 ? linear_stream<1, PRO_NONE, true> : nt == 2 ? linear_stream<2, PRO_NONE, true> : linear_stream<4, PRO_NONE, true>;
-        unsigned smem = 0;
+        if (flow) k = nt == 1 ? linear_flow<1, PRO_NONE> : nt == 2 ? linear_flow<2, PRO_NONE> : linear_flow<4, PRO_NONE>;
+        unsigned smem = flow ? kStreamWarps * kRing * 1024 : 0;
         if (fuse_norm) {
             k = pro == PRO_STREAMS ? linear_stream<1, PRO_STREAMS, false> : pro == PRO_GROUPS ? linear_stream<1, PRO_GROUPS, false> : linear_stream<1, PRO_NORM, false>;
+            if (flow) k = pro == PRO_STREAMS ? linear_flow<1, PRO_STREAMS> : pro == PRO_GROUPS ? linear_flow<1, PRO_GROUPS> : linear_flow<1, PRO_NORM>;
             p.streams = (int)norm->streams;
             p.norm_groups = (int)norm->groups;
-            smem = (unsigned)norm_smem;
-            ensure_max_dynamic_smem((const void*)k, 100 * 1024);
+            smem += (unsigned)norm_smem;
             p.eps = (float)norm->eps;
             p.ny_bf16 = norm->y->dtype == DT_BF16;
             p.y_scale = (float)norm->y_scale;
@@ -1390,6 +1524,7 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
             p.add_bf16 = norm->add && norm->add->dtype == DT_BF16;
             p.gate_ld = norm->gate ? norm->gate->shape[1] : 0;
         }
+        ensure_max_dynamic_smem((const void*)k, 150 * 1024);
         em.launch(k, grid, dim3(kStreamWarps * 32), smem, p,
                   {{&p.x[0], bx0}, {&p.x[1], bx1}, {&p.w[0], w0.buf}, {&p.w[1], bw1}, {&p.bias, bb}, {&p.y, y.buf}, {&p.mul, mul},
                    {&p.npost, fuse_norm ? buf_of(norm->post) : kNull}, {&p.nadd, fuse_norm ? buf_of(norm->add) : kNull},
@@ -1399,7 +1534,7 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
                    {&p.ngain, fuse_norm ? buf_of(norm->gain) : kNull}, {&p.nres, fuse_norm ? buf_of(norm->res) : kNull},
                    {&p.ngate, fuse_norm && norm->gate ? norm->gate->buf.at(norm->gate_off * 2) : kNull},
                    {&p.stream, fuse_norm ? buf_of(norm->stream) : kNull}, {&p.low, fuse_norm ? buf_of(low) : kNull}},
-                  "linear_stream", /*pdl=*/true);
+                  flow ? "linear_flow" : "linear_stream", /*pdl=*/true);
         return;
     }
     // Activation rows per tile and pieces along k: the choice with the smallest modelled time, waves × (64-k steps of a

@@ -2,13 +2,14 @@
 import numpy as np
 import pytest
 
+import mufevik_ref as ref
 from onyxia_b200 import backend as be
 from onyxia_b200 import ir, models
 from onyxia_b200.ir import HostTensor
 from gpu_util import cuda_backend, differential
 from lovuzen_util import to_bf16
 from test_gpu_kipizen import Experts
-from test_gpu_lovuzen import rel_err, run_linear
+from test_gpu_lovuzen import act, rel_err, run_linear
 
 pytestmark = pytest.mark.gpu
 
@@ -87,20 +88,52 @@ def test_generic_int4_products(act_dtype, m):
 
 @pytest.mark.parametrize("rows", [1, 3, 8, 9, 17, 32])
 def test_bf16_products_of_few_rows(rows):
-    """One, two and four CTAs per row tile; several tiles per CTA; k that ends inside a chunk, a second operand that begins inside a CTA's share;
-    a ring that wraps. Inputs are on the bf16 grid and products exact: f32 sums of k products are off by less than 2e-6 of the result's rms."""
+    """Matrices below and above the line to linear_flow: several tiles per CTA, k that ends inside a chunk and with some warps only, a second
+    operand that begins inside the warps' turn, rings that wrap. Inputs are on the bf16 grid and products exact: f32 sums of k products are off
+    by less than 2e-6 of the result's rms."""
     r = np.random.default_rng(rows)
-    for k, k1, n in ((4608, 0, 1152), (2056, 136, 24), (1152, 0, 15000), (1096, 0, 2400)):
+    for k, k1, n in ((4608, 0, 1152), (2056, 136, 5003), (1152, 0, 15000), (40, 0, 260000), (1096, 0, 2400)):
         x, w, more = to_bf16(r.standard_normal((rows, k))), to_bf16(r.standard_normal((n, k))), {}
         want = x.astype(np.float64) @ w.T.astype(np.float64)
         if k1:
             more = {"x1": to_bf16(r.standard_normal((rows, k1))), "w1": to_bf16(r.standard_normal((n, k1)))}
             want = want + more["x1"].astype(np.float64) @ more["w1"].T.astype(np.float64)
         assert rel_err(run_linear(ir.BF16, x, w, **more), want) < 2e-6, (k, n)
-    x, w = to_bf16(r.standard_normal((rows, 2304))), to_bf16(r.standard_normal((130, 2304)) / 48)
+    x, w = to_bf16(r.standard_normal((rows, 2304))), to_bf16(r.standard_normal((4402, 2304)) / 48)
     z = x.astype(np.float64) @ w.T.astype(np.float64)
     g, u = np.minimum(z[:, ::2], 1.5), np.clip(z[:, 1::2], -1.5, 1.5)
     assert rel_err(run_linear(ir.BF16, x, w, glu=(1.7, 1.5, 1.0)), g / (1 + np.exp(-1.7 * g)) * (u + 1)) < 3e-6
+
+
+@pytest.mark.parametrize("rows", [1, 7, 8, 9])
+def test_norms_in_front_of_a_large_matrix(rows):
+    """Every norm that runs as the prologue, in front of 20 MB and more. Tolerances as for small matrices: the norm's operand is rounded to bf16."""
+    r = np.random.default_rng(rows)
+    eps, n, of = 1e-3, 19999, HostTensor.from_numpy
+    for kind, width in (("residual", 520), ("streams", 528), ("groups", 544)):
+        y, w, m = to_bf16(0.02 * r.standard_normal((rows, width))).astype(np.float32), to_bf16(r.standard_normal(width)), to_bf16(r.standard_normal((n, width)))
+        S = 3 if kind == "streams" else 1
+        b, feed = ir.GraphBuilder(), {"y": of(y)}
+        ins, y64 = [b.input("y", ir.F32, [rows, width])], y.astype(np.float64)
+        if kind == "groups":
+            w, gate = np.tile(w[:136], 4), to_bf16(r.standard_normal((rows, width)))
+            ins += [b.constant(of(w)), b.input("gate", ir.BF16, [rows, width])]
+            feed["gate"], attrs = act(gate, ir.BF16), {"norm_groups": 4, "gate": 1, "gate_offset": 0}
+            want = ref.rms_norm(y64.reshape(rows, 4, 136), w[:136], eps).reshape(rows, width) * gate
+        else:
+            res = (0.1 * r.standard_normal((rows, S, width))).astype(np.float32)
+            ins += [b.constant(of(w)), b.input("res", ir.F32, [rows, S * width])]
+            feed["res"], attrs = of(res.reshape(rows, -1)), {"residual": 1}
+            want = ref.rms_norm(y64, w, eps) + res[:, 0]
+            if S > 1:
+                mix, out, take = r.standard_normal((S, S)), r.standard_normal(S), r.standard_normal(S)
+                ins.append(b.constant(of(np.concatenate([mix.reshape(-1), out, take]).astype(np.float32))))
+                attrs.update(pre=1, streams=S)
+                new = out[None, :, None] * y64[:, None] + np.einsum("st,rsw->rtw", mix, res.astype(np.float64))
+                want = ref.rms_norm(np.einsum("t,rtw->rw", take, new), w, eps)
+        b.output("out", b.composite("onyxia.Linear", dict(attrs, epsilon=eps, norm=1, stream=0), ins + [b.constant(act(m, ir.BF16))], [(ir.F32, [rows, n])])[0])
+        got = be.run_once(cuda_backend(), b.finish(), feed)[0][1].numpy()
+        assert rel_err(got, want @ m.T.astype(np.float64)) < 6e-3, kind
 
 
 @pytest.mark.parametrize("rows", [40, 300, 1100])
@@ -117,7 +150,7 @@ def test_bf16_products_in_persistent_tiles(rows):
 
 @pytest.mark.parametrize("n", [1, 8, 9, 32, 70, 600])
 def test_experts_with_long_products(n):
-    """Weights that go through the rings several times, pieces of the second product over clusters; grouped tiles of many experts. `check` compares with
+    """Long sums of both products, pieces of the second one over clusters; grouped tiles of many experts. `check` compares with
     the plain implementation at the tolerance of its own tests."""
     m = Experts("bf16", 1160, 12, 3, 840)
     m.check(m.rows(n))
@@ -154,8 +187,8 @@ def test_prefill_attention_with_kept_scores(heads, kv, d, past, seq, window):
 
 
 @pytest.mark.parametrize("rows,k,k1,n", [(1100, 2056, 0, 9000), (700, 1032, 1032, 12000), (2048, 1152, 0, 4610)])
-def test_bf16_products_of_pairs_of_ctas(rows, k, k1, n):
-    """Enough tiles for pairs; tiles that end inside either CTA's half in both directions, several rounds per pair, rings that wrap."""
+def test_bf16_products_of_several_rounds_per_cta(rows, k, k1, n):
+    """More tiles than SMs: tiles that end early in both directions, several rounds per CTA, a second operand, rings that wrap."""
     r = np.random.default_rng(rows)
     x, w, more = to_bf16(r.standard_normal((rows, k))), to_bf16(r.standard_normal((n, k)) / np.sqrt(k)), {}
     z = x.astype(np.float64) @ w.T.astype(np.float64)
