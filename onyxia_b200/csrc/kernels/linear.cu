@@ -1643,11 +1643,14 @@ void emit_grouped_linear(Emitter& em, const GroupedLinearDesc& d, const TRef& x,
     p.out_tiles = (int)mt;
     const long long tiles = tiles_of(p.nb) * mt;  // at most
     if (tiles >= INT32_MAX) throw std::runtime_error("grouped product: too many tiles");
-    p.stages = (int)std::min<size_t>(8, (p.nb <= 128 ? 108 * 1024 : 208 * 1024) / stage);
+    // Tiles of 32 rows are bound by the weights' bytes: four CTAs of two stages per SM instead of two of five, so that more tiles run side by side
+    // and few are left for a second round. 64 tokens, 16 experts, 4 096 × 2 560 and 2 560 × 2 048: 65 → 60 µs a product; three CTAs 64, five 60.
+    const int resident = p.nb == 32 ? 4 : p.nb <= 128 ? 2 : 1;
+    p.stages = (int)std::min<size_t>(8, (resident == 4 ? 48 * 1024 : resident == 2 ? 108 * 1024 : 208 * 1024) / stage);
     const size_t smem = stage * p.stages + 1024 + (2 * p.stages + 4) * 8 + 16;
     const auto kernel = d.glu ? linear_tc<EPI_GLU, false> : linear_tc<EPI_PLAIN, false>;
     ensure_max_dynamic_smem((const void*)kernel, 220 * 1024);
-    LaunchRec& rec = em.launch(kernel, dim3((unsigned)std::min<long long>(tiles, (long long)sm_count() * (p.nb <= 128 ? 2 : 1))), dim3(kTcThreads), (unsigned)smem, p,
+    LaunchRec& rec = em.launch(kernel, dim3((unsigned)std::min<long long>(tiles, (long long)sm_count() * resident)), dim3(kTcThreads), (unsigned)smem, p,
                                {{&p.bias, kNull}, {&p.y, y.buf}, {&p.partial, kNull}, {&p.err, Buf{kSlotErr, 0}}, {&p.counts, counts.buf}}, "grouped_tc",
                                /*pdl=*/true);
     auto add_map = [&](int i, const Buf& b, int64_t rows, uint32_t box) {
