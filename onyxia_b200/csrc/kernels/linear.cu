@@ -463,14 +463,16 @@ template <int NT, int NORM, bool BLOCKS> __global__ void __launch_bounds__(kStre
     }
 }
 
-// The same for matrices of more bytes than all rings hold (2 CTAs per SM × 64 KB): a warp's chunks pass through a ring in shared memory by
-// 16-byte asynchronous copies, eight of them in flight instead of one batch of four between two waits. Every lane copies, and reads back, only
-// the two pieces of a chunk that are its own MMA fragment, so nothing but the lane's own copies has to be waited for. The ring is filled
-// ahead of the grid dependency and runs on across row tiles.
-// 1 row: 5376 × 43 008 gated 123 → 89 µs (5.2 TB/s), 5376 × 32 768 92 → 68, 21 504 × 5376 90 → 80; 8 rows: 1152 × 32 768 31 → 22. Below that
-// size the products are faster alone, too, but not behind one another: decode steps of small models took 3 % longer with it (13.8 against
-// 13.4 ms for 48 steps of the 1b size).
+// The same for matrices of more than 19.4 MB (64 KB per CTA, two per SM): a warp's chunks pass through a ring in shared memory by 16-byte
+// asynchronous copies, eight of them in flight instead of one batch of four between two waits. Every lane copies, and reads back, only the pieces
+// of a chunk that are its own MMA fragments, so nothing but the lane's own copies has to be waited for. The ring is filled ahead of the grid
+// dependency (activations behind it) and runs on across row tiles. Up to eight rows that no prologue makes travel with their weights: loaded a
+// chunk ahead into registers, they held every chunk up by an L2 read (1 row × 21 504 × 5376 92 µs, now 50).
+// 1 row: 5376 × 43 008 gated 123 → 77 µs (6.0 TB/s), 5376 × 16 896 56 → 34; 8 rows: 5376 × 32 768 62 (activations in registers: 92), 1152 × 32 768
+// 31 → 22. Below that size the products are faster alone, too, but not behind one another: decode steps of small models took 3 % longer with it
+// (13.8 against 13.4 ms for 48 steps of the 1b size, activations in registers).
 constexpr int kRing = 8;  // 32-k chunks (1 KB) that a warp has in flight
+constexpr int flow_slot(bool ring_x) { return ring_x ? 1536 : 1024; }  // bytes, with the chunk's activations (up to eight rows) or without
 template <int NT, int NORM> __global__ void __launch_bounds__(kStreamWarps * 32, 2) linear_flow(const __grid_constant__ LinP p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ float red[2][kStreamWarps][16][NT * 8 + 1];
@@ -481,19 +483,27 @@ template <int NT, int NORM> __global__ void __launch_bounds__(kStreamWarps * 32,
     const int my_tiles = (int)blockIdx.x < tiles ? (tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
     // the chunk that is asked for next: its number in the tile, and the row tile
-    unsigned char* slots = smem + warp * kRing * 1024 + lane * 16;
+    constexpr bool kRingX = NT == 1 && NORM == PRO_NONE;
+    constexpr int kSlot = flow_slot(kRingX);
+    unsigned char* slots = smem + warp * kRing * kSlot + lane * 16;
     const unsigned ring = smem_u32(slots);
     int f_at = warp, f_tile = (int)blockIdx.x, f_slot = 0, f_left = my_tiles * per_tile;
-    auto fetch = [&]() {
+    auto fetch = [&](bool weights, bool acts) {
         if (f_left-- > 0) {
             const long long r0 = (long long)f_tile * 16 + g;
             const int op = f_at >= c0;
             const long long k = (long long)(op ? f_at - c0 : f_at) * 32 + t * 8, K = p.k[op];
             const bf16* w = (const bf16*)p.w[op] + r0 * K + k;
             const bool live = f_at < chunks && k < K;
-            const unsigned to = ring + (unsigned)f_slot * 1024;
-            cp_async16(to, live && r0 < p.out ? w : (const bf16*)p.w[0], live && r0 < p.out);
-            cp_async16(to + 512, live && r0 + 8 < p.out ? w + 8 * K : (const bf16*)p.w[0], live && r0 + 8 < p.out);
+            const unsigned to = ring + (unsigned)f_slot * kSlot;
+            if (weights) {
+                cp_async16(to, live && r0 < p.out ? w : (const bf16*)p.w[0], live && r0 < p.out);
+                cp_async16(to + 512, live && r0 + 8 < p.out ? w + 8 * K : (const bf16*)p.w[0], live && r0 + 8 < p.out);
+            }
+            if (acts) {
+                const bool met = live && g < p.rows;
+                cp_async16(to + 1024, (const bf16*)p.x[met ? op : 0] + (met ? g * K + k : 0), met);
+            }
             f_slot = f_slot + 1 == kRing ? 0 : f_slot + 1;
             f_at += kStreamWarps;
             if (f_at >= per_tile * kStreamWarps) {
@@ -501,13 +511,18 @@ template <int NT, int NORM> __global__ void __launch_bounds__(kStreamWarps * 32,
                 f_tile += (int)gridDim.x;
             }
         }
-        cp_async_commit();
+        if (acts || !kRingX) cp_async_commit();
     };
     pdl_trigger();
 #pragma unroll
-    for (int i = 0; i < kRing; i++) fetch();  // constants: ahead of the launches in front of this one
+    for (int i = 0; i < kRing; i++) fetch(true, false);  // constants: ahead of the launches in front of this one
     pdl_wait();
-    bf16* xs = reinterpret_cast<bf16*>(smem + kStreamWarps * kRing * 1024);
+    if constexpr (kRingX) {
+        f_at = warp, f_tile = (int)blockIdx.x, f_slot = 0, f_left = my_tiles * per_tile;
+#pragma unroll
+        for (int i = 0; i < kRing; i++) fetch(false, true);
+    }
+    bf16* xs = reinterpret_cast<bf16*>(smem + kStreamWarps * kRing * kSlot);
     const int stride = ((int)p.k[0] + 63) / 64 * 64 + 32;  // 64 bytes off a multiple of 128: conflict-free fragment loads
     if constexpr (NORM == PRO_NORM) {
         if (p.ny_bf16) norm_prologue<true>(p, xs, stride, norm_red);
@@ -535,7 +550,7 @@ template <int NT, int NORM> __global__ void __launch_bounds__(kStreamWarps * 32,
         }
     };
     int slot = 0;
-    if (NORM == PRO_NONE && my_tiles > 0) load_x(warp);
+    if (NORM == PRO_NONE && !kRingX && my_tiles > 0) load_x(warp);
     for (int done = 0; done < my_tiles; done++) {
         float acc[NT][4];
 #pragma unroll
@@ -544,13 +559,14 @@ template <int NT, int NORM> __global__ void __launch_bounds__(kStreamWarps * 32,
             for (int e = 0; e < 4; e++) acc[n][e] = 0.f;
         for (int i = 0; i < per_tile; i++) {
             cp_async_wait<kRing - 1>();
-            const uint4 a = *reinterpret_cast<const uint4*>(slots + slot * 1024), b = *reinterpret_cast<const uint4*>(slots + slot * 1024 + 512);
+            const uint4 a = *reinterpret_cast<const uint4*>(slots + slot * kSlot), b = *reinterpret_cast<const uint4*>(slots + slot * kSlot + 512);
+            if (kRingX) xv[0] = *reinterpret_cast<const uint4*>(slots + slot * kSlot + 1024);
             slot = slot + 1 == kRing ? 0 : slot + 1;
             if (NORM != PRO_NONE) load_x(i * kStreamWarps + warp);
             uint4 x[NT];
 #pragma unroll
             for (int n = 0; n < NT; n++) x[n] = xv[n];
-            if (NORM == PRO_NONE) {
+            if (NORM == PRO_NONE && !kRingX) {
                 if (i + 1 < per_tile) load_x((i + 1) * kStreamWarps + warp);
                 else if (done + 1 < my_tiles) load_x(warp);
             }
@@ -559,7 +575,7 @@ template <int NT, int NORM> __global__ void __launch_bounds__(kStreamWarps * 32,
                 mma_bf16(acc[n], a.x, b.x, a.y, b.y, x[n].x, x[n].y);
                 mma_bf16(acc[n], a.z, b.z, a.w, b.w, x[n].z, x[n].w);
             }
-            fetch();  // into the slot that has just been read
+            fetch(true, kRingX);  // into the slot that has just been read
         }
         const int half = done & 1;  // the other half is written before the next tile's meeting, which everybody comes to behind this tile's sums
 #pragma unroll
@@ -1508,7 +1524,7 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
         auto k = nt == 1 ? linear_stream<1, PRO_NONE, false> : nt == 2 ? linear_stream<2, PRO_NONE, false> : linear_stream<4, PRO_NONE, false>;
         if (blocks) k = nt == 1 ? linear_stream<1, PRO_NONE, true> : nt == 2 ? linear_stream<2, PRO_NONE, true> : linear_stream<4, PRO_NONE, true>;
         if (flow) k = nt == 1 ? linear_flow<1, PRO_NONE> : nt == 2 ? linear_flow<2, PRO_NONE> : linear_flow<4, PRO_NONE>;
-        unsigned smem = flow ? kStreamWarps * kRing * 1024 : 0;
+        unsigned smem = flow ? kStreamWarps * kRing * flow_slot(nt == 1 && !fuse_norm) : 0;
         if (fuse_norm) {
             k = pro == PRO_STREAMS ? linear_stream<1, PRO_STREAMS, false> : pro == PRO_GROUPS ? linear_stream<1, PRO_GROUPS, false> : linear_stream<1, PRO_NORM, false>;
             if (flow) k = pro == PRO_STREAMS ? linear_flow<1, PRO_STREAMS> : pro == PRO_GROUPS ? linear_flow<1, PRO_GROUPS> : linear_flow<1, PRO_NORM>;
