@@ -217,7 +217,11 @@ class OnyxiaError(RuntimeError):
 
 
 def whole_words(code: str, values) -> array.array:
-    """The values in one buffer of type "q" (int64) or "i" (int32). As with ctypes' integers, too large ones keep their low bits."""
+    """The values in one buffer of type "q" (int64) or "i" (int32). As with ctypes' integers, too large ones keep their low bits, and
+    what has no length is refused."""
+    len(values)
+    if isinstance(values, (bytes, bytearray)):  # ids of a vocabulary of bytes; `array` would take them for the buffer's own memory
+        values = list(values)
     try:
         return array.array(code, values)
     except OverflowError:
@@ -227,6 +231,7 @@ def whole_words(code: str, values) -> array.array:
 
 def int_words(code: str, values) -> array.array:
     """The same for anything that int() makes a whole number of."""
+    len(values)
     try:
         return whole_words(code, values)
     except TypeError:

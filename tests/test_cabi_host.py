@@ -196,6 +196,18 @@ def test_words_keep_what_ctypes_took():
         _ffi.whole_words("q", [1.5])
 
 
+def test_words_of_bytes_are_their_values():
+    """Ids of a vocabulary of bytes, at lengths that are and are not whole words of memory; iterators stay refused."""
+    for n in (0, 1, 5, 8, 16):
+        raw = bytes(range(49, 49 + n))
+        for kind in (bytes, bytearray, memoryview):
+            assert list(_ffi.whole_words("q", kind(raw))) == list(raw) == list(_ffi.int_words("q", kind(raw)))
+            assert list(_ffi.int_words("i", kind(raw))) == list(raw)
+    for words in (_ffi.whole_words, _ffi.int_words):
+        with pytest.raises(TypeError):
+            words("q", iter([1, 2.5, 3]))
+
+
 def test_half_precision_widens_exactly():
     bits = np.arange(65536, dtype=np.uint16)[1:]  # an odd count: a tail behind the eights
     want, got = bits.view(np.float16).astype(np.float32), np.empty(65535, np.float32)
