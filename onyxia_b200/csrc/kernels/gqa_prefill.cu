@@ -407,7 +407,13 @@ template <int D> __global__ void __launch_bounds__(kSThreads, 1) gqa_prefill_sco
     // ── probabilities: two rows per warp, eight scores per lane and step ──
     const int eights = nkb * kKB / 8;
     for (int i = 0; i < kSRows / kSWarps; i++) {
-        uint4* row = reinterpret_cast<uint4*>(Sc + (warp * (kSRows / kSWarps) + i) * ss);
+        const int at = warp * (kSRows / kSWarps) + i;
+        uint4* row = reinterpret_cast<uint4*>(Sc + at * ss);
+        const long long s = s0 + (at & 15), qpos = past_b + s;
+        if (s >= p.S || min(qpos, T - 1) < (p.window >= 0 ? qpos - p.window : 0)) {  // a row that sees nothing
+            for (int c = lane; c < eights; c += 32) row[c] = make_uint4(0, 0, 0, 0);
+            continue;
+        }
         __half2 most = __halves2half2(__ushort_as_half(0xFC00), __ushort_as_half(0xFC00));
         for (int c = lane; c < eights; c += 32) {
             const uint4 v = row[c];
@@ -416,11 +422,8 @@ template <int D> __global__ void __launch_bounds__(kSThreads, 1) gqa_prefill_sco
         float m = fmaxf(__low2float(most), __high2float(most));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        const __half hmax = __float2half_rn(m);  // an f16 value already
-        if (m == -INFINITY) {                    // a row that sees nothing
-            for (int c = lane; c < eights; c += 32) row[c] = make_uint4(0, 0, 0, 0);
-            continue;
-        }
+        // An f16 value already. It is −∞ where every visible score is NaN or −∞: the differences, and with them the row's outputs, are NaN then.
+        const __half hmax = __float2half_rn(m);
         unsigned long long sum = 0;  // every term is a multiple of 2^-24 not above 1: added as integers
         for (int c = lane; c < eights; c += 32) {
             const uint4 v = row[c];

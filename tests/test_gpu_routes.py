@@ -201,3 +201,28 @@ def test_bf16_products_of_several_rounds_per_cta(rows, k, k1, n):
         z = z + bias
         g, u = np.minimum(z[:, ::2], 2.0), np.clip(z[:, 1::2], -2.0, 2.0)
         assert rel_err(run_linear(ir.BF16, x, w, bias=bias, glu=(1.7, 2.0, 1.0)), g / (1 + np.exp(-1.7 * g)) * (u + 1)) < 3e-6
+
+
+@pytest.mark.parametrize("d,past,seq,window", [(64, 90, 33, -1), (128, 0, 70, 40), (256, 300, 20, 100)])
+def test_kept_scores_with_values_that_are_not_finite(d, past, seq, window):
+    """Rows whose visible scores are NaN, all minus infinity, or infinite in part, and a NaN among the keys: kept scores (two heads per key head) give
+    what the kernel that walks the keys three times gives for the same heads with a key head each, bit for bit in the other rows too."""
+    pairs, feed = models.build_gqa(2, 4, 2, d, past, seq, ir.F16, window, False, seed=d)
+    single, _ = models.build_gqa(2, 4, 4, d, past, seq, ir.F16, window, False, seed=d)
+    x = {n: t.numpy().copy() for n, t in feed.items()}
+    q, k = x["q"].reshape(2, seq, 4, d), x["k"].reshape(2, seq, 2, d)
+    k[..., 0], x["past_key"][..., 0] = 100, 100
+    q[..., 0] = 0
+    q[0, 3, 1] = np.nan           # every score of the row
+    q[0, 5, 2, 0] = -60000        # every score overflows to minus infinity
+    q[1, 7, 0, 1] = 60000         # scores of both signs
+    k[1, 9, 1, 2] = np.nan        # one key
+    feed = {n: HostTensor.from_numpy(v) for n, v in x.items()}
+    got = be.run_once(cuda_backend(), pairs, feed)[0][1].numpy().reshape(2, seq, 4, d)
+    for n in ("k", "v"):
+        feed[n] = HostTensor.from_numpy(np.repeat(x[n].reshape(2, seq, 2, d), 2, axis=2).reshape(2, seq, 4 * d))
+    for n in ("past_key", "past_value"):
+        feed[n] = HostTensor.from_numpy(np.repeat(x[n], 2, axis=1))
+    want = be.run_once(cuda_backend(), single, feed)[0][1].numpy().reshape(2, seq, 4, d)
+    assert np.isnan(got[0, 3, 1]).all() and np.isnan(got[0, 5, 2]).all() and np.isnan(got[1, 9, 2]).all()
+    assert np.array_equal(got, want, equal_nan=True) and np.isfinite(got[:, :3]).all()
