@@ -513,7 +513,7 @@ template <int D> void launch_prefill(Emitter& em, PrefillP& p, long long B, long
     constexpr int RS = D + kPad;
     // Two heads per key head and scores that fit beside the stages (200 KB: 2047 positions at a head size of 256, all visible) take the kernel
     // that forms them once; longer ranges walk the keys three times.
-    const long long seen = p.window >= 0 ? std::min(p.T, p.window + kBM) : p.T;  // keys that a CTA's rows see, at most
+    const long long seen = p.window >= 0 && p.window < p.T - kBM ? p.window + kBM : p.T;  // keys that a CTA's rows see, at most (any window: no overflow)
     p.score_stride = (int)((std::min<long long>(seen, 1 << 20) + kKB - 1) / kKB * kKB) + 8;  // 16 bytes off a multiple of 128: conflict-free
     const size_t kept = ((size_t)2 * kKB * RS + (size_t)kSRows * p.score_stride) * 2;
     if (H / p.KV % 2 == 0 && dyn_t.slot == kSlotNull && kept <= 200 * 1024) {

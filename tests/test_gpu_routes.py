@@ -226,3 +226,10 @@ def test_kept_scores_with_values_that_are_not_finite(d, past, seq, window):
     want = be.run_once(cuda_backend(), single, feed)[0][1].numpy().reshape(2, seq, 4, d)
     assert np.isnan(got[0, 3, 1]).all() and np.isnan(got[0, 5, 2]).all() and np.isnan(got[1, 9, 2]).all()
     assert np.array_equal(got, want, equal_nan=True) and np.isfinite(got[:, :3]).all()
+
+
+def test_windows_up_to_the_largest_number():
+    """A window beyond all positions sees what no window sees, up to the type's largest value."""
+    feeds = [models.build_gqa(1, 4, 2, 64, 40, 30, ir.F16, w, True, seed=1) for w in (-1, 70, 2 ** 63 - 17, 2 ** 63 - 16, 2 ** 63 - 1)]
+    want, *got = [be.run_once(cuda_backend(), m, f)[0][1].numpy() for m, f in feeds]
+    assert all(np.array_equal(g, want) for g in got)
