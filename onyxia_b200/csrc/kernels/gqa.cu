@@ -22,8 +22,8 @@
 //   gqa_pv       one warp per key again: p = exp(s − max)/Σ, acc += p·v; the
 //                last CTA to finish adds the partial accumulators in split order
 //                and stores the output row
-// When the present buffer is not the past buffer, gqa_copy_past fills it first; what follows appends in place, with the decode kernels
-// where they take the shape.
+// When the present buffer is not the past buffer, gqa_copy_past fills it first, and the three launches append in place. Single tokens
+// on a cache that was in place all along take the decode kernels, whose sums are in f32; here they are in f64.
 // "Last CTA" is decided by an arrival counter per query; nothing ever waits.
 //
 // KV tensors are [B, KV, T, D] views of buffers that hold `cap ≥ T` rows per
@@ -381,26 +381,15 @@ template <int DT> static void emit_gqa_t(Emitter& em, const GqaDesc& d, const TR
                    {&cp.seqlens, seqlens.buf}},
                   "gqa_copy_past", /*pdl=*/true);
     }
-    // With a bucket the true length travels through the plan's per-run scalars. A step that has copied its cache goes on like one that
-    // appends in place; its decode launch may not start ahead of the copy.
+    // With a bucket the true length travels through the plan's per-run scalars.
     const bool dyn = d.t_bucket > 0 && d.in_place && !bias;
     const long long Tsz = dyn ? d.t_bucket : T;
-    Buf dyn_t = dyn || (!d.in_place && S == 1 && P > 0 && !bias) ? em.dyn(T) : null;
-    if (S == 1 && P > 0 && !bias && !d.in_place) {
-        GqaDesc now = d;
-        now.in_place = true;
-        if (emit_gqa_decode(em, now, q, k, v, seqlens, cos, sin, out, present_k, present_v, dyn_t, T)) {
-            em.recs.back().pdl = false;
-            em.recs.back().pop = nullptr;
-            return;
-        }
-    }
+    Buf dyn_t = dyn ? em.dyn(T) : null;
     if (dyn && S == 1 && emit_gqa_decode(em, d, q, k, v, seqlens, cos, sin, out, present_k, present_v, dyn_t, Tsz)) return;
     GqaPrepP pp{};
     pp.B = B; pp.S = S; pp.H = H; pp.KV = KV; pp.D = D; pp.T = T;
     pp.pres_cap = pres_cap;
     if (dyn) pp.T = 0;
-    else dyn_t = null;
     pp.half = d.rot_half;
     pp.cache_rows = d.cache_rows;
     pp.clear = d.in_place ? 1 : P > 0 ? 0 : 2;
