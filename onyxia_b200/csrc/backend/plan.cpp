@@ -528,7 +528,6 @@ bool Session::update_plan(Plan& plan, const Bindings& bindings_in, const std::ve
     }
     plan.scratch_bytes = scratch;
     plan.bindings = bindings;
-    plan.runs_here = 0;
     finish_outputs(plan);
     fuse_persistent(plan);
     plans_updated++;
@@ -1026,12 +1025,9 @@ Plan* Session::plan_for(const std::vector<std::pair<std::string, DTensor>>& name
             plans_reused++;
             break;
         }
-    // A plan is patched for a new binding while its bindings come once each (a length that grows at every step). One whose binding has come
-    // back (decode steps beside prompts, batches of a few sizes) is kept as it is, graph included, and a new one is built beside it: patched,
-    // it would be lowered, captured and instantiated again at every change between the two (about 0.5 ms each on small models).
     if (!plan)
         for (auto it = plans_.begin(); it != plans_.end(); ++it)
-            if ((*it)->structure == key && (*it)->runs_here < 2) {
+            if ((*it)->structure == key) {
                 // patching may leave the plan half-updated when it gives up: such a plan is dropped
                 if (update_plan(**it, bindings, inputs, kv_in_place)) {
                     plans_.splice(plans_.begin(), plans_, it);
@@ -1045,7 +1041,7 @@ Plan* Session::plan_for(const std::vector<std::pair<std::string, DTensor>>& name
         if (shapes_only) return nullptr;  // a full build needs the real inputs
         plans_.push_front(build_plan(bindings, inputs, kv_in_place));
         plan = plans_.front().get();
-        while (plans_.size() > 8) plans_.pop_back();
+        while (plans_.size() > 6) plans_.pop_back();
     }
     return plan;
 }
@@ -1067,7 +1063,6 @@ std::vector<std::pair<std::string, DTensor>> Session::run(const std::vector<std:
     std::vector<DTensor> inputs;
     double t_bound = t_start;
     Plan* plan = plan_for(named, inputs, false, &t_bound);
-    plan->runs_here++;
 
     const double t_planned = now_us();
     std::vector<BufferRef> out_bufs;

@@ -82,7 +82,6 @@ struct Plan {
     std::vector<dim3> graph_grids, graph_clusters;
     std::vector<const void*> graph_funcs;
     uint64_t uses = 0;
-    uint64_t runs_here = 0;  // with the present binding
     ~Plan();
 };
 

@@ -241,3 +241,27 @@ def test_single_tokens_behind_a_copied_cache_keep_their_sums_in_64_bits(d):
     module, feed = models.build_gqa(3, 8, 2, d, 900, 1, ir.F16, -1, True, seed=d)
     got, want = differential(module, feed, atol=4e-3, rtol=4e-3)
     assert (got[0][1].numpy() != want[0][1].numpy()).mean() <= 2e-4
+
+
+def test_plans_of_changing_sizes_share_one():
+    """Sizes that come twice each, as the rows of a serving batch do: one plan is patched for all of them, and its memory is that of the largest."""
+    k, n, nb = 1024, 512, 32
+    r = np.random.default_rng(0)
+    b = ir.GraphBuilder()
+    rows = b.sym("rows")
+    ins = [b.input("a", ir.F16, [rows, k]), b.constant(HostTensor(ir.U4, [n, nb, 32], r.integers(0, 256, n * nb * 16, dtype=np.uint8))),
+           b.constant(HostTensor.from_numpy(r.uniform(0.005, 0.02, n * nb).astype(np.float16)))]
+    y = b.composite("com.microsoft.MatMulNBits", {"K": k, "N": n, "bits": 4, "block_size": 32}, ins, [(ir.F16, [rows, n])])[0]
+    b.output("y", b.composite("Gelu", {"approximate": "tanh"}, [y], [(ir.F16, [rows, n])])[0])
+    s = cuda_backend().prepare(b.finish())
+    held = []
+    for m in (600, 590, 400, 64, 300, 33, 500, 20, 280, 599):
+        a = s.upload(HostTensor.from_numpy(r.standard_normal((m, k)).astype(np.float16)))
+        for _ in range(2):
+            s.run({"a": a})
+        s.wait_idle()
+        del a
+        held.append(s.resident_bytes())
+    stats = s.plan_stats()
+    assert stats["built"] == 1 and stats["updated"] == 9
+    assert max(held) <= held[0]
