@@ -613,6 +613,19 @@ __global__ void __launch_bounds__(kWideThreads, 1) nbits_gemm_wide(const __grid_
     if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
+// Whether the weights are widened once. A pass of nbits_gemm_tc costs 8 µs and more besides its steps, the GEMM a pass over 2.6 bytes per weight and
+// half-filled rounds: short k pays from two passes on, long k with many of them. Measured on 150 sizes, nbits_gemm_tc → widened once, µs: k 1152 and 13 824
+// weight rows 46 → 33 (257 activation rows), 158 → 83 (1536); k 1536 and 12 288: 42 → 45 (512), 63 → 55 (768); k 2048 and 8192: 42 → 36 (257); k 2560 and 20 480:
+// 85 → 112 (257), 190 → 183 (1024), 381 → 320 (2047); k 3072 and 8192: 43 → 53 (257), 95 → 95 (1024); k 4096 and 4096: 32 → 37 (257), 70 → 61 (1024); k 6912 and
+// 1152: 20.3 → 21.7 (512), 40 → 35 (1024), 79 → 47 (2047); k 5376 and 8192: 60 → 77 (257), 261 → 270 (2047); k 5376 and 43 008: 266 → 386 (257), 2380 → 2510
+// (4096); k 21 504 and 5376: 130 → 430 (257), whose panels are too few tiles for the SMs.
+bool wide_pays(long long m, long long k, long long n) {
+    if (m <= 256) return false;
+    if (k <= 1280) return true;
+    if (k <= 2048) return n <= 8192 || m >= 640;
+    return m >= 1024 && (k <= 4096 || (k <= 7168 && n <= 2048));
+}
+
 // `t`: the launch of nbits_gemm_tc for these rows (its pieces of k are kept).
 void emit_wide(Emitter& em, const NBitsGroup& gr, const TRef& x, const TRef& tiles, const TcP& t) {
     const Buf null{kSlotNull, 0};
@@ -754,12 +767,7 @@ void emit_nbits_gemm_tc(Emitter& em, const NBitsGroup& gr, const TRef& x, const 
     if (debug) std::fprintf(stderr, "nbits_gemm_tc: m %lld k_tiles %d grid %u mb %d: %d pieces over %lld of the row blocks\n", gr.m, p.k_tiles, grid, mb, splits, tail);
     p.n_full = (int)n_full;
     p.splits = splits;
-    // two passes and more: measured on both sides beside nbits_gemm_wide
-    static const long long wide_from = [] {
-        const char* e = std::getenv("ONYXIA_GEMM_WIDE_FROM");  // diagnostics: activation rows from which the weights are widened into scratch
-        return e ? std::atoll(e) : 257LL;
-    }();
-    if (gr.m >= wide_from && gr.m < 65536 && gr.k % 8 == 0 && x.buf.off % 16 == 0) return emit_wide(em, gr, x, tiles, p);
+    if (wide_pays(gr.m, gr.k, (long long)p.row_tiles * 16) && gr.m < 65536 && gr.k % 8 == 0 && x.buf.off % 16 == 0) return emit_wide(em, gr, x, tiles, p);
     p.n_pad = tail * 128;
     const Buf partial = splits > 1 ? em.scratch((size_t)splits * mb * p.n_pad * sizeof(float)) : null;
     for (long long m0 = 0; m0 < gr.m; m0 += mb) {

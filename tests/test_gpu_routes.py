@@ -265,3 +265,19 @@ def test_plans_of_changing_sizes_share_one():
     stats = s.plan_stats()
     assert stats["built"] == 1 and stats["updated"] == 9
     assert max(held) <= held[0]
+
+
+def kernels_of(module, feed):
+    """Names of the kernels that a run launches."""
+    s = cuda_backend().prepare(module)
+    s.enable_profiling(True)
+    s.run({n: s.upload(t) for n, t in feed.items()})
+    return {kernel for kernel, _, _ in s.take_timings()}
+
+
+@pytest.mark.parametrize("m,k,n,wide", [(256, 512, 64, False), (257, 1280, 64, True), (257, 1288, 8192, True), (639, 2048, 8193, False), (640, 2048, 8193, True),
+                                        (1023, 2056, 64, False), (1024, 4096, 2064, True), (1024, 4104, 2048, True), (1024, 4104, 2049, False), (1024, 7176, 64, False)])
+def test_where_int4_weights_are_widened_once(m, k, n, wide):
+    module, act = models.build_matmul_nbits(m, k, n, act_dtype=ir.F16, seed=m)
+    names = kernels_of(module, {"a": act})
+    assert ("nbits_gemm_wide" in names) == wide and ("nbits_gemm_tc" in names) != wide
