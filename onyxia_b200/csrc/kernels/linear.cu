@@ -1519,8 +1519,12 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
     if (d.rows <= 32) {
         const long long tiles = (d.out + 15) / 16 * d.blocks;
         const dim3 grid((unsigned)std::min<long long>(tiles, 2 * sm_count()));
-        const bool flow = !blocks && d.out * (d.k[0] + d.k[1]) * 2 > 2LL * sm_count() * kStreamWarps * kRing * 1024;
         const int nt = d.rows <= 8 ? 1 : d.rows <= 16 ? 2 : 4;
+        // More than eight rows read their activations from L2 a chunk ahead, beside a first-level cache that the ring leaves little of: linear_stream
+        // → linear_flow, µs, 16 rows: k 5376, 21 504 weight rows 102 → 66 (9 rows 78 → 64); k 6912, 8192: 41 → 37; k 9216, 8192: 53 → 54; k 12 288, 8192: 67 → 83;
+        // k 16 896, 5376: 83 → 103. 32 rows: k 6912, 8192: 61 → 45; k 12 288, 8192: 98 → 98; k 14 336, 8192: 112 → 118.
+        const bool flow = !blocks && d.out * (d.k[0] + d.k[1]) * 2 > 2LL * sm_count() * kStreamWarps * kRing * 1024 &&
+                          (nt == 1 || d.k[0] + d.k[1] <= (nt == 2 ? 8192 : 12288));
         auto k = nt == 1 ? linear_stream<1, PRO_NONE, false> : nt == 2 ? linear_stream<2, PRO_NONE, false> : linear_stream<4, PRO_NONE, false>;
         if (blocks) k = nt == 1 ? linear_stream<1, PRO_NONE, true> : nt == 2 ? linear_stream<2, PRO_NONE, true> : linear_stream<4, PRO_NONE, true>;
         if (flow) k = nt == 1 ? linear_flow<1, PRO_NONE> : nt == 2 ? linear_flow<2, PRO_NONE> : linear_flow<4, PRO_NONE>;

@@ -281,3 +281,16 @@ def test_where_int4_weights_are_widened_once(m, k, n, wide):
     module, act = models.build_matmul_nbits(m, k, n, act_dtype=ir.F16, seed=m)
     names = kernels_of(module, {"a": act})
     assert ("nbits_gemm_wide" in names) == wide and ("nbits_gemm_tc" in names) != wide
+
+
+@pytest.mark.parametrize("dtype,rows,k,n,kernel", [(ir.BF16, 8, 9216, 1100, "linear_flow"), (ir.BF16, 16, 8192, 1200, "linear_flow"), (ir.BF16, 9, 8200, 1200, "linear_stream"),
+                                                   (ir.BF16, 17, 8200, 1200, "linear_flow"), (ir.BF16, 32, 12288, 800, "linear_flow"), (ir.BF16, 32, 12296, 800, "linear_stream")])
+def test_where_few_rows_take_the_ring(dtype, rows, k, n, kernel):
+    """The line itself, and the product on both sides of it: f32 sums of exact products, as in the test above."""
+    r = np.random.default_rng(k)
+    x, w = to_bf16(r.standard_normal((rows, k))), to_bf16(r.standard_normal((n, k)))
+    b = ir.GraphBuilder()
+    b.output("y", b.composite("onyxia.Linear", {}, [b.input("x", dtype, [rows, k]), b.constant(act(w, dtype))], [(ir.F32, [rows, n])])[0])
+    module, feed = b.finish(), {"x": act(x, dtype)}
+    assert kernels_of(module.clone(), feed) == {kernel}
+    assert rel_err(be.run_once(cuda_backend(), module, feed)[0][1].numpy(), x.astype(np.float64) @ w.T.astype(np.float64)) < 2e-6
