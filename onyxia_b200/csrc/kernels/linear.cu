@@ -978,6 +978,9 @@ template <int M, int R> __global__ void __launch_bounds__(kThreads, 2) linear_ro
 // `linear_reduce` adds the pieces in order. k, ldx and x_off are multiples of 4. 303 rows: 31 – 33 TFLOP/s, 313 and 146 µs for the two sizes
 // above (linear_simt, one scalar shared-memory read per two FMAs and no cut along k: 569 and 1046 µs).
 constexpr int kF32Threads = 128;
+// Its epilogue of 32 values per thread stands against few steps where k is short. linear_simt → linear_f32, µs: 40 rows × 64 weight rows, k 16: 7 → 15, k 64:
+// 12 → 18, k 128: 19 → 21, k 192 (64 rows): 26 → 24, k 256: 32 → 27; 1000 × 4096, k 64: 40 → 46, k 192: 91 → 82.
+static bool f32_pays(long long k) { return k >= 192; }
 __global__ void __launch_bounds__(kF32Threads) linear_f32(const __grid_constant__ LinP p) {
     __shared__ __align__(16) float ws[2][16][68], xs[2][16][68];
     const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
@@ -1497,7 +1500,7 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
                   {{&p.mul, mul}, {&p.x[0], bx0}, {&p.x[1], bx1}, {&p.w[0], w0.buf}, {&p.w[1], bw1}, {&p.bias, bb}, {&p.y, y.buf}}, "linear_rows_f32", /*pdl=*/true);
         return;
     }
-    if (!tc_type && quads) {
+    if (!tc_type && quads && f32_pays(d.k[0] + d.k[1])) {
         const dim3 tiles((unsigned)((d.out + 63) / 64 * d.blocks), (unsigned)((d.rows + 63) / 64));
         const long long steps = (d.k[0] + 15) / 16 + (d.k[1] + 15) / 16, ctas = (long long)tiles.x * tiles.y;
         // five CTAs fit an SM; pieces of at least 16 steps until three per SM are there
@@ -1634,7 +1637,7 @@ void emit_grouped_linear(Emitter& em, const GroupedLinearDesc& d, const TRef& x,
     auto tiles_of = [&](int64_t size) { return std::min<int64_t>(d.rows / size + std::min(d.groups, d.rows), d.rows); };
     const bool tc_type = w.dtype == DT_BF16;
     if (!tc_type || d.k % 8 != 0) {
-        const bool quads = !tc_type && d.k % 4 == 0 && w.buf.off % 16 == 0;
+        const bool quads = !tc_type && d.k % 4 == 0 && w.buf.off % 16 == 0 && f32_pays(d.k);
         const auto k = quads ? linear_f32 : tc_type ? linear_simt<bf16> : linear_simt<float>;
         em.launch(k, dim3((unsigned)((d.out + 63) / 64), (unsigned)tiles_of(64)), dim3(quads ? kF32Threads : 256), 0, p,
                   {{&p.x[0], x.buf}, {&p.x[1], kNull}, {&p.w[0], w.buf}, {&p.w[1], kNull}, {&p.bias, kNull}, {&p.y, y.buf}, {&p.counts, counts.buf}},

@@ -294,3 +294,16 @@ def test_where_few_rows_take_the_ring(dtype, rows, k, n, kernel):
     module, feed = b.finish(), {"x": act(x, dtype)}
     assert kernels_of(module.clone(), feed) == {kernel}
     assert rel_err(be.run_once(cuda_backend(), module, feed)[0][1].numpy(), x.astype(np.float64) @ w.T.astype(np.float64)) < 2e-6
+
+
+@pytest.mark.parametrize("rows,k,kernel", [(1, 16, "linear_simt"), (40, 64, "linear_simt"), (33, 188, "linear_simt"), (2, 192, "linear_f32"), (40, 192, "linear_f32"),
+                                           (8, 508, "linear_f32"), (8, 512, "linear_rows_f32")])
+def test_where_f32_products_take_register_tiles(rows, k, kernel):
+    """The line itself, and sums of k products of f32 on both sides of it: off by less than (k + 2) · 2^-24 of the sum of magnitudes."""
+    r = np.random.default_rng(k)
+    x, w = r.standard_normal((rows, k)).astype(np.float32), r.standard_normal((70, k)).astype(np.float32)
+    b = ir.GraphBuilder()
+    b.output("y", b.composite("onyxia.Linear", {}, [b.input("x", ir.F32, [rows, k]), b.constant(HostTensor.from_numpy(w))], [(ir.F32, [rows, 70])])[0])
+    module, feed = b.finish(), {"x": HostTensor.from_numpy(x)}
+    assert kernels_of(module.clone(), feed) - {"linear_reduce"} == {kernel}
+    assert rel_err(be.run_once(cuda_backend(), module, feed)[0][1].numpy(), x.astype(np.float64) @ w.T.astype(np.float64)) < 2e-6
