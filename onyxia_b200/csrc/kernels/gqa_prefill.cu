@@ -512,14 +512,19 @@ template <int D> void launch_prefill(Emitter& em, PrefillP& p, long long B, long
                                      Buf out, Buf dyn_t) {
     constexpr int RS = D + kPad;
     // Two heads per key head and scores that fit beside the stages (200 KB: 2047 positions at a head size of 256, all visible) take the kernel
-    // that forms them once; longer ranges walk the keys three times.
+    // that forms them once; longer ranges walk the keys three times, and so do short ones: one CTA of 16 warps for two heads has the SM to itself,
+    // where three or more of the other kernel's share it (at a head size of 256, one). Three walks → kept scores, µs for heads : key heads : size, positions,
+    // all visible: 4:1:256 64 13.5 → 17.3, 128 17.8 → 19.2, 192 23.5 → 21.9, 512 50 → 35; 8:4:64 32 9.7 → 13.2, 128 15.7 → 15.6, 256 24 → 17; 32:16:128 eight
+    // sequences of 64 56 → 70, 256 270 → 270, 384 471 → 445. A second round that few CTAs are left for: 16:8:64 320 (160 CTAs) 28 → 30, 384 (192) 33 → 33.
     const long long seen = p.window >= 0 && p.window < p.T - kBM ? p.window + kBM : p.T;  // keys that a CTA's rows see, at most (any window: no overflow)
     p.score_stride = (int)((std::min<long long>(seen, 1 << 20) + kKB - 1) / kKB * kKB) + 8;  // 16 bytes off a multiple of 128: conflict-free
     const size_t kept = ((size_t)2 * kKB * RS + (size_t)kSRows * p.score_stride) * 2;
-    if (H / p.KV % 2 == 0 && dyn_t.slot == kSlotNull && kept <= 200 * 1024) {
+    const long long ctas = (S + kBM - 1) / kBM * (H / 2) * B, sms = sm_count();
+    const bool pays = seen >= (D == 256 ? 160 : 256) && (D == 256 || seen >= 512 || ctas <= sms || 4 * ctas >= 5 * sms);
+    if (H / p.KV % 2 == 0 && dyn_t.slot == kSlotNull && kept <= 200 * 1024 && pays) {
         ensure_max_dynamic_smem((const void*)gqa_prefill_scores<D>, 200 * 1024);
         em.launch(gqa_prefill_scores<D>, dim3((unsigned)((S + kBM - 1) / kBM), (unsigned)(H / 2), (unsigned)B), dim3(kSThreads), (unsigned)kept, p,
-                  {{&p.q, q}, {&p.pk, pk}, {&p.pv, pv}, {&p.seqlens, seqlens}, {&p.out, out}, {&p.dyn_t, dyn_t}}, "gqa_prefill_tc", /*pdl=*/true);
+                  {{&p.q, q}, {&p.pk, pk}, {&p.pv, pv}, {&p.seqlens, seqlens}, {&p.out, out}, {&p.dyn_t, dyn_t}}, "gqa_prefill_scores", /*pdl=*/true);
         return;
     }
     const size_t smem = (size_t)(kBM + 4 * kKB) * RS * 2;

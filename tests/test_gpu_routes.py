@@ -176,7 +176,8 @@ def test_gelu_of_every_half():
 
 
 @pytest.mark.parametrize("heads,kv,d,past,seq,window", [(4, 1, 256, 0, 100, -1), (8, 2, 64, 300, 40, 70), (3, 3, 128, 50, 33, -1), (6, 2, 128, 0, 700, 129),
-                                                        (2, 1, 64, 1, 16, 0)])
+                                                        (2, 1, 64, 1, 16, 0), (8, 2, 64, 300, 40, -1), (6, 2, 128, 0, 700, 300), (4, 1, 256, 0, 200, -1),
+                                                        (2, 1, 64, 300, 16, 260)])
 def test_prefill_attention_with_kept_scores(heads, kv, d, past, seq, window):
     """Pairs of heads and single ones, windows shorter and longer than a block, ranges that end inside a block, a query tile that is not full;
     the bounds are those of the kernel's own tests (every rounding of the decomposition is repeated, sums differ in the last bits)."""
@@ -203,7 +204,7 @@ def test_bf16_products_of_several_rounds_per_cta(rows, k, k1, n):
         assert rel_err(run_linear(ir.BF16, x, w, bias=bias, glu=(1.7, 2.0, 1.0)), g / (1 + np.exp(-1.7 * g)) * (u + 1)) < 3e-6
 
 
-@pytest.mark.parametrize("d,past,seq,window", [(64, 90, 33, -1), (128, 0, 70, 40), (256, 300, 20, 100)])
+@pytest.mark.parametrize("d,past,seq,window", [(64, 240, 33, -1), (128, 100, 300, 250), (256, 300, 20, 150)])
 def test_kept_scores_with_values_that_are_not_finite(d, past, seq, window):
     """Rows whose visible scores are NaN, all minus infinity, or infinite in part, and a NaN among the keys: kept scores (two heads per key head) give
     what the kernel that walks the keys three times gives for the same heads with a key head each, bit for bit in the other rows too."""
@@ -230,7 +231,7 @@ def test_kept_scores_with_values_that_are_not_finite(d, past, seq, window):
 
 def test_windows_up_to_the_largest_number():
     """A window beyond all positions sees what no window sees, up to the type's largest value."""
-    feeds = [models.build_gqa(1, 4, 2, 64, 40, 30, ir.F16, w, True, seed=1) for w in (-1, 70, 2 ** 63 - 17, 2 ** 63 - 16, 2 ** 63 - 1)]
+    feeds = [models.build_gqa(1, 4, 2, 64, 300, 30, ir.F16, w, True, seed=1) for w in (-1, 330, 2 ** 63 - 17, 2 ** 63 - 16, 2 ** 63 - 1)]
     want, *got = [be.run_once(cuda_backend(), m, f)[0][1].numpy() for m, f in feeds]
     assert all(np.array_equal(g, want) for g in got)
 
@@ -307,3 +308,11 @@ def test_where_f32_products_take_register_tiles(rows, k, kernel):
     module, feed = b.finish(), {"x": HostTensor.from_numpy(x)}
     assert kernels_of(module.clone(), feed) - {"linear_reduce"} == {kernel}
     assert rel_err(be.run_once(cuda_backend(), module, feed)[0][1].numpy(), x.astype(np.float64) @ w.T.astype(np.float64)) < 2e-6
+
+
+@pytest.mark.parametrize("heads,kv,d,seq,window,batch,kept", [(4, 1, 256, 159, -1, 1, False), (4, 1, 256, 160, -1, 1, True), (8, 4, 64, 255, -1, 1, False), (8, 4, 64, 256, -1, 1, True),
+                                                              (4, 2, 128, 300, 239, 1, False), (4, 2, 128, 300, 240, 1, True), (16, 8, 64, 320, -1, 1, False), (16, 8, 64, 384, -1, 1, True),
+                                                              (16, 8, 64, 256, -1, 1, True), (3, 3, 64, 300, -1, 1, False)])
+def test_where_prompt_attention_keeps_its_scores(heads, kv, d, seq, window, batch, kept):
+    names = kernels_of(*models.build_gqa(batch, heads, kv, d, 0, seq, ir.F16, window, True, seed=1))
+    assert ("gqa_prefill_scores" in names) == kept and ("gqa_prefill_tc" in names) != kept
