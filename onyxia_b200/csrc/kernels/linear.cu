@@ -633,10 +633,11 @@ template <int EPI, bool ONE> __global__ void __launch_bounds__(kTcThreads) linea
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * S + 4);
     const unsigned finished = smem_u32(bars + 2 * S), read = finished + 16;
     pdl_trigger();
-    int row_tiles = p.row_tiles;
+    int row_tiles = p.row_tiles, group = 0, group_row = 0, group_live = 0;
     if (p.groups) {  // the counts come from an earlier launch
         pdl_wait();
-        row_tiles = count_tiles(p, nb);
+        if (!ONE) row_tiles = count_tiles(p, nb);
+        else if (!locate_group(p, (int)blockIdx.x, nb, &group, &group_row, &group_live)) return;  // the grid covers the most tiles that any counts give
     }
     const int first = ONE ? 0 : (int)blockIdx.x, total = ONE ? 1 : row_tiles * p.out_tiles * p.splits;
     if (tid == 0) {
@@ -672,7 +673,15 @@ template <int EPI, bool ONE> __global__ void __launch_bounds__(kTcThreads) linea
         }
         q.n0 = x * nb;
         q.live = (int)min((long long)nb, p.rows - q.n0);
-        if (p.groups) locate_group(p, x, nb, &q.group, &q.n0, &q.live);
+        if (p.groups) {
+            if (!ONE) {
+                locate_group(p, x, nb, &q.group, &q.n0, &q.live);
+            } else {
+                q.group = group;
+                q.n0 = group_row;
+                q.live = group_live;
+            }
+        }
         q.block = p.blocks > 1 ? y / block_tiles : 0;
         q.m0 = (y - q.block * block_tiles) * 128;
         q.lo = (int)((unsigned)(all * q.piece) / (unsigned)p.splits);
@@ -1666,14 +1675,18 @@ void emit_grouped_linear(Emitter& em, const GroupedLinearDesc& d, const TRef& x,
     p.out_tiles = (int)mt;
     const long long tiles = tiles_of(p.nb) * mt;  // at most
     if (tiles >= INT32_MAX) throw std::runtime_error("grouped product: too many tiles");
-    // Tiles of 32 rows are bound by the weights' bytes: four CTAs of two stages per SM instead of two of five, so that more tiles run side by side
-    // and few are left for a second round. 64 tokens, 16 experts, 4 096 × 2 560 and 2 560 × 2 048: 65 → 60 µs a product; three CTAs 64, five 60.
-    const int resident = p.nb == 32 ? 4 : p.nb <= 128 ? 2 : 1;
+    // Tiles of 32 rows are bound by the weights' bytes: where more are expected than two CTAs of five stages per SM take at once, four of two stages, so
+    // that few are left for a second round.
+    const double expected = std::max((double)std::min(d.groups, d.rows), (double)d.rows / p.nb + 0.5 * (double)std::min(d.groups, d.rows)) * (double)mt;
+    const int resident = p.nb == 32 && expected > 2.0 * sm_count() ? 4 : p.nb <= 128 ? 2 : 1;
+    // A CTA per tile where a group has few rows: what a persistent CTA spends on finding its tiles stands beside few, short ones.
+    const bool one = d.rows < 64 * d.groups;
     p.stages = (int)std::min<size_t>(8, (resident == 4 ? 48 * 1024 : resident == 2 ? 108 * 1024 : 208 * 1024) / stage);
     const size_t smem = stage * p.stages + 1024 + (2 * p.stages + 4) * 8 + 16;
-    const auto kernel = d.glu ? linear_tc<EPI_GLU, false> : linear_tc<EPI_PLAIN, false>;
+    const auto kernel = one ? (d.glu ? linear_tc<EPI_GLU, true> : linear_tc<EPI_PLAIN, true>) : (d.glu ? linear_tc<EPI_GLU, false> : linear_tc<EPI_PLAIN, false>);
     ensure_max_dynamic_smem((const void*)kernel, 220 * 1024);
-    LaunchRec& rec = em.launch(kernel, dim3((unsigned)std::min<long long>(tiles, (long long)sm_count() * resident)), dim3(kTcThreads), (unsigned)smem, p,
+    const dim3 grid = one ? dim3((unsigned)tiles_of(p.nb), (unsigned)mt) : dim3((unsigned)std::min<long long>(tiles, (long long)sm_count() * resident));
+    LaunchRec& rec = em.launch(kernel, grid, dim3(kTcThreads), (unsigned)smem, p,
                                {{&p.bias, kNull}, {&p.y, y.buf}, {&p.partial, kNull}, {&p.err, Buf{kSlotErr, 0}}, {&p.counts, counts.buf}}, "grouped_tc",
                                /*pdl=*/true);
     auto add_map = [&](int i, const Buf& b, int64_t rows, uint32_t box) {

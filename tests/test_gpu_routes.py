@@ -316,3 +316,10 @@ def test_where_f32_products_take_register_tiles(rows, k, kernel):
 def test_where_prompt_attention_keeps_its_scores(heads, kv, d, seq, window, batch, kept):
     names = kernels_of(*models.build_gqa(batch, heads, kv, d, 0, seq, ir.F16, window, True, seed=1))
     assert ("gqa_prefill_scores" in names) == kept and ("gqa_prefill_tc" in names) != kept
+
+
+@pytest.mark.parametrize("n", [40, 64, 200, 700])
+def test_experts_with_more_small_tiles_than_ctas(n):
+    """Tiles of 32 rows in four CTAs per SM, a CTA per tile and none for the tiles that the counts do not give; persistent ones where groups have many rows."""
+    m = Experts("bf16", 264, 24, 3, 1100)
+    m.check(m.rows(n))
