@@ -22,8 +22,9 @@
 //   gqa_pv       one warp per key again: p = exp(s − max)/Σ, acc += p·v; the
 //                last CTA to finish adds the partial accumulators in split order
 //                and stores the output row
-// When the present buffer is not the past buffer, gqa_copy_past fills it first, and the three launches append in place. Single tokens
-// on a cache that was in place all along take the decode kernels, whose sums are in f32; here they are in f64.
+// When the present buffer is not the past buffer, gqa_copy_past fills it first (gqa_prepare itself where the cache is small), and the three
+// launches append in place. Single tokens on a cache that was in place all along take the decode kernels, whose sums are in f32; here they
+// are in f64.
 // "Last CTA" is decided by an arrival counter per query; nothing ever waits.
 //
 // KV tensors are [B, KV, T, D] views of buffers that hold `cap ≥ T` rows per
@@ -52,6 +53,8 @@ struct GqaPrepP {
     const void* q;
     const void* k;
     const void* v;
+    const void* past_k;  // of a small cache that is copied here
+    const void* past_v;
     const int* seqlens;
     const void* cos;
     const void* sin;
@@ -60,9 +63,10 @@ struct GqaPrepP {
     void* present_v;
     ErrWord* err;
     const long long* dyn_t;  // when set, the present length T is read from here
-    long long B, S, H, KV, D, T, pres_cap, half, cache_rows;
+    long long B, S, H, KV, D, P, T, past_cap, pres_cap, half, cache_rows;
     long long nq;    // threads that rotate q (0 without rotary)
     long long nkv;   // threads that write the new rows
+    long long ncopy; // threads that copy the past
     int clear, node;  // clear: what lies beyond a ragged row's tokens is zeroed here (2: in front of them too)
 };
 
@@ -79,7 +83,7 @@ __device__ __forceinline__ float rope_elem(const void* x, long long base, long l
 
 template <int DT> __global__ void gqa_prepare(const GqaPrepP p) {
     pdl_enter();
-    const long long total = p.nq + p.nkv;
+    const long long total = p.nq + p.nkv + p.ncopy;
     const long long T = p.dyn_t ? *p.dyn_t : p.T;
     for (long long i = global_tid(); i < total; i += global_threads()) {
         if (i < p.nq) {
@@ -95,6 +99,17 @@ template <int DT> __global__ void gqa_prepare(const GqaPrepP p) {
             continue;
         }
         long long r = i - p.nq;
+        if (r >= p.nkv) {  // a small cache's past, and zeros behind the rows that are written above
+            r -= p.nkv;
+            const long long e = r % p.D, t = (r / p.D) % T, head = r / (p.D * T), b = head / p.KV;
+            const long long tot = (long long)p.seqlens[b] + 1, past_b = tot - p.S > 0 ? tot - p.S : 0;
+            if (t >= past_b && t < past_b + p.S) continue;
+            const bool held = t < p.P && t < past_b;
+            const long long from = (head * p.past_cap + t) * p.D + e, to = (head * p.pres_cap + t) * p.D + e;
+            st<DT>(p.present_k, to, held ? ld<DT>(p.past_k, from) : 0.f);
+            st<DT>(p.present_v, to, held ? ld<DT>(p.past_v, from) : 0.f);
+            continue;
+        }
         long long e = r % p.D, j = (r / p.D) % p.S, kvh = (r / (p.D * p.S)) % p.KV, b = r / (p.D * p.S * p.KV);
         long long tot = (long long)p.seqlens[b] + 1, past_b = tot - p.S > 0 ? tot - p.S : 0;
         long long pres_base = (b * p.KV + kvh) * p.pres_cap * p.D;
@@ -364,11 +379,15 @@ template <int DT> static void emit_gqa_t(Emitter& em, const GqaDesc& d, const TR
     const int esz = DT == DT_F16 ? 2 : 4;
     Buf null{kSlotNull, 0};
 
-    const long long pres_cap = present_k.cap ? present_k.cap : T;
-    if (!d.in_place && P > 0) {
+    const long long pres_cap = present_k.cap ? present_k.cap : T, past_cap = past_k.cap ? past_k.cap : P;
+    // A small cache is copied by gqa_prepare, an element per thread: a launch of its own takes longer. Whole attention, copy beside the new rows →
+    // by a launch of its own: 8 heads of 32, 4 key heads, 16 rows 13.1 → 14.7 µs; 8 of 64, 16 rows and 20 new ones 9.6 → 10.5; one key head of 256, 100
+    // rows 27.0 → 28.9, 500 rows (128 000 elements) 46.0 → 45.2; 16 of 128, 100 rows (207 000) 23.6 → 22.0.
+    const bool small = !d.in_place && P > 0 && B * KV * T * D <= 1 << 16;
+    if (!d.in_place && P > 0 && !small) {
         GqaCopyP cp{};
         cp.S = S; cp.P = P; cp.T = T;
-        cp.past_cap = past_k.cap ? past_k.cap : P;
+        cp.past_cap = past_cap;
         cp.pres_cap = pres_cap;
         cp.row_bytes = D * esz;
         cp.KV = (int)KV;
@@ -387,7 +406,8 @@ template <int DT> static void emit_gqa_t(Emitter& em, const GqaDesc& d, const TR
     Buf dyn_t = dyn ? em.dyn(T) : null;
     if (dyn && S == 1 && emit_gqa_decode(em, d, q, k, v, seqlens, cos, sin, out, present_k, present_v, dyn_t, Tsz)) return;
     GqaPrepP pp{};
-    pp.B = B; pp.S = S; pp.H = H; pp.KV = KV; pp.D = D; pp.T = T;
+    pp.B = B; pp.S = S; pp.H = H; pp.KV = KV; pp.D = D; pp.P = P; pp.T = T;
+    pp.past_cap = past_cap;
     pp.pres_cap = pres_cap;
     if (dyn) pp.T = 0;
     pp.half = d.rot_half;
@@ -396,9 +416,10 @@ template <int DT> static void emit_gqa_t(Emitter& em, const GqaDesc& d, const TR
     pp.node = em.node;
     pp.nq = d.rot_half ? B * S * H * D : 0;
     pp.nkv = B * KV * S * D;
+    pp.ncopy = small ? B * KV * T * D : 0;
     Buf qrot = d.rot_half ? em.scratch((size_t)(B * S * H * D * esz)) : null;
-    em.launch(gqa_prepare<DT>, dim3(grid_for(pp.nq + pp.nkv, 256)), dim3(256), 0, pp,
-              {{&pp.q, q.buf}, {&pp.k, k.buf}, {&pp.v, v.buf},
+    em.launch(gqa_prepare<DT>, dim3(grid_for(pp.nq + pp.nkv + pp.ncopy, 256)), dim3(256), 0, pp,
+              {{&pp.q, q.buf}, {&pp.k, k.buf}, {&pp.v, v.buf}, {&pp.past_k, small ? past_k.buf : null}, {&pp.past_v, small ? past_v.buf : null},
                {&pp.seqlens, seqlens.buf}, {&pp.cos, cos ? cos->buf : null}, {&pp.sin, sin ? sin->buf : null},
                {&pp.q_rot, qrot}, {&pp.present_k, present_k.buf}, {&pp.present_v, present_v.buf}, {&pp.err, Buf{kSlotErr, 0}},
                {&pp.dyn_t, dyn_t}},

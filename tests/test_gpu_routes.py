@@ -323,3 +323,19 @@ def test_experts_with_more_small_tiles_than_ctas(n):
     """Tiles of 32 rows in four CTAs per SM, a CTA per tile and none for the tiles that the counts do not give; persistent ones where groups have many rows."""
     m = Experts("bf16", 264, 24, 3, 1100)
     m.check(m.rows(n))
+
+
+@pytest.mark.parametrize("dtype,d,past,seq,alone", [(ir.F16, 32, 1, 1, False), (ir.F32, 256, 40, 3, False), (ir.F16, 64, 255, 1, False), (ir.F16, 64, 256, 1, True),
+                                                    (ir.F32, 64, 251, 12, True), (ir.F16, 128, 100, 20, False)])
+def test_small_caches_are_copied_beside_the_new_rows(dtype, d, past, seq, alone):
+    """Up to 2^16 elements the launch that writes the new rows copies the past: bit for bit, zeros behind ragged rows, the line itself."""
+    module, feed = models.build_gqa(2, 4, 2, d, past, seq, dtype, -1, True, seed=d + seq)
+    valid = [past, past // 3]
+    feed["seqlens_k"] = HostTensor.from_numpy(np.array([v + seq - 1 for v in valid], np.int32))
+    assert ("gqa_copy_past" in kernels_of(module.clone(), feed)) == alone
+    tol = dict(atol=4e-3, rtol=4e-3) if dtype == ir.F16 else dict(atol=2e-4, rtol=1e-3)
+    got = {n: t.numpy() for n, t in differential(module, feed, **tol)[0]}
+    for name in ("key", "value"):
+        for b, v in enumerate(valid):
+            assert np.array_equal(got["present_" + name][b, :, :v], feed["past_" + name].numpy()[b, :, :v])
+            assert not got["present_" + name][b, :, v + seq:].any()
