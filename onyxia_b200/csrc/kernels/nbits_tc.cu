@@ -393,8 +393,8 @@ __global__ void __launch_bounds__(256) nbits_gemm_reduce(const TcReduceP p) {
 }
 
 // ───────────────────────────── many activation rows ─────────────────────────────
-// nbits_gemm_tc widens a weight again for every 256 activation rows, which is what sets its pace (1.3 µs per 128 k and CTA). Above that
-// the weights are widened once into scratch, as f16 rows that a plain tcgen05 GEMM takes by TMA.
+// nbits_gemm_tc widens a weight again for every 256 activation rows, which is what sets its pace (1.3 µs per 128 k and CTA). Where that costs
+// more (wide_pays) the weights are widened once into scratch, as f16 rows that a plain tcgen05 GEMM takes by TMA.
 struct WidenP {
     const unsigned char* tiles;  // of this panel
     __half* w;                   // [row tiles · 16][k_tiles · 128]
@@ -613,25 +613,47 @@ __global__ void __launch_bounds__(kWideThreads, 1) nbits_gemm_wide(const __grid_
     if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
-// Whether the weights are widened once. A pass of nbits_gemm_tc costs 8 µs and more besides its steps, the GEMM a pass over 2.6 bytes per weight and
-// half-filled rounds: short k pays from two passes on, long k with many of them. Measured on 150 sizes, nbits_gemm_tc → widened once, µs: k 1152 and 13 824
-// weight rows 46 → 33 (257 activation rows), 158 → 83 (1536); k 1536 and 12 288: 42 → 45 (512), 63 → 55 (768); k 2048 and 8192: 42 → 36 (257); k 2560 and 20 480:
-// 85 → 112 (257), 190 → 183 (1024), 381 → 320 (2047); k 3072 and 8192: 43 → 53 (257), 95 → 95 (1024); k 4096 and 4096: 32 → 37 (257), 70 → 61 (1024); k 6912 and
-// 1152: 20.3 → 21.7 (512), 40 → 35 (1024), 79 → 47 (2047); k 5376 and 8192: 60 → 77 (257), 261 → 270 (2047); k 5376 and 43 008: 266 → 386 (257), 2380 → 2510
-// (4096); k 21 504 and 5376: 130 → 430 (257), whose panels are too few tiles for the SMs.
-bool wide_pays(long long m, long long k, long long n) {
-    if (m <= 256) return false;
-    if (k <= 1280) return true;
-    if (k <= 2048) return n <= 8192 || m >= 640;
-    return m >= 1024 && (k <= 4096 || (k <= 7168 && n <= 2048));
+// Row tiles of a panel: at most 64 MB of widened weights, which stay in L2 until the product reads them.
+int panel_tiles(const TcP& t) { return (int)std::max<long long>(8, (64LL << 20) / ((long long)t.k_tiles * 128 * 32) / 8 * 8); }
+
+// Few tiles: the pieces of k go to CTAs of their own where that, with the partial sums' trip (5 TB/s) and a second launch, is shorter.
+bool pieces_apart(const TcP& t, long long m, int count) {
+    const long long slots = sm_count(), ctas = (m + kWideRows - 1) / kWideRows * ((count + 7) / 8);
+    const double step_us = 0.45;  // 128 k of a tile
+    const double joined = (double)((ctas + slots - 1) / slots) * t.k_tiles * step_us;
+    const double apart = (double)((ctas * t.splits + slots - 1) / slots) * ((double)t.k_tiles / t.splits * step_us + 1.0) + 3.0 +
+                         (double)t.splits * m * ((count + 7) / 8 * 128) * 8.0 / 5e6;
+    return t.splits > 1 && t.n_full == 0 && apart < joined;
 }
 
-// `t`: the launch of nbits_gemm_tc for these rows (its pieces of k are kept).
+// Whether the weights are widened once, for m rows whose launches of nbits_gemm_tc are `t`. Both sides as sums of what they do, fitted to 459 times of
+// either (51 sizes, k 512 … 21 504, 512 … 61 440 weight rows, 257 … 4096 activation rows: residuals 4 % and 6 %; two other sweeps, of grouped
+// products, 5 … 8 %). With a tenth of margin nothing measured is slower than nbits_gemm_tc alone. nbits_gemm_tc → widened once, µs, at 257, 1024 and 4096
+// rows: k 1152, 13 824 weight rows 48 → 39, 109 → 63, 431 → 194; k 2560, 20 480: 99 → (119), 217 → (196), 858 → 574; k 5376, 5376: 58 → (55), 126 → (114), 499 → 322;
+// k 5376, 43 008: 289 → (389), 620 → (795), 2469 → (2388); k 6912, 1152: 39 → 33, 82 → 58, 332 → 99; k 21 504, 5376: 148 → (270), 308 → (430), 1219 → (1282);
+// in brackets: not taken.
+bool wide_pays(const TcP& t, long long m) {
+    const long long slots = sm_count(), grid = (t.row_tiles + 7) / 8, tail = grid - t.n_full;
+    const double out_mb = (double)m * t.row_tiles * 32.0 / 1e6;
+    const long long full = (t.n_full + slots - 1) / slots, cut = tail > 0 ? (tail * t.splits + slots - 1) / slots : 0;  // rounds of CTAs
+    const double steps = (double)full * t.k_tiles + (double)cut * t.k_tiles / t.splits, sums_mb = t.splits > 1 ? (double)t.splits * t.mb * tail * 128 * 8.0 / 1e6 : 0.0;
+    const double passes_us = (double)((m + t.mb - 1) / t.mb) * (3.65 + 1.036 * steps + 11.1 * (double)full + 6.5 * (double)cut + 0.12 * sums_mb) + 0.59 * out_mb;
+    double wide_us = 5.5 + 0.38 * out_mb;
+    for (int first = 0, size = panel_tiles(t); first < t.row_tiles; first += size) {
+        const int count = std::min(size, t.row_tiles - first), pieces = pieces_apart(t, m, count) ? t.splits : 1;
+        const long long o_tiles = (count + 7) / 8, rounds = ((m + kWideRows - 1) / kWideRows * o_tiles * pieces + slots - 1) / slots;
+        wide_us += 2.5 * (pieces > 1 ? 3 : 2) + 0.69 * (double)rounds * t.k_tiles / pieces + 0.23 * (double)count * 16 * t.k_tiles * 128 * 2.5 / 1e6;
+        if (pieces > 1) wide_us += 0.14 * (double)pieces * m * o_tiles * 128 * 8.0 / 1e6;
+    }
+    return wide_us < 0.9 * passes_us;
+}
+
+// `t`: the launch of nbits_gemm_tc for these rows (its pieces of k are kept). The activations come by tensor map alone: their offset in the
+// buffer is checked by the caller, and buffers (arena granules, the pool's, a caller's whole tensors) begin on 256 bytes.
 void emit_wide(Emitter& em, const NBitsGroup& gr, const TRef& x, const TRef& tiles, const TcP& t) {
     const Buf null{kSlotNull, 0};
-    // panels of at most 64 MB of widened weights: they stay in L2 until the product reads them
     const long long ld = (long long)t.k_tiles * 128;
-    const int per_panel = (int)std::max<long long>(8, (64LL << 20) / (ld * 32) / 8 * 8);
+    const int per_panel = panel_tiles(t);
     const Buf wide = em.scratch((size_t)std::min(per_panel, (t.row_tiles + 7) / 8 * 8) * 16 * ld * 2);
     for (int first = 0; first < t.row_tiles; first += per_panel) {
         const int count = std::min(per_panel, t.row_tiles - first);
@@ -657,13 +679,8 @@ void emit_wide(Emitter& em, const NBitsGroup& gr, const TRef& x, const TRef& til
         p.m_tiles = (int)((gr.m + kWideRows - 1) / kWideRows);
         p.o_tiles = (count + 7) / 8;
         p.n_pad = (long long)p.o_tiles * 128;
-        // Few tiles: the pieces of k go to CTAs of their own where that, with the partial sums' trip (5 TB/s) and a second launch, is shorter
         const long long slots = sm_count(), ctas = (long long)p.m_tiles * p.o_tiles;
-        const double step_us = 0.45;  // 128 k of a tile
-        const double joined = (double)((ctas + slots - 1) / slots) * t.k_tiles * step_us;
-        const double apart = (double)((ctas * t.splits + slots - 1) / slots) * ((double)t.k_tiles / t.splits * step_us + 1.0) + 3.0 +
-                             (double)t.splits * gr.m * p.n_pad * 8.0 / 5e6;
-        p.apart = t.splits > 1 && t.n_full == 0 && apart < joined;
+        p.apart = pieces_apart(t, gr.m, count);
         const Buf partial = p.apart ? em.scratch((size_t)p.splits * gr.m * p.n_pad * 4) : null;
         const size_t smem = kWideStages * kWideStage + 1024 + (2 * kWideStages + 4) * 8 + 16;
         ensure_max_dynamic_smem((const void*)nbits_gemm_wide, 220 * 1024);
@@ -767,7 +784,7 @@ void emit_nbits_gemm_tc(Emitter& em, const NBitsGroup& gr, const TRef& x, const 
     if (debug) std::fprintf(stderr, "nbits_gemm_tc: m %lld k_tiles %d grid %u mb %d: %d pieces over %lld of the row blocks\n", gr.m, p.k_tiles, grid, mb, splits, tail);
     p.n_full = (int)n_full;
     p.splits = splits;
-    if (wide_pays(gr.m, gr.k, (long long)p.row_tiles * 16) && gr.m < 65536 && gr.k % 8 == 0 && x.buf.off % 16 == 0) return emit_wide(em, gr, x, tiles, p);
+    if (gr.m > 256 && gr.m < 65536 && gr.k % 8 == 0 && x.buf.off % 16 == 0 && wide_pays(p, gr.m)) return emit_wide(em, gr, x, tiles, p);
     p.n_pad = tail * 128;
     const Buf partial = splits > 1 ? em.scratch((size_t)splits * mb * p.n_pad * sizeof(float)) : null;
     for (long long m0 = 0; m0 < gr.m; m0 += mb) {

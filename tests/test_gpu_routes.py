@@ -276,12 +276,24 @@ def kernels_of(module, feed):
     return {kernel for kernel, _, _ in s.take_timings()}
 
 
-@pytest.mark.parametrize("m,k,n,wide", [(256, 512, 64, False), (257, 1280, 64, True), (257, 1288, 8192, True), (639, 2048, 8193, False), (640, 2048, 8193, True),
-                                        (1023, 2056, 64, False), (1024, 4096, 2064, True), (1024, 4104, 2048, True), (1024, 4104, 2049, False), (1024, 7176, 64, False)])
+@pytest.mark.parametrize("m,k,n,wide", [(256, 512, 64, False), (257, 128, 64, True), (257, 1152, 6912, True), (257, 4096, 1024, True), (512, 4096, 1024, False),
+                                        (257, 5376, 2048, True), (512, 5376, 2048, False), (1024, 5376, 2048, True), (512, 8192, 2048, False)])
 def test_where_int4_weights_are_widened_once(m, k, n, wide):
     module, act = models.build_matmul_nbits(m, k, n, act_dtype=ir.F16, seed=m)
     names = kernels_of(module, {"a": act})
     assert ("nbits_gemm_wide" in names) == wide and ("nbits_gemm_tc" in names) != wide
+
+
+@pytest.mark.parametrize("m,parts,k,n,zp", [(400, 2, 1000, 200, True), (512, 2, 1152, 1536, False), (400, 2, 136, 4104, True), (384, 2, 1152, 29300, True),
+                                            (1024, 4, 4096, 2064, False), (1024, 5, 6912, 1152, True)])
+def test_weights_widened_once_give_the_bits_of_the_passes(m, parts, k, n, zp):
+    """The same rows in pieces of 129 to 256, which take the passes: pieces of k and whole k, k that ends inside a block, two panels, zero points."""
+    module, act = models.build_matmul_nbits(m, k, n, act_dtype=ir.F16, seed=n, with_zp=zp)
+    got = be.run_once(cuda_backend(), module, {"a": act})[0][1].numpy()
+    for rows in np.array_split(np.arange(m), parts):
+        part, _ = models.build_matmul_nbits(len(rows), k, n, act_dtype=ir.F16, seed=n, with_zp=zp)
+        feed = {"a": HostTensor.from_numpy(act.numpy()[rows].copy())}
+        assert np.array_equal(got[rows], be.run_once(cuda_backend(), part, feed)[0][1].numpy())
 
 
 @pytest.mark.parametrize("dtype,rows,k,n,kernel", [(ir.BF16, 8, 9216, 1100, "linear_flow"), (ir.BF16, 16, 8192, 1200, "linear_flow"), (ir.BF16, 9, 8200, 1200, "linear_stream"),
