@@ -184,14 +184,20 @@ def gemv_sweep(backend, shapes, ms, peak, reps=10):
                     s.run(feed)
                 us = s.timer_stop() * 1e3 / (reps * copies)
                 fused = (s.launch_count() - n0) < reps * copies
+                names = set()
+                if m > 256:  # sizes decide which of two kernels runs
+                    s.enable_profiling(True)
+                    s.run(feed)
+                    names = {kernel for kernel, _, _ in s.take_timings()}
                 del s
-                return us, fused
+                return us, fused, "nbits_stream" if m <= 8 else "nbits_gemm_wide" if "nbits_gemm_wide" in names else "nbits_gemm_tc"
 
-            us, fused = time_on(backend)
-            entry_kernel = "persist_step" if fused else ("nbits_stream" if m <= 8 else "nbits_gemm_tc" if m <= 256 else "nbits_gemm_wide")
+            us, fused, entry_kernel = time_on(backend)
+            if fused:
+                entry_kernel = "persist_step"
             other = None
             if fused:  # the same products, one launch each
-                us2, _ = time_on(plain)
+                us2, _, _ = time_on(plain)
                 other = {"kernel": "nbits_stream", "us_per_launch": us2}
                 if us2 < us:
                     other = {"kernel": "persist_step", "us_per_launch": us}

@@ -198,7 +198,6 @@ __device__ __forceinline__ double erf_as_f(float xf) {  // Abramowitz–Stegun 7
 }
 
 // gelu(x) in the working type, before the last rounding.
-// gelu(x) in the working type, before the last rounding.
 template <int DT> __device__ __forceinline__ float gelu_value(const GeluP& p, float x) {
     float inner;
     if (p.tanh_approx) {  // decomp.rs:192-202

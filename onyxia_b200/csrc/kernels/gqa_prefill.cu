@@ -16,7 +16,7 @@
 //   pass 3  p = round16(e / Σ) becomes the A operand of the P·V product straight from the score
 //           tile's accumulator registers; V rows are the B operand through ldmatrix.trans; the four
 //           key groups' f32 partial outputs are added in group order through shared memory
-// Where the scores of two heads' rows fit in shared memory they are kept there instead (gqa_prefill_scores).
+// Where the scores of two heads' rows fit in shared memory and the range is not short they are kept there instead (gqa_prefill_scores).
 // K (and V in pass 3) blocks of 64 keys are staged by cp.async into padded shared-memory rows, two
 // stages deep. Products are exact f16 × f16 and are added in f32 by the tensor core (the interpreter
 // adds in f64): results differ from it by an f16 spacing on a small share of the elements, like the
@@ -511,9 +511,9 @@ template <int D> __global__ void __launch_bounds__(kSThreads, 1) gqa_prefill_sco
 template <int D> void launch_prefill(Emitter& em, PrefillP& p, long long B, long long S, long long H, Buf q, Buf pk, Buf pv, Buf seqlens,
                                      Buf out, Buf dyn_t) {
     constexpr int RS = D + kPad;
-    // Two heads per key head and scores that fit beside the stages (200 KB: 2047 positions at a head size of 256, all visible) take the kernel
-    // that forms them once; longer ranges walk the keys three times, and so do short ones: one CTA of 16 warps for two heads has the SM to itself,
-    // where three or more of the other kernel's share it (at a head size of 256, one). Three walks → kept scores, µs for heads : key heads : size, positions,
+    // Two heads per key head and scores that fit beside the stages (200 KB, a line drawn below the SM's 227: 2047 positions at a head size of
+    // 256, all visible) take the kernel that forms them once; longer ranges walk the keys three times, and so do short ones: one CTA of 16 warps
+    // for two heads has the SM to itself, where three or more of the other kernel's share it (at a head size of 256, one). Three walks → kept scores, µs for heads : key heads : size, positions,
     // all visible: 4:1:256 64 13.5 → 17.3, 128 17.8 → 19.2, 192 23.5 → 21.9, 512 50 → 35; 8:4:64 32 9.7 → 13.2, 128 15.7 → 15.6, 256 24 → 17; 32:16:128 eight
     // sequences of 64 56 → 70, 256 270 → 270, 384 471 → 445. A second round that few CTAs are left for: 16:8:64 320 (160 CTAs) 28 → 30, 384 (192) 33 → 33.
     const long long seen = p.window >= 0 && p.window < p.T - kBM ? p.window + kBM : p.T;  // keys that a CTA's rows see, at most (any window: no overflow)

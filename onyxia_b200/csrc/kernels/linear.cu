@@ -5,13 +5,13 @@
 //                   a row), eight warps share a row tile's k. Weight loads run one batch ahead and start before the
 //                   grid dependency resolves. For up to eight rows the residual norm that makes x runs as the
 //                   prologue, in every CTA.
-//   linear_flow     the same for large matrices: more of their weights in flight, through shared memory.
+//   linear_flow     the same for large matrices (above eight rows where k is not long): more of their weights in flight, through shared memory.
 //   linear_tc       more rows: tcgen05 GEMM. Weights are the MMA's A operand (128 rows), activations its B operand
 //                   (32–256 rows), both loaded by TMA into 128-byte-swizzled stages; accumulator in tensor memory.
 //                   Grids that would leave SMs idle are cut along k; `linear_reduce` adds the pieces in order.
-//   linear_rows_f32 f32 (true 32-bit), up to 32 rows: warps stream whole weight rows.
-//   linear_f32      f32, more rows: register-blocked tiles.
-//   linear_simt     f32 and bf16 shapes whose rows are not 16-byte aligned.
+//   linear_rows_f32 f32 (true 32-bit), up to 32 rows and k of 512 and more: warps stream whole weight rows.
+//   linear_f32      f32, more rows or shorter k: register-blocked tiles.
+//   linear_simt     f32 of short k, and f32 and bf16 shapes whose rows are not 16-byte aligned.
 //
 // linear_tc, linear_f32 and linear_simt also run grouped: activation rows sorted by group, one weight matrix per group, the groups'
 // row counts known on the device only. A CTA finds its group from the counts; the grid covers the most tiles
@@ -467,7 +467,9 @@ template <int NT, int NORM, bool BLOCKS> __global__ void __launch_bounds__(kStre
 // asynchronous copies, eight of them in flight instead of one batch of four between two waits. Every lane copies, and reads back, only the pieces
 // of a chunk that are its own MMA fragments, so nothing but the lane's own copies has to be waited for. The ring is filled ahead of the grid
 // dependency (activations behind it) and runs on across row tiles. Up to eight rows that no prologue makes travel with their weights: loaded a
-// chunk ahead into registers, they held every chunk up by an L2 read (1 row × 21 504 × 5376 92 µs, now 50).
+// chunk ahead into registers, they held every chunk up by an L2 read (1 row × 21 504 × 5376 92 µs, now 50). The weights of the first eight chunks
+// belong to the group of the first chunk's activations, so the first wait is for all of them; later ones are for a chunk each. 9 to 32 rows
+// still come chunk by chunk from L2, which is why long k does not take this kernel (see its rule).
 // 1 row: 5376 × 43 008 gated 123 → 77 µs (6.0 TB/s), 5376 × 16 896 56 → 34; 8 rows: 5376 × 32 768 62 (activations in registers: 92), 1152 × 32 768
 // 31 → 22. Below that size the products are faster alone, too, but not behind one another: decode steps of small models took 3 % longer with it
 // (13.8 against 13.4 ms for 48 steps of the 1b size, activations in registers).
@@ -1570,7 +1572,9 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
         return;
     }
     // Activation rows per tile and pieces along k: the choice with the smallest modelled time, waves × (64-k steps of a
-    // CTA × cost of a step + set-up and drain), plus the trip of the partial sums and a second launch where k is cut.
+    // CTA × cost of a step + set-up and drain), plus the trip of the partial sums and a second launch where k is cut. The costs are those of a CTA
+    // per tile, which one round still has; of more rounds the persistent form hides part of what a wave is charged. At 64 rows the choice was within 10 %
+    // of the best at six sizes (2560 → 5120: 13.9 µs, the best 12.6).
     const long long mt = (d.out + 127) / 128 * d.blocks, steps = (d.k[0] + 63) / 64 + (d.k[1] + 63) / 64;
     double best = 1e300;
     for (int nb : {32, 64, 128, 256}) {
@@ -1653,7 +1657,8 @@ void emit_grouped_linear(Emitter& em, const GroupedLinearDesc& d, const TRef& x,
                   "grouped_simt", /*pdl=*/true);
         return;
     }
-    // Rows per tile: whole tiles plus half a tile per group are expected to be filled.
+    // Rows per tile: whole tiles plus half a tile per group are expected to be filled. (The costs count two CTAs per SM up to 128 rows; the four that
+    // tiles of 32 rows may have below are not modelled.)
     const long long mt = (d.out + 127) / 128, steps = (d.k + 63) / 64;
     double best = 1e300;
     for (int nb : {32, 64, 128, 256}) {

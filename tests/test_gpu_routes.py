@@ -51,7 +51,7 @@ def widened(packed, scales, n, nb, zero=8.0):
     return ((q - zero) * scales.astype(np.float64).reshape(n, nb, 1)).astype(scales.dtype).astype(np.float64).reshape(n, nb * 32)
 
 
-@pytest.mark.parametrize("m,k,n", [(257, 1152, 1536), (300, 1000, 200), (513, 136, 4104), (384, 6912, 4760)])
+@pytest.mark.parametrize("m,k,n", [(257, 1152, 1536), (300, 1000, 200), (513, 136, 4104), (384, 6912, 4760), (300, 1152, 29300)])
 def test_many_rows_against_weights_widened_once(m, k, n):
     """Tiles that end inside a tile, k that ends inside a block and inside a step, one and two panels of weights, whole k and pieces of it.
     After one rounding to f16 nearly all outputs equal the f64 sum's (the bound of the other kernel's test), none is further than an ulp of
