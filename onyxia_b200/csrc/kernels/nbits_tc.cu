@@ -628,10 +628,10 @@ bool pieces_apart(const TcP& t, long long m, int count) {
 
 // Whether the weights are widened once, for m rows whose launches of nbits_gemm_tc are `t`. Both sides as sums of what they do, fitted to 459 times of
 // either (51 sizes, k 512 … 21 504, 512 … 61 440 weight rows, 257 … 4096 activation rows: residuals 4 % and 6 %; two other sweeps, of grouped
-// products, 5 … 8 %). With a tenth of margin nothing measured is slower than nbits_gemm_tc alone; 0.631 of its time in the geometric mean, 0.627 with the
-// better of the two at each size. nbits_gemm_tc → widened once, µs, at 257, 1024 and 4096 rows: k 1152, 13 824 weight rows 48 → 39, 109 → 63, 431 → 194; k 2560, 20 480: 99 → (119), 217 → (196), 858 → 574; k 5376, 5376: 58 → (55), 126 → (114), 499 → 322;
-// k 5376, 43 008: 289 → (389), 620 → (795), 2469 → (2388); k 6912, 1152: 39 → 33, 82 → 58, 332 → 99; k 21 504, 5376: 148 → (270), 308 → (430), 1219 → (1282);
-// in brackets: not taken.
+// products, 5 … 8 %). With a tenth of margin nothing measured is slower than nbits_gemm_tc alone; 0.631 of its time in the geometric mean, 0.627 with
+// the better of the two at each size. nbits_gemm_tc → widened once, µs, at 257, 1024 and 4096 rows, in brackets what is not taken: k 1152, 13 824 weight
+// rows 48 → 39, 109 → 63, 431 → 194; k 2560, 20 480: 99 → (119), 217 → (196), 858 → 574; k 5376, 5376: 58 → (55), 126 → (114), 499 → 322; k 5376,
+// 43 008: 289 → (389), 620 → (795), 2469 → (2388); k 6912, 1152: 39 → 33, 82 → 58, 332 → 99; k 21 504, 5376: 148 → (270), 308 → (430), 1219 → (1282).
 bool wide_pays(const TcP& t, long long m) {
     const long long slots = sm_count(), grid = (t.row_tiles + 7) / 8, tail = grid - t.n_full;
     const double out_mb = (double)m * t.row_tiles * 32.0 / 1e6;
