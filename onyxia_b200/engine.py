@@ -45,7 +45,7 @@ class Engine:
         out = np.empty((wanted, self.vocab), dtype=np.float32) if logits else None
         ptr = out.ctypes.data_as(C.POINTER(C.c_float)) if logits else None
         arr = C.cast(words.buffer_info()[0] if spans else C.byref(_ffi.EngineEntry()), C.POINTER(_ffi.EngineEntry))
-        check(self._lib.ox_engine_forward(self._h, arr, len(spans), ptr, out.size if logits else 0))
+        check(self._lib.ox_engine_forward(self._h, arr, len(entries), ptr, out.size if logits else 0))
         return out
 
     def release(self, seq: int) -> None:

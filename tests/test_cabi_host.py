@@ -208,6 +208,27 @@ def test_words_of_bytes_are_their_values():
             words("q", iter([1, 2.5, 3]))
 
 
+def test_entries_reach_the_library_as_they_were_given():
+    """Entries of lists, arrays and bytes, without and with wanted places, as the library reads them; an iterator of entries is refused."""
+    from onyxia_b200.engine import Engine
+    seen = []
+
+    class Library:
+        def ox_engine_forward(self, h, entries, n, logits, cap):
+            seen.append([(e.id, e.tokens[:e.n_tokens], e.want[:e.n_want] if e.n_want else []) for e in entries[:n]])
+            return 0
+
+    engine = Engine.__new__(Engine)
+    engine._lib, engine._h, engine.vocab = Library(), None, 3
+    given = [(7, b"12345678", [1, 7]), (-2, np.array([2 ** 40, 5]), ()), (2 ** 33, [9], b"\0"), (0, (4, 2.0), [])]
+    assert engine.forward(given).shape == (3, 3) and engine.forward(given, logits=False) is None and engine.forward([]).shape == (0, 3)
+    want = [(7, list(b"12345678"), [1, 7]), (-2, [2 ** 40, 5], []), (2 ** 33, [9], [0]), (0, [4, 2], [])]
+    assert seen == [want, want, []]
+    with pytest.raises(TypeError):
+        engine.forward(iter(given))
+    assert len(seen) == 3
+
+
 def test_half_precision_widens_exactly():
     bits = np.arange(65536, dtype=np.uint16)[1:]  # an odd count: a tail behind the eights
     want, got = bits.view(np.float16).astype(np.float32), np.empty(65535, np.float32)
