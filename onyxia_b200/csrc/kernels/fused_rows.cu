@@ -286,8 +286,13 @@ void emit_gelu(Emitter& em, const TRef& x, const TRef& y, bool tanh_approx, cons
             std::lock_guard<std::mutex> lock(mu);
             bool& done = filled[{dev, p.tanh_approx}];
             if (!done) {
-                gelu_fill_lut<<<64, 256>>>(p);
-                done = cudaDeviceSynchronize() == cudaSuccess;
+                // on a stream of its own: waiting for the device would break a graph that another thread is recording
+                cudaStream_t stream = nullptr;
+                if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) == cudaSuccess) {
+                    gelu_fill_lut<<<64, 256, 0, stream>>>(p);
+                    done = cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(stream) == cudaSuccess;
+                    cudaStreamDestroy(stream);
+                }
                 if (!done) cudaGetLastError();
             }
             ready = done;

@@ -1,4 +1,8 @@
 """Kernels that a rule on sizes picks, at the sizes where the rule changes and where their tiles and pieces end."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -173,6 +177,35 @@ def test_gelu_of_every_half():
             got = be.run_once(cuda_backend(), b.finish(), {"x": HostTensor.from_numpy(x), "m": HostTensor.from_numpy(m)})
             outs.append([v.numpy()[:65536] for _, v in got])
         assert np.array_equal(outs[0][0], outs[1][0], equal_nan=True) and np.array_equal(outs[0][1], outs[1][1], equal_nan=True)
+
+
+def test_gelu_beside_another_streams_capture():
+    """The table's first use in a process leaves a graph that is being recorded on another stream as it is."""
+    code = """if True:
+        import numpy as np
+        import torch
+        from onyxia_b200 import backend as be, ir
+        from onyxia_b200.ir import HostTensor
+        n = 1 << 20
+        b = ir.GraphBuilder()
+        b.output("y", b.composite("Gelu", {"approximate": "tanh"}, [b.input("x", ir.F16, [n])], [(ir.F16, [n])])[0])
+        s = be.CudaBackend((0,)).prepare(b.finish())
+        x = s.upload(HostTensor.from_numpy(np.ones(n, np.float16)))
+        t, graph = torch.zeros(4, device="cuda"), torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(torch.cuda.Stream()):
+            graph.capture_begin(capture_error_mode="relaxed")
+            t += 1
+            s.run({"x": x})
+            t += 1
+            graph.capture_end()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert t.tolist() == [2.0] * 4
+    """
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout
 
 
 @pytest.mark.parametrize("heads,kv,d,past,seq,window", [(4, 1, 256, 0, 100, -1), (8, 2, 64, 300, 40, 70), (3, 3, 128, 50, 33, -1), (6, 2, 128, 0, 700, 129),
