@@ -621,6 +621,9 @@ constexpr int kTcPanelA = 128 * 128; // bytes: 128 weight rows × 64 k
 // Rows × k × weight rows: 4096 × 1152 × 13 824 gated 217 → 136 µs (959 TFLOP/s), 2048 × 2560 × 20 480 gated 246 → 201, 2048 × 5376 × 16 896
 // 353 → 347 against a CTA per tile, whose fill and drain stood beside 18, 40 and 84 steps. ONE: as many CTAs as tiles and pieces, which the grid's
 // axes count; the loop's code is not there. 64 rows × 2560 × 5120 cut along k: 14.1 → 13.2 µs against the kernel that had no loop, either.
+// What the loop saves per tile is little beside 256 and more steps, and its tiles are dealt out ahead of time: 5376 weight rows, k 21 504: 1000 rows 248 →
+// 243 µs, 2047 480–497 → 517, 4096 966 → 1036 (a CTA per tile in this form 977), 8192 2193 → 2168; 2560 weight rows, k 16 384: within 3 % either way. Neither k
+// nor the number of rounds tells those sizes apart, so there is no rule for them.
 //
 // What the epilogue does: EPI_PLAIN bias only, EPI_GLU the gated unit, EPI_ACT functions of columns and factors. Kernels of their own: the
 // paths of one are short enough to stay in the instruction cache.
