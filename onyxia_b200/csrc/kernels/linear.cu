@@ -625,6 +625,11 @@ constexpr int kTcPanelA = 128 * 128; // bytes: 128 weight rows × 64 k
 // 243 µs, 2047 480–497 → 517, 4096 966 → 1036 (a CTA per tile in this form 977), 8192 2193 → 2168; 2560 weight rows, k 16 384: within 3 % either way. Neither k
 // nor the number of rounds tells those sizes apart, so there is no rule for them.
 //
+// The warps that copy and that issue products do their steps in few dependent instructions: stage and parity are carried along, descriptors advance by addition, the next
+// stage's barrier is asked before this stage's products are issued. With the step counter divided and reduced by the number of stages (five runtime divisions a step) a
+// step could not take less than 0.36 µs whatever its size: 400 × 5376 × 5376 42.8 → 33.5 µs, 1046 × 2560 × 4160 40.6 → 30.2, 512 × 1152 × 1152 11.8 → 8.5, 64 × 2560 × 4160
+// with its reduction 12.5 → 11.3; 2048 × 5376 × 16 896, bound by what comes to an SM, 329 either way.
+//
 // What the epilogue does: EPI_PLAIN bias only, EPI_GLU the gated unit, EPI_ACT functions of columns and factors. Kernels of their own: the
 // paths of one are short enough to stay in the instruction cache.
 enum : int { EPI_PLAIN, EPI_GLU, EPI_ACT };
@@ -696,71 +701,84 @@ template <int EPI, bool ONE> __global__ void __launch_bounds__(kTcThreads) linea
     bool ok = true;
 
     if (warp == 4) {
-        int done = 0;  // steps so far
+        // Stage and parity are carried along: the divisions of a step counter took longer than the copies of the step.
+        RingAt at;
+        bool round = false;  // the ring's first round waits for nothing
         bool waited = p.groups != 0;
+        const unsigned full = smem_u32(bars), empty = full + S * 8, data = smem_u32(smem);
         for (int t = first; t < total; t += (int)gridDim.x) {
             const Tile q = tile_of(t);
-            if (lane == 0) {
-                const int w0 = (q.group + q.block) * (int)p.out + q.m0, x0 = (int)(p.x_off + q.block * p.x_step);
-                auto load_w = [&](int i) {
-                    const int s = (done + i) % S, c = q.lo + i, op = c >= s0;
-                    mbar_expect_tx(smem_u32(bars + s), (unsigned)stage_bytes);
-                    tma_load_2d(smem_u32(smem + (size_t)s * stage_bytes), p.maps[op * 2 + 1], (op ? c - s0 : c) * 64, w0, smem_u32(bars + s));
-                };
-                auto load_x = [&](int i) {
-                    const int s = (done + i) % S, c = q.lo + i, op = c >= s0;
-                    tma_load_2d(smem_u32(smem + (size_t)s * stage_bytes + kTcPanelA), p.maps[op * 2], (op ? c - s0 : c) * 64 + x0, q.n0, smem_u32(bars + s));
-                };
-                int i = 0;
-                if (!waited) {
-                    const int head = min(S, q.steps);
-                    for (; i < head; i++) load_w(i);  // constants: may overlap the launches before this one
-                    pdl_wait();
-                    for (i = 0; i < head; i++) load_x(i);
-                }
-                for (; ok && i < q.steps; i++) {
-                    const int n = done + i;
-                    if (n >= S && !mbar_wait(smem_u32(bars + S + n % S), ((n / S) - 1) & 1)) {
-                        ok = false;
-                        break;
-                    }
-                    load_w(i);
-                    load_x(i);
-                }
-                done += i;
-            } else if (!waited) {
+            const int w0 = (q.group + q.block) * (int)p.out + q.m0, x0 = (int)(p.x_off + q.block * p.x_step);
+            auto load_w = [&](unsigned s, int i) {
+                const int c = q.lo + i, op = c >= s0;
+                mbar_expect_tx(full + s * 8, (unsigned)stage_bytes);
+                tma_load_2d(data + s * stage_bytes, p.maps[op * 2 + 1], (op ? c - s0 : c) * 64, w0, full + s * 8);
+            };
+            auto load_x = [&](unsigned s, int i) {
+                const int c = q.lo + i, op = c >= s0;
+                tma_load_2d(data + s * stage_bytes + kTcPanelA, p.maps[op * 2], (op ? c - s0 : c) * 64 + x0, q.n0, full + s * 8);
+            };
+            int i = 0;
+            if (!waited) {
+                const int head = min(S, q.steps);
+                if (elect_one())
+                    for (int h = 0; h < head; h++) load_w(h, h);  // constants: may overlap the launches before this one
+                __syncwarp();
                 pdl_wait();
+                for (; i < head; i++) {
+                    if (elect_one()) load_x(i, i);
+                    __syncwarp();
+                    at.next(S);
+                }
+                round = head == S;
+                waited = true;
             }
-            waited = true;
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) break;
+            for (; i < q.steps; i++) {
+                if (round && !mbar_wait(empty + at.s * 8, at.parity ^ 1)) {
+                    ok = false;
+                    break;
+                }
+                if (elect_one()) {
+                    load_w(at.s, i);
+                    load_x(at.s, i);
+                }
+                __syncwarp();
+                at.next(S);
+                if (at.s == 0) round = true;
+            }
+            if (!__all_sync(0xffffffffu, ok)) break;
         }
         // every copy has landed before this CTA's shared memory can be given away
-        if (lane == 0)
-            for (int n = max(0, done - S); n < done; n++)
-                if (!mbar_wait(smem_u32(bars + n % S), (n / S) & 1)) ok = false;
+        for (unsigned n = 0; n < (round ? (unsigned)S : at.s); n++)
+            if (!mbar_wait(full + n * 8, n < at.s ? at.parity : at.parity ^ 1)) ok = false;
     } else if (warp == 5) {
         pdl_wait();
         const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(nb >> 3) << 17) | (8u << 24);  // bf16 × bf16 → f32, M 128 × N nb
-        int n = 0, j = 0;
+        RingAt at;
+        bool ready = false;
+        int j = 0;
+        const unsigned full = smem_u32(bars), empty = full + S * 8, step16 = (unsigned)stage_bytes >> 4;
+        const unsigned long long a0 = umma_kmajor_desc(smem_u32(smem)), b0 = umma_kmajor_desc(smem_u32(smem) + kTcPanelA);
         for (int t = first; t < total; t += (int)gridDim.x, j++) {
             const int piece = ONE ? (int)blockIdx.z : t / row_tiles / p.out_tiles, steps = (int)((unsigned)(all * (piece + 1)) / (unsigned)p.splits) - (int)((unsigned)(all * piece) / (unsigned)p.splits);
             const unsigned d = tmem + (unsigned)((j & 1) * nb);
             if (!ONE && j >= 2 && ok && !mbar_wait(read + (j & 1) * 8, ((j >> 1) - 1) & 1)) ok = false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int i = 0; i < steps; i++, n++) {
-                const int s = n % S;
-                if (ok && !mbar_wait(smem_u32(bars + s), (n / S) & 1)) ok = false;
+            for (int i = 0; i < steps; i++) {
+                if (ok && !ready && !mbar_wait(full + at.s * 8, at.parity)) ok = false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (lane == 0 && ok) {
-                    const unsigned a0 = smem_u32(smem + (size_t)s * stage_bytes), b0 = a0 + kTcPanelA;
+                const unsigned long long a = a0 + at.s * step16, b = b0 + at.s * step16;  // descriptors count in 16 bytes
+                const unsigned done = empty + at.s * 8;
+                at.next(S);
+                ready = mbar_test(full + at.s * 8, at.parity);  // the answer is there when the products have been issued
+                if (elect_one() && ok) {
 #pragma unroll
-                    for (int e = 0; e < 4; e++) umma_bf16(d, umma_kmajor_desc(a0 + e * 32), umma_kmajor_desc(b0 + e * 32), idesc, i > 0 || e > 0);
-                    umma_commit(smem_u32(bars + S + s));
+                    for (int e = 0; e < 4; e++) umma_bf16(d, a + e * 2, b + e * 2, idesc, i > 0 || e > 0);
+                    umma_commit(done);
                 }
                 __syncwarp();
             }
-            if (lane == 0) umma_commit(finished + (j & 1) * 8);
+            if (elect_one()) umma_commit(finished + (j & 1) * 8);
             __syncwarp();
         }
     } else {

@@ -25,6 +25,16 @@ __device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
         : "memory");
     return ok != 0;
 }
+// Whether the phase is complete now: try_wait may hold the thread for microseconds.
+__device__ __forceinline__ bool mbar_test(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 // False when the phase did not complete within about a second.
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
     if (mbar_try(bar, parity)) return true;
@@ -33,6 +43,24 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
         if (mbar_try(bar, parity)) return true;
     return false;
 }
+
+// One lane of a converged warp. The compiler knows that its branch is taken by one lane: operands that have to be in uniform registers (copies,
+// matrix instructions, their barriers) get there without a loop over lanes.
+__device__ __forceinline__ bool elect_one() {
+    unsigned p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
+}
+// A place in a ring of `n` stages and the parity of its current round.
+struct RingAt {
+    unsigned s = 0, parity = 0;
+    __device__ __forceinline__ void next(unsigned n) {
+        if (++s == n) {
+            s = 0;
+            parity ^= 1;
+        }
+    }
+};
 
 // ── TMA: one 2-D tile; x must keep the copy on a 16-byte boundary ──
 __device__ __forceinline__ void tma_load_2d(unsigned dst, const void* map, int x, int y, unsigned bar) {
