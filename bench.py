@@ -442,7 +442,7 @@ def lovuzen_costs(cfg, rows, seqs, past, wanted):
     return {"linear": (lin_b, lin_f), "attn": (att_b, att_f), "gates": (gate_b, gate_f), "scan": (scan_b, 0), "norm": (norm_b, 0)}
 
 
-_FAMILY = {"linear_stream": "linear", "linear_flow": "linear", "linear_tc": "linear", "linear_reduce": "linear", "linear_simt": "linear",
+_FAMILY = {"linear_stream": "linear", "linear_flow": "linear", "linear_tc": "linear", "linear_pair": "linear", "linear_reduce": "linear", "linear_simt": "linear",
            "paged_attn_prefill": "attn", "paged_attn_decode": "attn", "paged_attn_simt": "attn", "recurrence_step": "gates",
            "recurrence_gates": "gates", "recurrence_scan": "scan", "residual_norm": "norm",
            "linear_rows_f32": "linear", "linear_f32": "linear", "nbits_widen": "linear", "nbits_gemm_wide": "linear",
@@ -583,7 +583,7 @@ def kipizen_costs(cfg, rows, seqs, past, wanted):
 
 _FAMILY.update({"paged_kv_prefill": "attn", "paged_kv_decode": "attn", "paged_kv_simt": "attn", "lightning_step": "lightning_step",
                 "lightning_chunk": "lightning_chunks", "lightning_scan": "lightning_chunks", "lightning_out": "lightning_chunks",
-                "moe_stream_up": "experts", "moe_stream_down": "experts", "grouped_tc": "experts", "moe_top": "routing", "moe_route": "routing", "moe_sort": "routing",
+                "moe_stream_up": "experts", "moe_stream_down": "experts", "grouped_tc": "experts", "grouped_pair": "experts", "moe_top": "routing", "moe_route": "routing", "moe_sort": "routing",
                 "moe_combine": "routing"})
 
 

@@ -9,118 +9,25 @@
 //   linear_tc       more rows: tcgen05 GEMM. Weights are the MMA's A operand (128 rows), activations its B operand
 //                   (32–256 rows), both loaded by TMA into 128-byte-swizzled stages; accumulator in tensor memory.
 //                   Grids that would leave SMs idle are cut along k; `linear_reduce` adds the pieces in order.
+//   linear_pair     products of many rows and groups of many rows (linear_pair.cu).
 //   linear_rows_f32 f32 (true 32-bit), up to 32 rows and k of 512 and more: warps stream whole weight rows.
 //   linear_f32      f32, more rows or shorter k: register-blocked tiles.
 //   linear_simt     f32 of short k, and f32 and bf16 shapes whose rows are not 16-byte aligned.
 //
-// linear_tc, linear_f32 and linear_simt also run grouped: activation rows sorted by group, one weight matrix per group, the groups'
+// linear_tc, linear_pair, linear_f32 and linear_simt also run grouped: activation rows sorted by group, one weight matrix per group, the groups'
 // row counts known on the device only. A CTA finds its group from the counts; the grid covers the most tiles
 // that any counts can give.
 //
 // Bytes per launch: out · k · 2 once per 256 activation rows; FLOPs 2 · rows · out · k.
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 
-#include "tc_util.cuh"
+#include "linear.cuh"
 
 namespace oxk {
 
 namespace {
-
-struct LinP {
-    alignas(64) unsigned char maps[4][128];  // x0, w0, x1, w1 (linear_tc)
-    const void* x[2];
-    const void* w[2];
-    const float* bias;
-    void* y;
-    float* partial;
-    ErrWord* err;
-    // residual norm (linear_stream prologue)
-    const void* ny;
-    const float *nw, *ngain, *nres;
-    const bf16* ngate;
-    const float *npost, *noffset;
-    const void* nadd;
-    float* stream;
-    bf16* low;
-    long long gate_ld, ny_ld;
-    float eps, y_scale, add_scale;
-    int ny_bf16, pre, add_bf16, streams, norm_groups;
-    const float *connect, *npost2;
-    const void* ny2;
-    long long rows, out, k[2];
-    // block-diagonal products: x rows are ldx apart, block b reads its columns from x_off + b · x_step on; y rows are ldy apart
-    const void* mul;
-    long long ldx, x_off, x_step, ldy, mul_ld;
-    int blocks;
-    int y_bf16, fast, glu;  // fast: the operands are bf16
-    float alpha, limit, shift;
-    int act[2];           // functions of the columns before and from act_split on; none from act_end on
-    long long act_split, act_end;
-    int nb, stages, splits, node;  // linear_tc
-    int row_tiles, out_tiles;      // tiles of activation rows (not grouped) and of weight rows
-    const int* counts;    // grouped: rows of every group
-    int groups;
-};
-
-// Grouped: the `tile`-th tile of `size` rows, counted group by group → its group, first row and rows. Called by whole warps.
-__device__ __forceinline__ bool locate_group(const LinP& p, int tile, int size, int* group, int* row, int* live) {
-    const int lane = threadIdx.x & 31;
-    int tiles = 0, rows = 0;
-    for (int g0 = 0; g0 < p.groups; g0 += 32) {
-        const int n = g0 + lane < p.groups ? p.counts[g0 + lane] : 0, mine = (n + size - 1) / size;
-        int t_inc = mine, r_inc = n;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, t_inc, o), r = __shfl_up_sync(0xffffffffu, r_inc, o);
-            if (lane >= o) {
-                t_inc += t;
-                r_inc += r;
-            }
-        }
-        const unsigned hit = __ballot_sync(0xffffffffu, tiles + t_inc > tile);
-        if (hit) {
-            const int at = __ffs(hit) - 1;
-            const int count = __shfl_sync(0xffffffffu, n, at);
-            const int first = (tile - tiles - (__shfl_sync(0xffffffffu, t_inc, at) - __shfl_sync(0xffffffffu, mine, at))) * size;
-            *group = g0 + at;
-            *row = rows + __shfl_sync(0xffffffffu, r_inc, at) - count + first;
-            *live = min(size, count - first);
-            return true;
-        }
-        tiles += __shfl_sync(0xffffffffu, t_inc, 31);
-        rows += __shfl_sync(0xffffffffu, r_inc, 31);
-    }
-    return false;
-}
-
-// Grouped: tiles of `size` rows over all groups. Called by whole warps.
-__device__ __forceinline__ int count_tiles(const LinP& p, int size) {
-    int tiles = 0;
-    for (int g = threadIdx.x & 31; g < p.groups; g += 32) tiles += (p.counts[g] + size - 1) / size;
-    return __reduce_add_sync(0xffffffffu, tiles);
-}
-
-__device__ __forceinline__ float glu_value(const LinP& p, float gate, float up) {
-    const float g = fminf(gate, p.limit), u = fminf(fmaxf(up, -p.limit), p.limit);
-    return g * (p.y_bf16 ? sigmoid_fast(p.alpha * g) : sigmoid_f(p.alpha * g)) * (u + p.shift);
-}
-// act: per column range
-__device__ __forceinline__ float activate(const LinP& p, long long col, float v) {
-    const int f = col < p.act_end ? p.act[col >= p.act_split] : ACT_NONE;
-    if (f == ACT_NONE) return v;
-    if (f == ACT_SOFTPLUS) return p.fast ? softplus_fast(v) : softplus_f(v);
-    const float s = p.y_bf16 ? sigmoid_fast(v) : sigmoid_f(v);
-    return f == ACT_SILU ? v * s : s;
-}
-// The factor of a block-diagonal product's result; the matrix has the weights' type.
-template <typename T> __device__ __forceinline__ float factor(const LinP& p, long long row, long long col) {
-    return p.mul ? to_f(((const T*)p.mul)[row * p.mul_ld + col]) : 1.f;
-}
-__device__ __forceinline__ void put(const LinP& p, long long row, long long width, long long col, float v) {
-    if (p.y_bf16) ((bf16*)p.y)[row * width + col] = __float2bfloat16_rn(v);
-    else ((float*)p.y)[row * width + col] = v;
-}
 
 // ───────────────────────────── decode ───────────────────────────────────
 constexpr int kStreamWarps = 8, kThreads = kStreamWarps * 32;
@@ -617,22 +524,14 @@ constexpr int kTcThreads = 192;      // warps 0-3 epilogue, 4 TMA, 5 MMA
 constexpr int kTcPanelA = 128 * 128; // bytes: 128 weight rows × 64 k
 
 // A persistent CTA works through tiles (piece of k slowest, activation tiles fastest: they share a weight tile while it is in L2); loads and
-// MMAs run on into the next tile while the epilogue of the last one empties the other of two accumulators.
-// Rows × k × weight rows: 4096 × 1152 × 13 824 gated 217 → 136 µs (959 TFLOP/s), 2048 × 2560 × 20 480 gated 246 → 201, 2048 × 5376 × 16 896
-// 353 → 347 against a CTA per tile, whose fill and drain stood beside 18, 40 and 84 steps. ONE: as many CTAs as tiles and pieces, which the grid's
-// axes count; the loop's code is not there. 64 rows × 2560 × 5120 cut along k: 14.1 → 13.2 µs against the kernel that had no loop, either.
-// What the loop saves per tile is little beside 256 and more steps, and its tiles are dealt out ahead of time: 5376 weight rows, k 21 504: 1000 rows 248 →
-// 243 µs, 2047 480–497 → 517, 4096 966 → 1036 (a CTA per tile in this form 977), 8192 2193 → 2168; 2560 weight rows, k 16 384: within 3 % either way. Neither k
-// nor the number of rounds tells those sizes apart, so there is no rule for them.
+// MMAs run on into the next tile while the epilogue of the last one empties the other of two accumulators. ONE: as many CTAs as tiles and pieces, which the
+// grid's axes count; the loop's code is not there. 64 rows × 2560 × 5120 cut along k: 14.1 → 13.2 µs against the kernel that had no loop. Most products with more tiles than
+// that belong to pairs of CTAs (linear_pair.cu); here remain those of few rows, of groups of few rows, and block-diagonal ones.
 //
 // The warps that copy and that issue products do their steps in few dependent instructions: stage and parity are carried along, descriptors advance by addition, the next
 // stage's barrier is asked before this stage's products are issued. With the step counter divided and reduced by the number of stages (five runtime divisions a step) a
 // step could not take less than 0.36 µs whatever its size: 400 × 5376 × 5376 42.8 → 33.5 µs, 1046 × 2560 × 4160 40.6 → 30.2, 512 × 1152 × 1152 11.8 → 8.5, 64 × 2560 × 4160
 // with its reduction 12.5 → 11.3; 2048 × 5376 × 16 896, bound by what comes to an SM, 329 either way.
-//
-// What the epilogue does: EPI_PLAIN bias only, EPI_GLU the gated unit, EPI_ACT functions of columns and factors. Kernels of their own: the
-// paths of one are short enough to stay in the instruction cache.
-enum : int { EPI_PLAIN, EPI_GLU, EPI_ACT };
 template <int EPI, bool ONE> __global__ void __launch_bounds__(kTcThreads) linear_tc(const __grid_constant__ LinP p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -1592,38 +1491,74 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
                   flow ? "linear_flow" : "linear_stream", /*pdl=*/true);
         return;
     }
-    // Activation rows per tile and pieces along k: the choice with the smallest modelled time, waves × (64-k steps of a
-    // CTA × cost of a step + set-up and drain), plus the trip of the partial sums and a second launch where k is cut. The costs are those of a CTA
-    // per tile, which one round still has; of more rounds the persistent form hides part of what a wave is charged. At 64 rows the choice was within 10 %
-    // of the best at six sizes (2560 → 5120: 13.9 µs, the best 12.6).
+    // Which kernel, activation rows per tile and pieces along k: the choice with the smallest modelled time. A CTA alone on its SM has a step of 64 k in `one` µs,
+    // waves of two (up to 128 rows) in `two`; epilogues grow with the tile; where k is cut, the trip of the partial sums and a second launch are added. The
+    // constants are fitted to 560 launches of 45 sizes (64 … 4096 rows, k 16 … 10 240, 1152 … 32 768 weight rows): of one of them (200 × 2560 × 4096, 10 %) is the choice
+    // more than 3 % behind the best form.
     const long long mt = (d.out + 127) / 128 * d.blocks, steps = (d.k[0] + 63) / 64 + (d.k[1] + 63) / 64;
     double best = 1e300;
     for (int nb : {32, 64, 128, 256}) {
         if (nb > 32 && nb / 2 >= d.rows) break;
         const int resident = nb <= 128 ? 2 : 1;
-        const long long slots = (long long)sm_count() * resident, tiles = mt * ((d.rows + nb - 1) / nb);
+        const long long tiles = mt * ((d.rows + nb - 1) / nb);
+        const double one = nb == 32 ? 0.19 : nb == 64 ? 0.21 : nb == 128 ? 0.24 : 0.35, two = nb == 32 ? 0.21 : nb == 64 ? 0.285 : nb == 128 ? 0.4 : 0.34;
+        const double epilogue = 5.8 * nb / 256;
         for (int sp = 1; sp <= (d.rows < 65536 ? 16 : 1) && sp * 2 <= std::max<long long>(steps, 2); sp++) {
-            const long long waves = (tiles * sp + slots - 1) / slots;
-            // measured: a 64-k step of the CTAs that share an SM, and what a wave costs besides its steps
-            const double step_us = nb == 32 ? 0.36 : nb == 64 ? 0.38 : nb == 128 ? 0.42 : 0.45;
-            double us = (double)waves * ((double)((steps + sp - 1) / sp) * step_us + (nb == 256 ? 10.0 : 7.0));
-            if (sp > 1) us += 3.0 + (double)(sp + 1) * d.rows * p.ldy * 4.0 / 3e6;
-            if (us < best * (sp > 1 ? 0.97 : 1.0)) {
+            const long long waves = (tiles * sp + sm_count() * resident - 1) / (sm_count() * resident), piece = (steps + sp - 1) / sp;
+            double us = 4.1 + (tiles * sp <= sm_count() ? piece * one + 0.9 + epilogue : waves * (piece * two + 0.9 + epilogue / 2) + epilogue / 2);
+            if (sp > 1) us += 1.4 + (double)(sp + 1) * d.rows * p.ldy * 4.0 / 5.6e6;
+            if (us < best) {
                 best = us;
                 p.nb = nb;
                 p.splits = sp;
             }
         }
     }
-    if (const char* e = std::getenv("ONYXIA_LINEAR_TILE")) {  // diagnostics: "rows,pieces"
-        int nb = 0, sp = 0;
-        if (std::sscanf(e, "%d,%d", &nb, &sp) == 2 && (nb == 32 || nb == 64 || nb == 128 || nb == 256) && sp >= 1 && sp <= 16 && sp * 2 <= std::max<long long>(steps, 2)) {
+    // Pairs of CTAs: a step is bound by the bytes that come to an SM, 128 weight rows and half a tile's activation rows. Any multiple of 16 rows, so that the last round
+    // of tiles is as full as the others.
+    bool pair = false;
+    for (int nb = 256; nb >= 64 && !blocks; nb -= 16) {
+        const double rounds = std::ceil((double)((d.rows + nb - 1) / nb * ((d.out + 255) / 256)) / (sm_count() / 2)), us = pair_us(rounds, steps, nb);
+        if (us < best) {
+            best = us;
+            pair = true;
             p.nb = nb;
-            p.splits = sp;
+            p.splits = 1;
         }
     }
-    const size_t stage = kTcPanelA + (size_t)p.nb * 128;
+    if (const char* e = std::getenv("ONYXIA_LINEAR_TILE")) {  // diagnostics: "rows,pieces"; no pieces: pairs of CTAs
+        int nb = 0, sp = 0;
+        if (std::sscanf(e, "%d,%d", &nb, &sp) == 2 && (nb == 32 || nb == 64 || nb == 128 || nb == 256) && sp >= 1 && sp <= 16 && sp * 2 <= std::max<long long>(steps, 2)) {
+            pair = false;
+            p.nb = nb;
+            p.splits = sp;
+        } else if (!blocks && sp == 0 && nb >= 16 && nb <= 256 && nb % 16 == 0) {
+            pair = true;
+            p.nb = nb;
+            p.splits = 1;
+        }
+    }
+    auto add_maps = [&](LaunchRec& rec, uint32_t box) {
+        auto add = [&](int i, const Buf& b, int64_t k, int64_t rows, uint32_t high) {
+            rec.tmaps.push_back(TmapReloc{(uint32_t)(offsetof(LinP, maps) + 128 * i), b, (uint64_t)k, (uint64_t)rows, (uint64_t)k * 2, 64u, high});
+        };
+        add(0, bx0, blocks ? ldx : d.k[0], d.rows, box);
+        add(1, w0.buf, d.k[0], d.blocks * d.out, 128u);
+        if (d.k[1]) {
+            add(2, bx1, d.k[1], d.rows, box);
+            add(3, bw1, d.k[1], d.out, 128u);
+        }
+    };
     p.row_tiles = (int)((d.rows + p.nb - 1) / p.nb);
+    if (pair) {
+        p.out_tiles = (int)((d.out + 255) / 256);
+        p.box = p.nb / 2;
+        add_maps(launch_pair(em, p, d.glu ? EPI_GLU : d.act[0] || d.act[1] ? EPI_ACT : EPI_PLAIN,
+                             {{&p.bias, bb}, {&p.y, y.buf}, {&p.mul, kNull}, {&p.err, Buf{kSlotErr, 0}}}, y.buf.off, "linear_pair"),
+                 (uint32_t)p.box);
+        return;
+    }
+    const size_t stage = kTcPanelA + (size_t)p.nb * 128;
     p.out_tiles = (int)mt;
     const long long tiles = mt * p.row_tiles * p.splits;
     if (tiles >= INT32_MAX) throw std::runtime_error("onyxia.Linear: too many tiles");
@@ -1639,15 +1574,7 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
     const Buf partial = p.splits > 1 ? em.scratch((size_t)p.splits * d.rows * p.ldy * 4) : kNull;
     LaunchRec& rec = em.launch(kernel, one ? dim3((unsigned)p.row_tiles, (unsigned)mt, (unsigned)p.splits) : dim3((unsigned)slots), dim3(kTcThreads), (unsigned)smem, p,
                                {{&p.bias, bb}, {&p.y, y.buf}, {&p.mul, mul}, {&p.partial, partial}, {&p.err, Buf{kSlotErr, 0}}}, "linear_tc", /*pdl=*/true);
-    auto add_map = [&](int i, const Buf& b, int64_t k, int64_t rows, uint32_t box) {
-        rec.tmaps.push_back(TmapReloc{(uint32_t)(offsetof(LinP, maps) + 128 * i), b, (uint64_t)k, (uint64_t)rows, (uint64_t)k * 2, 64u, box});
-    };
-    add_map(0, bx0, blocks ? ldx : d.k[0], d.rows, (uint32_t)p.nb);
-    add_map(1, w0.buf, d.k[0], d.blocks * d.out, 128u);
-    if (d.k[1]) {
-        add_map(2, bx1, d.k[1], d.rows, (uint32_t)p.nb);
-        add_map(3, bw1, d.k[1], d.out, 128u);
-    }
+    add_maps(rec, (uint32_t)p.nb);
     if (p.splits > 1) reduce(partial);
 }
 
@@ -1678,24 +1605,45 @@ void emit_grouped_linear(Emitter& em, const GroupedLinearDesc& d, const TRef& x,
                   "grouped_simt", /*pdl=*/true);
         return;
     }
-    // Rows per tile: whole tiles plus half a tile per group are expected to be filled. (The costs count two CTAs per SM up to 128 rows; the four that
-    // tiles of 32 rows may have below are not modelled.)
+    // Rows per tile: a group of so many rows that they spread over more than a tile is expected to fill whole tiles and half a one. The costs are those of
+    // emit_linear; tiles of 32 rows may have four CTAs per SM below, which is not modelled. Of 16 groups, k 1152 → 3456 gated: pairs of CTAs from 100 rows per group on (160:
+    // 45 → 36 µs, 1024: 143 → 114); k 1728 → 1152, from 250 (33 → 28; 160 rows would take 25 against 23); k 2560 → 4096 gated, from 62 (74 → 66).
     const long long mt = (d.out + 127) / 128, steps = (d.k + 63) / 64;
+    const double met = (double)std::min(d.groups, d.rows), mean = (double)d.rows / met;
+    auto parts = [&](double nb) { return mean + 2.0 * std::sqrt(mean) <= nb ? 1.0 : mean / nb + 0.5; };
     double best = 1e300;
     for (int nb : {32, 64, 128, 256}) {
-        const long long slots = (long long)sm_count() * (nb <= 128 ? 2 : 1);
-        const double groups = (double)std::min(d.groups, d.rows), tiles = std::max(groups, (double)d.rows / nb + 0.5 * groups);
-        const double step_us = nb == 32 ? 0.36 : nb == 64 ? 0.38 : nb == 128 ? 0.42 : 0.45;
-        const double waves = std::max(1.0, tiles * (double)mt / (double)slots);
-        const double us = waves * ((double)steps * step_us + (nb == 256 ? 10.0 : 7.0));
+        const double two = nb == 32 ? 0.21 : nb == 64 ? 0.285 : nb == 128 ? 0.4 : 0.34, epilogue = 5.8 * nb / 256;
+        const double waves = std::ceil(met * parts(nb) * (double)mt / (double)(sm_count() * (nb <= 128 ? 2 : 1)));
+        const double us = 4.1 + waves * ((double)steps * two + 0.9 + epilogue / 2) + epilogue / 2;
         if (us < best) {
             best = us;
             p.nb = nb;
         }
     }
-    if (const char* e = std::getenv("ONYXIA_GROUPED_TILE")) {  // diagnostics: rows
+    const double pair_rounds = std::max(1.0, met * parts(256) * (double)((d.out + 255) / 256) / (sm_count() / 2) + 0.5);
+    bool pair = pair_us(pair_rounds, steps, mean / parts(256)) < best;
+    if (pair) p.nb = 256;
+    if (const char* e = std::getenv("ONYXIA_GROUPED_TILE")) {  // diagnostics: rows; below zero: pairs of CTAs
         const int nb = std::atoi(e);
-        if (nb == 32 || nb == 64 || nb == 128 || nb == 256) p.nb = nb;
+        pair = nb < 0 && nb >= -256 && nb % 16 == 0;
+        if (pair || nb == 32 || nb == 64 || nb == 128 || nb == 256) p.nb = std::abs(nb);
+    }
+    auto add_maps = [&](LaunchRec& rec, uint32_t box) {
+        auto add = [&](int i, const Buf& b, int64_t rows, uint32_t high) {
+            rec.tmaps.push_back(TmapReloc{(uint32_t)(offsetof(LinP, maps) + 128 * i), b, (uint64_t)d.k, (uint64_t)rows, (uint64_t)d.k * 2, 64u, high});
+        };
+        add(0, x.buf, d.rows, box);
+        add(1, w.buf, d.groups * d.out, 128u);
+    };
+    if (pair) {
+        p.out_tiles = (int)((d.out + 255) / 256);
+        p.row_tiles = (int)tiles_of(p.nb);  // at most
+        p.box = 32;
+        add_maps(launch_pair(em, p, d.glu ? EPI_GLU : EPI_PLAIN,
+                             {{&p.bias, kNull}, {&p.y, y.buf}, {&p.mul, kNull}, {&p.err, Buf{kSlotErr, 0}}, {&p.counts, counts.buf}}, y.buf.off, "grouped_pair"),
+                 (uint32_t)p.box);
+        return;
     }
     const size_t stage = kTcPanelA + (size_t)p.nb * 128;
     p.out_tiles = (int)mt;
@@ -1715,11 +1663,7 @@ void emit_grouped_linear(Emitter& em, const GroupedLinearDesc& d, const TRef& x,
     LaunchRec& rec = em.launch(kernel, grid, dim3(kTcThreads), (unsigned)smem, p,
                                {{&p.bias, kNull}, {&p.y, y.buf}, {&p.partial, kNull}, {&p.err, Buf{kSlotErr, 0}}, {&p.counts, counts.buf}}, "grouped_tc",
                                /*pdl=*/true);
-    auto add_map = [&](int i, const Buf& b, int64_t rows, uint32_t box) {
-        rec.tmaps.push_back(TmapReloc{(uint32_t)(offsetof(LinP, maps) + 128 * i), b, (uint64_t)d.k, (uint64_t)rows, (uint64_t)d.k * 2, 64u, box});
-    };
-    add_map(0, x.buf, d.rows, (uint32_t)p.nb);
-    add_map(1, w.buf, d.groups * d.out, 128u);
+    add_maps(rec, (uint32_t)p.nb);
 }
 
 }  // namespace oxk

@@ -237,6 +237,44 @@ def test_bf16_products_of_several_rounds_per_cta(rows, k, k1, n):
         assert rel_err(run_linear(ir.BF16, x, w, bias=bias, glu=(1.7, 2.0, 1.0)), g / (1 + np.exp(-1.7 * g)) * (u + 1)) < 3e-6
 
 
+@pytest.mark.parametrize("rows,k,k1,n,out", [(257, 1160, 0, 13830, ir.F32), (700, 72, 0, 9001, ir.BF16), (1999, 1152, 136, 2370, ir.BF16), (2048, 16, 0, 2560, ir.F32), (3001, 520, 0, 1536, ir.BF16)])
+def test_bf16_products_by_pairs_of_ctas(rows, k, k1, n, out):
+    """Tiles that end inside a CTA's weight rows or in the first CTA of a pair, odd columns, last tiles of few rows, a k below one step, a second operand inside the ring,
+    tiles of sizes between the powers of two, several rounds. Products are exact; f32 sums as above, a bf16 result is off by half a unit of eight digits."""
+    r = np.random.default_rng(rows)
+    x, w, more = to_bf16(r.standard_normal((rows, k))), to_bf16(r.standard_normal((n, k)) / np.sqrt(k)), {}
+    z = x.astype(np.float64) @ w.T.astype(np.float64)
+    if k1:
+        more = {"x1": to_bf16(r.standard_normal((rows, k1))), "w1": to_bf16(r.standard_normal((n, k1)) / np.sqrt(k))}
+        z = z + more["x1"].astype(np.float64) @ more["w1"].T.astype(np.float64)
+    b = ir.GraphBuilder()
+    b.output("y", b.composite("onyxia.Linear", {}, [b.input("x", ir.BF16, [rows, k]), b.constant(act(w, ir.BF16))], [(out, [rows, n])])[0])
+    assert kernels_of(b.finish(), {"x": act(x, ir.BF16)}) == {"linear_pair"}
+    bias = to_bf16(r.standard_normal(n))
+    assert rel_err(run_linear(ir.BF16, x, w, bias=bias, out_dtype=out, **more).astype(np.float64), z + bias) < (2e-6 if out == ir.F32 else 2.0 ** -9)
+    if n % 2 == 0 and not k1:
+        g, u = np.minimum(z[:, ::2], 2.0), np.clip(z[:, 1::2], -2.0, 2.0)
+        assert rel_err(run_linear(ir.BF16, x, w, glu=(1.7, 2.0, 1.0), out_dtype=out).astype(np.float64), g / (1 + np.exp(-1.7 * g)) * (u + 1)) < (3e-6 if out == ir.F32 else 2.0 ** -9)
+    b, z = ir.GraphBuilder(), x.astype(np.float64) @ w.T.astype(np.float64)
+    attrs = {"act": "silu", "act_rest": "softplus", "act_split": n // 3, "act_end": n - 5}
+    b.output("y", b.composite("onyxia.Linear", attrs, [b.input("x", ir.BF16, [rows, k]), b.constant(act(w, ir.BF16))], [(out, [rows, n])])[0])
+    z[:, :n // 3] /= 1 + np.exp(-z[:, :n // 3])
+    z[:, n // 3:n - 5] = np.log1p(np.exp(z[:, n // 3:n - 5]))
+    got = be.run_once(cuda_backend(), b.finish(), {"x": act(x, ir.BF16)})[0][1].numpy().astype(np.float64)
+    assert rel_err(got, z) < (3e-6 if out == ir.F32 else 2.0 ** -9)
+
+
+@pytest.mark.parametrize("n,experts,top,width,ff", [(700, 3, 2, 1160, 1100), (1500, 5, 1, 1160, 1096), (600, 4, 4, 264, 1700), (4000, 40, 2, 264, 1100)])
+def test_experts_by_pairs_of_ctas(n, experts, top, width, ff):
+    """Groups of a few parts each, some of hardly a row more than a tile, more groups than a warp's search takes at once."""
+    m = Experts("bf16", width, experts, top, ff)
+    h = m.rows(n)
+    m.check(h)
+    m.s.enable_profiling(True)
+    m.check(h)
+    assert "grouped_pair" in {kernel for kernel, _, _ in m.s.take_timings()}
+
+
 @pytest.mark.parametrize("d,past,seq,window", [(64, 240, 33, -1), (128, 100, 300, 250), (256, 300, 20, 150)])
 def test_kept_scores_with_values_that_are_not_finite(d, past, seq, window):
     """Rows whose visible scores are NaN, all minus infinity, or infinite in part, and a NaN among the keys: kept scores (two heads per key head) give
