@@ -35,8 +35,8 @@
 #include <cstdio>
 #include <cstdlib>
 
-#include "common.cuh"
 #include "kernels.hpp"
+#include "tc_util.cuh"
 
 namespace oxk {
 
@@ -47,7 +47,6 @@ constexpr int kMmaWarp = kProducerWarps;  // the warp that issues the MMAs
 constexpr int kThreadsTc = (kMmaWarp + 1) * 32;
 constexpr int kTileWt = 1024, kTileSt = 128, kTileZt = 64;
 constexpr int kPanelA = 128 * 128;  // bytes: 128 rows × 64 k of f16
-constexpr long long kWaitCyclesTc = 2000000000LL;
 
 struct TcP {
     alignas(64) unsigned char xmap[128];  // tensor map over the activations [M, K] (box 64 k × mb rows), when use_tma
@@ -68,23 +67,7 @@ struct TcP {
     long long n_pad;             // weight rows of the tail blocks (128 per block)
 };
 
-__device__ __forceinline__ unsigned s_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool bar_try_tc(unsigned bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool bar_wait_tc(unsigned bar, unsigned parity) {
-    if (bar_try_tc(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (clock64() - t0 < kWaitCyclesTc)
-        if (bar_try_tc(bar, parity)) return true;
-    return false;
-}
+__device__ __forceinline__ unsigned s_addr(const void* p) { return smem_u32(p); }
 __device__ __forceinline__ void bar_arrive(unsigned bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -111,10 +94,8 @@ __device__ __forceinline__ uint4 widen_tc(unsigned w, __half2 sub_lo, __half2 ad
     return o;
 }
 
-// Shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1 024 bytes apart.
-__device__ __forceinline__ unsigned long long umma_desc(unsigned smem_byte_addr) {
-    return (unsigned long long)((smem_byte_addr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
+// f16 × f16 → f32, one CTA.
+__device__ __forceinline__ void umma_f16(unsigned d, unsigned long long a, unsigned long long b, unsigned idesc, bool accumulate) { umma_bf16(d, a, b, idesc, accumulate); }
 
 __global__ void __launch_bounds__(kThreadsTc, 2) nbits_gemm_tc(const __grid_constant__ TcP p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -126,8 +107,6 @@ __global__ void __launch_bounds__(kThreadsTc, 2) nbits_gemm_tc(const __grid_cons
     const int stage_bytes = 2 * kPanelA + 2 * panel_b;  // A panels, then B panels
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + (size_t)S * stage_bytes);  // full[S], empty[S], done
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * S + 1);
-
-    pdl_enter();
 
     if (tid == 0) {
         for (int s = 0; s < S; s++) {
@@ -149,6 +128,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2) nbits_gemm_tc(const __grid_cons
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned tmem = *tmem_slot;
+    pdl_trigger();  // the tensor memory is taken: what starts now may wait for it, but does not keep it from this kernel
 
     // CTAs 0 … n_full − 1 own a whole row block; the ones after them share the tail blocks, `splits` CTAs each
     const int tail_j = (int)blockIdx.x - p.n_full;
@@ -186,10 +166,13 @@ __global__ void __launch_bounds__(kThreadsTc, 2) nbits_gemm_tc(const __grid_cons
             }
             return r;
         };
-        Rec next = fetch(0);
+        Rec next = fetch(0);  // weights are constants: may overlap the launches before this one
+        pdl_wait();
+        RingAt at;  // carried along: a division by the number of stages is a long chain
         for (int i = 0; i < steps; i++) {
-            const int s = i % S;
-            if (i >= S && ok && !bar_wait_tc(s_addr(bars + S + s), ((i / S) - 1) & 1)) ok = false;
+            const unsigned s = at.s;
+            if (i >= S && ok && !mbar_wait(s_addr(bars + S + s), at.parity ^ 1)) ok = false;
+            at.next(S);
             unsigned char* stage = smem + (size_t)s * stage_bytes;
             ox_trace(p.err, 41);
             if (p.use_tma) {
@@ -250,38 +233,32 @@ __global__ void __launch_bounds__(kThreadsTc, 2) nbits_gemm_tc(const __grid_cons
     } else {
         // ── MMA issuer ──
         const unsigned idesc = (1u << 4) | ((unsigned)(mb >> 3) << 17) | (8u << 24);  // f16 × f16 → f32, K-major, N = mb, M = 128
+        pdl_wait();
+        RingAt at, acc;  // acc: the accumulator of a step
+        const unsigned full = s_addr(bars), empty = full + S * 8, step16 = (unsigned)stage_bytes >> 4;
+        const unsigned long long a0 = umma_kmajor_desc(s_addr(smem)), b0 = umma_kmajor_desc(s_addr(smem) + 2 * kPanelA);
         for (int i = 0; i < steps; i++) {
-            const int s = i % S;
-            if (ok && !bar_wait_tc(s_addr(bars + s), (i / S) & 1)) ok = false;
+            if (ok && !mbar_wait(full + at.s * 8, at.parity)) ok = false;
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the asynchronous copies landed through the generic proxy
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (lane == 0) {
-                ox_trace_here(p.err, 44);
-                const unsigned a0 = s_addr(smem + (size_t)s * stage_bytes), b0 = a0 + 2 * kPanelA;
+            const unsigned long long da = a0 + at.s * step16, db = b0 + at.s * step16;  // descriptors count in 16 bytes
+            const unsigned d = tmem + acc.s * (unsigned)mb;
+            if (elect_one()) {
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const unsigned long long da = umma_desc(a0 + (j >> 2) * kPanelA + (j & 3) * 32);
-                    const unsigned long long db = umma_desc(b0 + (j >> 2) * panel_b + (j & 3) * 32);
-                    const unsigned accumulate = (i >= p.n_acc || j > 0) ? 1u : 0u;  // the first step of each accumulator overwrites it
-                    asm volatile(
-                        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n" ::"r"(tmem + (unsigned)((i % p.n_acc) * mb)),
-                        "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u)
-                        : "memory");
-                }
-                // the stage is free once these MMAs have read it
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s_addr(bars + S + s)) : "memory");
-                ox_trace_here(p.err, 45);
-                if (i == steps - 1)
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s_addr(bars + 2 * S)) : "memory");
+                for (int j = 0; j < 8; j++)  // the first step of each accumulator overwrites it
+                    umma_f16(d, da + (j >> 2) * (kPanelA >> 4) + (j & 3) * 2, db + (j >> 2) * ((unsigned)panel_b >> 4) + (j & 3) * 2, idesc, i >= p.n_acc || j > 0);
+                umma_commit(empty + at.s * 8);  // the stage is free once these MMAs have read it
+                if (i == steps - 1) umma_commit(s_addr(bars + 2 * S));
             }
             __syncwarp();
+            at.next(S);
+            acc.next(p.n_acc);
         }
     }
 
     // ── epilogue: warps 0-3 read their quarter of the 128 accumulator lanes ──
     if (warp < 4) {
-        if (ok && steps > 0 && !bar_wait_tc(s_addr(bars + 2 * S), 0)) ok = false;
+        if (ok && steps > 0 && !mbar_wait(s_addr(bars + 2 * S), 0)) ok = false;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int row_in_cta = warp * 32 + lane;           // weight row = accumulator lane
         const int rtg = rt0 + (row_in_cta >> 4);
@@ -442,11 +419,15 @@ struct WideP {
     int k_tiles, n_full, splits; // as in nbits_gemm_tc: row blocks before n_full take all of k, the others that many pieces
     int apart;                   // pieces are CTAs' work of their own; nbits_gemm_reduce adds them up
     int m_tiles, o_tiles, node;
+    int y_odd;                   // rows of some result do not begin on four bytes
 };
 // Persistent CTAs, 128 weight rows × 128 activation rows per tile. Every sum is formed as nbits_gemm_tc forms it, bit for bit: 128-k steps go in
 // turn into two accumulators, which are added in f32 (the tensor core adds without rounding to nearest: shorter chains), and the pieces
 // of k are added in f64. A piece's accumulators are read, half of the columns per group of four warps, while the next piece runs in the other two.
-// 2047 rows through six layers of the 1B architecture (24 products): 1.06 ms and 0.13 ms of widening; nbits_gemm_tc and its reductions took 3.75.
+// A result of one piece is an f32 value: it is rounded as such, without the way through f64, and two rows are stored at a time. With that and the rings' stage and parity
+// carried along instead of divided out of a counter (both kernels), widening included, the same bits, µs: 2047 × 1152 × 13 824 107 → 84, 2047 × 6912 × 1152 59 → 50, 4096 × 5376 ×
+// 5376 340 → 293, 512 × 1152 × 13 824 41 → 35; nbits_gemm_tc, which also takes its tensor memory and first weights before the launches in front of it end, 64 × 4096 × 5376
+// 18.7 → 16.3, 64 × 5376 × 43 008 78 → 72, 16 × 5376 × 43 008 70 → 62. What is left in the wide kernel is the 32 KB that a step brings to an SM (64 bytes a cycle).
 __global__ void __launch_bounds__(kWideThreads, 1) nbits_gemm_wide(const __grid_constant__ WideP p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -454,7 +435,6 @@ __global__ void __launch_bounds__(kWideThreads, 1) nbits_gemm_wide(const __grid_
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + kWideStages * kWideStage);  // full, empty, finished[2], read[2]
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * kWideStages + 4);
     const unsigned full = s_addr(bars), empty = full + kWideStages * 8, finished = empty + kWideStages * 8, read = finished + 16;
-    pdl_trigger();
     if (tid == 0) {
         for (int s = 0; s < 2 * kWideStages + 2; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + s * 8) : "memory");
         for (int s = 0; s < 2; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(read + s * 8) : "memory");
@@ -468,6 +448,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) nbits_gemm_wide(const __grid_
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned tmem = *tmem_slot;
+    pdl_trigger();
     pdl_wait();
     const int units = p.m_tiles * p.o_tiles * (p.apart ? p.splits : 1);  // activation tiles fastest, pieces slowest
     // a unit's tile and pieces; a piece's 128-k steps
@@ -487,108 +468,71 @@ __global__ void __launch_bounds__(kWideThreads, 1) nbits_gemm_wide(const __grid_
     auto first_step = [&](const Unit& q, int piece) { return (int)((long long)p.k_tiles * piece / q.pieces); };
     bool ok = true;
     if (warp == 8) {
-        if (lane == 0) {
-            int done = 0;
-            for (int u = (int)blockIdx.x; u < units && ok; u += (int)gridDim.x) {
-                const Unit q = unit_of(u);
-                const int lo = first_step(q, q.from) * 2, hi = first_step(q, q.to) * 2;  // 64-k steps; pieces follow one another
-                for (int i = lo; i < hi; i++, done++) {
-                    const int s = done % kWideStages;
-                    if (done >= kWideStages && !bar_wait_tc(empty + s * 8, ((done / kWideStages) - 1) & 1)) {
-                        ok = false;
-                        break;
-                    }
-                    const unsigned bar = full + s * 8, dst = s_addr(smem + s * kWideStage);
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((unsigned)kWideStage) : "memory");
-#pragma unroll
-                    for (int op = 0; op < 2; op++)
-                        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                                         dst + op * kPanelA),
-                                     "l"(reinterpret_cast<unsigned long long>(&p.maps[op])), "r"(i * 64), "r"(op ? q.m0 : q.o0), "r"(bar)
-                                     : "memory");
+        RingAt at;
+        bool round = false;  // the ring's first round waits for nothing
+        const unsigned data = s_addr(smem);
+        for (int u = (int)blockIdx.x; u < units; u += (int)gridDim.x) {
+            const Unit q = unit_of(u);
+            const int lo = first_step(q, q.from) * 2, hi = first_step(q, q.to) * 2;  // 64-k steps; pieces follow one another
+            for (int i = lo; i < hi; i++) {
+                if (round && !mbar_wait(empty + at.s * 8, at.parity ^ 1)) {
+                    ok = false;
+                    break;
                 }
+                const unsigned bar = full + at.s * 8, dst = data + at.s * kWideStage;
+                if (elect_one()) {
+                    mbar_expect_tx(bar, (unsigned)kWideStage);
+                    tma_load_2d(dst, p.maps[0], i * 64, q.o0, bar);
+                    tma_load_2d(dst + kPanelA, p.maps[1], i * 64, q.m0, bar);
+                }
+                __syncwarp();
+                at.next(kWideStages);
+                if (at.s == 0) round = true;
             }
-            // every copy has landed before this CTA's shared memory can be given away
-            for (int n = max(0, done - kWideStages); n < done; n++)
-                if (!bar_wait_tc(full + n % kWideStages * 8, (n / kWideStages) & 1)) ok = false;
+            if (!__all_sync(0xffffffffu, ok)) break;
         }
+        // every copy has landed before this CTA's shared memory can be given away
+        for (unsigned n = 0; n < (round ? (unsigned)kWideStages : at.s); n++)
+            if (!mbar_wait(full + n * 8, n < at.s ? at.parity : at.parity ^ 1)) ok = false;
     } else if (warp == 9) {
         const unsigned idesc = (1u << 4) | ((kWideRows >> 3) << 17) | (8u << 24);  // f16 × f16 → f32, M 128 × N 128
-        int done = 0, j = 0;
+        RingAt at;
+        bool ready = false;
+        int j = 0;
+        const unsigned long long a0 = umma_kmajor_desc(s_addr(smem)), b0 = umma_kmajor_desc(s_addr(smem) + kPanelA);
         for (int u = (int)blockIdx.x; u < units; u += (int)gridDim.x) {
             const Unit q = unit_of(u);
             for (int piece = q.from; piece < q.to; piece++, j++) {
                 const int n = first_step(q, piece + 1) - first_step(q, piece);
                 const unsigned d = tmem + (unsigned)((j & 1) * 2 * kWideRows);
-                if (j >= 2 && ok && !bar_wait_tc(read + (j & 1) * 8, ((j >> 1) - 1) & 1)) ok = false;
+                if (j >= 2 && ok && !mbar_wait(read + (j & 1) * 8, ((j >> 1) - 1) & 1)) ok = false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int i = 0; i < 2 * n; i++, done++) {
-                    const int s = done % kWideStages;
-                    if (ok && !bar_wait_tc(full + s * 8, (done / kWideStages) & 1)) ok = false;
+                for (int i = 0; i < 2 * n; i++) {
+                    if (ok && !ready && !mbar_wait(full + at.s * 8, at.parity)) ok = false;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (lane == 0 && ok) {
-                        const unsigned a0 = s_addr(smem + s * kWideStage), b0 = a0 + kPanelA;
+                    const unsigned long long a = a0 + at.s * (kWideStage >> 4), b = b0 + at.s * (kWideStage >> 4);  // descriptors count in 16 bytes
+                    const unsigned done = empty + at.s * 8, to = d + (unsigned)((i >> 1 & 1) * kWideRows);
+                    at.next(kWideStages);
+                    ready = mbar_test(full + at.s * 8, at.parity);  // the answer is there when the products have been issued
+                    if (elect_one() && ok) {
 #pragma unroll
-                        for (int e = 0; e < 4; e++)
-                            asm volatile(
-                                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                                " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n" ::"r"(d + (unsigned)((i >> 1 & 1) * kWideRows)),
-                                "l"(umma_desc(a0 + e * 32)), "l"(umma_desc(b0 + e * 32)), "r"(idesc), "r"(i >= 4 || (i & 1) || e > 0 ? 1u : 0u), "r"(0u)
-                                : "memory");
-                        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(empty + s * 8) : "memory");
+                        for (int e = 0; e < 4; e++) umma_f16(to, a + e * 2, b + e * 2, idesc, i >= 4 || (i & 1) || e > 0);
+                        umma_commit(done);
                     }
                     __syncwarp();
                 }
-                if (lane == 0) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(finished + (j & 1) * 8) : "memory");
+                if (elect_one()) umma_commit(finished + (j & 1) * 8);
                 __syncwarp();
             }
         }
     } else {
         constexpr int kCols = kWideRows / 2;
-        const int lanes = (warp & 3) * 32, col0 = (warp >> 2) * kCols;
+        const int lanes = (warp & 3) * 32, col0 = (warp >> 2) * kCols, odd = lane & 1;
         int j = 0;
         for (int u = (int)blockIdx.x; u < units; u += (int)gridDim.x) {
             const Unit q = unit_of(u);
             const long long m0 = q.m0 + col0;
             const int row_in_panel = q.o0 + lanes + lane, rtg = p.rt_first + (row_in_panel >> 4);
-            double sum[kCols];
-#pragma unroll
-            for (int e = 0; e < kCols; e++) sum[e] = 0.0;
-            for (int piece = q.from; piece < q.to; piece++, j++) {
-                const int accs = min(2, first_step(q, piece + 1) - first_step(q, piece));
-                if (ok && !bar_wait_tc(finished + (j & 1) * 8, (j >> 1) & 1)) ok = false;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const unsigned d = tmem + (unsigned)((j & 1) * 2 * kWideRows + col0) + ((unsigned)lanes << 16);
-#pragma unroll
-                for (int c = 0; c < kCols; c += 16) {
-                    float part[16];
-#pragma unroll
-                    for (int e = 0; e < 16; e++) part[e] = 0.f;
-                    for (int a = 0; a < accs; a++) {
-                        unsigned v[16];
-                        asm volatile(
-                            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-                            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                              "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                            : "r"(d + (unsigned)(a * kWideRows + c)));
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                        for (int e = 0; e < 16; e++) part[e] += __uint_as_float(v[e]);
-                    }
-#pragma unroll
-                    for (int e = 0; e < 16; e++) sum[c + e] += (double)part[e];
-                }
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) bar_arrive(read + (j & 1) * 8);
-            }
-            if (p.apart) {
-                float* part = p.partial + ((size_t)q.from * p.m + m0) * p.n_pad + row_in_panel;
-#pragma unroll
-                for (int e = 0; e < kCols; e++)
-                    if (ok && m0 + e < p.m) part[(size_t)e * p.n_pad] = (float)sum[e];  // one piece: an f32 value
-                continue;
-            }
             int seg = 0;
             long long row;
             if (p.interleave2) {
@@ -600,11 +544,100 @@ __global__ void __launch_bounds__(kWideThreads, 1) nbits_gemm_wide(const __grid_
                 row = (long long)(rtg - p.seg_rt0[seg]) * 16 + (row_in_panel & 15);
             }
             const long long width = p.seg_n[seg];
-            __half* y = p.y[seg] + m0 * width + row;
             const bool row_ok = ok && rtg < p.row_tiles && row < width;
+            const int there = (int)min((long long)kCols, p.m - m0);  // activation rows of these columns that exist
+            // 16 columns of a piece: its two accumulators added in f32
+            auto part_of = [&](int piece, int c, float (&part)[16]) {
+                const int accs = min(2, first_step(q, piece + 1) - first_step(q, piece));
+                const unsigned d = tmem + (unsigned)((j & 1) * 2 * kWideRows + col0 + c) + ((unsigned)lanes << 16);
 #pragma unroll
-            for (int e = 0; e < kCols; e++)
-                if (row_ok && m0 + e < p.m) y[e * width] = __double2half(sum[e]);
+                for (int e = 0; e < 16; e++) part[e] = 0.f;
+                for (int a = 0; a < accs; a++) {
+                    unsigned v[16];
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+                          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                        : "r"(d + (unsigned)(a * kWideRows)));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int e = 0; e < 16; e++) part[e] += __uint_as_float(v[e]);
+                }
+            };
+            auto piece_begin = [&] {
+                if (ok && !mbar_wait(finished + (j & 1) * 8, (j >> 1) & 1)) ok = false;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            };
+            auto piece_end = [&] {
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) bar_arrive(read + (j & 1) * 8);
+                j++;
+            };
+            // 16 columns as f16. Rows of neighbouring lanes are neighbours and of one segment: of two columns the even lane stores both rows of the first, the odd
+            // lane of the second, where that is 32-bit aligned.
+            auto store = [&](int c, const __half (&h)[16]) {
+                if (!p.y_odd) {  // for all lanes alike: half of them may be of another segment
+                    unsigned w[8];
+#pragma unroll
+                    for (int e = 0; e < 8; e++) {
+                        const unsigned mine = __half_as_ushort(odd ? h[2 * e + 1] : h[2 * e]), got = __shfl_xor_sync(0xffffffffu, (unsigned)__half_as_ushort(odd ? h[2 * e] : h[2 * e + 1]), 1);
+                        w[e] = odd ? got | mine << 16 : mine | got << 16;
+                    }
+                    __half* y = p.y[seg] + (m0 + c + odd) * width + (row & ~1ll);
+#pragma unroll
+                    for (int e = 0; e < 8; e++, y += 2 * width)
+                        if (row_ok && c + 2 * e + odd < there) *reinterpret_cast<unsigned*>(y) = w[e];
+                } else {
+                    __half* y = p.y[seg] + (m0 + c) * width + row;
+#pragma unroll
+                    for (int e = 0; e < 16; e++, y += width)
+                        if (row_ok && c + e < there) *y = h[e];
+                }
+                __syncwarp();
+            };
+            if (q.to - q.from == 1) {  // one piece: its f32 sums are the results, or the partial sums
+                piece_begin();
+#pragma unroll
+                for (int c = 0; c < kCols; c += 16) {
+                    float part[16];
+                    part_of(q.from, c, part);
+                    if (p.apart) {
+                        float* to = p.partial + ((size_t)q.from * p.m + m0 + c) * p.n_pad + row_in_panel;
+#pragma unroll
+                        for (int e = 0; e < 16; e++, to += p.n_pad)
+                            if (ok && c + e < there) *to = part[e];
+                    } else {
+                        __half h[16];
+#pragma unroll
+                        for (int e = 0; e < 16; e++) h[e] = __float2half_rn(part[e]);
+                        store(c, h);
+                    }
+                }
+                piece_end();
+                continue;
+            }
+            double sum[kCols];
+#pragma unroll
+            for (int e = 0; e < kCols; e++) sum[e] = 0.0;
+            for (int piece = q.from; piece < q.to; piece++) {
+                piece_begin();
+#pragma unroll
+                for (int c = 0; c < kCols; c += 16) {
+                    float part[16];
+                    part_of(piece, c, part);
+#pragma unroll
+                    for (int e = 0; e < 16; e++) sum[c + e] += (double)part[e];
+                }
+                piece_end();
+            }
+#pragma unroll
+            for (int c = 0; c < kCols; c += 16) {
+                __half h[16];
+#pragma unroll
+                for (int e = 0; e < 16; e++) h[e] = __double2half(sum[c + e]);
+                store(c, h);
+            }
         }
     }
     if (!ok && lane == 0) report(p.err, ERR_WAIT_TIMEOUT, p.node, (long long)blockIdx.x, (long long)warp);
@@ -628,7 +661,7 @@ bool pieces_apart(const TcP& t, long long m, int count) {
 
 // Whether the weights are widened once, for m rows whose launches of nbits_gemm_tc are `t`. Both sides as sums of what they do, fitted to 459 times of
 // either (51 sizes, k 512 … 21 504, 512 … 61 440 weight rows, 257 … 4096 activation rows: residuals 4 % and 6 %; two other sweeps, of grouped
-// products, 5 … 8 %). With a tenth of margin nothing measured is slower than nbits_gemm_tc alone; 0.631 of its time in the geometric mean, 0.627 with
+// products, 5 … 8 %; by the kernels of that time, of which both have lost 5 … 20 % since). With a tenth of margin nothing measured is slower than nbits_gemm_tc alone; 0.631 of its time in the geometric mean, 0.627 with
 // the better of the two at each size. nbits_gemm_tc → widened once, µs, at 257, 1024 and 4096 rows, in brackets what is not taken: k 1152, 13 824 weight
 // rows 48 → 39, 109 → 63, 431 → 194; k 2560, 20 480: 99 → (119), 217 → (196), 858 → 574; k 5376, 5376: 58 → (55), 126 → (114), 499 → 322; k 5376,
 // 43 008: 289 → (389), 620 → (795), 2469 → (2388); k 6912, 1152: 39 → 33, 82 → 58, 332 → 99; k 21 504, 5376: 148 → (270), 308 → (430), 1219 → (1282).
@@ -677,6 +710,7 @@ void emit_wide(Emitter& em, const NBitsGroup& gr, const TRef& x, const TRef& til
         for (int i = 0; i < 3; i++) p.seg_n[i] = t.seg_n[i];
         for (int i = 0; i < 4; i++) p.seg_rt0[i] = t.seg_rt0[i];
         p.m_tiles = (int)((gr.m + kWideRows - 1) / kWideRows);
+        for (int i = 0; i < gr.n_seg; i++) p.y_odd |= gr.y[i].buf.off % 4 != 0 || p.seg_n[i] % 2 != 0;
         p.o_tiles = (count + 7) / 8;
         p.n_pad = (long long)p.o_tiles * 128;
         const long long slots = sm_count(), ctas = (long long)p.m_tiles * p.o_tiles;
