@@ -345,6 +345,8 @@ void ox_f16_to_f32(const void* src, float* dst, size_t n);
 void ox_llm_reset(ox_llm*);
 ox_status ox_llm_step(ox_llm*, const int64_t* ids, int32_t n_ids, int64_t* token_out, void* logits_out, size_t logits_cap,
                       size_t* logits_written);
+/* The same step, its logits as f32 whatever they are stored in; `cap` and `written` count values. */
+ox_status ox_llm_step_f32(ox_llm*, const int64_t* ids, int32_t n_ids, float* logits, size_t cap, size_t* written);
 /* `n_new` greedy tokens in one call: the first step runs `ids` (a prompt, or one token), every later step takes its
  * input id from the previous step's argmax on the device. Every step still uploads its attention mask from host
  * memory and sends its token id to (pinned) host memory, but the host does not wait in between: the steps are

@@ -142,6 +142,7 @@ SIGNATURES = {
     "ox_f16_to_f32": (None, [C.c_void_p, C.POINTER(C.c_float), C.c_size_t]),
     "ox_llm_step": (C.c_int32, [_P, C.POINTER(C.c_int64), C.c_int32, C.POINTER(C.c_int64), C.c_void_p, C.c_size_t,
                                 C.POINTER(C.c_size_t)]),
+    "ox_llm_step_f32": (C.c_int32, [_P, C.POINTER(C.c_int64), C.c_int32, C.POINTER(C.c_float), C.c_size_t, C.POINTER(C.c_size_t)]),
     "ox_llm_generate": (C.c_int32, [_P, C.POINTER(C.c_int64), C.c_int32, C.c_int32, C.POINTER(C.c_int64)]),
     "ox_llm_step_sampled": (C.c_int32, [_P, C.POINTER(C.c_int64), C.c_int32, C.c_float, C.c_int64, C.c_float, C.c_float,
                                         C.POINTER(C.c_int64)]),

@@ -147,15 +147,21 @@ DTensor Engine::forward(const std::vector<Entry>& entries, const DTensor* ids_de
         std::copy(q.pages.begin(), q.pages.end(), table.begin() + (long)(i * width));
     }
     const int64_t R = (int64_t)entries.size();
+    // what describes the step, in one copy
+    std::vector<Session::HostPart> parts = {{DType::I32, {R, 4}, info.data(), info.size() * 4},
+                                            {DType::I32, {R, (int64_t)width}, table.data(), table.size() * 4},
+                                            {DType::I64, {(int64_t)want.size()}, want.data(), want.size() * 8}};
+    if (!ids_dev) parts.push_back({DType::I64, {rows}, ids.data(), ids.size() * 8});
+    const std::vector<DTensor> step = s_.upload_together(parts);
     std::vector<std::pair<std::string, DTensor>> feed;
     feed.reserve(names_.size());
     for (size_t i = 0; i < names_.size(); i++) {
         const std::string& n = names_[i];
         DTensor t;
-        if (n == "input_ids") t = ids_dev ? *ids_dev : s_.upload(DType::I64, {rows}, ids.data(), ids.size() * 8);
-        else if (n == "seq_info") t = s_.upload(DType::I32, {R, 4}, info.data(), info.size() * 4);
-        else if (n == "page_table") t = s_.upload(DType::I32, {R, (int64_t)width}, table.data(), table.size() * 4);
-        else if (n == "logit_rows") t = s_.upload(DType::I64, {(int64_t)want.size()}, want.data(), want.size() * 8);
+        if (n == "input_ids") t = ids_dev ? *ids_dev : step[3];
+        else if (n == "seq_info") t = step[0];
+        else if (n == "page_table") t = step[1];
+        else if (n == "logit_rows") t = step[2];
         else if (state_[i].buf) t = state_[i];
         else fail(ErrKind::Binding, "input '" + n + "' is not one the engine can fill");
         feed.emplace_back(n, std::move(t));

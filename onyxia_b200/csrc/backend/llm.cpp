@@ -49,6 +49,25 @@ std::vector<int64_t> input_shape(const Module& m, size_t i, const Bindings& b) {
     catch (const ox::Error& e) { return (ox_status)ox::set_error(e); }                    \
     catch (const std::exception& e) { return (ox_status)ox::set_error(ErrKind::Runtime, e.what()); }
 
+namespace oxrt {
+// Eight values per instruction where the processor has it (a 262 144-word row of logits: 350 µs through numpy, 42 µs here).
+#if defined(__x86_64__)
+__attribute__((target("avx,f16c"))) static size_t widen_eights(const uint16_t* src, float* dst, size_t n) {
+    size_t i = 0;
+    for (; i + 8 <= n; i += 8) _mm256_storeu_ps(dst + i, _mm256_cvtph_ps(_mm_loadu_si128((const __m128i*)(src + i))));
+    return i;
+}
+#endif
+void widen_f16(const void* src, float* dst, size_t n) {
+    const uint16_t* h = (const uint16_t*)src;
+    size_t i = 0;
+#if defined(__x86_64__)
+    if (__builtin_cpu_supports("f16c") && __builtin_cpu_supports("avx")) i = widen_eights(h, dst, n);
+#endif
+    for (; i < n; i++) dst[i] = __half2float(__ushort_as_half(h[i]));
+}
+}  // namespace oxrt
+
 extern "C" {
 
 ox_status ox_llm_create(ox_session* session, int64_t max_seq_len, ox_llm** out) {
@@ -81,22 +100,7 @@ int32_t ox_llm_logits_dtype(const ox_llm* l) {
     const Module& m = l->s->module();
     return (int32_t)m.values[m.outputs[(size_t)l->logits_out].second].ty.dtype;
 }
-// Eight values per instruction where the processor has it (a 262 144-word row of logits: 350 µs through numpy, 42 µs here).
-#if defined(__x86_64__)
-__attribute__((target("avx,f16c"))) static size_t widen_eights(const uint16_t* src, float* dst, size_t n) {
-    size_t i = 0;
-    for (; i + 8 <= n; i += 8) _mm256_storeu_ps(dst + i, _mm256_cvtph_ps(_mm_loadu_si128((const __m128i*)(src + i))));
-    return i;
-}
-#endif
-void ox_f16_to_f32(const void* src, float* dst, size_t n) {
-    const uint16_t* h = (const uint16_t*)src;
-    size_t i = 0;
-#if defined(__x86_64__)
-    if (__builtin_cpu_supports("f16c") && __builtin_cpu_supports("avx")) i = widen_eights(h, dst, n);
-#endif
-    for (; i < n; i++) dst[i] = __half2float(__ushort_as_half(h[i]));
-}
+void ox_f16_to_f32(const void* src, float* dst, size_t n) { oxrt::widen_f16(src, dst, n); }
 void ox_llm_reset(ox_llm* l) {
     if (l->engine && l->past > 0) l->engine->release(0);
     l->past = 0;
@@ -113,12 +117,16 @@ struct SamplingArgs {
 };
 ox_status llm_step(ox_llm* l, const int64_t* ids, int32_t n_ids, int64_t* token_out, void* logits_out, size_t logits_cap,
                    size_t* logits_written, const SamplingArgs* sampling, const oxrt::DTensor* ids_dev = nullptr,
-                   oxrt::DTensor* token_dev = nullptr);
+                   oxrt::DTensor* token_dev = nullptr, float* logits_f32 = nullptr);
 }  // namespace
 
 ox_status ox_llm_step(ox_llm* l, const int64_t* ids, int32_t n_ids, int64_t* token_out, void* logits_out, size_t logits_cap,
                       size_t* logits_written) {
     return llm_step(l, ids, n_ids, token_out, logits_out, logits_cap, logits_written, nullptr);
+}
+
+ox_status ox_llm_step_f32(ox_llm* l, const int64_t* ids, int32_t n_ids, float* logits, size_t cap, size_t* written) {
+    return llm_step(l, ids, n_ids, nullptr, nullptr, cap, written, nullptr, nullptr, nullptr, logits);
 }
 
 // The same step with the next token drawn on the device by temperature / top-k / top-p sampling
@@ -163,7 +171,7 @@ ox_status ox_llm_generate(ox_llm* l, const int64_t* ids, int32_t n_ids, int32_t 
 
 namespace {
 ox_status llm_step(ox_llm* l, const int64_t* ids, int32_t n_ids, int64_t* token_out, void* logits_out, size_t logits_cap,
-                   size_t* logits_written, const SamplingArgs* sampling, const oxrt::DTensor* ids_dev, oxrt::DTensor* token_dev) {
+                   size_t* logits_written, const SamplingArgs* sampling, const oxrt::DTensor* ids_dev, oxrt::DTensor* token_dev, float* logits_f32) {
     OX_TRY
     if (n_ids <= 0) fail(ErrKind::Shape, "Cannot step with empty input_ids");
     if (l->past + n_ids > l->max_seq_len)
@@ -185,6 +193,7 @@ ox_status llm_step(ox_llm* l, const int64_t* ids, int32_t n_ids, int64_t* token_
         if (token_dev) *token_dev = tok;
         if (token_out) s.download(tok, token_out, sizeof(int64_t), nullptr);
         if (logits_out) s.download(logits, logits_out, logits_cap, logits_written);
+        if (logits_f32) s.download_f32(logits, logits_f32, logits_cap, logits_written);
         return OX_OK;
     }
     Bindings b;
@@ -275,15 +284,16 @@ ox_status llm_step(ox_llm* l, const int64_t* ids, int32_t n_ids, int64_t* token_
         s.download(tok, host.data(), host.size() * sizeof(int64_t), &written);
         *token_out = host[(size_t)tok.numel() - 1];
     }
-    if (logits_out) {
+    if (logits_out || logits_f32) {
         // the last position's row
         const int64_t vocab = logits.shape.back(), rows = logits.numel() / vocab;
         const size_t row_bytes = dtype_storage_bytes(logits.dtype, (uint64_t)vocab);
-        if (logits_cap < row_bytes) fail(ErrKind::Shape, "logits buffer too small");
+        if (logits_cap < (logits_f32 ? (size_t)vocab : row_bytes)) fail(ErrKind::Shape, "logits buffer too small");
         oxrt::DTensor last = logits;
         last.shape = {vocab};
         last.offset += (size_t)(rows - 1) * row_bytes;
-        s.download(last, logits_out, logits_cap, logits_written);
+        if (logits_f32) s.download_f32(last, logits_f32, logits_cap, logits_written);
+        else s.download(last, logits_out, logits_cap, logits_written);
     }
     return OX_OK;
     OX_CATCH

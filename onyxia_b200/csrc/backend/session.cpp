@@ -1,4 +1,7 @@
 // Session: prepare-time analysis, per-binding plans, execution.
+#ifdef __linux__
+#include <sys/mman.h>
+#endif
 #include "session.hpp"
 
 #include <algorithm>
@@ -152,6 +155,11 @@ Session::~Session() {
         cudaEventDestroy(r.b);
     }
     for (auto e : prof_free_) cudaEventDestroy(e);
+    if (land_pinned_) {
+        cudaFreeHost(land_pinned_);
+        for (auto e : land_events_)
+            if (e) cudaEventDestroy(e);
+    }
     if (stage_pinned_) {
         cudaFreeHost(stage_pinned_);
         for (auto e : stage_events_) cudaEventDestroy(e);
@@ -693,6 +701,33 @@ DTensor Session::upload(DType dtype, const std::vector<int64_t>& shape, const vo
     return t;
 }
 
+// The tensors of one step in one buffer and one copy (a copy and its event are 4 µs of the host and 5 of the device, whatever they move): one tensor begins
+// on 256 bytes after the other. More than a staging slot holds goes up tensor by tensor.
+std::vector<DTensor> Session::upload_together(const std::vector<HostPart>& parts) {
+    std::vector<DTensor> out;
+    size_t total = 0;
+    for (auto& p : parts) total += (p.nbytes + 255) / 256 * 256;
+    if (total > kStageBytes) {
+        for (auto& p : parts) out.push_back(upload(p.dtype, p.shape, p.bytes, p.nbytes));
+        return out;
+    }
+    std::vector<uint8_t> flat(total);
+    size_t at = 0;
+    for (auto& p : parts) {
+        DTensor t;
+        t.dtype = p.dtype;
+        t.shape = p.shape;
+        t.offset = at;
+        if (t.nbytes() != p.nbytes) fail(ErrKind::Interp, "tensor data size mismatch");
+        if (p.nbytes) std::memcpy(flat.data() + at, p.bytes, p.nbytes);
+        at += (p.nbytes + 255) / 256 * 256;
+        out.push_back(std::move(t));
+    }
+    const DTensor all = upload(DType::U8, {(int64_t)total}, flat.data(), total);
+    for (auto& t : out) t.buf = all.buf;
+    return out;
+}
+
 DTensor Session::zeros(DType dtype, const std::vector<int64_t>& shape) {
     OX_CUDA(cudaSetDevice(device_));
     DTensor t;
@@ -786,6 +821,55 @@ void Session::download(const DTensor& t, void* dst, size_t cap, size_t* written)
     OX_CUDA(cudaStreamSynchronize(stream_));
     if (written) *written = nbytes;
     check_device_error();
+}
+
+void Session::download_f32(const DTensor& t, float* dst, size_t cap, size_t* written) {
+    if (t.dtype == DType::F32) {
+        download(t, dst, cap * sizeof(float), written);
+        if (written) *written /= sizeof(float);
+        return;
+    }
+    if (t.dtype != DType::F16 || t.cap) fail(ErrKind::DType, "a dense f32 or f16 tensor is wanted");
+    OX_CUDA(cudaSetDevice(device_));
+    const size_t n = (size_t)t.numel();
+    if (cap < n) fail(ErrKind::Runtime, "download buffer too small: " + std::to_string(cap) + " < " + std::to_string(n) + " values");
+    if (n) {
+        populate(dst, n * sizeof(float));
+        land(t, n * 2, [&](size_t at, const uint8_t* from, size_t bytes) { widen_f16(from, dst + at / 2, bytes / 2); });
+    }
+    OX_CUDA(cudaStreamSynchronize(stream_));
+    if (written) *written = n;
+    check_device_error();
+}
+
+// Pages of a destination that has just been allocated, while the device still works on what will be copied there: one after the other as they
+// are written, they take 340 µs per MB (populated at once, 84). Nothing is lost where the kernel does not know the advice.
+void Session::populate(void* dst, size_t nbytes) {
+#ifdef __linux__
+    const uintptr_t page = 4096, first = ((uintptr_t)dst + page - 1) / page * page, last = ((uintptr_t)dst + nbytes) / page * page;
+    if (last > first) madvise((void*)first, last - first, 23 /* MADV_POPULATE_WRITE */);
+#endif
+}
+
+// A dense tensor through two pinned chunks, `take(offset, bytes, n)` called in order: values are widened out of one while the other lands, without the copy into
+// memory of the caller's that cudaMemcpyAsync ends with. (As a plain copy this way is no faster than the driver's own: 8 × 32 768 values 12.6 against 12.0 ms per 33 steps.)
+template <class F> void Session::land(const DTensor& t, size_t nbytes, F&& take) {
+    if (!land_pinned_) {
+        OX_CUDA(cudaMallocHost((void**)&land_pinned_, 2 * kLandBytes));
+        for (auto& e : land_events_) OX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    const size_t chunks = (nbytes + kLandBytes - 1) / kLandBytes;
+    auto ask = [&](size_t i) {
+        OX_CUDA(cudaMemcpyAsync(land_pinned_ + (i & 1) * kLandBytes, (const uint8_t*)t.ptr() + i * kLandBytes, std::min(kLandBytes, nbytes - i * kLandBytes),
+                                cudaMemcpyDeviceToHost, stream_));
+        OX_CUDA(cudaEventRecord(land_events_[i & 1], stream_));
+    };
+    ask(0);
+    for (size_t i = 0; i < chunks; i++) {
+        if (i + 1 < chunks) ask(i + 1);
+        OX_CUDA(cudaEventSynchronize(land_events_[i & 1]));
+        take(i * kLandBytes, land_pinned_ + (i & 1) * kLandBytes, std::min(kLandBytes, nbytes - i * kLandBytes));
+    }
 }
 
 void Session::download_async(const DTensor& t, void* pinned_dst) {

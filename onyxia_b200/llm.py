@@ -138,7 +138,7 @@ class NativeLlmSession:
         h = C.c_void_p()
         _ffi.check(self._lib.ox_llm_create(self.session._h, max_seq_len, C.byref(h)))
         self._h = h
-        self._raw = np.empty(1 << 20, dtype=np.uint8)  # a step's logits as they are stored
+        self._room = (1 << 20) // (2 if self._lib.ox_llm_logits_dtype(h) == ir.F16 else 4)  # values; their number once a step has given it
 
     def step_greedy(self, ids) -> int:
         C = self._C
@@ -172,14 +172,12 @@ class NativeLlmSession:
         C = self._C
         from . import _ffi
         arr = _ffi.whole_words("q", ids)
-        buf = self._raw
-        written = C.c_size_t()
-        _ffi.check(self._lib.ox_llm_step(self._h, C.cast(arr.buffer_info()[0], C.POINTER(C.c_int64)), len(arr), None,
-                                         buf.ctypes.data_as(C.c_void_p), buf.size, C.byref(written)))
-        if self._lib.ox_llm_logits_dtype(self._h) != ir.F16:
-            return buf[:written.value].view(np.float32).copy()
-        out = np.empty(written.value // 2, dtype=np.float32)
-        self._lib.ox_f16_to_f32(buf.ctypes.data_as(C.c_void_p), out.ctypes.data_as(C.POINTER(C.c_float)), out.size)
+        out, written = np.empty(self._room, dtype=np.float32), C.c_size_t()
+        _ffi.check(self._lib.ox_llm_step_f32(self._h, C.cast(arr.buffer_info()[0], C.POINTER(C.c_int64)), len(arr), out.ctypes.data_as(C.POINTER(C.c_float)), out.size,
+                                             C.byref(written)))
+        if out.size > written.value:
+            self._room = written.value
+            return out[:written.value].copy()
         return out
 
     def sequence_length(self) -> int:

@@ -1,4 +1,5 @@
 """Kernels that a rule on sizes picks, at the sizes where the rule changes and where their tiles and pieces end."""
+import ctypes
 import os
 import subprocess
 import sys
@@ -8,7 +9,7 @@ import pytest
 
 import mufevik_ref as ref
 from onyxia_b200 import backend as be
-from onyxia_b200 import ir, models
+from onyxia_b200 import ir, llm, models
 from onyxia_b200.ir import HostTensor
 from gpu_util import cuda_backend, differential
 from lovuzen_util import to_bf16
@@ -422,3 +423,18 @@ def test_small_caches_are_copied_beside_the_new_rows(dtype, d, past, seq, alone)
         for b, v in enumerate(valid):
             assert np.array_equal(got["present_" + name][b, :, :v], feed["past_" + name].numpy()[b, :, :v])
             assert not got["present_" + name][b, :, v + seq:].any()
+
+
+@pytest.mark.parametrize("model,vocab", [("c1", 300), ("1b", 130), ("1b", 131072), ("1b", 131073), ("1b", 300001)])
+def test_logits_as_f32(model, vocab):
+    """Logits of one chunk, of whole chunks and of a tail, widened as they land: the stored values themselves. The first step does not know how many there are."""
+    cfg = models.config_c1() if model == "c1" else models.config_gemma3_1b()
+    cfg.layers, cfg.vocab = 1, vocab
+    module, ids = models.build_decoder(cfg, seed=3), [5, 7, 11]
+    a, b = (llm.NativeLlmSession(cuda_backend(), module.clone(), 16) for _ in range(2))
+    for i in ids:
+        raw, written = np.empty(4 * vocab, np.uint8), ctypes.c_size_t()
+        assert a._lib.ox_llm_step(a._h, (ctypes.c_int64 * 1)(i), 1, None, raw.ctypes.data_as(ctypes.c_void_p), raw.size, ctypes.byref(written)) == 0
+        want = raw[:written.value].view(np.float32 if model == "c1" else np.float16).astype(np.float32)
+        got = b.step_logits([i])
+        assert got.shape == (vocab,) and np.array_equal(got, want)
