@@ -58,6 +58,9 @@ template <typename T> __device__ __forceinline__ float head_factor(const KvP& p,
 // queries `q` of sequences with several new tokens are prepared.
 void emit_talking_heads(Emitter&, const PagedKvDesc&, KvP p, const TRef& proj, const TRef& turns, Buf q, const TRef& keys, const TRef& values,
                         const TRef& seqs, const TRef& pages, const TRef& out);
+// Prompts on tcgen05 (paged_kv_prefill.cu), with values or, without, `lse` only; `ptrs`: fields of KvP by their offset.
+bool kv_prefill_fits(const PagedKvDesc&, const TRef& keys, const TRef* values, int64_t out_off);
+void emit_kv_prefill(Emitter&, const PagedKvDesc&, const KvP&, const TRef& keys, const TRef* values, std::initializer_list<std::pair<size_t, Buf>> ptrs);
 // The form of the prefill kernel that leaves `lse` only.
 void emit_kv_lse(Emitter&, const PagedKvDesc&, KvP p, Buf q, Buf lse, const TRef& keys, const TRef& seqs, const TRef& pages);
 

@@ -8,8 +8,8 @@
 // keeps the length of a vector: the mean square is taken in front of it. Angles are reduced in 64-bit turns.
 //
 //   paged_kv_prepare, paged_kv_turn   rotated, normed queries; the new keys and values go to the pools
-//   paged_kv_prefill   sequences with several new tokens: 64 (token, head) rows per CTA share each tile of 64 keys;
-//                      `mma.sync`, online softmax, only the tiles that the window reaches
+//   paged_kv_prefill   sequences with several new tokens: on tcgen05 (paged_kv_prefill.cu) where a page holds 64 keys and more; here for smaller
+//                      pages: 64 (token, head) rows per CTA share each tile of 64 keys, `mma.sync`. Online softmax, only the tiles that the window reaches
 //   paged_kv_decode    sequences with one new token, the window's keys split over CTAs and warps, all of the above in one launch
 //   paged_kv_simt      f32, and shapes the tensor-core kernels do not take
 //
@@ -654,8 +654,14 @@ void emit_paged_kv_attention(Emitter& em, const PagedKvDesc& d, const TRef& proj
     }
     if (!decode_only) {
         const int64_t tq = kPreRows / rep;
-        ensure_max_dynamic_smem((const void*)dc.prefill, 220 * 1024);
-        launch(dc.prefill, dim3((unsigned)((rows + tq - 1) / tq + n_seqs), (unsigned)d.kv_heads), kPreThreads, (unsigned)dc.pre_smem, none, "paged_kv_prefill");
+        if (kv_prefill_fits(d, keys, &values, out.buf.off)) {
+            emit_kv_prefill(em, d, p, keys, &values,
+                            {{offsetof(KvP, keys), keys.buf}, {offsetof(KvP, values), values.buf}, {offsetof(KvP, q), q}, {offsetof(KvP, sinks), sink}, {offsetof(KvP, temps), temps},
+                             {offsetof(KvP, gate), gate}, {offsetof(KvP, out), out.buf}, {offsetof(KvP, seqs), seqs.buf}, {offsetof(KvP, table), pages.buf}, {offsetof(KvP, err), Buf{kSlotErr, 0}}});
+        } else {
+            ensure_max_dynamic_smem((const void*)dc.prefill, 220 * 1024);
+            launch(dc.prefill, dim3((unsigned)((rows + tq - 1) / tq + n_seqs), (unsigned)d.kv_heads), kPreThreads, (unsigned)dc.pre_smem, none, "paged_kv_prefill");
+        }
     }
     if (decode_only || n_seqs > 1) {
         const int nh = rep > 8;  // two groups of eight heads per CTA
@@ -686,6 +692,9 @@ void emit_kv_lse(Emitter& em, const PagedKvDesc& d, KvP p, Buf q, Buf lse, const
     const DimChoice dc = dim_choice(d.dim);
     const int64_t tq = kPreRows / (d.heads / d.kv_heads);
     const Buf none{kSlotNull, 0}, temps = d.temps ? d.temps->buf : none;
+    if (kv_prefill_fits(d, keys, nullptr, 0))
+        return emit_kv_prefill(em, d, p, keys, nullptr, {{offsetof(KvP, keys), keys.buf}, {offsetof(KvP, q), q}, {offsetof(KvP, temps), temps}, {offsetof(KvP, lse), lse}, {offsetof(KvP, seqs), seqs.buf},
+                                                         {offsetof(KvP, table), pages.buf}, {offsetof(KvP, err), Buf{kSlotErr, 0}}});
     ensure_max_dynamic_smem((const void*)dc.lse, 220 * 1024);
     em.launch(dc.lse, dim3((unsigned)((p.rows + tq - 1) / tq + p.n_seqs), (unsigned)d.kv_heads), dim3(kPreThreads), (unsigned)dc.lse_smem, p,
               {{&p.keys, keys.buf}, {&p.values, none}, {&p.q, q}, {&p.temps, temps}, {&p.lse, lse}, {&p.seqs, seqs.buf}, {&p.table, pages.buf}, {&p.err, Buf{kSlotErr, 0}}},

@@ -1,0 +1,330 @@
+// Prompts over paged keys and values in bf16 on tcgen05: scores and sums of values in tensor memory.
+//
+// A CTA owns 128 (token, head) rows of one key head and walks over their keys 64 at a time. Per 64 keys: 4 · dim / 64 products of 128 × 64 make the scores, two threads per
+// row cap, mask and weigh them, 4 products of 128 × vdim add the weights' share of the values; the scores of the next 64 keys are made under the weights of these. Keys and
+// values come by TMA, a page's rows are the rows of a tensor map; two of either are on their way.
+//
+// What bounds it is the chain of a step, about 1.3 µs in a CTA alone on its SM (256 dimensions: shared memory), of which the products are 0.7; a short prompt's longest tiles are as long
+// as the launch. The `mma.sync` kernel, which remains for pages of less than 64 keys, had four warps per SM at this size. µs, before → now: 4096 tokens, 4 heads of 256 over one key
+// head, capped 245 → 91 (rows by one thread each: 104); 1999 tokens, the same 127 → 49; 2048 tokens, 16 heads of 128 over 4, the softmax's sums alone 94 → 35.
+#include "paged_kv.cuh"
+
+namespace oxk {
+
+namespace {
+
+constexpr int kRows = 128, kKeys = 64, kSoft = 256, kThreads = kSoft + 64;  // warps 0-7 softmax, 8 copies, 9 issues products
+constexpr int kHalf = kKeys / 2;                                            // keys of a row per thread
+constexpr unsigned kPanelQ = kRows * 128, kPanelKv = kKeys * 128;  // bytes: rows × 64 dimensions
+
+struct PreP {
+    alignas(64) unsigned char maps[2][128];  // keys, values: [rows of the pool, dim | vdim]
+    KvP kv;
+    int kp, vp;  // panels of 64 dimensions
+};
+
+// Rows of weights in tensor memory (two per column) × values, of which 64 stand side by side for a key.
+__device__ __forceinline__ void umma_weights(unsigned d, unsigned a, unsigned long long b, unsigned idesc, bool accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n}\n" ::"r"(d),
+        "r"(a), "l"(b), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(0u)
+        : "memory");
+}
+// Shared-memory matrix descriptor, 128-byte swizzle, 64 elements of the wide axis side by side: groups of eight keys 1 024 bytes apart, the next 64
+// elements a panel further.
+__device__ __forceinline__ unsigned long long umma_wide_desc(unsigned smem_byte_addr) {
+    return (unsigned long long)((smem_byte_addr & 0x3FFFFu) >> 4) | ((unsigned long long)(kPanelKv >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ void tmem_ld32(unsigned (&v)[32], unsigned from) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, "
+        "%21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
+          "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]),
+          "=r"(v[30]), "=r"(v[31])
+        : "r"(from));
+}
+__device__ __forceinline__ void tmem_ld16(unsigned (&v)[16], unsigned from) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
+          "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(from));
+}
+__device__ __forceinline__ void tmem_st16(unsigned to, const unsigned (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};\n" ::"r"(v[0]), "r"(v[1]), "r"(v[2]),
+        "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(to)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+// CAPPED: scores are capped. LSE: no values; the softmax's sums are the result.
+template <bool CAPPED, bool LSE> __global__ void __launch_bounds__(kThreads, 2) paged_kv_prefill_tc(const __grid_constant__ PreP pp) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const KvP& p = pp.kv;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kp = pp.kp, vp = LSE ? 0 : pp.vp;
+    const unsigned k_stage = kp * kPanelKv, v_stage = vp * kPanelKv;
+    const unsigned sq0 = smem_u32(smem), sk = sq0 + kp * kPanelQ, sv = sk + 2 * k_stage, bars = sv + 2 * v_stage;
+    // two barriers each: keys there, free, values there, free, scores there, weights there; and one for the sums
+    const unsigned k_full = bars, k_free = bars + 16, v_full = bars + 32, v_free = bars + 48, s_full = bars + 64, w_full = bars + 80, o_done = bars + 96;
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(smem + (bars + 104 - sq0));
+    float* shared = reinterpret_cast<float*>(smem + (bars + 112 - sq0));  // [turn][half of the keys][row]: what the two threads of a row tell each other
+    if (tid == 0) {
+        for (int i = 0; i < 13; i++) mbar_init(bars + i * 8, i == 10 || i == 11 ? kSoft / 32 : 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    pdl_wait();
+    const int rep = p.heads / p.kv_heads, tq = kRows / rep, g = blockIdx.y;
+    int seq, first;
+    // long rows first: the last tiles of a sequence see the most keys
+    if (!locate_tile(p.seqs, p.n_seqs, (int)gridDim.x - 1 - (int)blockIdx.x, tq, &seq, &first)) return;
+    const SeqRow sq = load_seq(p.seqs, seq);
+    const int n_tok = min(tq, sq.len - first), pos0 = sq.past + first, last = pos0 + n_tok - 1;
+    // Scores in two turns of 64 columns, weights in two of 32, sums. Up to 128 dimensions weights take their scores' place, so that two CTAs fit an SM.
+    const bool apart = vp > 2;
+    const unsigned cols = LSE ? 128 : apart ? 512 : 256;
+    if (warp == 9) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    for (int i = tid; i < kRows * kp * 8; i += kThreads) {
+        const int r = i / (kp * 8), c = i % (kp * 8), tok = r / rep, h = g * rep + r % rep;
+        const bool live = tok < n_tok && c * 8 < p.dim;
+        const bf16* src = (const bf16*)p.q;
+        cp_async16(sq0 + (c >> 3) * kPanelQ + r * 128 + (((c & 7) ^ (r & 7)) << 4), live ? src + ((long long)(sq.start + first + tok) * p.heads + h) * p.dim + c * 8 : src, live);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads them
+    before_sync();
+    __syncthreads();
+    after_sync();
+    pdl_trigger();  // the tensor memory is taken: nothing that starts now can keep it from this CTA
+    const unsigned tmem = *tmem_slot, t_weights = apart ? tmem + 128 : tmem, weights_turn = apart ? 32 : kKeys, t_sum = tmem + (apart ? 192 : 128);
+    const int kt0 = first_key(p, pos0) / kKeys, n = last / kKeys + 1 - kt0;
+    bool ok = true;
+
+    if (warp == 8) {
+        RingAt at;
+        for (int i = 0; i < n && ok; i++) {
+            const int j0 = (kt0 + i) * kKeys, row = (int)key_row(p, page_of(p, seq, j0), g, j0);
+            if (i >= 2 && !mbar_wait(k_free + at.s * 8, at.parity ^ 1)) ok = false;
+            if (ok && elect_one()) {
+                mbar_expect_tx(k_full + at.s * 8, k_stage);
+                for (int c = 0; c < kp; c++) tma_load_2d(sk + at.s * k_stage + c * kPanelKv, pp.maps[0], c * 64, row, k_full + at.s * 8);
+            }
+            __syncwarp();
+            if constexpr (!LSE) {
+                if (i >= 2 && ok && !mbar_wait(v_free + at.s * 8, at.parity ^ 1)) ok = false;
+                if (ok && elect_one()) {
+                    mbar_expect_tx(v_full + at.s * 8, v_stage);
+                    for (int c = 0; c < vp; c++) tma_load_2d(sv + at.s * v_stage + c * kPanelKv, pp.maps[1], c * 64, row, v_full + at.s * 8);
+                }
+                __syncwarp();
+            }
+            ok = __all_sync(0xffffffffu, ok);
+            at.next(2);
+        }
+    } else if (warp == 9) {
+        const unsigned base = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);  // bf16 × bf16 → f32, M 128
+        const unsigned by_keys = base | ((kKeys >> 3) << 17), by_values = base | (1u << 16) | ((unsigned)(vp * 8) << 17);  // the values' wide axis is the result's
+        const unsigned long long dq = umma_kmajor_desc(sq0), dk = umma_kmajor_desc(sk), dv = umma_wide_desc(sv);
+        RingAt ahead, at;
+        auto scores = [&] {
+            if (ok && !mbar_wait(k_full + ahead.s * 8, ahead.parity)) ok = false;
+            after_sync();
+            if (ok && elect_one()) {
+                const unsigned long long k = dk + ahead.s * (k_stage >> 4);
+                for (int c = 0; c < kp; c++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) umma_bf16(tmem + ahead.s * kKeys, dq + c * (kPanelQ >> 4) + e * 2, k + c * (kPanelKv >> 4) + e * 2, by_keys, c > 0 || e > 0);
+                umma_commit(k_free + ahead.s * 8);
+                umma_commit(s_full + ahead.s * 8);
+            }
+            __syncwarp();
+            ahead.next(2);
+        };
+        scores();
+        for (int i = 0; i < n; i++) {
+            if (i + 1 < n) {
+                // the other turn's scores were read by the threads that wrote its weights; where these have their place, products have to be done with them
+                if (!LSE && !apart && i > 0 && ok && !mbar_wait(o_done, (unsigned)(i - 1) & 1)) ok = false;
+                scores();
+            }
+            if (ok && !mbar_wait(w_full + at.s * 8, at.parity)) ok = false;
+            if constexpr (!LSE) {
+                if (ok && !mbar_wait(v_full + at.s * 8, at.parity)) ok = false;
+                after_sync();
+                if (ok && elect_one()) {
+                    const unsigned long long v = dv + at.s * (v_stage >> 4);
+#pragma unroll
+                    for (int e = 0; e < kKeys / 16; e++) umma_weights(t_sum, t_weights + at.s * weights_turn + e * 8, v + e * 128, by_values, i > 0 || e > 0);
+                    umma_commit(v_free + at.s * 8);
+                    umma_commit(o_done);
+                }
+                __syncwarp();
+            }
+            at.next(2);
+        }
+    } else {
+        // two threads per row, each with half of the keys
+        const int r = tid & (kRows - 1), part = tid / kRows, tok = r / rep, head = g * rep + r % rep;
+        const bool live = tok < n_tok;
+        const int pos = live ? pos0 + tok : last, low = first_key(p, pos), last_low = first_key(p, last);  // rows without a token compute something harmless
+        const float mul2 = p.mul2 * temp_of(p, head), cap2 = p.cap2;
+        const unsigned lanes = (unsigned)((warp & 3) * 32) << 16;
+        // what both threads of a row know: by the two warps that share its rows
+        auto both = [&](int turn, float mine) {
+            float* at = shared + turn * 2 * kRows + r;
+            at[part * kRows] = mine;
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 3)) : "memory");
+            return at[(part ^ 1) * kRows];
+        };
+        float m = kNoScore, l = 0.f;
+        RingAt at;
+        for (int i = 0; i < n; i++) {
+            const int j0 = (kt0 + i) * kKeys, mine0 = j0 + part * kHalf;
+            if (ok && !mbar_wait(s_full + at.s * 8, at.parity)) ok = false;
+            after_sync();
+            float s[kHalf];
+            {
+                unsigned v[32];
+                tmem_ld32(v, tmem + lanes + at.s * kKeys + part * kHalf);
+                tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < kHalf; e++) {
+                    const float x = __uint_as_float(v[e]) * mul2;
+                    s[e] = CAPPED ? cap2 - __fdividef(2.f * cap2, 1.f + exp2f(x)) : x;
+                }
+            }
+            if (j0 + kKeys - 1 > pos0 || j0 < last_low) {
+#pragma unroll
+                for (int e = 0; e < kHalf; e++)
+                    if (mine0 + e > pos || mine0 + e < low) s[e] = -INFINITY;
+            }
+            float top = m;
+#pragma unroll
+            for (int e = 0; e < kHalf; e++) top = fmaxf(top, s[e]);
+            top = fmaxf(top, both(i & 1, top));
+            // Weights are taken against a maximum that may be up to 2^8 behind: the sums are divided by their weights' sum in the end, whatever it was taken against.
+            // Both warps of a row see the same tops.
+            if (__any_sync(0xffffffffu, top > m + 8.f)) {
+                const float keep = exp2f(m - top);
+                m = top;
+                l *= keep;
+                if (!LSE && i > 0) {
+                    if (ok && !mbar_wait(o_done, (unsigned)(i - 1) & 1)) ok = false;
+                    after_sync();
+#pragma unroll 1
+                    for (int c = part * 16; c < vp * 64; c += 32) {
+                        unsigned v[16];
+                        tmem_ld16(v, t_sum + lanes + c);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int e = 0; e < 16; e++) v[e] = __float_as_uint(__uint_as_float(v[e]) * keep);
+                        tmem_st16(t_sum + lanes + c, v);
+                    }
+                }
+            }
+            unsigned w[kHalf / 2];
+#pragma unroll
+            for (int e = 0; e < kHalf / 2; e++) {
+                const float a = exp2f(s[2 * e] - m), b = exp2f(s[2 * e + 1] - m);
+                l += a + b;
+                w[e] = pack_bf16(a, b);
+            }
+            if constexpr (!LSE) {
+                // Where weights take their scores' place: both threads of the row have read these. Elsewhere: the products that read this turn's last weights were issued
+                // before these scores.
+                tmem_st16(t_weights + lanes + at.s * weights_turn + part * (kHalf / 2), w);
+                if (j0 + kKeys - 1 > last) {  // what lies behind the last key may be no number, which a weight of 0 would not cancel
+                    if (ok && !mbar_wait(v_full + at.s * 8, at.parity)) ok = false;
+                    const int dead = j0 + kKeys - 1 - last;
+                    for (int u = tid; u < dead * vp * 8; u += kSoft) {
+                        const unsigned to = sv + at.s * v_stage + (u >> 3) / dead * kPanelKv + (kKeys - dead + (u >> 3) % dead) * 128 + (u & 7) * 16;
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(to), "r"(0) : "memory");
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                }
+                tmem_st_wait();
+            }
+            before_sync();
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(w_full + at.s * 8) : "memory");
+            at.next(2);
+        }
+        l += both(n & 1, l);
+        const long long token = sq.start + first + tok;
+        if constexpr (LSE) {
+            if (live && ok && part == 0) p.lse[token * p.heads + head] = m + log2f(l);
+        } else {
+            if (ok && !mbar_wait(o_done, (unsigned)(n - 1) & 1)) ok = false;
+            after_sync();
+            float f = 1.f / l;
+            if (p.sink && live) {
+                const float s = sink_of(p, head) * kLog2e, top = fmaxf(m, s), keep = exp2f(m - top);
+                f = keep / (l * keep + exp2f(s - top));
+            }
+            if (live) f *= gate_of<bf16>(p, token, head);
+            bf16* out = (bf16*)p.out + (token * p.heads + head) * p.vdim;
+#pragma unroll 1
+            for (int c = part * 32; c < vp * 64; c += 64) {
+                unsigned v[32];
+                tmem_ld32(v, t_sum + lanes + c);
+                tmem_ld_wait();
+                if (live && ok) {
+#pragma unroll
+                    for (int e = 0; e < 32; e += 8)
+                        if (c + e < p.vdim) {
+                            uint4 q;
+                            q.x = pack_bf16(__uint_as_float(v[e]) * f, __uint_as_float(v[e + 1]) * f);
+                            q.y = pack_bf16(__uint_as_float(v[e + 2]) * f, __uint_as_float(v[e + 3]) * f);
+                            q.z = pack_bf16(__uint_as_float(v[e + 4]) * f, __uint_as_float(v[e + 5]) * f);
+                            q.w = pack_bf16(__uint_as_float(v[e + 6]) * f, __uint_as_float(v[e + 7]) * f);
+                            *reinterpret_cast<uint4*>(out + c + e) = q;
+                        }
+                }
+                __syncwarp();
+            }
+        }
+    }
+    if (!ok && lane == 0) report(p.err, ERR_WAIT_TIMEOUT, p.node, (long long)blockIdx.x, (long long)warp);
+    before_sync();
+    __syncthreads();
+    if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+}
+
+}  // namespace
+
+bool kv_prefill_fits(const PagedKvDesc& d, const TRef& keys, const TRef* values, int64_t out_off) {
+    const int64_t rows = keys.shape[0] * d.kv_heads * d.page;
+    return d.page >= kKeys && d.dim % 8 == 0 && d.dim <= 256 && d.heads / d.kv_heads <= kRows && rows < INT32_MAX && keys.buf.off % 16 == 0 &&
+           (!values || (d.vdim % 8 == 0 && d.vdim <= 256 && values->buf.off % 16 == 0 && out_off % 16 == 0));
+}
+
+void emit_kv_prefill(Emitter& em, const PagedKvDesc& d, const KvP& kv, const TRef& keys, const TRef* values, std::initializer_list<std::pair<size_t, Buf>> ptrs) {
+    PreP p{};
+    p.kv = kv;
+    p.kp = (int)((d.dim + 63) / 64);
+    p.vp = (int)((d.vdim + 63) / 64);
+    const int64_t tq = kRows / (d.heads / d.kv_heads), rows = keys.shape[0] * d.kv_heads * d.page;
+    const int smem = 1024 + p.kp * (int)(kPanelQ + 2 * kPanelKv) + (values ? p.vp * 2 * (int)kPanelKv : 0) + 112 + 4 * kRows * 4;
+    void (*const k)(const PreP) = values ? (kv.cap2 > 0.f ? paged_kv_prefill_tc<true, false> : paged_kv_prefill_tc<false, false>)
+                                         : (kv.cap2 > 0.f ? paged_kv_prefill_tc<true, true> : paged_kv_prefill_tc<false, true>);
+    ensure_max_dynamic_smem((const void*)k, 200 * 1024);
+    LaunchRec& rec = em.launch(k, dim3((unsigned)((kv.rows + tq - 1) / tq + kv.n_seqs), (unsigned)d.kv_heads), dim3(kThreads), (unsigned)smem, p, {},
+                               values ? "paged_kv_prefill" : "talk_lse", /*pdl=*/true);
+    for (auto& pr : ptrs) rec.relocs.push_back(Reloc{(uint32_t)(offsetof(PreP, kv) + pr.first), pr.second});
+    rec.tmaps.push_back(TmapReloc{(uint32_t)offsetof(PreP, maps), keys.buf, (uint64_t)d.dim, (uint64_t)rows, (uint64_t)d.dim * 2, 64u, (uint32_t)kKeys});
+    if (values)
+        rec.tmaps.push_back(TmapReloc{(uint32_t)offsetof(PreP, maps) + 128, values->buf, (uint64_t)d.vdim, (uint64_t)rows, (uint64_t)kv.ldv * 2, 64u, (uint32_t)kKeys});
+}
+
+}  // namespace oxk

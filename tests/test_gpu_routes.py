@@ -13,7 +13,7 @@ from onyxia_b200 import ir, llm, models
 from onyxia_b200.ir import HostTensor
 from gpu_util import cuda_backend, differential
 from lovuzen_util import to_bf16
-from test_gpu_kipizen import Experts
+from test_gpu_kipizen import Attention, Experts, piece, row_err
 from test_gpu_lovuzen import act, rel_err, run_linear
 
 pytestmark = pytest.mark.gpu
@@ -438,3 +438,25 @@ def test_logits_as_f32(model, vocab):
         want = raw[:written.value].view(np.float32 if model == "c1" else np.float16).astype(np.float32)
         got = b.step_logits([i])
         assert got.shape == (vocab,) and np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("heads,kv,dim,vdim,window,softcap,rising", [(4, 1, 256, 256, 0, 30.0, 0.0), (20, 1, 72, 136, 100, 0.0, 0.0), (3, 3, 128, 64, 0, 0.0, 0.3), (2, 1, 192, 200, 65, 0.0, 0.3),
+                                                                    (64, 1, 64, 64, 0, 4.0, 0.0), (5, 5, 16, 8, 1, 0.0, 0.0)])
+def test_prompts_over_pages_in_tensor_memory(heads, kv, dim, vdim, window, softcap, rising):
+    """Unwritten places of the pools hold no numbers. Tiles of 128 rows that heads do not fill evenly, two tokens per tile, portions that begin inside a page, windows that leave
+    tiles out, sums in either place of the tensor memory; scores that rise by more than 2^8 within a row, so that the sums are taken against a new maximum."""
+    T = 330
+    a = Attention("bf16", heads, kv, dim, vdim, scale=1.0 if rising else 2.0 / np.sqrt(dim), softcap=softcap, window=window, norm=int(not rising), sink=int(not rising))
+    a.pools = [a.s.upload(act(np.full((40, kv, 64, d), np.nan), ir.BF16)) for d in (dim, vdim)]
+    q, k, v = a.random(T)
+    if rising:
+        k = to_bf16(0.05 * k)
+        q[..., 0], k[..., 0] = 1.0, to_bf16(rising * np.arange(T))[:, None]
+    x, want, got, at = (q, k, v), a.want(q, k, v), [], 0
+    a.s.enable_profiling(True)
+    for n in (2, 129, 70, T - 201):
+        got.append(a.step([(0, *piece(x, at, at + n)), (8, *piece(x, at, at + 5))])[0])
+        at += n
+    assert any("paged_kv_prefill" == kernel for kernel, _, _ in a.s.take_timings())
+    err = row_err(np.concatenate(got), want)
+    assert np.isfinite(err).all() and err.max() < 1.5e-2, (int(err.argmax()), float(err.max()))
