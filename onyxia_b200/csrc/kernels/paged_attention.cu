@@ -6,13 +6,13 @@
 // and both products read the same tile: half the bytes of separate keys and values.
 //
 //   paged_prepare         query norm, temperature and scale → q'; the new keys and r go to the pool
-//   paged_attn_prefill    sequences with several new tokens: 64 (token, head) rows per CTA share each key tile; `mma.sync`,
-//                         online softmax
+//   paged_attn_prefill    sequences with several new tokens: on tcgen05 (paged_kv_prefill.cu) where a page holds 64 keys and more; here for
+//                         smaller pages: 64 (token, head) rows per CTA share each key tile; `mma.sync`, online softmax
 //   paged_attn_decode     sequences with one new token, keys split over CTAs and warps, all of the above in one launch
 //   paged_attn_simt       f32, and shapes the tensor-core kernels do not take
 //
 // Decode reads past · kv_heads · dim · 2 bytes (+ 4 per token) per sequence; prefill 4 · S · T · heads · dim FLOPs.
-#include "paged_util.cuh"
+#include "paged_kv.cuh"
 
 namespace oxk {
 
@@ -662,8 +662,27 @@ void emit_paged_attention(Emitter& em, const PagedAttnDesc& d, const TRef& proj,
     }
     if (!decode_only) {
         const int64_t tq = kPreRows / rep;
-        ensure_max_dynamic_smem((const void*)dc.prefill, 220 * 1024);
-        launch(dc.prefill, dim3((unsigned)((rows + tq - 1) / tq + n_seqs), (unsigned)d.kv_heads), kPreThreads, (unsigned)pre_smem, none, "paged_attn_prefill");
+        KvP kv{};
+        kv.rows = rows;
+        kv.n_seqs = p.n_seqs;
+        kv.width = p.width;
+        kv.n_pages = p.n_pages;
+        kv.shift = p.shift;
+        kv.heads = p.heads;
+        kv.kv_heads = p.kv_heads;
+        kv.dim = kv.vdim = p.dim;
+        kv.nd = p.nd;
+        kv.out_scale = p.out_scale;
+        kv.node = em.node;
+        if (kv_prefill_fits(kv, pool, &pool, out.buf.off) && key_scale.buf.off % 16 == 0) {
+            emit_kv_prefill(em, kv, pool, &pool,
+                            {{offsetof(KvP, kscale), key_scale.buf}, {offsetof(KvP, bias), bb}, {offsetof(KvP, q), q}, {offsetof(KvP, out), out.buf}, {offsetof(KvP, seqs), seqs.buf},
+                             {offsetof(KvP, table), pages.buf}, {offsetof(KvP, err), err}},
+                            "paged_attn_prefill");
+        } else {
+            ensure_max_dynamic_smem((const void*)dc.prefill, 220 * 1024);
+            launch(dc.prefill, dim3((unsigned)((rows + tq - 1) / tq + n_seqs), (unsigned)d.kv_heads), kPreThreads, (unsigned)pre_smem, none, "paged_attn_prefill");
+        }
     }
     if (decode_only || n_seqs > 1) {
         const int nh = rep > 8;  // two groups of eight heads per CTA

@@ -29,6 +29,11 @@ struct KvP {
     int norm, sink, append;
     int singles;                 // prepare: also sequences with one new token
     const float* temps;          // [heads]: factors of the scores, or null
+    // keys that are the values, as they were projected (paged_attention.cu): a factor per key [pages, page], scores added by distance [heads, nd] (null: none), a
+    // factor of the results
+    const float *kscale, *bias;
+    int nd;
+    float out_scale;
     float* lse;                  // [rows, heads]: base-2 logarithm of the softmax's sum (the prefill kernel's form that has no values)
 };
 
@@ -59,8 +64,8 @@ template <typename T> __device__ __forceinline__ float head_factor(const KvP& p,
 void emit_talking_heads(Emitter&, const PagedKvDesc&, KvP p, const TRef& proj, const TRef& turns, Buf q, const TRef& keys, const TRef& values,
                         const TRef& seqs, const TRef& pages, const TRef& out);
 // Prompts on tcgen05 (paged_kv_prefill.cu), with values or, without, `lse` only; `ptrs`: fields of KvP by their offset.
-bool kv_prefill_fits(const PagedKvDesc&, const TRef& keys, const TRef* values, int64_t out_off);
-void emit_kv_prefill(Emitter&, const PagedKvDesc&, const KvP&, const TRef& keys, const TRef* values, std::initializer_list<std::pair<size_t, Buf>> ptrs);
+bool kv_prefill_fits(const KvP&, const TRef& keys, const TRef* values, int64_t out_off);
+void emit_kv_prefill(Emitter&, const KvP&, const TRef& keys, const TRef* values, std::initializer_list<std::pair<size_t, Buf>> ptrs, const char* label);
 // The form of the prefill kernel that leaves `lse` only.
 void emit_kv_lse(Emitter&, const PagedKvDesc&, KvP p, Buf q, Buf lse, const TRef& keys, const TRef& seqs, const TRef& pages);
 

@@ -654,10 +654,11 @@ void emit_paged_kv_attention(Emitter& em, const PagedKvDesc& d, const TRef& proj
     }
     if (!decode_only) {
         const int64_t tq = kPreRows / rep;
-        if (kv_prefill_fits(d, keys, &values, out.buf.off)) {
-            emit_kv_prefill(em, d, p, keys, &values,
+        if (kv_prefill_fits(p, keys, &values, out.buf.off)) {
+            emit_kv_prefill(em, p, keys, &values,
                             {{offsetof(KvP, keys), keys.buf}, {offsetof(KvP, values), values.buf}, {offsetof(KvP, q), q}, {offsetof(KvP, sinks), sink}, {offsetof(KvP, temps), temps},
-                             {offsetof(KvP, gate), gate}, {offsetof(KvP, out), out.buf}, {offsetof(KvP, seqs), seqs.buf}, {offsetof(KvP, table), pages.buf}, {offsetof(KvP, err), Buf{kSlotErr, 0}}});
+                             {offsetof(KvP, gate), gate}, {offsetof(KvP, out), out.buf}, {offsetof(KvP, seqs), seqs.buf}, {offsetof(KvP, table), pages.buf}, {offsetof(KvP, err), Buf{kSlotErr, 0}}},
+                            "paged_kv_prefill");
         } else {
             ensure_max_dynamic_smem((const void*)dc.prefill, 220 * 1024);
             launch(dc.prefill, dim3((unsigned)((rows + tq - 1) / tq + n_seqs), (unsigned)d.kv_heads), kPreThreads, (unsigned)dc.pre_smem, none, "paged_kv_prefill");
@@ -692,9 +693,9 @@ void emit_kv_lse(Emitter& em, const PagedKvDesc& d, KvP p, Buf q, Buf lse, const
     const DimChoice dc = dim_choice(d.dim);
     const int64_t tq = kPreRows / (d.heads / d.kv_heads);
     const Buf none{kSlotNull, 0}, temps = d.temps ? d.temps->buf : none;
-    if (kv_prefill_fits(d, keys, nullptr, 0))
-        return emit_kv_prefill(em, d, p, keys, nullptr, {{offsetof(KvP, keys), keys.buf}, {offsetof(KvP, q), q}, {offsetof(KvP, temps), temps}, {offsetof(KvP, lse), lse}, {offsetof(KvP, seqs), seqs.buf},
-                                                         {offsetof(KvP, table), pages.buf}, {offsetof(KvP, err), Buf{kSlotErr, 0}}});
+    if (kv_prefill_fits(p, keys, nullptr, 0))
+        return emit_kv_prefill(em, p, keys, nullptr, {{offsetof(KvP, keys), keys.buf}, {offsetof(KvP, q), q}, {offsetof(KvP, temps), temps}, {offsetof(KvP, lse), lse}, {offsetof(KvP, seqs), seqs.buf},
+                                                         {offsetof(KvP, table), pages.buf}, {offsetof(KvP, err), Buf{kSlotErr, 0}}}, "talk_lse");
     ensure_max_dynamic_smem((const void*)dc.lse, 220 * 1024);
     em.launch(dc.lse, dim3((unsigned)((p.rows + tq - 1) / tq + p.n_seqs), (unsigned)d.kv_heads), dim3(kPreThreads), (unsigned)dc.lse_smem, p,
               {{&p.keys, keys.buf}, {&p.values, none}, {&p.q, q}, {&p.temps, temps}, {&p.lse, lse}, {&p.seqs, seqs.buf}, {&p.table, pages.buf}, {&p.err, Buf{kSlotErr, 0}}},

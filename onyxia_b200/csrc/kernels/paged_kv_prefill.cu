@@ -6,7 +6,8 @@
 //
 // What bounds it is the chain of a step, about 1.3 µs in a CTA alone on its SM (256 dimensions: shared memory), of which the products are 0.7; a short prompt's longest tiles are as long
 // as the launch. The `mma.sync` kernel, which remains for pages of less than 64 keys, had four warps per SM at this size. µs, before → now: 4096 tokens, 4 heads of 256 over one key
-// head, capped 245 → 91 (rows by one thread each: 104); 1999 tokens, the same 127 → 49; 2048 tokens, 16 heads of 128 over 4, the softmax's sums alone 94 → 35.
+// head, capped 245 → 91 (rows by one thread each: 104); 1999 tokens, the same 127 → 49; 2048 tokens, 16 heads of 128 over 4, the softmax's sums alone 94 → 35; keys that are the
+// values, 32 heads of 128 over 16, four portions of 2048 tokens 2862 → 846.
 #include "paged_kv.cuh"
 
 namespace oxk {
@@ -64,20 +65,24 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 __device__ __forceinline__ void before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// CAPPED: scores are capped. LSE: no values; the softmax's sums are the result.
-template <bool CAPPED, bool LSE> __global__ void __launch_bounds__(kThreads, 2) paged_kv_prefill_tc(const __grid_constant__ PreP pp) {
+// KEYS: keys are the values, scores have a factor per key and an addend by distance. LSE: no values; the softmax's sums are the result.
+enum : int { FORM_PLAIN, FORM_CAPPED, FORM_KEYS };
+template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) paged_kv_prefill_tc(const __grid_constant__ PreP pp) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const KvP& p = pp.kv;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kp = pp.kp, vp = LSE ? 0 : pp.vp;
+    constexpr bool KEYS = FORM == FORM_KEYS;
+    constexpr int NS = KEYS ? 3 : 2;  // tiles on their way: keys that are values are kept until both products have read them
     const unsigned k_stage = kp * kPanelKv, v_stage = vp * kPanelKv;
-    const unsigned sq0 = smem_u32(smem), sk = sq0 + kp * kPanelQ, sv = sk + 2 * k_stage, bars = sv + 2 * v_stage;
-    // two barriers each: keys there, free, values there, free, scores there, weights there; and one for the sums
-    const unsigned k_full = bars, k_free = bars + 16, v_full = bars + 32, v_free = bars + 48, s_full = bars + 64, w_full = bars + 80, o_done = bars + 96;
-    unsigned* tmem_slot = reinterpret_cast<unsigned*>(smem + (bars + 104 - sq0));
-    float* shared = reinterpret_cast<float*>(smem + (bars + 112 - sq0));  // [turn][half of the keys][row]: what the two threads of a row tell each other
+    const unsigned sq0 = smem_u32(smem), sk = sq0 + kp * kPanelQ, sv = KEYS ? sk : sk + NS * k_stage, bars = sk + NS * k_stage + (KEYS ? 0 : NS * v_stage);
+    // barriers: keys there, free (three each), values there, free, scores there, weights there (two each), sums
+    const unsigned k_full = bars, k_free = bars + 24, v_full = KEYS ? k_full : bars + 48, v_free = bars + 64, s_full = bars + 80, w_full = bars + 96, o_done = bars + 112;
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(smem + (bars + 120 - sq0));
+    float* shared = reinterpret_cast<float*>(smem + (bars + 128 - sq0));  // [turn][half of the keys][row]: what the two threads of a row tell each other
+    float *scale_s = shared + 4 * kRows, *bias_s = scale_s + NS * kKeys;  // KEYS: [tile][key], [head][distance]
     if (tid == 0) {
-        for (int i = 0; i < 13; i++) mbar_init(bars + i * 8, i == 10 || i == 11 ? kSoft / 32 : 1);
+        for (int i = 0; i < 15; i++) mbar_init(bars + i * 8, i == 12 || i == 13 ? kSoft / 32 : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     pdl_wait();
@@ -101,6 +106,9 @@ template <bool CAPPED, bool LSE> __global__ void __launch_bounds__(kThreads, 2) 
         cp_async16(sq0 + (c >> 3) * kPanelQ + r * 128 + (((c & 7) ^ (r & 7)) << 4), live ? src + ((long long)(sq.start + first + tok) * p.heads + h) * p.dim + c * 8 : src, live);
     }
     cp_async_commit();
+    if constexpr (KEYS)
+        if (p.bias)
+            for (int i = tid; i < rep * p.nd; i += kThreads) bias_s[i] = p.bias[(long long)g * rep * p.nd + i] * kLog2e;
     cp_async_wait<0>();
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads them
     before_sync();
@@ -114,15 +122,21 @@ template <bool CAPPED, bool LSE> __global__ void __launch_bounds__(kThreads, 2) 
     if (warp == 8) {
         RingAt at;
         for (int i = 0; i < n && ok; i++) {
-            const int j0 = (kt0 + i) * kKeys, row = (int)key_row(p, page_of(p, seq, j0), g, j0);
-            if (i >= 2 && !mbar_wait(k_free + at.s * 8, at.parity ^ 1)) ok = false;
+            const int j0 = (kt0 + i) * kKeys;
+            const long long pg = page_of(p, seq, j0);
+            const int row = (int)key_row(p, pg, g, j0);
+            if (i >= NS && !mbar_wait(k_free + at.s * 8, at.parity ^ 1)) ok = false;
             if (ok && elect_one()) {
-                mbar_expect_tx(k_full + at.s * 8, k_stage);
+                mbar_expect_tx(k_full + at.s * 8, k_stage + (KEYS ? kKeys * 4 : 0));
+                if constexpr (KEYS)  // a page's factors follow one another
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(scale_s + at.s * kKeys)),
+                                 "l"(p.kscale + (pg << p.shift) + (j0 & ((1 << p.shift) - 1))), "r"(kKeys * 4), "r"(k_full + at.s * 8)
+                                 : "memory");
                 for (int c = 0; c < kp; c++) tma_load_2d(sk + at.s * k_stage + c * kPanelKv, pp.maps[0], c * 64, row, k_full + at.s * 8);
             }
             __syncwarp();
-            if constexpr (!LSE) {
-                if (i >= 2 && ok && !mbar_wait(v_free + at.s * 8, at.parity ^ 1)) ok = false;
+            if constexpr (!LSE && !KEYS) {
+                if (i >= NS && ok && !mbar_wait(v_free + at.s * 8, at.parity ^ 1)) ok = false;
                 if (ok && elect_one()) {
                     mbar_expect_tx(v_full + at.s * 8, v_stage);
                     for (int c = 0; c < vp; c++) tma_load_2d(sv + at.s * v_stage + c * kPanelKv, pp.maps[1], c * 64, row, v_full + at.s * 8);
@@ -130,25 +144,26 @@ template <bool CAPPED, bool LSE> __global__ void __launch_bounds__(kThreads, 2) 
                 __syncwarp();
             }
             ok = __all_sync(0xffffffffu, ok);
-            at.next(2);
+            at.next(NS);
         }
     } else if (warp == 9) {
         const unsigned base = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);  // bf16 × bf16 → f32, M 128
         const unsigned by_keys = base | ((kKeys >> 3) << 17), by_values = base | (1u << 16) | ((unsigned)(vp * 8) << 17);  // the values' wide axis is the result's
         const unsigned long long dq = umma_kmajor_desc(sq0), dk = umma_kmajor_desc(sk), dv = umma_wide_desc(sv);
-        RingAt ahead, at;
+        RingAt tile_ahead, ahead, tile, at;  // tiles, and turns of scores and weights
         auto scores = [&] {
-            if (ok && !mbar_wait(k_full + ahead.s * 8, ahead.parity)) ok = false;
+            if (ok && !mbar_wait(k_full + tile_ahead.s * 8, tile_ahead.parity)) ok = false;
             after_sync();
             if (ok && elect_one()) {
-                const unsigned long long k = dk + ahead.s * (k_stage >> 4);
+                const unsigned long long k = dk + tile_ahead.s * (k_stage >> 4);
                 for (int c = 0; c < kp; c++)
 #pragma unroll
                     for (int e = 0; e < 4; e++) umma_bf16(tmem + ahead.s * kKeys, dq + c * (kPanelQ >> 4) + e * 2, k + c * (kPanelKv >> 4) + e * 2, by_keys, c > 0 || e > 0);
-                umma_commit(k_free + ahead.s * 8);
+                if (!KEYS) umma_commit(k_free + tile_ahead.s * 8);
                 umma_commit(s_full + ahead.s * 8);
             }
             __syncwarp();
+            tile_ahead.next(NS);
             ahead.next(2);
         };
         scores();
@@ -160,17 +175,18 @@ template <bool CAPPED, bool LSE> __global__ void __launch_bounds__(kThreads, 2) 
             }
             if (ok && !mbar_wait(w_full + at.s * 8, at.parity)) ok = false;
             if constexpr (!LSE) {
-                if (ok && !mbar_wait(v_full + at.s * 8, at.parity)) ok = false;
+                if (ok && !mbar_wait(v_full + tile.s * 8, tile.parity)) ok = false;
                 after_sync();
                 if (ok && elect_one()) {
-                    const unsigned long long v = dv + at.s * (v_stage >> 4);
+                    const unsigned long long v = dv + tile.s * (v_stage >> 4);
 #pragma unroll
                     for (int e = 0; e < kKeys / 16; e++) umma_weights(t_sum, t_weights + at.s * weights_turn + e * 8, v + e * 128, by_values, i > 0 || e > 0);
-                    umma_commit(v_free + at.s * 8);
+                    umma_commit((KEYS ? k_free : v_free) + tile.s * 8);
                     umma_commit(o_done);
                 }
                 __syncwarp();
             }
+            tile.next(NS);
             at.next(2);
         }
     } else {
@@ -187,21 +203,38 @@ template <bool CAPPED, bool LSE> __global__ void __launch_bounds__(kThreads, 2) 
             asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 3)) : "memory");
             return at[(part ^ 1) * kRows];
         };
-        float m = kNoScore, l = 0.f;
-        RingAt at;
+        const float* bias = bias_s + r % rep * p.nd;
+        float m = KEYS ? -INFINITY : kNoScore, l = 0.f;  // KEYS: key 0 is there for every row
+        RingAt at, tile;
         for (int i = 0; i < n; i++) {
             const int j0 = (kt0 + i) * kKeys, mine0 = j0 + part * kHalf;
             if (ok && !mbar_wait(s_full + at.s * 8, at.parity)) ok = false;
+            if constexpr (KEYS)  // the factors
+                if (ok && !mbar_wait(k_full + tile.s * 8, tile.parity)) ok = false;
             after_sync();
             float s[kHalf];
             {
                 unsigned v[32];
                 tmem_ld32(v, tmem + lanes + at.s * kKeys + part * kHalf);
                 tmem_ld_wait();
+                if constexpr (KEYS) {
+                    const float* f = scale_s + tile.s * kKeys + part * kHalf;
 #pragma unroll
-                for (int e = 0; e < kHalf; e++) {
-                    const float x = __uint_as_float(v[e]) * mul2;
-                    s[e] = CAPPED ? cap2 - __fdividef(2.f * cap2, 1.f + exp2f(x)) : x;
+                    for (int e = 0; e < kHalf; e++) s[e] = __uint_as_float(v[e]) * f[e];
+                    if (p.bias && pos0 - (j0 + kKeys - 1) >= p.nd - 1) {  // one addend per head for the whole tile
+                        const float far = bias[p.nd - 1];
+#pragma unroll
+                        for (int e = 0; e < kHalf; e++) s[e] += far;
+                    } else if (p.bias) {
+#pragma unroll
+                        for (int e = 0; e < kHalf; e++) s[e] += bias[min(max(pos - (mine0 + e), 0), p.nd - 1)];
+                    }
+                } else {
+#pragma unroll
+                    for (int e = 0; e < kHalf; e++) {
+                        const float x = __uint_as_float(v[e]) * mul2;
+                        s[e] = FORM == FORM_CAPPED ? cap2 - __fdividef(2.f * cap2, 1.f + exp2f(x)) : x;
+                    }
                 }
             }
             if (j0 + kKeys - 1 > pos0 || j0 < last_low) {
@@ -245,10 +278,10 @@ template <bool CAPPED, bool LSE> __global__ void __launch_bounds__(kThreads, 2) 
                 // before these scores.
                 tmem_st16(t_weights + lanes + at.s * weights_turn + part * (kHalf / 2), w);
                 if (j0 + kKeys - 1 > last) {  // what lies behind the last key may be no number, which a weight of 0 would not cancel
-                    if (ok && !mbar_wait(v_full + at.s * 8, at.parity)) ok = false;
+                    if (ok && !mbar_wait(v_full + tile.s * 8, tile.parity)) ok = false;
                     const int dead = j0 + kKeys - 1 - last;
                     for (int u = tid; u < dead * vp * 8; u += kSoft) {
-                        const unsigned to = sv + at.s * v_stage + (u >> 3) / dead * kPanelKv + (kKeys - dead + (u >> 3) % dead) * 128 + (u & 7) * 16;
+                        const unsigned to = sv + tile.s * v_stage + (u >> 3) / dead * kPanelKv + (kKeys - dead + (u >> 3) % dead) * 128 + (u & 7) * 16;
                         asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(to), "r"(0) : "memory");
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -258,6 +291,7 @@ template <bool CAPPED, bool LSE> __global__ void __launch_bounds__(kThreads, 2) 
             before_sync();
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(w_full + at.s * 8) : "memory");
+            tile.next(NS);
             at.next(2);
         }
         l += both(n & 1, l);
@@ -268,11 +302,12 @@ template <bool CAPPED, bool LSE> __global__ void __launch_bounds__(kThreads, 2) 
             if (ok && !mbar_wait(o_done, (unsigned)(n - 1) & 1)) ok = false;
             after_sync();
             float f = 1.f / l;
-            if (p.sink && live) {
+            if (!KEYS && p.sink && live) {
                 const float s = sink_of(p, head) * kLog2e, top = fmaxf(m, s), keep = exp2f(m - top);
                 f = keep / (l * keep + exp2f(s - top));
             }
-            if (live) f *= gate_of<bf16>(p, token, head);
+            if (KEYS) f *= p.out_scale;
+            else if (live) f *= gate_of<bf16>(p, token, head);
             bf16* out = (bf16*)p.out + (token * p.heads + head) * p.vdim;
 #pragma unroll 1
             for (int c = part * 32; c < vp * 64; c += 64) {
@@ -303,28 +338,36 @@ template <bool CAPPED, bool LSE> __global__ void __launch_bounds__(kThreads, 2) 
 
 }  // namespace
 
-bool kv_prefill_fits(const PagedKvDesc& d, const TRef& keys, const TRef* values, int64_t out_off) {
-    const int64_t rows = keys.shape[0] * d.kv_heads * d.page;
-    return d.page >= kKeys && d.dim % 8 == 0 && d.dim <= 256 && d.heads / d.kv_heads <= kRows && rows < INT32_MAX && keys.buf.off % 16 == 0 &&
-           (!values || (d.vdim % 8 == 0 && d.vdim <= 256 && values->buf.off % 16 == 0 && out_off % 16 == 0));
+static int prefill_smem(const KvP& kv, bool keys, bool lse) {
+    const int kp = (kv.dim + 63) / 64, vp = (kv.vdim + 63) / 64, tiles = keys ? 3 : 2;
+    return 1024 + kp * (int)(kPanelQ + tiles * kPanelKv) + (keys || lse ? 0 : vp * tiles * (int)kPanelKv) + 128 + 4 * kRows * 4 +
+           (keys ? tiles * kKeys * 4 + kv.heads / kv.kv_heads * kv.nd * 4 : 0);
 }
 
-void emit_kv_prefill(Emitter& em, const PagedKvDesc& d, const KvP& kv, const TRef& keys, const TRef* values, std::initializer_list<std::pair<size_t, Buf>> ptrs) {
+bool kv_prefill_fits(const KvP& kv, const TRef& keys, const TRef* values, int64_t out_off) {
+    const int64_t rows = (int64_t)kv.n_pages * kv.kv_heads << kv.shift;
+    return 1 << kv.shift >= kKeys && kv.dim % 8 == 0 && kv.dim <= 256 && kv.heads / kv.kv_heads <= kRows && rows < INT32_MAX && keys.buf.off % 16 == 0 &&
+           (!values || (kv.vdim % 8 == 0 && kv.vdim <= 256 && values->buf.off % 16 == 0 && out_off % 16 == 0)) &&
+           prefill_smem(kv, values == &keys, !values) <= 200 * 1024;
+}
+
+// `values` = &keys: the form whose keys are the values.
+void emit_kv_prefill(Emitter& em, const KvP& kv, const TRef& keys, const TRef* values, std::initializer_list<std::pair<size_t, Buf>> ptrs, const char* label) {
     PreP p{};
     p.kv = kv;
-    p.kp = (int)((d.dim + 63) / 64);
-    p.vp = (int)((d.vdim + 63) / 64);
-    const int64_t tq = kRows / (d.heads / d.kv_heads), rows = keys.shape[0] * d.kv_heads * d.page;
-    const int smem = 1024 + p.kp * (int)(kPanelQ + 2 * kPanelKv) + (values ? p.vp * 2 * (int)kPanelKv : 0) + 112 + 4 * kRows * 4;
-    void (*const k)(const PreP) = values ? (kv.cap2 > 0.f ? paged_kv_prefill_tc<true, false> : paged_kv_prefill_tc<false, false>)
-                                         : (kv.cap2 > 0.f ? paged_kv_prefill_tc<true, true> : paged_kv_prefill_tc<false, true>);
+    p.kp = (kv.dim + 63) / 64;
+    p.vp = (kv.vdim + 63) / 64;
+    const int64_t tq = kRows / (kv.heads / kv.kv_heads), rows = (int64_t)kv.n_pages * kv.kv_heads << kv.shift;
+    void (*const k)(const PreP) = values == &keys   ? paged_kv_prefill_tc<FORM_KEYS, false>
+                                  : kv.cap2 > 0.f ? (values ? paged_kv_prefill_tc<FORM_CAPPED, false> : paged_kv_prefill_tc<FORM_CAPPED, true>)
+                                                  : (values ? paged_kv_prefill_tc<FORM_PLAIN, false> : paged_kv_prefill_tc<FORM_PLAIN, true>);
     ensure_max_dynamic_smem((const void*)k, 200 * 1024);
-    LaunchRec& rec = em.launch(k, dim3((unsigned)((kv.rows + tq - 1) / tq + kv.n_seqs), (unsigned)d.kv_heads), dim3(kThreads), (unsigned)smem, p, {},
-                               values ? "paged_kv_prefill" : "talk_lse", /*pdl=*/true);
+    LaunchRec& rec = em.launch(k, dim3((unsigned)((kv.rows + tq - 1) / tq + kv.n_seqs), (unsigned)kv.kv_heads), dim3(kThreads),
+                               (unsigned)prefill_smem(kv, values == &keys, !values), p, {}, label, /*pdl=*/true);
     for (auto& pr : ptrs) rec.relocs.push_back(Reloc{(uint32_t)(offsetof(PreP, kv) + pr.first), pr.second});
-    rec.tmaps.push_back(TmapReloc{(uint32_t)offsetof(PreP, maps), keys.buf, (uint64_t)d.dim, (uint64_t)rows, (uint64_t)d.dim * 2, 64u, (uint32_t)kKeys});
-    if (values)
-        rec.tmaps.push_back(TmapReloc{(uint32_t)offsetof(PreP, maps) + 128, values->buf, (uint64_t)d.vdim, (uint64_t)rows, (uint64_t)kv.ldv * 2, 64u, (uint32_t)kKeys});
+    rec.tmaps.push_back(TmapReloc{(uint32_t)offsetof(PreP, maps), keys.buf, (uint64_t)kv.dim, (uint64_t)rows, (uint64_t)kv.dim * 2, 64u, (uint32_t)kKeys});
+    if (values && values != &keys)
+        rec.tmaps.push_back(TmapReloc{(uint32_t)offsetof(PreP, maps) + 128, values->buf, (uint64_t)kv.vdim, (uint64_t)rows, (uint64_t)kv.ldv * 2, 64u, (uint32_t)kKeys});
 }
 
 }  // namespace oxk

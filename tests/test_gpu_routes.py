@@ -9,12 +9,13 @@ import pytest
 
 import mufevik_ref as ref
 from onyxia_b200 import backend as be
-from onyxia_b200 import ir, llm, models
+from onyxia_b200 import ir, llm, lovuzen, models
 from onyxia_b200.ir import HostTensor
 from gpu_util import cuda_backend, differential
 from lovuzen_util import to_bf16
 from test_gpu_kipizen import Attention, Experts, piece, row_err
-from test_gpu_lovuzen import act, rel_err, run_linear
+import test_gpu_lovuzen
+from test_gpu_lovuzen import act, attention_want, rel_err, run_linear
 
 pytestmark = pytest.mark.gpu
 
@@ -460,3 +461,22 @@ def test_prompts_over_pages_in_tensor_memory(heads, kv, dim, vdim, window, softc
     assert any("paged_kv_prefill" == kernel for kernel, _, _ in a.s.take_timings())
     err = row_err(np.concatenate(got), want)
     assert np.isfinite(err).all() and err.max() < 1.5e-2, (int(err.argmax()), float(err.max()))
+
+
+@pytest.mark.parametrize("heads,kv,dim,far", [(32, 16, 128, 128), (20, 1, 72, 40), (2, 1, 256, 300)])
+def test_prompts_whose_keys_are_their_values(heads, kv, dim, far):
+    """Unwritten places of the pool and of its factors hold no numbers; tiles nearer than the farthest addend, across it and behind it; three tiles in the ring."""
+    r, T, rows = np.random.default_rng(dim), 420, 12
+    q, k = to_bf16(r.standard_normal((T, heads, dim))), to_bf16(r.standard_normal((T, kv, dim)))
+    q_w, k_w, bias = to_bf16(1 + 0.3 * r.standard_normal(heads * dim)), to_bf16(1 + 0.3 * r.standard_normal(kv * dim)), r.standard_normal((rows, heads))
+    kw = dict(scale=2.0 / np.sqrt(dim), temp=(0.4, 30))
+    a = test_gpu_lovuzen.Attention("bf16", heads, kv, dim, lovuzen.distance_bias(bias, far), q_w, k_w, **kw)
+    a.pool = a.s.upload(act(np.full(a.pool.shape, np.nan), ir.BF16))
+    a.scales = a.s.upload(HostTensor.from_numpy(np.full(a.scales.shape, np.nan, np.float32)))
+    got, at = [], 0
+    for n in (3, 130, T - 133):
+        got.append(a.step([(0, q[at:at + n], k[at:at + n]), (8, q[at:at + 5], k[at:at + 5])])[0])
+        at += n
+    got, want = np.concatenate(got), attention_want(q, k, bias, far, q_w, k_w, **kw)
+    err = np.sqrt(((got - want) ** 2).mean(axis=(1, 2))) / np.sqrt((want ** 2).mean())
+    assert np.isfinite(err).all() and err.max() < 1e-2, (int(err.argmax()), float(err.max()))
