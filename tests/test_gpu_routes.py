@@ -480,3 +480,24 @@ def test_prompts_whose_keys_are_their_values(heads, kv, dim, far):
     got, want = np.concatenate(got), attention_want(q, k, bias, far, q_w, k_w, **kw)
     err = np.sqrt(((got - want) ** 2).mean(axis=(1, 2))) / np.sqrt((want ** 2).mean())
     assert np.isfinite(err).all() and err.max() < 1e-2, (int(err.argmax()), float(err.max()))
+
+
+@pytest.mark.parametrize("width", [4, 1020, 1028, 3072, 4100, 6144, 6148])
+def test_residual_norms_of_rows_in_registers(width):
+    """Widths at the ends of a thread's packs and beyond them; everything that a norm in front of or behind the sum can take. f32 sums of at most 6148 squares."""
+    r, rows, of, eps = np.random.default_rng(width), 5, HostTensor.from_numpy, 1e-4
+    t = {n: r.standard_normal((rows, width)).astype(np.float32) for n in ("y", "res", "add", "gate")}
+    v = {n: (1 + 0.2 * r.standard_normal(width)).astype(np.float32) for n in ("w", "gain", "post", "offset")}
+    x = {n: a.astype(np.float64) for n, a in {**t, **v}.items()}
+    for pre in (0, 1):
+        b = ir.GraphBuilder()
+        i = {n: b.input(n, ir.F32, [rows, width]) for n in t}
+        if pre:
+            ins, attrs = [i["y"], b.constant(of(v["w"])), i["res"], b.constant(of(v["post"])), i["add"], b.constant(of(v["offset"]))], {"residual": 1, "post": 1, "add": 1, "offset": 1, "add_scale": 0.3}
+            want = ref.rms_norm(ref.rms_norm(x["y"], x["post"], eps) + x["res"] + 0.3 * x["add"] + x["offset"], x["w"], eps)
+        else:
+            ins, attrs = [i["y"], b.constant(of(v["w"])), i["res"], b.constant(of(v["gain"])), i["gate"]], {"residual": 1, "gain": 1, "gate": 1, "gate_offset": 0}
+            want = ref.rms_norm(x["y"], x["w"], eps) * x["gain"] * x["gate"] + x["res"]
+        b.output("out", b.composite("onyxia.ResidualNorm", dict(attrs, epsilon=eps, pre=pre), ins, [(ir.F32, [rows, width])])[0])
+        got = be.run_once(cuda_backend(), b.finish(), {n: of(a) for n, a in t.items()})[0][1].numpy()
+        assert rel_err(got, want) < 1e-6, pre
