@@ -501,3 +501,15 @@ def test_residual_norms_of_rows_in_registers(width):
         b.output("out", b.composite("onyxia.ResidualNorm", dict(attrs, epsilon=eps, pre=pre), ins, [(ir.F32, [rows, width])])[0])
         got = be.run_once(cuda_backend(), b.finish(), {n: of(a) for n, a in t.items()})[0][1].numpy()
         assert rel_err(got, want) < 1e-6, pre
+
+
+@pytest.mark.parametrize("dtype,shape,axis", [(np.float16, (50, 24), 0), (np.float16, (50, 23), 0), (np.int64, (7, 2), 0), (np.int64, (7, 3), 0), (np.uint8, (9, 16), 0), (np.uint8, (9, 5), 0),
+                                              (np.float32, (3, 11, 8), 1), (np.float32, (3, 11, 6), 1), (np.float32, (6, 40), 1), (np.float16, (5, 7000), 0)])
+def test_slices_gathered_in_units(dtype, shape, axis):
+    """Slices of whole 16-byte units and others, along the first axis and behind it, indexes counted from the end."""
+    r = np.random.default_rng(len(shape))
+    data, idx = r.integers(0, 100, shape).astype(dtype), r.integers(-shape[axis], shape[axis], (3, 7)).astype(np.int64)
+    b = ir.GraphBuilder()
+    b.output("y", b.gather(b.constant(HostTensor.from_numpy(data)), b.input("i", ir.I64, [3, 7]), axis=axis))
+    got = be.run_once(cuda_backend(), b.finish(), {"i": HostTensor.from_numpy(idx)})[0][1].numpy()
+    assert np.array_equal(got, np.take(data, np.where(idx < 0, idx + shape[axis], idx), axis=axis))
