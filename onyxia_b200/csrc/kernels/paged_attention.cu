@@ -92,8 +92,9 @@ template <typename T> __global__ void __launch_bounds__(128) paged_prepare(const
 }
 
 // ───────────────────────────── any shape ────────────────────────────────
-// One CTA per (row, head); key chunks of 128.
-template <typename T> __global__ void __launch_bounds__(128) paged_attn_simt(const PagedP p) {
+// One CTA per (row, head); key chunks of 128, two threads per key, a thread per value dimension. Loads one behind the
+// other are what it takes: with 128 threads, a whole key and two dimensions each, 34 launches over 3 sequences of 100 tokens, 4 heads of 256, took 36.5 µs each, now 19.7.
+template <typename T> __global__ void __launch_bounds__(kAnyThreads) paged_attn_simt(const PagedP p) {
     extern __shared__ float sm[];  // q[dim], acc[dim], w[128]
     __shared__ float red[32];
     pdl_enter();
@@ -102,32 +103,32 @@ template <typename T> __global__ void __launch_bounds__(128) paged_attn_simt(con
     if (row >= sq.start + sq.len) return;
     const int pos = sq.past + row - sq.start, g = h / (p.heads / p.kv_heads);
     float *q = sm, *acc = sm + p.dim, *w = acc + p.dim;
-    for (int i = tid; i < p.dim; i += 128) {
+    for (int i = tid; i < p.dim; i += kAnyThreads) {
         q[i] = to_f(((const T*)p.q)[((long long)row * p.heads + h) * p.dim + i]);
         acc[i] = 0.f;
     }
     float m = -INFINITY, l = 0.f;
     __syncthreads();
     for (int j0 = 0; j0 <= pos; j0 += 128) {
-        const int j = j0 + tid;
+        const int j = j0 + (tid >> 1), half = tid & 1;
         float sc = -INFINITY;
+        const long long pg = j <= pos ? page_of(p, s, j) : 0;
+        float d = j <= pos ? dot_of_half(q, (const T*)p.pool + key_row(p, pg, g, j) * p.dim, p.dim, half) : 0.f;
+        d += __shfl_xor_sync(0xffffffffu, d, 1);
         if (j <= pos) {
-            const long long pg = page_of(p, s, j);
-            const T* k = (const T*)p.pool + key_row(p, pg, g, j) * p.dim;
-            const float d = dot_in_order(q, k, p.dim, 0.f);
             sc = d * p.kscale[scale_at(p, pg, j)];
             if (p.bias) sc += p.bias[(long long)h * p.nd + min(pos - j, p.nd - 1)];
         }
         const float m2 = fmaxf(m, block_max(sc, red));
         const float e = expf(sc - m2), keep = expf(m - m2);
-        w[tid] = e;
-        l = l * keep + block_sum(e, red);  // (its barriers order the stores to w)
+        if (half == 0) w[tid >> 1] = e;
+        l = l * keep + block_sum(half == 0 ? e : 0.f, red);  // (its barriers order the stores to w)
         m = m2;
         const int live = min(128, pos + 1 - j0);
-        for (int i = tid; i < p.dim; i += 128) acc[i] = weigh_in_order(p, (const T*)p.pool, s, g, j0, live, p.dim, i, w, acc[i] * keep);
+        for (int i = tid; i < p.dim; i += kAnyThreads) acc[i] = weigh_in_order(p, (const T*)p.pool, s, g, j0, live, p.dim, i, w, acc[i] * keep);
         __syncthreads();
     }
-    for (int i = tid; i < p.dim; i += 128) ((T*)p.out)[((long long)row * p.heads + h) * p.dim + i] = from_f<T>(acc[i] / l * p.out_scale);
+    for (int i = tid; i < p.dim; i += kAnyThreads) ((T*)p.out)[((long long)row * p.heads + h) * p.dim + i] = from_f<T>(acc[i] / l * p.out_scale);
 }
 
 // ───────────────────────────── prefill ──────────────────────────────────
@@ -657,7 +658,7 @@ void emit_paged_attention(Emitter& em, const PagedAttnDesc& d, const TRef& proj,
         const unsigned smem = (unsigned)((2 * d.dim + 128) * 4);
         const PagedKernel k = bf ? paged_attn_simt<bf16> : paged_attn_simt<float>;
         ensure_max_dynamic_smem((const void*)k, 220 * 1024);
-        launch(k, dim3((unsigned)rows, (unsigned)d.heads), 128, smem, none, "paged_attn_simt");
+        launch(k, dim3((unsigned)rows, (unsigned)d.heads), kAnyThreads, smem, none, "paged_attn_simt");
         return;
     }
     if (!decode_only) {

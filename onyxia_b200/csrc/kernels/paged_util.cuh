@@ -20,13 +20,20 @@ template <class P> __device__ __forceinline__ long long page_of(const P& p, int 
 template <class P> __device__ __forceinline__ long long key_row(const P& p, long long pg, int g, int pos) {
     return ((pg * p.kv_heads + g) << p.shift) + (pos & ((1 << p.shift) - 1));
 }
+// Threads of the kernels for any shape: two for each of 128 keys.
+constexpr int kAnyThreads = 256;
+// Half of a dot product: the first or the second n / 2 (a multiple of four) elements.
+template <typename T> __device__ __forceinline__ float dot_of_half(const float* x, const T* w, int n, int half) {
+    const int cut = n / 2 & ~3;
+    return half ? dot_in_order(x + cut, w + cut, n - cut, 0.f) : dot_in_order(x, w, cut, 0.f);
+}
 // a + Σ w[jj] · (element i of the rows of positions j0 + jj), one after the other; `ld` elements per row. Several loads of a page in flight.
 template <typename T, class P>
 __device__ __forceinline__ float weigh_in_order(const P& p, const T* pool, int seq, int g, int j0, int live, long long ld, int i, const float* w, float a) {
     for (int jj = 0; jj < live;) {
         const int end = min(live, ((j0 + jj) | ((1 << p.shift) - 1)) + 1 - j0);
         const T* v = pool + key_row(p, page_of(p, seq, j0 + jj), g, j0 + jj) * ld + i;
-#pragma unroll 8
+#pragma unroll 16
         for (; jj < end; jj++, v += ld) a = fmaf(w[jj], to_f(*v), a);
     }
     return a;
