@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 import mufevik_ref as ref
+from oracle import ref as oracle
 from onyxia_b200 import backend as be
 from onyxia_b200 import ir, llm, lovuzen, models
 from onyxia_b200.ir import HostTensor
@@ -513,3 +514,16 @@ def test_slices_gathered_in_units(dtype, shape, axis):
     b.output("y", b.gather(b.constant(HostTensor.from_numpy(data)), b.input("i", ir.I64, [3, 7]), axis=axis))
     got = be.run_once(cuda_backend(), b.finish(), {"i": HostTensor.from_numpy(idx)})[0][1].numpy()
     assert np.array_equal(got, np.take(data, np.where(idx < 0, idx + shape[axis], idx), axis=axis))
+
+
+@pytest.mark.parametrize("width", [8, 264, 2056, 8192, 8200, 12])
+def test_norms_of_eights(width):
+    """Rows of one group of eight, of a part of a warp, of all threads, and those that other kernels take: the oracle's bits, also of squares that overflow and of what is no number."""
+    r = np.random.default_rng(width)
+    x, w = (4 * r.standard_normal((6, width))).astype(np.float16), (1 + 0.1 * r.standard_normal(width)).astype(np.float16)
+    x[1, width // 2], x[2, 0], x[3, width - 1], x[4] = 300.0, np.inf, np.nan, 0.0
+    b = ir.GraphBuilder()
+    b.output("y", b.composite("SimplifiedLayerNormalization", {"epsilon": 1e-6}, [b.input("x", ir.F16, list(x.shape)), b.input("w", ir.F16, [width])], [(ir.F16, list(x.shape))])[0])
+    module, feed = b.finish(), {"x": HostTensor.from_numpy(x), "w": HostTensor.from_numpy(w)}
+    got, want = be.run_once(cuda_backend(), module.clone(), feed)[0][1].numpy(), be.run_once(oracle.RefBackend(), module, feed)[0][1].numpy()
+    assert np.array_equal(got, want, equal_nan=True)
