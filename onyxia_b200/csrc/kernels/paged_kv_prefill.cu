@@ -76,13 +76,13 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
     constexpr int NS = KEYS ? 3 : 2;  // tiles on their way: keys that are values are kept until both products have read them
     const unsigned k_stage = kp * kPanelKv, v_stage = vp * kPanelKv;
     const unsigned sq0 = smem_u32(smem), sk = sq0 + kp * kPanelQ, sv = KEYS ? sk : sk + NS * k_stage, bars = sk + NS * k_stage + (KEYS ? 0 : NS * v_stage);
-    // barriers: keys there, free (three each), values there, free, scores there, weights there (two each), sums
+    // barriers: keys there, free (three each), values there, free, scores there, weights there, sums (two each)
     const unsigned k_full = bars, k_free = bars + 24, v_full = KEYS ? k_full : bars + 48, v_free = bars + 64, s_full = bars + 80, w_full = bars + 96, o_done = bars + 112;
-    unsigned* tmem_slot = reinterpret_cast<unsigned*>(smem + (bars + 120 - sq0));
-    float* shared = reinterpret_cast<float*>(smem + (bars + 128 - sq0));  // [turn][half of the keys][row]: what the two threads of a row tell each other
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(smem + (bars + 128 - sq0));
+    float* shared = reinterpret_cast<float*>(smem + (bars + 144 - sq0));  // [turn][half of the keys][row]: what the two threads of a row tell each other
     float *scale_s = shared + 4 * kRows, *bias_s = scale_s + NS * kKeys;  // KEYS: [tile][key], [head][distance]
     if (tid == 0) {
-        for (int i = 0; i < 15; i++) mbar_init(bars + i * 8, i == 12 || i == 13 ? kSoft / 32 : 1);
+        for (int i = 0; i < 16; i++) mbar_init(bars + i * 8, i == 12 || i == 13 ? kSoft / 32 : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     pdl_wait();
@@ -118,6 +118,10 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
     const unsigned tmem = *tmem_slot, t_weights = apart ? tmem + 128 : tmem, weights_turn = apart ? 32 : kKeys, t_sum = tmem + (apart ? 192 : 128);
     const int kt0 = first_key(p, pos0) / kKeys, n = last / kKeys + 1 - kt0;
     bool ok = true;
+    // Waits until the products of tile i are in the sums. Tiles take turns at two barriers. Who has the scores of tile i knows the products of tile i - 2 and of all before it to be
+    // done, so the barrier of tile i - 1 or i cannot be a round behind. (With one barrier for all tiles, parity alone takes the end of tile i - 2 for that of tile i while
+    // tile i - 1 is open.)
+    auto added = [&](int i) { return mbar_wait(o_done + (i & 1) * 8, (unsigned)(i >> 1) & 1); };
 
     if (warp == 8) {
         RingAt at;
@@ -170,7 +174,7 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
         for (int i = 0; i < n; i++) {
             if (i + 1 < n) {
                 // the other turn's scores were read by the threads that wrote its weights; where these have their place, products have to be done with them
-                if (!LSE && !apart && i > 0 && ok && !mbar_wait(o_done, (unsigned)(i - 1) & 1)) ok = false;
+                if (!LSE && !apart && i > 0 && ok && !added(i - 1)) ok = false;
                 scores();
             }
             if (ok && !mbar_wait(w_full + at.s * 8, at.parity)) ok = false;
@@ -182,7 +186,7 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
 #pragma unroll
                     for (int e = 0; e < kKeys / 16; e++) umma_weights(t_sum, t_weights + at.s * weights_turn + e * 8, v + e * 128, by_values, i > 0 || e > 0);
                     umma_commit((KEYS ? k_free : v_free) + tile.s * 8);
-                    umma_commit(o_done);
+                    umma_commit(o_done + at.s * 8);
                 }
                 __syncwarp();
             }
@@ -253,7 +257,7 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
                 m = top;
                 l *= keep;
                 if (!LSE && i > 0) {
-                    if (ok && !mbar_wait(o_done, (unsigned)(i - 1) & 1)) ok = false;
+                    if (ok && !added(i - 1)) ok = false;
                     after_sync();
 #pragma unroll 1
                     for (int c = part * 16; c < vp * 64; c += 32) {
@@ -299,7 +303,7 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
         if constexpr (LSE) {
             if (live && ok && part == 0) p.lse[token * p.heads + head] = m + log2f(l);
         } else {
-            if (ok && !mbar_wait(o_done, (unsigned)(n - 1) & 1)) ok = false;
+            if (ok && !added(n - 1)) ok = false;
             after_sync();
             float f = 1.f / l;
             if (!KEYS && p.sink && live) {
@@ -340,7 +344,7 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
 
 static int prefill_smem(const KvP& kv, bool keys, bool lse) {
     const int kp = (kv.dim + 63) / 64, vp = (kv.vdim + 63) / 64, tiles = keys ? 3 : 2;
-    return 1024 + kp * (int)(kPanelQ + tiles * kPanelKv) + (keys || lse ? 0 : vp * tiles * (int)kPanelKv) + 128 + 4 * kRows * 4 +
+    return 1024 + kp * (int)(kPanelQ + tiles * kPanelKv) + (keys || lse ? 0 : vp * tiles * (int)kPanelKv) + 144 + 4 * kRows * 4 +
            (keys ? tiles * kKeys * 4 + kv.heads / kv.kv_heads * kv.nd * 4 : 0);
 }
 

@@ -483,6 +483,40 @@ def test_prompts_whose_keys_are_their_values(heads, kv, dim, far):
     assert np.isfinite(err).all() and err.max() < 1e-2, (int(err.argmax()), float(err.max()))
 
 
+@pytest.mark.parametrize("form,heads,dim,vdim", [("plain", 4, 64, 128), ("plain", 4, 128, 256), ("capped", 4, 128, 128), ("capped", 4, 64, 192), ("keys", 64, 64, 64), ("keys", 64, 128, 128), ("keys", 64, 192, 192)])
+def test_prompts_whose_maxima_rise_for_some_rows(form, heads, dim, vdim):
+    """Warps of one CTA that take a new maximum in every tile, and are late for it, beside warps that never do: one to four tiles, either place of the weights. The sums of
+    the others have to wait for the tile before the last as well. Every run gives the same bits."""
+    r, T = np.random.default_rng(dim + vdim), 256
+    place, tile = np.arange(T), np.arange(T) // 64
+    k, v = to_bf16(0.1 * r.standard_normal((T, 1, dim))), to_bf16(r.standard_normal((T, 1, vdim)))
+    q = to_bf16(0.1 * r.standard_normal((T, heads, dim)))
+    if form == "keys":  # 64 heads: a warp's rows are half of a token's; their addends fall with the distance
+        bias = np.zeros((heads, T), np.float32)
+        bias[:32] = -0.25 * np.arange(T)
+        a = test_gpu_lovuzen.Attention("bf16", heads, 1, dim, bias, np.ones(heads * dim, np.float32), np.ones(dim, np.float32), scale=0.2)
+        qn, kn = (ref.rms_norm(x.reshape(T, -1).astype(np.float64), 1.0, 1e-5).reshape(x.shape) for x in (q, k))
+        far = np.maximum(place[:, None] - place[None], 0)
+        score, v, x = np.einsum("thd,jd->htj", qn, kn[:, 0]) * 0.2 + bias[:, far], k, (q, k)
+    else:  # four heads: a warp's rows are eight tokens'; every other eight see scores that rise by 10 from tile to tile
+        a = Attention("bf16", heads, 1, dim, vdim, scale=1.0, softcap=60.0 if form == "capped" else 0.0, norm=0, sink=0)
+        q[..., 0], k[..., 0] = (place // 8 % 2)[:, None], (10 * tile)[:, None]
+        score, x = np.einsum("thd,jd->htj", q.astype(np.float64), k[:, 0].astype(np.float64)), (q, k, v)
+        if form == "capped":
+            score = 60.0 * np.tanh(score / 60.0)
+    score = np.where(place[None] <= place[:, None], score, -np.inf)
+    w = np.exp(score - score.max(-1, keepdims=True))
+    want = np.einsum("htj,jd->thd", w / w.sum(-1, keepdims=True), v[:, 0].astype(np.float64))
+    first = None
+    for run in range(60):
+        got = a.step([(0, *x)])[0]
+        first = got if first is None else first
+        assert np.array_equal(got, first), run
+        a.past.pop(0)  # the same pages once more
+    err = row_err(first, want)
+    assert err.max() < 1.5e-2, (int(err.argmax()), float(err.max()))
+
+
 @pytest.mark.parametrize("width", [4, 1020, 1028, 3072, 4100, 6144, 6148])
 def test_residual_norms_of_rows_in_registers(width):
     """Widths at the ends of a thread's packs and beyond them; everything that a norm in front of or behind the sum can take. f32 sums of at most 6148 squares."""
