@@ -633,7 +633,7 @@ template <int EPI, bool ONE> __global__ void __launch_bounds__(kTcThreads) linea
                 waited = true;
             }
             for (; i < q.steps; i++) {
-                if (round && !mbar_wait(empty + at.s * 8, at.parity ^ 1)) {
+                if (!__all_sync(0xffffffffu, !round || mbar_wait(empty + at.s * 8, at.parity ^ 1))) {
                     ok = false;
                     break;
                 }

@@ -167,7 +167,7 @@ template <int EPI, bool YB> __global__ void __launch_bounds__(kPairThreads, 1) l
             const int y0 = weights ? q.group * (int)p.out + q.m * 256 + (int)rank * 128 : q.n0 + (int)rank * (q.n >> 1);
             const unsigned bytes = 2 * (kPanelA + (unsigned)boxes * box_bytes);
             for (int i = 0; i < steps; i++) {
-                if (round && !ready && !mbar_wait(empty + at.s * 8, at.parity ^ 1)) {
+                if (!__all_sync(0xffffffffu, !round || ready || mbar_wait(empty + at.s * 8, at.parity ^ 1))) {
                     ok = false;
                     break;
                 }

@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) nbits_gemm_wide(const __grid_
             const Unit q = unit_of(u);
             const int lo = first_step(q, q.from) * 2, hi = first_step(q, q.to) * 2;  // 64-k steps; pieces follow one another
             for (int i = lo; i < hi; i++) {
-                if (round && !mbar_wait(empty + at.s * 8, at.parity ^ 1)) {
+                if (!__all_sync(0xffffffffu, !round || mbar_wait(empty + at.s * 8, at.parity ^ 1))) {
                     ok = false;
                     break;
                 }

@@ -130,7 +130,7 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
             const long long pg = page_of(p, seq, j0);
             const int row = (int)key_row(p, pg, g, j0);
             if (i >= NS && !mbar_wait(k_free + at.s * 8, at.parity ^ 1)) ok = false;
-            if (ok && elect_one()) {
+            if (elect_one() && ok) {
                 mbar_expect_tx(k_full + at.s * 8, k_stage + (KEYS ? kKeys * 4 : 0));
                 if constexpr (KEYS)  // a page's factors follow one another
                     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(scale_s + at.s * kKeys)),
@@ -141,7 +141,7 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
             __syncwarp();
             if constexpr (!LSE && !KEYS) {
                 if (i >= NS && ok && !mbar_wait(v_free + at.s * 8, at.parity ^ 1)) ok = false;
-                if (ok && elect_one()) {
+                if (elect_one() && ok) {
                     mbar_expect_tx(v_full + at.s * 8, v_stage);
                     for (int c = 0; c < vp; c++) tma_load_2d(sv + at.s * v_stage + c * kPanelKv, pp.maps[1], c * 64, row, v_full + at.s * 8);
                 }
@@ -158,7 +158,7 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
         auto scores = [&] {
             if (ok && !mbar_wait(k_full + tile_ahead.s * 8, tile_ahead.parity)) ok = false;
             after_sync();
-            if (ok && elect_one()) {
+            if (elect_one() && ok) {
                 const unsigned long long k = dk + tile_ahead.s * (k_stage >> 4);
                 for (int c = 0; c < kp; c++)
 #pragma unroll
@@ -181,7 +181,7 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
             if constexpr (!LSE) {
                 if (ok && !mbar_wait(v_full + tile.s * 8, tile.parity)) ok = false;
                 after_sync();
-                if (ok && elect_one()) {
+                if (elect_one() && ok) {
                     const unsigned long long v = dv + tile.s * (v_stage >> 4);
 #pragma unroll
                     for (int e = 0; e < kKeys / 16; e++) umma_weights(t_sum, t_weights + at.s * weights_turn + e * 8, v + e * 128, by_values, i > 0 || e > 0);

@@ -45,7 +45,8 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
 }
 
 // One lane of a converged warp. The compiler knows that its branch is taken by one lane: operands that have to be in uniform registers (copies,
-// matrix instructions, their barriers) get there without a loop over lanes.
+// matrix instructions, their barriers) get there without a loop over lanes. All 32 lanes have to come: a wait may run out for some lanes and not for others, so
+// what it found is never a condition in front of this, and a loop is left by a vote.
 __device__ __forceinline__ bool elect_one() {
     unsigned p;
     asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
