@@ -443,7 +443,7 @@ def lovuzen_costs(cfg, rows, seqs, past, wanted):
 
 
 _FAMILY = {"linear_stream": "linear", "linear_flow": "linear", "linear_tc": "linear", "linear_pair": "linear", "linear_reduce": "linear", "linear_simt": "linear",
-           "paged_attn_prefill": "attn", "paged_attn_decode": "attn", "paged_attn_simt": "attn", "recurrence_step": "gates",
+           "paged_attn_prefill": "attn", "paged_attn_prefill_mma": "attn", "paged_attn_decode": "attn", "paged_attn_simt": "attn", "recurrence_step": "gates",
            "recurrence_gates": "gates", "recurrence_scan": "scan", "residual_norm": "norm",
            "linear_rows_f32": "linear", "linear_f32": "linear", "nbits_widen": "linear", "nbits_gemm_wide": "linear",
            "nbits_stream": "linear", "nbits_gemm_tc": "linear", "nbits_gemm_reduce": "linear", "persist_step": "persist_step"}
@@ -581,7 +581,7 @@ def kipizen_costs(cfg, rows, seqs, past, wanted):
             "experts": (exp_b, exp_f), "routing": (route_b, route_f), "norm": (norm_b, 0)}
 
 
-_FAMILY.update({"paged_kv_prefill": "attn", "paged_kv_decode": "attn", "paged_kv_simt": "attn", "lightning_step": "lightning_step",
+_FAMILY.update({"paged_kv_prefill": "attn", "paged_kv_prefill_mma": "attn", "paged_kv_decode": "attn", "paged_kv_simt": "attn", "lightning_step": "lightning_step",
                 "lightning_chunk": "lightning_chunks", "lightning_scan": "lightning_chunks", "lightning_out": "lightning_chunks",
                 "moe_stream_up": "experts", "moe_stream_down": "experts", "grouped_tc": "experts", "grouped_pair": "experts", "moe_top": "routing", "moe_route": "routing", "moe_sort": "routing",
                 "moe_combine": "routing"})
@@ -727,7 +727,7 @@ def mufevik_costs(cfg, rows, seqs, past, wanted):
     return {k: tuple(v) for k, v in c.items()}
 
 
-_FAMILY.update({"talk_lse": "attn", "talk_prefill": "attn", "talk_prefill_any": "attn", "talk_merge": "attn", "talk_scores": "attn", "talk_values": "attn", "gated_linear_step": "gated_step", "gated_linear_decay": "gated_chunks",
+_FAMILY.update({"talk_lse": "attn", "talk_lse_mma": "attn", "talk_prefill": "attn", "talk_prefill_any": "attn", "talk_merge": "attn", "talk_scores": "attn", "talk_values": "attn", "gated_linear_step": "gated_step", "gated_linear_decay": "gated_chunks",
                 "gated_linear_chunk": "gated_chunks", "gated_linear_scan": "gated_chunks", "gated_linear_out": "gated_chunks", "delta_step": "delta_step", "delta_keep": "conv",
                 "delta_chunk": "delta_chunks", "delta_scan": "delta_chunks", "delta_out": "delta_chunks", "streams_norm": "norm", "groups_norm": "norm"})
 

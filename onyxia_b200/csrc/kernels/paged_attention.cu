@@ -682,7 +682,7 @@ void emit_paged_attention(Emitter& em, const PagedAttnDesc& d, const TRef& proj,
                             "paged_attn_prefill");
         } else {
             ensure_max_dynamic_smem((const void*)dc.prefill, 220 * 1024);
-            launch(dc.prefill, dim3((unsigned)((rows + tq - 1) / tq + n_seqs), (unsigned)d.kv_heads), kPreThreads, (unsigned)pre_smem, none, "paged_attn_prefill");
+            launch(dc.prefill, dim3((unsigned)((rows + tq - 1) / tq + n_seqs), (unsigned)d.kv_heads), kPreThreads, (unsigned)pre_smem, none, "paged_attn_prefill_mma");
         }
     }
     if (decode_only || n_seqs > 1) {

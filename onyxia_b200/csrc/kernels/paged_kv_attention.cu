@@ -662,7 +662,7 @@ void emit_paged_kv_attention(Emitter& em, const PagedKvDesc& d, const TRef& proj
                             "paged_kv_prefill");
         } else {
             ensure_max_dynamic_smem((const void*)dc.prefill, 220 * 1024);
-            launch(dc.prefill, dim3((unsigned)((rows + tq - 1) / tq + n_seqs), (unsigned)d.kv_heads), kPreThreads, (unsigned)dc.pre_smem, none, "paged_kv_prefill");
+            launch(dc.prefill, dim3((unsigned)((rows + tq - 1) / tq + n_seqs), (unsigned)d.kv_heads), kPreThreads, (unsigned)dc.pre_smem, none, "paged_kv_prefill_mma");
         }
     }
     if (decode_only || n_seqs > 1) {
@@ -700,7 +700,7 @@ void emit_kv_lse(Emitter& em, const PagedKvDesc& d, KvP p, Buf q, Buf lse, const
     ensure_max_dynamic_smem((const void*)dc.lse, 220 * 1024);
     em.launch(dc.lse, dim3((unsigned)((p.rows + tq - 1) / tq + p.n_seqs), (unsigned)d.kv_heads), dim3(kPreThreads), (unsigned)dc.lse_smem, p,
               {{&p.keys, keys.buf}, {&p.values, none}, {&p.q, q}, {&p.temps, temps}, {&p.lse, lse}, {&p.seqs, seqs.buf}, {&p.table, pages.buf}, {&p.err, Buf{kSlotErr, 0}}},
-              "talk_lse", /*pdl=*/true);
+              "talk_lse_mma", /*pdl=*/true);
 }
 
 }  // namespace oxk

@@ -7,10 +7,11 @@ import sys
 import numpy as np
 import pytest
 
+import kipizen_ref
 import mufevik_ref as ref
 from oracle import ref as oracle
 from onyxia_b200 import backend as be
-from onyxia_b200 import ir, llm, lovuzen, models
+from onyxia_b200 import ir, kipizen, llm, lovuzen, models
 from onyxia_b200.ir import HostTensor
 from gpu_util import cuda_backend, differential
 from lovuzen_util import to_bf16
@@ -561,3 +562,76 @@ def test_norms_of_eights(width):
     module, feed = b.finish(), {"x": HostTensor.from_numpy(x), "w": HostTensor.from_numpy(w)}
     got, want = be.run_once(cuda_backend(), module.clone(), feed)[0][1].numpy(), be.run_once(oracle.RefBackend(), module, feed)[0][1].numpy()
     assert np.array_equal(got, want, equal_nan=True)
+
+
+def prompt_over_pages(op, attrs, rows, before, pools, after, out, portions):
+    """A prompt in portions through one attention node in bf16 whose pools hold no numbers yet: its results and the kernels that ran. `before` and `after`: constants around the
+    pools and the description of the step; `out`: heads and their width."""
+    b = ir.GraphBuilder()
+    N, R, TW, n_pages = b.sym("n"), b.sym("r"), b.sym("w"), pools[0][1][0]
+    ins = [b.input("proj", ir.BF16, [N, rows.shape[1]])] + [b.constant(HostTensor.from_numpy(np.asarray(c, np.float32))) for c in before]
+    ins += [b.input(f"pool{i}", dt, shape) for i, (dt, shape) in enumerate(pools)] + [b.input("seqs", ir.I32, [R, 4]), b.input("table", ir.I32, [R, TW])]
+    outs = b.composite(op, attrs, ins + [b.constant(HostTensor.from_numpy(np.asarray(c, np.float32))) for c in after], [(ir.BF16, [N, out[0] * out[1]])] + pools)
+    for i, v in enumerate(outs):
+        b.output(f"out{i}", v)
+    s = cuda_backend().prepare(b.finish())
+    held = [s.upload(act(np.full(shape, np.nan), dt)) for dt, shape in pools]
+    table = s.upload(HostTensor.from_numpy(np.random.default_rng(0).permutation(n_pages).astype(np.int32)[None]))
+    s.enable_profiling(True)
+    got, at = [], 0
+    for n in portions:
+        feed = {"proj": s.upload(act(rows[at:at + n], ir.BF16)), "seqs": s.upload(HostTensor.from_numpy(np.array([[0, n, at, 0]], np.int32))), "table": table}
+        o = dict(s.run({**feed, **{f"pool{i}": t for i, t in enumerate(held)}}))
+        got.append(s.download(o["out0"]).numpy())
+        held, at = [o[f"out{i + 1}"] for i in range(len(pools))], at + n
+    return np.concatenate(got).reshape(-1, *out), {kernel for kernel, _, _ in s.take_timings()}
+
+
+@pytest.mark.parametrize("page", [16, 32, 64])
+@pytest.mark.parametrize("heads,kv,dim,vdim,window,softcap", [(4, 2, 72, 136, 50, 0.0), (16, 1, 256, 256, 0, 30.0), (3, 3, 16, 8, 0, 0.0)])
+def test_prompts_over_pages_of_any_size(page, heads, kv, dim, vdim, window, softcap):
+    """Tiles of 64 keys over several pages take the `mma.sync` kernel."""
+    r, T, scale = np.random.default_rng(page), 200, 2.0 / np.sqrt(dim)
+    q, k, v = (to_bf16(r.standard_normal((T, n, d))) for n, d in ((heads, dim), (kv, dim), (kv, vdim)))
+    attrs = {"heads": heads, "kv_heads": kv, "dim": dim, "vdim": vdim, "rot_dims": 0, "window": window, "scale": scale, "softcap": softcap, "epsilon": 1e-5, "norm": 0, "sink": 1,
+             "q_offset": 0, "k_offset": heads * dim, "v_offset": (heads + kv) * dim}
+    rows = np.concatenate([x.reshape(T, -1) for x in (q, k, v)], axis=1)
+    n = 256 // page
+    got, kernels = prompt_over_pages("onyxia.PagedKVAttention", attrs, rows, [kipizen.turns_per_position(0, 100.0, 1.0)], [(ir.BF16, [n, kv, page, d]) for d in (dim, vdim)], [],
+                                     (heads, vdim), (3, 130, 67))
+    assert ("paged_kv_prefill" in kernels) == (page == 64) and ("paged_kv_prefill_mma" in kernels) == (page < 64)
+    err = row_err(got, kipizen_ref.attention(*(x.astype(np.float64) for x in (q, k, v)), scale, softcap or None, window or None))
+    assert np.isfinite(err).all() and err.max() < 1.5e-2, (int(err.argmax()), float(err.max()))
+
+
+@pytest.mark.parametrize("page,heads,kv,dim,far", [(16, 32, 16, 128, 128), (32, 20, 1, 72, 40), (16, 2, 1, 256, 300), (64, 20, 1, 72, 40), (64, 8, 1, 64, 5500)])
+def test_prompts_whose_keys_are_their_values_over_pages_of_any_size(page, heads, kv, dim, far):
+    """Pages of less than 64 keys, and more addends by distance than stand beside the tiles in shared memory, take the `mma.sync` kernel."""
+    r, T, kw = np.random.default_rng(page), 200, dict(scale=2.0 / np.sqrt(dim), temp=(0.4, 30))
+    q, k = (to_bf16(r.standard_normal((T, n, dim))) for n in (heads, kv))
+    q_w, k_w, bias = to_bf16(1 + 0.3 * r.standard_normal(heads * dim)), to_bf16(1 + 0.3 * r.standard_normal(kv * dim)), r.standard_normal((12, heads))
+    attrs = {"heads": heads, "kv_heads": kv, "dim": dim, "q_offset": 0, "k_offset": heads * dim, "scale": kw["scale"], "epsilon": 1e-5, "temp_coef": 0.4, "temp_every": 30.0, "out_scale": 1.0}
+    rows = np.concatenate([x.reshape(T, -1) for x in (q, k)], axis=1)
+    got, kernels = prompt_over_pages("onyxia.PagedAttention", attrs, rows, [q_w, k_w, lovuzen.distance_bias(bias, far)], [(ir.BF16, [256 // page, kv, page, dim]), (ir.F32, [256 // page, page])],
+                                     [], (heads, dim), (3, 130, 67))
+    mma = page < 64 or far == 5500
+    assert ("paged_attn_prefill_mma" in kernels) == mma and ("paged_attn_prefill" in kernels) == (not mma)
+    want = attention_want(q, k, bias, far, q_w, k_w, **kw)
+    err = np.sqrt(((got - want) ** 2).mean(axis=(1, 2))) / np.sqrt((want ** 2).mean())
+    assert np.isfinite(err).all() and err.max() < 1e-2, (int(err.argmax()), float(err.max()))
+
+
+@pytest.mark.parametrize("page", [16, 32, 64])
+@pytest.mark.parametrize("heads,kv,dim,vdim", [(4, 2, 64, 128), (20, 1, 72, 136)])
+def test_mixed_heads_over_pages_of_any_size(page, heads, kv, dim, vdim):
+    """The softmax's sums alone come from the `mma.sync` kernel where a tile lies in several pages."""
+    r, T, scale = np.random.default_rng(page), 200, 1.5 / np.sqrt(dim)
+    q, k, v = (to_bf16(r.standard_normal((T, n, d))) for n, d in ((heads, dim), (kv, dim), (kv, vdim)))
+    temp, talk = to_bf16(r.uniform(0.5, 2, heads)), to_bf16(0.6 * np.eye(heads) + 0.5 * r.standard_normal((heads, heads)) / np.sqrt(heads))
+    attrs = {"heads": heads, "kv_heads": kv, "dim": dim, "vdim": vdim, "rot_dims": 0, "scale": scale, "temps": 1, "talk": 1, "q_offset": 0, "k_offset": heads * dim, "v_offset": (heads + kv) * dim}
+    rows = np.concatenate([x.reshape(T, -1) for x in (q, k, v)], axis=1)
+    got, kernels = prompt_over_pages("onyxia.PagedKVAttention", attrs, rows, [kipizen.turns_per_position(0, 100.0, 1.0)], [(ir.BF16, [256 // page, kv, page, d]) for d in (dim, vdim)],
+                                     [temp, talk], (heads, vdim), (3, 130, 67))
+    assert ("talk_lse" in kernels) == (page == 64) and ("talk_lse_mma" in kernels) == (page < 64)
+    err = row_err(got, ref.talking_attention(*(x.astype(np.float64) for x in (q, k, v)), scale, temp.astype(np.float64), talk.astype(np.float64)))
+    assert np.isfinite(err).all() and err.max() < 2e-2, (int(err.argmax()), float(err.max()))
