@@ -583,7 +583,7 @@ def kipizen_costs(cfg, rows, seqs, past, wanted):
 
 _FAMILY.update({"paged_kv_prefill": "attn", "paged_kv_prefill_mma": "attn", "paged_kv_decode": "attn", "paged_kv_simt": "attn", "lightning_step": "lightning_step",
                 "lightning_chunk": "lightning_chunks", "lightning_scan": "lightning_chunks", "lightning_out": "lightning_chunks",
-                "moe_stream_up": "experts", "moe_stream_down": "experts", "grouped_tc": "experts", "grouped_pair": "experts", "moe_top": "routing", "moe_route": "routing", "moe_sort": "routing",
+                "moe_stream_up": "experts", "moe_stream_down": "experts", "grouped_tc": "experts", "grouped_pair": "experts", "moe_top": "routing", "moe_route": "routing", "moe_route_pairs": "routing", "moe_sort": "routing",
                 "moe_combine": "routing"})
 
 

@@ -425,21 +425,22 @@ __global__ void __launch_bounds__(kTopWarps * 32) moe_top(const MoeP p) {
     }
 }
 
-// A warp per token, since the choice is a chain of shuffles (two tokens per warp, one after the other, and half as many warps for the products: 64 rows of 2560 16.3 → 10.0 µs of a
-// step, 1999 of 1152 12.8 → 8.4, 2048 of 2560 19.3 → 14.2, 4096 of 1152, which are two rounds of CTAs now, 10.6 → 12.7).
-constexpr int kRouteRows = 16, kRouteWarps = kRouteRows;
-__global__ void __launch_bounds__(kRouteWarps * 32) moe_route(const MoeP p) {
-    constexpr int kBatch = 4;
+// WARPS 16: a warp per token, since the choice is a chain of shuffles. WARPS 8: two tokens per warp, one after the other, and half as many warps for the products; two such CTAs
+// share an SM. 64 rows of 2560 16.3 µs of a step with eight warps, 10.0 with sixteen; 1999 of 1152 12.8 → 8.4; 2048 of 2560 19.3 → 14.2; where CTAs of sixteen warps are more than
+// one round and those of eight are not, 4096 of 1152, 10.6 with eight and 12.7 with sixteen.
+constexpr int kRouteRows = 16;
+template <int WARPS> __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) moe_route(const MoeP p) {
+    constexpr int kBatch = 4, kEach = kRouteRows / WARPS;  // tokens of a warp
     extern __shared__ __align__(16) unsigned char smem[];  // count[experts], base[experts], z[rows][ld] [, the same once more]
-    __shared__ float red[kRouteWarps][16][kRouteRows + 1];
+    __shared__ float red[WARPS][16][kRouteRows + 1];
     pdl_trigger();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, E = p.experts, L = p.ld;
     int *count = reinterpret_cast<int*>(smem), *base = count + E;
     float* z = reinterpret_cast<float*>(base + E);
     const long long row0 = (long long)blockIdx.x * kRouteRows, K = p.width;
-    const int chunks = (int)((K + 31) / 32), per_tile = (chunks + kRouteWarps * kBatch - 1) / (kRouteWarps * kBatch), total = (L + 15) / 16 * per_tile;
+    const int chunks = (int)((K + 31) / 32), per_tile = (chunks + WARPS * kBatch - 1) / (WARPS * kBatch), total = (L + 15) / 16 * per_tile;
     const bf16* W = (const bf16*)p.router;
-    auto k_of = [&](int it, int j) { return (long long)(((it % per_tile) * kBatch + j) * kRouteWarps + warp) * 32 + t * 8; };
+    auto k_of = [&](int it, int j) { return (long long)(((it % per_tile) * kBatch + j) * WARPS + warp) * 32 + t * 8; };
     uint4 wl[kBatch], wh[kBatch];
     auto fetch = [&](int it) {
 #pragma unroll
@@ -452,7 +453,7 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route(const MoeP p) {
         }
     };
     fetch(0);  // constants: may overlap the launches before this one
-    for (int i = tid; i < E; i += kRouteWarps * 32) count[i] = 0;
+    for (int i = tid; i < E; i += WARPS * 32) count[i] = 0;
     pdl_wait();
     float acc[2][4];
     for (int it = 0; it < total; it++) {
@@ -495,27 +496,34 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_route(const MoeP p) {
         if (o < L && m < kRouteRows) {
             float s = 0.f;
 #pragma unroll
-            for (int w = 0; w < kRouteWarps; w++) s += red[w][tid & 15][m];
+            for (int w = 0; w < WARPS; w++) s += red[w][tid & 15][m];
             z[m * L + o] = s + p.router_bias[o];
             if (p.scores != MOE_CHOSEN) z[(kRouteRows + m) * L + o] = s + p.router_bias[o];
         }
         __syncthreads();
     }
-    int id;
-    float w;
-    const long long row = row0 + warp;
-    const float* raw = z + (kRouteRows + warp) * L;
-    choose(p, z + warp * L, raw, &id, &w);
-    if (p.gates && lane == 0 && row < p.rows) p.gates[row] = sigmoid_f(raw[E]);
-    const int place = row < p.rows && lane < p.top ? atomicAdd(count + id, 1) : 0;
+    int id[kEach], place[kEach];
+    float w[kEach];
+#pragma unroll
+    for (int h = 0; h < kEach; h++) {
+        const long long row = row0 + warp + h * WARPS;
+        const float* raw = z + (kRouteRows + warp + h * WARPS) * L;
+        choose(p, z + (warp + h * WARPS) * L, raw, id + h, w + h);
+        if (p.gates && lane == 0 && row < p.rows) p.gates[row] = sigmoid_f(raw[E]);
+        place[h] = row < p.rows && lane < p.top ? atomicAdd(count + id[h], 1) : 0;
+    }
     __syncthreads();
-    for (int i = tid; i < E; i += kRouteWarps * 32)
+    for (int i = tid; i < E; i += WARPS * 32)
         if (count[i]) base[i] = atomicAdd(p.counts + i, count[i]);
     __syncthreads();
-    if (row >= p.rows || lane >= p.top) return;
-    p.ids[row * p.top + lane] = id;
-    p.weights[row * p.top + lane] = w;
-    p.rank[row * p.top + lane] = base[id] + place;
+#pragma unroll
+    for (int h = 0; h < kEach; h++) {
+        const long long row = row0 + warp + h * WARPS;
+        if (row >= p.rows || lane >= p.top) continue;
+        p.ids[row * p.top + lane] = id[h];
+        p.weights[row * p.top + lane] = w[h];
+        p.rank[row * p.top + lane] = base[id[h]] + place[h];
+    }
 }
 
 // One CTA per token: its row goes to every chosen expert's part of the sorted rows; `rank` becomes the row there.
@@ -707,8 +715,12 @@ void emit_moe(Emitter& em, const MoeDesc& d, const ResidualNormDesc& norm, const
                   label, /*pdl=*/true);
     };
     if (route) {
-        ensure_max_dynamic_smem((const void*)moe_route, 64 * 1024);
-        launch(moe_route, (unsigned)((d.rows + kRouteRows - 1) / kRouteRows), kRouteWarps * 32, route_smem, "moe_route");
+        // one CTA of sixteen warps per SM: beyond one round of those, eight
+        const int64_t ctas = (d.rows + kRouteRows - 1) / kRouteRows;
+        const int warps = ctas > sm_count() ? 8 : 16;
+        void (*const k)(const MoeP) = warps == 8 ? moe_route<8> : moe_route<16>;
+        ensure_max_dynamic_smem((const void*)k, 64 * 1024);
+        launch(k, (unsigned)ctas, (unsigned)warps * 32, route_smem, warps == 8 ? "moe_route_pairs" : "moe_route");
     } else {
         const unsigned top_smem = (unsigned)((2 + kTopWarps) * d.experts * 4);
         ensure_max_dynamic_smem((const void*)moe_top, 200 * 1024);

@@ -6,6 +6,7 @@ import sys
 
 import numpy as np
 import pytest
+import torch
 
 import kipizen_ref
 import mufevik_ref as ref
@@ -17,6 +18,7 @@ from gpu_util import cuda_backend, differential
 from lovuzen_util import to_bf16
 from test_gpu_kipizen import Attention, Experts, piece, row_err
 import test_gpu_lovuzen
+import test_gpu_mufevik
 from test_gpu_lovuzen import act, attention_want, rel_err, run_linear
 
 pytestmark = pytest.mark.gpu
@@ -635,3 +637,15 @@ def test_mixed_heads_over_pages_of_any_size(page, heads, kv, dim, vdim):
     assert ("talk_lse" in kernels) == (page == 64) and ("talk_lse_mma" in kernels) == (page < 64)
     err = row_err(got, ref.talking_attention(*(x.astype(np.float64) for x in (q, k, v)), scale, temp.astype(np.float64), talk.astype(np.float64)))
     assert np.isfinite(err).all() and err.max() < 2e-2, (int(err.argmax()), float(err.max()))
+
+
+@pytest.mark.parametrize("more", [0, 1, 2400])
+@pytest.mark.parametrize("scores", ["chosen", "corrected"])
+def test_routing_in_one_round_and_more(more, scores):
+    """A warp per token as long as every SM has one CTA at most, two tokens per warp beyond; the last CTA has one token."""
+    n = 16 * torch.cuda.get_device_properties(0).multi_processor_count + more
+    m = Experts("bf16", 64, 8, 2, 40) if scores == "chosen" else test_gpu_mufevik.Experts("bf16", 64, 8, 2, 40, (4, 2), 72, correction=0.2 / 8)
+    m.s.enable_profiling(True)
+    m.check(m.rows(n))
+    kernels = {kernel for kernel, _, _ in m.s.take_timings()}
+    assert ("moe_route" in kernels) == (more == 0) and ("moe_route_pairs" in kernels) == (more > 0)
