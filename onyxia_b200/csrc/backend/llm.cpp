@@ -89,6 +89,7 @@ ox_status ox_llm_create(ox_session* session, int64_t max_seq_len, ox_llm** out) 
             if (l->names[i] == past) l->present_of[i] = (int)o;
     }
     if (l->logits_out < 0) fail(ErrKind::Binding, "output 'logits' missing");
+    if (m.values[m.outputs[(size_t)l->logits_out].second].ty.dtype == DType::F16) l->s->open_landing();  // not inside the first step
     *out = l.release();
     return OX_OK;
     OX_CATCH

@@ -155,11 +155,6 @@ Session::~Session() {
         cudaEventDestroy(r.b);
     }
     for (auto e : prof_free_) cudaEventDestroy(e);
-    if (land_pinned_) {
-        cudaFreeHost(land_pinned_);
-        for (auto e : land_events_)
-            if (e) cudaEventDestroy(e);
-    }
     if (stage_pinned_) {
         cudaFreeHost(stage_pinned_);
         for (auto e : stage_events_) cudaEventDestroy(e);
@@ -835,11 +830,18 @@ void Session::download_f32(const DTensor& t, float* dst, size_t cap, size_t* wri
     if (cap < n) fail(ErrKind::Runtime, "download buffer too small: " + std::to_string(cap) + " < " + std::to_string(n) + " values");
     if (n) {
         populate(dst, n * sizeof(float));
-        land(t, n * 2, [&](size_t at, const uint8_t* from, size_t bytes) { widen_f16(from, dst + at / 2, bytes / 2); });
+        // Values are widened out of one chunk while the next lands, without the copy into memory of the caller's that cudaMemcpyAsync ends with. (As a plain copy this way
+        // is no faster than the driver's own: 8 × 32 768 values 12.6 against 12.0 ms per 33 steps.)
+        OX_CUDA(landing_.land((const uint8_t*)t.ptr(), n * 2, stream_, [&](size_t at, const uint8_t* from, size_t bytes) { widen_f16(from, dst + at / 2, bytes / 2); }));
     }
     OX_CUDA(cudaStreamSynchronize(stream_));
     if (written) *written = n;
     check_device_error();
+}
+
+void Session::open_landing() {
+    OX_CUDA(cudaSetDevice(device_));
+    OX_CUDA(landing_.open());
 }
 
 // Pages of a destination that has just been allocated, while the device still works on what will be copied there: one after the other as they
@@ -849,27 +851,6 @@ void Session::populate(void* dst, size_t nbytes) {
     const uintptr_t page = 4096, first = ((uintptr_t)dst + page - 1) / page * page, last = ((uintptr_t)dst + nbytes) / page * page;
     if (last > first) madvise((void*)first, last - first, 23 /* MADV_POPULATE_WRITE */);
 #endif
-}
-
-// A dense tensor through two pinned chunks, `take(offset, bytes, n)` called in order: values are widened out of one while the other lands, without the copy into
-// memory of the caller's that cudaMemcpyAsync ends with. (As a plain copy this way is no faster than the driver's own: 8 × 32 768 values 12.6 against 12.0 ms per 33 steps.)
-template <class F> void Session::land(const DTensor& t, size_t nbytes, F&& take) {
-    if (!land_pinned_) {
-        OX_CUDA(cudaMallocHost((void**)&land_pinned_, 2 * kLandBytes));
-        for (auto& e : land_events_) OX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
-    const size_t chunks = (nbytes + kLandBytes - 1) / kLandBytes;
-    auto ask = [&](size_t i) {
-        OX_CUDA(cudaMemcpyAsync(land_pinned_ + (i & 1) * kLandBytes, (const uint8_t*)t.ptr() + i * kLandBytes, std::min(kLandBytes, nbytes - i * kLandBytes),
-                                cudaMemcpyDeviceToHost, stream_));
-        OX_CUDA(cudaEventRecord(land_events_[i & 1], stream_));
-    };
-    ask(0);
-    for (size_t i = 0; i < chunks; i++) {
-        if (i + 1 < chunks) ask(i + 1);
-        OX_CUDA(cudaEventSynchronize(land_events_[i & 1]));
-        take(i * kLandBytes, land_pinned_ + (i & 1) * kLandBytes, std::min(kLandBytes, nbytes - i * kLandBytes));
-    }
 }
 
 void Session::download_async(const DTensor& t, void* pinned_dst) {

@@ -3,6 +3,7 @@
 #pragma once
 #include <list>
 
+#include "landing.hpp"
 #include "runtime.hpp"
 #include "../kernels/persist.hpp"
 
@@ -103,6 +104,7 @@ public:
     std::vector<DTensor> upload_together(const std::vector<HostPart>& parts);
     // f32 values of a dense f32 or f16 tensor; `cap` and `written` count values.
     void download_f32(const DTensor& t, float* dst, size_t cap, size_t* written);
+    void open_landing();  // what the first download_f32 of f16 values would make
     std::vector<std::pair<std::string, DTensor>> run(const std::vector<std::pair<std::string, DTensor>>& inputs);
     void preplan(const std::vector<std::pair<std::string, DTensor>>& next_inputs);
     DTensor zeros(DType dtype, const std::vector<int64_t>& shape);
@@ -229,11 +231,7 @@ private:
     uint8_t* stage_pinned_ = nullptr;
     cudaEvent_t stage_events_[kStageSlots] = {};
     unsigned stage_cursor_ = 0;
-    // pinned chunks that values to be widened land in
-    static constexpr size_t kLandBytes = 256 * 1024;
-    uint8_t* land_pinned_ = nullptr;
-    cudaEvent_t land_events_[2] = {};
-    template <class F> void land(const DTensor& t, size_t nbytes, F&& take);
+    Landing landing_;  // of values to be widened
     static void populate(void* dst, size_t nbytes);
     // profiling: one event pair per launch, read back in take_timings
     struct ProfRec {
