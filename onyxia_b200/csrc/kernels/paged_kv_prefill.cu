@@ -4,10 +4,11 @@
 // row cap, mask and weigh them, 4 products of 128 × vdim add the weights' share of the values; the scores of the next 64 keys are made under the weights of these. Keys and
 // values come by TMA, a page's rows are the rows of a tensor map; two of either are on their way.
 //
-// What bounds it is the chain of a step, about 1.3 µs in a CTA alone on its SM (256 dimensions: shared memory), of which the products are 0.7; a short prompt's longest tiles are as long
-// as the launch. The `mma.sync` kernel, which remains for pages of less than 64 keys, had four warps per SM at this size. µs, before → now: 4096 tokens, 4 heads of 256 over one key
-// head, capped 245 → 91 (rows by one thread each: 104); 1999 tokens, the same 127 → 49; 2048 tokens, 16 heads of 128 over 4, the softmax's sums alone 94 → 35; keys that are the
-// values, 32 heads of 128 over 16, four portions of 2048 tokens 2862 → 846.
+// What bounds it is the chain of a step, about 1.3 µs in a CTA alone on its SM (256 dimensions: shared memory), of which the products are 0.7, and the sums' way through registers
+// in steps that bring a new maximum; a short prompt's longest tiles are as long as the launch. The `mma.sync` kernel, which remains for pages of less than 64 keys, had four warps per
+// SM at this size. µs, with it → here: 4096 tokens, 4 heads of 256 over one key head, capped 258 → 127; 1999 tokens, the same 133 → 70; 2048 tokens, 16 heads of 128 over 4,
+// 130 → 60, the softmax's sums alone 92 → 41; keys that are the values, 32 heads of 128 over 16, four portions of 2048 tokens 2830 → 1083. Errors against 64-bit results are the same to
+// four digits (scores of either spread, capped or not; 700 and 1999 tokens).
 #include "paged_kv.cuh"
 
 namespace oxk {
@@ -250,9 +251,10 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
 #pragma unroll
             for (int e = 0; e < kHalf; e++) top = fmaxf(top, s[e]);
             top = fmaxf(top, both(i & 1, top));
-            // Weights are taken against a maximum that may be up to 2^8 behind: the sums are divided by their weights' sum in the end, whatever it was taken against.
-            // Both warps of a row see the same tops.
-            if (__any_sync(0xffffffffu, top > m + 8.f)) {
+            // Weights are taken against the maximum itself: the key that stands out weighs 1, which bf16 holds. (Against a maximum up to 2^8 behind it is rounded, though sums are
+            // rarely taken anew then: 2048 tokens, 16 heads of 128 over 4, 51 µs against 60, but 1.85e-3 from 64-bit results against 1.65e-3 where single keys stand out, 2.08e-3
+            // against 2.02e-3 where none do.) Both warps of a row see the same tops.
+            if (__any_sync(0xffffffffu, top > m)) {
                 const float keep = exp2f(m - top);
                 m = top;
                 l *= keep;

@@ -649,3 +649,31 @@ def test_routing_in_one_round_and_more(more, scores):
     m.check(m.rows(n))
     kernels = {kernel for kernel, _, _ in m.s.take_timings()}
     assert ("moe_route" in kernels) == (more == 0) and ("moe_route_pairs" in kernels) == (more > 0)
+
+
+@pytest.mark.parametrize("form,vdim", [("plain", 128), ("plain", 256), ("capped", 64), ("sink", 128), ("keys", 64)])
+def test_prompts_where_one_late_key_stands_out(form, vdim):
+    """A key of the second tile that weighs 2^7.4 of the first tile's only key, between two bf16 values. Taken against the maximum it weighs 1, and only the other key's share of
+    2^-7.4 is rounded, by 2^-8 of it and less: results differ from the rounded exact ones where these are that close to the middle of two bf16 values, 1 % of them. (Taken against
+    the first tile's maximum: off by 2.8e-3 of a value, with 3.9e-3 … 7.8e-3 between two values, so four in ten.)"""
+    r, T, heads, dim, late = np.random.default_rng(vdim), 128, 4, 64, 5.15625
+    v, place = to_bf16(r.standard_normal((T, 1, vdim))), np.arange(T)
+    if form == "keys":
+        bias = np.full((heads, T), -100.0, np.float32)
+        bias[:, 0], bias[:, 64] = late, 0.0
+        a = test_gpu_lovuzen.Attention("bf16", heads, 1, dim, bias, np.ones(heads * dim, np.float32), np.ones(dim, np.float32), scale=0.0)
+        score = np.repeat(bias[0][np.maximum(place[:, None] - place[None], 0)][None], heads, axis=0)
+        x = (to_bf16(r.standard_normal((T, heads, dim))), v)
+    else:
+        cap, shift = 600.0 if form == "capped" else 0.0, 5.0 if form == "sink" else 0.0
+        a = Attention("bf16", heads, 1, dim, vdim, scale=1.0, softcap=cap, norm=0, sink=int(form == "sink"))
+        q, k = np.zeros((T, heads, dim), np.float32), np.zeros((T, 1, dim), np.float32)
+        q[..., 0], k[:, 0, 0] = 1.0, -100.0
+        k[0, 0, 0], k[64, 0, 0] = -shift, late - shift
+        score, x = np.einsum("thd,jd->htj", q.astype(np.float64), k[:, 0].astype(np.float64)), (q, k, v)
+        if cap:
+            score = cap * np.tanh(score / cap)
+    w = np.where(place[None] <= place[:, None], np.exp(score), 0.0)
+    want = np.einsum("htj,jd->thd", w / (w.sum(-1, keepdims=True) + (form == "sink")), v[:, 0].astype(np.float64))[64:]
+    got = a.step([(0, *x)])[0][64:]
+    assert (got != to_bf16(want)).mean() < 0.05
