@@ -1436,6 +1436,28 @@ void emit_residual_norm(Emitter& em, const ResidualNormDesc& d, const TRef* low,
               "residual_norm", /*pdl=*/true);
 }
 
+// Pieces of k that sums are at least cut into. The tensor core adds without rounding to nearest: a chain of n products of 64 k is about n · 6.7e-8 off, and pieces are added in f32.
+// The pieces are what a step of 0.36 … 0.45 µs makes worth it. By the costs of emit_linear fewer would often be faster, but then f32 results are further from 64-bit ones (303 × 2560 ×
+// 2560: 2.7e-6 off in one chain, 6.0e-7 in five pieces; 512 × 21 504 × 5376 2.5e-5 and 7.9e-6), and bf16 results of long k a little (512 × 21 504 × 5376 1.66178e-3 and 1.66161e-3).
+static int least_pieces(long long rows, long long weight_tiles, long long steps, long long ldy) {
+    double best = 1e300;
+    int pieces = 1;
+    for (int nb : {32, 64, 128, 256}) {
+        if (nb > 32 && nb / 2 >= rows) break;
+        const long long slots = (long long)sm_count() * (nb <= 128 ? 2 : 1), tiles = weight_tiles * ((rows + nb - 1) / nb);
+        const double step = nb == 32 ? 0.36 : nb == 64 ? 0.38 : nb == 128 ? 0.42 : 0.45;
+        for (int sp = 1; sp <= (rows < 65536 ? 16 : 1) && sp * 2 <= std::max<long long>(steps, 2); sp++) {
+            double us = (double)((tiles * sp + slots - 1) / slots) * ((double)((steps + sp - 1) / sp) * step + (nb == 256 ? 10.0 : 7.0));
+            if (sp > 1) us += 3.0 + (double)(sp + 1) * rows * ldy * 4.0 / 3e6;
+            if (us < best * (sp > 1 ? 0.97 : 1.0)) {
+                best = us;
+                pieces = sp;
+            }
+        }
+    }
+    return pieces;
+}
+
 void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x1, const TRef& w0, const TRef* w1, const TRef* bias,
                  const TRef& y, const ResidualNormDesc* norm, const TRef* low) {
     if (d.rows == 0) return;
@@ -1577,10 +1599,11 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
         return;
     }
     // Which kernel, activation rows per tile and pieces along k: the choice with the smallest modelled time. A CTA alone on its SM has a step of 64 k in `one` µs,
-    // waves of two (up to 128 rows) in `two`; epilogues grow with the tile; where k is cut, the trip of the partial sums and a second launch are added. The
+    // waves of two (up to 128 rows) in `two`; epilogues grow with the tile; where k is cut, the trip of the partial sums and a second launch are added. No fewer pieces than least_pieces. The
     // constants are fitted to 560 launches of 45 sizes (64 … 4096 rows, k 16 … 10 240, 1152 … 32 768 weight rows): of one of them (200 × 2560 × 4096, 10 %) is the choice
     // more than 3 % behind the best form.
     const long long mt = (d.out + 127) / 128 * d.blocks, steps = (d.k[0] + 63) / 64 + (d.k[1] + 63) / 64;
+    const int least = least_pieces(d.rows, mt, steps, p.ldy);
     double best = 1e300;
     for (int nb : {32, 64, 128, 256}) {
         if (nb > 32 && nb / 2 >= d.rows) break;
@@ -1588,7 +1611,7 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
         const long long tiles = mt * ((d.rows + nb - 1) / nb);
         const double one = nb == 32 ? 0.19 : nb == 64 ? 0.21 : nb == 128 ? 0.24 : 0.35, two = nb == 32 ? 0.21 : nb == 64 ? 0.285 : nb == 128 ? 0.4 : 0.34;
         const double epilogue = 5.8 * nb / 256;
-        for (int sp = 1; sp <= (d.rows < 65536 ? 16 : 1) && sp * 2 <= std::max<long long>(steps, 2); sp++) {
+        for (int sp = least; sp <= (d.rows < 65536 ? 16 : 1) && sp * 2 <= std::max<long long>(steps, 2); sp++) {
             const long long waves = (tiles * sp + sm_count() * resident - 1) / (sm_count() * resident), piece = (steps + sp - 1) / sp;
             double us = 4.1 + (tiles * sp <= sm_count() ? piece * one + 0.9 + epilogue : waves * (piece * two + 0.9 + epilogue / 2) + epilogue / 2);
             if (sp > 1) us += 1.4 + (double)(sp + 1) * d.rows * p.ldy * 4.0 / 5.6e6;
@@ -1599,10 +1622,10 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
             }
         }
     }
-    // Pairs of CTAs: a step is bound by the bytes that come to an SM, 128 weight rows and half a tile's activation rows. Any multiple of 16 rows, so that the last round
+    // Pairs of CTAs, which do not cut k: a step is bound by the bytes that come to an SM, 128 weight rows and half a tile's activation rows. Any multiple of 16 rows, so that the last round
     // of tiles is as full as the others.
     bool pair = false;
-    for (int nb = 256; nb >= 64 && !blocks; nb -= 16) {
+    for (int nb = 256; nb >= 64 && !blocks && least == 1; nb -= 16) {
         const double rounds = std::ceil((double)((d.rows + nb - 1) / nb * ((d.out + 255) / 256)) / (sm_count() / 2)), us = pair_us(rounds, steps, nb);
         if (us < best) {
             best = us;

@@ -677,3 +677,25 @@ def test_prompts_where_one_late_key_stands_out(form, vdim):
     want = np.einsum("htj,jd->thd", w / (w.sum(-1, keepdims=True) + (form == "sink")), v[:, 0].astype(np.float64))[64:]
     got = a.step([(0, *x)])[0][64:]
     assert (got != to_bf16(want)).mean() < 0.05
+
+
+@pytest.mark.parametrize("rows,k,n", [(303, 2560, 2560), (200, 2560, 4160), (2048, 6912, 1152)])
+def test_results_of_cut_chains(rows, k, n):
+    """A chain of tensor-core sums is 6.7e-8 off per 64 k; cut into two pieces and more, half of that and less."""
+    r = np.random.default_rng(rows)
+    x, w = to_bf16(r.standard_normal((rows, k), dtype=np.float32)), to_bf16(r.standard_normal((n, k), dtype=np.float32) / np.sqrt(k))
+    want = x.astype(np.float64) @ w.T.astype(np.float64)
+    assert rel_err(run_linear(ir.BF16, x, w).astype(np.float64), want) < 0.6 * 6.7e-8 * k / 64
+    assert rel_err(run_linear(ir.BF16, x, w, out_dtype=ir.BF16).astype(np.float64), want) < 2.0 ** -9
+
+
+@pytest.mark.parametrize("rows,k,n", [(1046, 5376, 514), (300, 21504, 270)])
+def test_pairs_of_ctas_sum_as_single_ones_do(rows, k, n, monkeypatch):
+    """Long chains as f32 results: the bits of linear_tc whose k is not cut, whatever the tile."""
+    r, got = np.random.default_rng(rows), []
+    x, w = to_bf16(r.standard_normal((rows, k), dtype=np.float32)), to_bf16(r.standard_normal((n, k), dtype=np.float32) / np.sqrt(k))
+    for tile in ("128,1", "256,0", "240,0", "96,0"):
+        monkeypatch.setenv("ONYXIA_LINEAR_TILE", tile)
+        got.append(run_linear(ir.BF16, x, w))
+    assert all(np.array_equal(got[0], g) for g in got[1:])
+    assert rel_err(got[0].astype(np.float64), x.astype(np.float64) @ w.T.astype(np.float64)) < 2 * 6.7e-8 * k / 64
