@@ -92,9 +92,10 @@ template <typename T> __global__ void __launch_bounds__(128) paged_prepare(const
 }
 
 // ───────────────────────────── any shape ────────────────────────────────
-// One CTA per (row, head); key chunks of 128, two threads per key, a thread per value dimension. Loads one behind the
-// other are what it takes: with 128 threads, a whole key and two dimensions each, 34 launches over 3 sequences of 100 tokens, 4 heads of 256, took 36.5 µs each, now 19.7.
-template <typename T> __global__ void __launch_bounds__(kAnyThreads) paged_attn_simt(const PagedP p) {
+// One CTA per (row, head); key chunks of 128, PER threads per key (any_threads_per_key), a thread per value dimension where there are as many. Loads one behind the
+// other are what it takes.
+template <typename T, int PER> __global__ void __launch_bounds__(kAnyKeys * PER) paged_attn_simt(const PagedP p) {
+    constexpr int kThreads = kAnyKeys * PER;
     extern __shared__ float sm[];  // q[dim], acc[dim], w[128]
     __shared__ float red[32];
     pdl_enter();
@@ -103,32 +104,37 @@ template <typename T> __global__ void __launch_bounds__(kAnyThreads) paged_attn_
     if (row >= sq.start + sq.len) return;
     const int pos = sq.past + row - sq.start, g = h / (p.heads / p.kv_heads);
     float *q = sm, *acc = sm + p.dim, *w = acc + p.dim;
-    for (int i = tid; i < p.dim; i += kAnyThreads) {
+    for (int i = tid; i < p.dim; i += kThreads) {
         q[i] = to_f(((const T*)p.q)[((long long)row * p.heads + h) * p.dim + i]);
         acc[i] = 0.f;
     }
     float m = -INFINITY, l = 0.f;
     __syncthreads();
     for (int j0 = 0; j0 <= pos; j0 += 128) {
-        const int j = j0 + (tid >> 1), half = tid & 1;
-        float sc = -INFINITY;
-        const long long pg = j <= pos ? page_of(p, s, j) : 0;
-        float d = j <= pos ? dot_of_half(q, (const T*)p.pool + key_row(p, pg, g, j) * p.dim, p.dim, half) : 0.f;
-        d += __shfl_xor_sync(0xffffffffu, d, 1);
+        const int j = j0 + tid / PER;
+        const bool first = tid % PER == 0;
+        float sc = -INFINITY, d = 0.f;
+        long long pg = 0;
+        if (j <= pos) {
+            pg = page_of(p, s, j);
+            const T* k = (const T*)p.pool + key_row(p, pg, g, j) * p.dim;
+            d = PER == 2 ? dot_of_half(q, k, p.dim, tid & 1) : dot_in_order(q, k, p.dim, 0.f);
+        }
+        if (PER == 2) d += __shfl_xor_sync(0xffffffffu, d, 1);
         if (j <= pos) {
             sc = d * p.kscale[scale_at(p, pg, j)];
             if (p.bias) sc += p.bias[(long long)h * p.nd + min(pos - j, p.nd - 1)];
         }
         const float m2 = fmaxf(m, block_max(sc, red));
         const float e = expf(sc - m2), keep = expf(m - m2);
-        if (half == 0) w[tid >> 1] = e;
-        l = l * keep + block_sum(half == 0 ? e : 0.f, red);  // (its barriers order the stores to w)
+        if (first) w[tid / PER] = e;
+        l = l * keep + block_sum(first ? e : 0.f, red);  // (its barriers order the stores to w)
         m = m2;
         const int live = min(128, pos + 1 - j0);
-        for (int i = tid; i < p.dim; i += kAnyThreads) acc[i] = weigh_in_order(p, (const T*)p.pool, s, g, j0, live, p.dim, i, w, acc[i] * keep);
+        for (int i = tid; i < p.dim; i += kThreads) acc[i] = weigh_in_order<8 * PER>(p, (const T*)p.pool, s, g, j0, live, p.dim, i, w, acc[i] * keep);
         __syncthreads();
     }
-    for (int i = tid; i < p.dim; i += kAnyThreads) ((T*)p.out)[((long long)row * p.heads + h) * p.dim + i] = from_f<T>(acc[i] / l * p.out_scale);
+    for (int i = tid; i < p.dim; i += kThreads) ((T*)p.out)[((long long)row * p.heads + h) * p.dim + i] = from_f<T>(acc[i] / l * p.out_scale);
 }
 
 // ───────────────────────────── prefill ──────────────────────────────────
@@ -656,9 +662,10 @@ void emit_paged_attention(Emitter& em, const PagedAttnDesc& d, const TRef& proj,
     if (!decode_only) launch(bf ? paged_prepare<bf16> : paged_prepare<float>, dim3((unsigned)rows), 128, 0, none, "paged_prepare");
     if (!tc) {
         const unsigned smem = (unsigned)((2 * d.dim + 128) * 4);
-        const PagedKernel k = bf ? paged_attn_simt<bf16> : paged_attn_simt<float>;
+        const int per = any_threads_per_key(d.dim);
+        const PagedKernel k = bf ? (per == 2 ? paged_attn_simt<bf16, 2> : paged_attn_simt<bf16, 1>) : per == 2 ? paged_attn_simt<float, 2> : paged_attn_simt<float, 1>;
         ensure_max_dynamic_smem((const void*)k, 220 * 1024);
-        launch(k, dim3((unsigned)rows, (unsigned)d.heads), kAnyThreads, smem, none, "paged_attn_simt");
+        launch(k, dim3((unsigned)rows, (unsigned)d.heads), (unsigned)(kAnyKeys * per), smem, none, "paged_attn_simt");
         return;
     }
     if (!decode_only) {

@@ -98,8 +98,9 @@ __global__ void __launch_bounds__(kTurnThreads) paged_kv_turn(const KvP p) {
 }
 
 // ───────────────────────────── any shape ────────────────────────────────
-// One CTA per (row, head); key chunks of 128, two threads per key, a thread per value dimension.
-template <typename T> __global__ void __launch_bounds__(kAnyThreads) paged_kv_simt(const KvP p) {
+// One CTA per (row, head); key chunks of 128, PER threads per key (any_threads_per_key).
+template <typename T, int PER> __global__ void __launch_bounds__(kAnyKeys * PER) paged_kv_simt(const KvP p) {
+    constexpr int kThreads = kAnyKeys * PER;
     extern __shared__ float sm[];  // q[dim], acc[vdim], w[128]
     __shared__ float red[32];
     pdl_enter();
@@ -108,30 +109,36 @@ template <typename T> __global__ void __launch_bounds__(kAnyThreads) paged_kv_si
     if (row >= sq.start + sq.len) return;
     const int pos = sq.past + row - sq.start, g = h / (p.heads / p.kv_heads);
     float *q = sm, *acc = sm + p.dim, *w = acc + p.vdim;
-    for (int i = tid; i < p.dim; i += kAnyThreads) q[i] = to_f(((const T*)p.q)[((long long)row * p.heads + h) * p.dim + i]);
-    for (int i = tid; i < p.vdim; i += kAnyThreads) acc[i] = 0.f;
+    for (int i = tid; i < p.dim; i += kThreads) q[i] = to_f(((const T*)p.q)[((long long)row * p.heads + h) * p.dim + i]);
+    for (int i = tid; i < p.vdim; i += kThreads) acc[i] = 0.f;
     float m = p.sink ? sink_of(p, h) : kNoScore, l = p.sink ? 1.f : 0.f;
     __syncthreads();
     for (int j0 = first_key(p, pos); j0 <= pos; j0 += 128) {
-        const int j = j0 + (tid >> 1), half = tid & 1;
-        float sc = -INFINITY;
-        float d = j <= pos ? dot_of_half(q, (const T*)p.keys + key_row(p, page_of(p, s, j), g, j) * p.dim, p.dim, half) : 0.f;
-        d += __shfl_xor_sync(0xffffffffu, d, 1);
+        const int j = j0 + tid / PER;
+        const bool first = tid % PER == 0;
+        float sc = -INFINITY, d = 0.f;
+        long long pg = 0;
+        if (j <= pos) {
+            pg = page_of(p, s, j);
+            const T* k = (const T*)p.keys + key_row(p, pg, g, j) * p.dim;
+            d = PER == 2 ? dot_of_half(q, k, p.dim, tid & 1) : dot_in_order(q, k, p.dim, 0.f);
+        }
+        if (PER == 2) d += __shfl_xor_sync(0xffffffffu, d, 1);
         if (j <= pos) {
             sc = d * p.scale * temp_of(p, h);
             if (p.cap > 0.f) sc = p.cap * tanhf(sc / p.cap);
         }
         const float m2 = fmaxf(m, block_max(sc, red));
         const float e = expf(sc - m2), keep = expf(m - m2);
-        if (half == 0) w[tid >> 1] = e;
-        l = l * keep + block_sum(half == 0 ? e : 0.f, red);  // (its barriers order the stores to w)
+        if (first) w[tid / PER] = e;
+        l = l * keep + block_sum(first ? e : 0.f, red);  // (its barriers order the stores to w)
         m = m2;
         const int live = min(128, pos + 1 - j0);
-        for (int i = tid; i < p.vdim; i += kAnyThreads) acc[i] = weigh_in_order(p, (const T*)p.values, s, g, j0, live, p.ldv, i, w, acc[i] * keep);
+        for (int i = tid; i < p.vdim; i += kThreads) acc[i] = weigh_in_order<8 * PER>(p, (const T*)p.values, s, g, j0, live, p.ldv, i, w, acc[i] * keep);
         __syncthreads();
     }
     const float f = gate_of<T>(p, row, h) / l;
-    for (int i = tid; i < p.vdim; i += kAnyThreads) ((T*)p.out)[((long long)row * p.heads + h) * p.vdim + i] = from_f<T>(acc[i] * f);
+    for (int i = tid; i < p.vdim; i += kThreads) ((T*)p.out)[((long long)row * p.heads + h) * p.vdim + i] = from_f<T>(acc[i] * f);
 }
 
 // ───────────────────────────── prefill ──────────────────────────────────
@@ -648,9 +655,10 @@ void emit_paged_kv_attention(Emitter& em, const PagedKvDesc& d, const TRef& proj
         launch(bf ? paged_kv_prepare<bf16> : paged_kv_prepare<float>, dim3((unsigned)rows), 128, (unsigned)(d.rot_dims * 4), none, "paged_kv_prepare");
     if (d.talk) return emit_talking_heads(em, d, p, proj, turns, q, keys, values, seqs, pages, out);
     if (!tc) {
-        const KvKernel k = bf ? paged_kv_simt<bf16> : paged_kv_simt<float>;
+        const int per = any_threads_per_key(widest);
+        const KvKernel k = bf ? (per == 2 ? paged_kv_simt<bf16, 2> : paged_kv_simt<bf16, 1>) : per == 2 ? paged_kv_simt<float, 2> : paged_kv_simt<float, 1>;
         ensure_max_dynamic_smem((const void*)k, 220 * 1024);
-        launch(k, dim3((unsigned)rows, (unsigned)d.heads), kAnyThreads, (unsigned)((d.dim + d.vdim + 128) * 4), none, "paged_kv_simt");
+        launch(k, dim3((unsigned)rows, (unsigned)d.heads), (unsigned)(kAnyKeys * per), (unsigned)((d.dim + d.vdim + 128) * 4), none, "paged_kv_simt");
         return;
     }
     if (!decode_only) {

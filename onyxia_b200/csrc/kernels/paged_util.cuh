@@ -20,20 +20,24 @@ template <class P> __device__ __forceinline__ long long page_of(const P& p, int 
 template <class P> __device__ __forceinline__ long long key_row(const P& p, long long pg, int g, int pos) {
     return ((pg * p.kv_heads + g) << p.shift) + (pos & ((1 << p.shift) - 1));
 }
-// Threads of the kernels for any shape: two for each of 128 keys.
-constexpr int kAnyThreads = 256;
+// The kernels for any shape take 128 keys at a time with PER threads for each, one or two.
+constexpr int kAnyKeys = 128;
 // Half of a dot product: the first or the second n / 2 (a multiple of four) elements.
 template <typename T> __device__ __forceinline__ float dot_of_half(const float* x, const T* w, int n, int half) {
     const int cut = n / 2 & ~3;
     return half ? dot_in_order(x + cut, w + cut, n - cut, 0.f) : dot_in_order(x, w, cut, 0.f);
 }
-// a + Σ w[jj] · (element i of the rows of positions j0 + jj), one after the other; `ld` elements per row. Several loads of a page in flight.
-template <typename T, class P>
+// Threads per key: two where that leaves a thread fewer value dimensions as well. f32, 4 heads over one key head of their own keys and values, µs with one → two: 256 dimensions, one token
+// behind 700 271 → 163, 100 tokens behind 300 each 211 → 160, a prompt of 1000 1048 → 927. At 128 and fewer half of 256 threads have no value to add up: prompts of 1000 of 64
+// 356 → 457, of 8 heads of 96 690 → 928, 500 tokens behind 100 each of 64 49 → 74.
+inline int any_threads_per_key(int64_t widest) { return widest > kAnyKeys ? 2 : 1; }
+// a + Σ w[jj] · (element i of the rows of positions j0 + jj), one after the other; `ld` elements per row. LOADS of a page in flight.
+template <int LOADS = 8, typename T, class P>
 __device__ __forceinline__ float weigh_in_order(const P& p, const T* pool, int seq, int g, int j0, int live, long long ld, int i, const float* w, float a) {
     for (int jj = 0; jj < live;) {
         const int end = min(live, ((j0 + jj) | ((1 << p.shift) - 1)) + 1 - j0);
         const T* v = pool + key_row(p, page_of(p, seq, j0 + jj), g, j0 + jj) * ld + i;
-#pragma unroll 16
+#pragma unroll LOADS
         for (; jj < end; jj++, v += ld) a = fmaf(w[jj], to_f(*v), a);
     }
     return a;

@@ -699,3 +699,17 @@ def test_pairs_of_ctas_sum_as_single_ones_do(rows, k, n, monkeypatch):
         got.append(run_linear(ir.BF16, x, w))
     assert all(np.array_equal(got[0], g) for g in got[1:])
     assert rel_err(got[0].astype(np.float64), x.astype(np.float64) @ w.T.astype(np.float64)) < 2 * 6.7e-8 * k / 64
+
+
+@pytest.mark.parametrize("kind", ["f32", "bf16"])
+@pytest.mark.parametrize("dim,vdim", [(127, 10), (128, 128), (129, 7), (20, 129), (6, 130)])
+def test_any_shape_by_one_or_two_threads_per_key(kind, dim, vdim):
+    """Either side of a thread per value dimension, halves of a key that are no multiple of four, more than one chunk of 128 keys, prompts and single tokens."""
+    a = Attention(kind, 3, 1, dim, vdim, scale=1.0 / np.sqrt(dim), norm=0, sink=1)
+    x, got, at = a.random(200), [], 0
+    want = a.want(*x)
+    for n in (1, 126, 1, 1, 1, 70):
+        got.append(a.step([(0, *piece(x, at, at + n))])[0])
+        at += n
+    err = row_err(np.concatenate(got), want)
+    assert err.max() < (1e-5 if kind == "f32" else 1e-2), (int(err.argmax()), float(err.max()))
