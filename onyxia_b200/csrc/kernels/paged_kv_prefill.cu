@@ -350,9 +350,14 @@ static int prefill_smem(const KvP& kv, bool keys, bool lse) {
            (keys ? tiles * kKeys * 4 + kv.heads / kv.kv_heads * kv.nd * 4 : 0);
 }
 
+// Where no sequence has more keys than a tile there is nothing to overlap, and a tile of 128 rows is the emptier: the `mma.sync` kernel stays. µs of a step with it → here, keys and values:
+// one prompt of 33 tokens, 16 heads of 128 over 4, 19.7 → 22.6; 64 prompts of 32, 8 heads of 64 over 8, 32.8 → 38.4; 64 sequences of 60 with two tokens more, 32 heads of 128 over 16,
+// 40.7 → 49.6; keys that are the values, the same 52.0 → 64.8, prompts of 8, 8 heads of 64 over 8, 19.8 → 23.5. Up to twice a tile: 16 prompts of 128, 16 heads over 4, 49 → 38; one of 100, 4 heads of
+// 256, 26.2 → 25.2; keys that are the values, where heads share none, 16 prompts of 128, 8 heads of 64, 31.2 → 36.4, so there twice a tile is the line. Of 160 tokens and more every
+// form is faster here (16 heads of 128 over 4, 25.8 → 23.9; 260: 31.0 → 25.0).
 bool kv_prefill_fits(const KvP& kv, const TRef& keys, const TRef* values, int64_t out_off) {
-    const int64_t rows = (int64_t)kv.n_pages * kv.kv_heads << kv.shift;
-    return 1 << kv.shift >= kKeys && kv.dim % 8 == 0 && kv.dim <= 256 && kv.heads / kv.kv_heads <= kRows && rows < INT32_MAX && keys.buf.off % 16 == 0 &&
+    const int64_t rows = (int64_t)kv.n_pages * kv.kv_heads << kv.shift, longest = (int64_t)kv.width << kv.shift;
+    return longest > (values == &keys && kv.heads == kv.kv_heads ? 2 * kKeys : kKeys) && 1 << kv.shift >= kKeys && kv.dim % 8 == 0 && kv.dim <= 256 && kv.heads / kv.kv_heads <= kRows && rows < INT32_MAX && keys.buf.off % 16 == 0 &&
            (!values || (kv.vdim % 8 == 0 && kv.vdim <= 256 && values->buf.off % 16 == 0 && out_off % 16 == 0)) &&
            prefill_smem(kv, values == &keys, !values) <= 200 * 1024;
 }

@@ -713,3 +713,31 @@ def test_any_shape_by_one_or_two_threads_per_key(kind, dim, vdim):
         at += n
     err = row_err(np.concatenate(got), want)
     assert err.max() < (1e-5 if kind == "f32" else 1e-2), (int(err.argmax()), float(err.max()))
+
+
+@pytest.mark.parametrize("form,heads,kv,tokens,mma", [("values", 4, 1, 64, True), ("values", 4, 1, 65, False), ("values", 3, 3, 65, False), ("keys", 4, 1, 64, True), ("keys", 4, 1, 65, False),
+                                                      ("keys", 3, 3, 128, True), ("keys", 3, 3, 129, False), ("sums", 4, 2, 64, True), ("sums", 4, 2, 65, False)])
+def test_where_prompts_are_short(form, heads, kv, tokens, mma):
+    """Sequences of one page take the `mma.sync` kernel; heads that share no keys which are their values, of two."""
+    r, dim, scale, page = np.random.default_rng(tokens), 64, 0.25, 64
+    n = -(-tokens // page)
+    q, k, v = (to_bf16(r.standard_normal((tokens, g, dim))) for g in (heads, kv, kv))
+    turns, f64 = kipizen.turns_per_position(0, 100.0, 1.0), np.float64
+    attrs = {"heads": heads, "kv_heads": kv, "dim": dim, "scale": scale, "q_offset": 0, "k_offset": heads * dim, "epsilon": 1e-5}
+    values, pool = {"vdim": dim, "rot_dims": 0, "v_offset": (heads + kv) * dim}, (ir.BF16, [n, kv, page, dim])
+    rows = np.concatenate([x.reshape(tokens, -1) for x in ((q, k) if form == "keys" else (q, k, v))], axis=1)
+    if form == "keys":
+        one, bias = np.ones(heads * dim, np.float32), r.standard_normal((12, heads))
+        got, kernels = prompt_over_pages("onyxia.PagedAttention", dict(attrs, temp_coef=0.0, temp_every=0.0, out_scale=1.0), rows, [one, one[:kv * dim], lovuzen.distance_bias(bias, 40)],
+                                         [pool, (ir.F32, [n, page])], [], (heads, dim), (tokens,))
+        want, name = attention_want(q, k, bias, 40, one, one[:kv * dim], scale=scale), "paged_attn_prefill"
+    elif form == "values":
+        got, kernels = prompt_over_pages("onyxia.PagedKVAttention", dict(attrs, **values, window=0, softcap=0.0, norm=0, sink=0), rows, [turns], [pool, pool], [], (heads, dim), (tokens,))
+        want, name = kipizen_ref.attention(q.astype(f64), k.astype(f64), v.astype(f64), scale, sink=False), "paged_kv_prefill"
+    else:
+        temp, talk = to_bf16(r.uniform(0.5, 2, heads)), to_bf16(np.eye(heads) + 0.3 * r.standard_normal((heads, heads)))
+        got, kernels = prompt_over_pages("onyxia.PagedKVAttention", dict(attrs, **values, temps=1, talk=1), rows, [turns], [pool, pool], [temp, talk], (heads, dim), (tokens,))
+        want, name = ref.talking_attention(q.astype(f64), k.astype(f64), v.astype(f64), scale, temp.astype(f64), talk.astype(f64)), "talk_lse"
+    assert (name + "_mma" in kernels) == mma and (name in kernels) == (not mma)
+    err = row_err(got, want)
+    assert np.isfinite(err).all() and err.max() < 2e-2, (int(err.argmax()), float(err.max()))
