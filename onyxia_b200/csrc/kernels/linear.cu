@@ -1436,10 +1436,10 @@ void emit_residual_norm(Emitter& em, const ResidualNormDesc& d, const TRef* low,
               "residual_norm", /*pdl=*/true);
 }
 
-// Pieces of k that sums are at least cut into. The tensor core adds without rounding to nearest: a chain of n products of 64 k is about n · 6.7e-8 off, and pieces are added in f32.
-// The pieces are what a step of 0.36 … 0.45 µs makes worth it. By the costs of emit_linear fewer would often be faster, but then f32 results are further from 64-bit ones (303 × 2560 ×
-// 2560: 2.7e-6 off in one chain, 6.0e-7 in five pieces; 512 × 21 504 × 5376 2.5e-5 and 7.9e-6), and bf16 results of long k a little (512 × 21 504 × 5376 1.66178e-3 and 1.66161e-3).
-static int least_pieces(long long rows, long long weight_tiles, long long steps, long long ldy) {
+// Pieces of k that sums are cut into, whatever the kernel and the tile: results of a size have the same bits with all of them. The tensor core adds without rounding to nearest: a chain of
+// n products of 64 k is about n · 6.7e-8 off, and pieces are added in f32. They are as many as a step of 0.36 … 0.45 µs makes worth it. By the costs of emit_linear others would often be
+// faster, but fewer are further from 64-bit results (303 × 2560 × 2560 in f32: 2.7e-6 off in one chain, 6.0e-7 in five pieces; 512 × 21 504 × 5376 2.5e-5 and 7.9e-6).
+static int pieces_of_k(long long rows, long long weight_tiles, long long steps, long long ldy) {
     double best = 1e300;
     int pieces = 1;
     for (int nb : {32, 64, 128, 256}) {
@@ -1598,12 +1598,13 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
                   flow ? "linear_flow" : "linear_stream", /*pdl=*/true);
         return;
     }
-    // Which kernel, activation rows per tile and pieces along k: the choice with the smallest modelled time. A CTA alone on its SM has a step of 64 k in `one` µs,
-    // waves of two (up to 128 rows) in `two`; epilogues grow with the tile; where k is cut, the trip of the partial sums and a second launch are added. No fewer pieces than least_pieces. The
+    // Which kernel and activation rows per tile: the choice with the smallest modelled time. A CTA alone on its SM has a step of 64 k in `one` µs,
+    // waves of two (up to 128 rows) in `two`; epilogues grow with the tile. The
     // constants are fitted to 560 launches of 45 sizes (64 … 4096 rows, k 16 … 10 240, 1152 … 32 768 weight rows): of one of them (200 × 2560 × 4096, 10 %) is the choice
     // more than 3 % behind the best form.
     const long long mt = (d.out + 127) / 128 * d.blocks, steps = (d.k[0] + 63) / 64 + (d.k[1] + 63) / 64;
-    const int least = least_pieces(d.rows, mt, steps, p.ldy);
+    p.splits = pieces_of_k(d.rows, mt, steps, p.ldy);
+    const int sp = p.splits;
     double best = 1e300;
     for (int nb : {32, 64, 128, 256}) {
         if (nb > 32 && nb / 2 >= d.rows) break;
@@ -1611,27 +1612,22 @@ void emit_linear(Emitter& em, const LinearDesc& d, const TRef* x0, const TRef* x
         const long long tiles = mt * ((d.rows + nb - 1) / nb);
         const double one = nb == 32 ? 0.19 : nb == 64 ? 0.21 : nb == 128 ? 0.24 : 0.35, two = nb == 32 ? 0.21 : nb == 64 ? 0.285 : nb == 128 ? 0.4 : 0.34;
         const double epilogue = 5.8 * nb / 256;
-        for (int sp = least; sp <= (d.rows < 65536 ? 16 : 1) && sp * 2 <= std::max<long long>(steps, 2); sp++) {
-            const long long waves = (tiles * sp + sm_count() * resident - 1) / (sm_count() * resident), piece = (steps + sp - 1) / sp;
-            double us = 4.1 + (tiles * sp <= sm_count() ? piece * one + 0.9 + epilogue : waves * (piece * two + 0.9 + epilogue / 2) + epilogue / 2);
-            if (sp > 1) us += 1.4 + (double)(sp + 1) * d.rows * p.ldy * 4.0 / 5.6e6;
-            if (us < best) {
-                best = us;
-                p.nb = nb;
-                p.splits = sp;
-            }
+        const long long waves = (tiles * sp + sm_count() * resident - 1) / (sm_count() * resident), piece = (steps + sp - 1) / sp;
+        const double us = 4.1 + (tiles * sp <= sm_count() ? piece * one + 0.9 + epilogue : waves * (piece * two + 0.9 + epilogue / 2) + epilogue / 2);
+        if (us < best) {
+            best = us;
+            p.nb = nb;
         }
     }
     // Pairs of CTAs, which do not cut k: a step is bound by the bytes that come to an SM, 128 weight rows and half a tile's activation rows. Any multiple of 16 rows, so that the last round
     // of tiles is as full as the others.
     bool pair = false;
-    for (int nb = 256; nb >= 64 && !blocks && least == 1; nb -= 16) {
+    for (int nb = 256; nb >= 64 && !blocks && sp == 1; nb -= 16) {
         const double rounds = std::ceil((double)((d.rows + nb - 1) / nb * ((d.out + 255) / 256)) / (sm_count() / 2)), us = pair_us(rounds, steps, nb);
         if (us < best) {
             best = us;
             pair = true;
             p.nb = nb;
-            p.splits = 1;
         }
     }
     if (const char* e = std::getenv("ONYXIA_LINEAR_TILE")) {  // diagnostics: "rows,pieces"; no pieces: pairs of CTAs
