@@ -431,16 +431,17 @@ __global__ void __launch_bounds__(kTopWarps * 32) moe_top(const MoeP p) {
 constexpr int kRouteRows = 16;
 template <int WARPS> __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) moe_route(const MoeP p) {
     constexpr int kBatch = 4, kEach = kRouteRows / WARPS;  // tokens of a warp
+    constexpr int kAlong = 8, kTiles = WARPS == 8 ? 2 : 1;  // warps along k, and tiles of eight tokens of each: sums have one order in both forms
     extern __shared__ __align__(16) unsigned char smem[];  // count[experts], base[experts], z[rows][ld] [, the same once more]
-    __shared__ float red[WARPS][16][kRouteRows + 1];
+    __shared__ float red[kAlong][16][kRouteRows + 1];
     pdl_trigger();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, E = p.experts, L = p.ld;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, E = p.experts, L = p.ld, along = warp % kAlong, tile0 = warp / kAlong;
     int *count = reinterpret_cast<int*>(smem), *base = count + E;
     float* z = reinterpret_cast<float*>(base + E);
     const long long row0 = (long long)blockIdx.x * kRouteRows, K = p.width;
-    const int chunks = (int)((K + 31) / 32), per_tile = (chunks + WARPS * kBatch - 1) / (WARPS * kBatch), total = (L + 15) / 16 * per_tile;
+    const int chunks = (int)((K + 31) / 32), per_tile = (chunks + kAlong * kBatch - 1) / (kAlong * kBatch), total = (L + 15) / 16 * per_tile;
     const bf16* W = (const bf16*)p.router;
-    auto k_of = [&](int it, int j) { return (long long)(((it % per_tile) * kBatch + j) * WARPS + warp) * 32 + t * 8; };
+    auto k_of = [&](int it, int j) { return (long long)(((it % per_tile) * kBatch + j) * kAlong + along) * 32 + t * 8; };
     uint4 wl[kBatch], wh[kBatch];
     auto fetch = [&](int it) {
 #pragma unroll
@@ -455,23 +456,23 @@ template <int WARPS> __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) m
     fetch(0);  // constants: may overlap the launches before this one
     for (int i = tid; i < E; i += WARPS * 32) count[i] = 0;
     pdl_wait();
-    float acc[2][4];
+    float acc[kTiles][4];
     for (int it = 0; it < total; it++) {
         if (it % per_tile == 0) {
 #pragma unroll
-            for (int n = 0; n < 2; n++)
+            for (int n = 0; n < kTiles; n++)
 #pragma unroll
                 for (int e = 0; e < 4; e++) acc[n][e] = 0.f;
         }
-        uint4 a[kBatch], b[kBatch], xv[kBatch][2];
+        uint4 a[kBatch], b[kBatch], xv[kBatch][kTiles];
 #pragma unroll
         for (int j = 0; j < kBatch; j++) {
             a[j] = wl[j];
             b[j] = wh[j];
             const long long k = k_of(it, j);
 #pragma unroll
-            for (int n = 0; n < 2; n++) {
-                const long long row = row0 + n * 8 + g;
+            for (int n = 0; n < kTiles; n++) {
+                const long long row = row0 + (tile0 + n) * 8 + g;
                 xv[j][n] = k < K && row < p.rows ? *reinterpret_cast<const uint4*>((const bf16*)p.h + row * K + k) : make_uint4(0, 0, 0, 0);
             }
         }
@@ -479,24 +480,24 @@ template <int WARPS> __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) m
 #pragma unroll
         for (int j = 0; j < kBatch; j++)
 #pragma unroll
-            for (int n = 0; n < 2; n++) {
+            for (int n = 0; n < kTiles; n++) {
                 mma_bf16(acc[n], a[j].x, b[j].x, a[j].y, b[j].y, xv[j][n].x, xv[j][n].y);
                 mma_bf16(acc[n], a[j].z, b[j].z, a[j].w, b[j].w, xv[j][n].z, xv[j][n].w);
             }
         if (it % per_tile != per_tile - 1) continue;
 #pragma unroll
-        for (int n = 0; n < 2; n++) {
-            red[warp][g][n * 8 + t * 2] = acc[n][0];
-            red[warp][g][n * 8 + t * 2 + 1] = acc[n][1];
-            red[warp][g + 8][n * 8 + t * 2] = acc[n][2];
-            red[warp][g + 8][n * 8 + t * 2 + 1] = acc[n][3];
+        for (int n = 0; n < kTiles; n++) {
+            red[along][g][(tile0 + n) * 8 + t * 2] = acc[n][0];
+            red[along][g][(tile0 + n) * 8 + t * 2 + 1] = acc[n][1];
+            red[along][g + 8][(tile0 + n) * 8 + t * 2] = acc[n][2];
+            red[along][g + 8][(tile0 + n) * 8 + t * 2 + 1] = acc[n][3];
         }
         __syncthreads();
         const int o = it / per_tile * 16 + (tid & 15), m = tid >> 4;
         if (o < L && m < kRouteRows) {
             float s = 0.f;
 #pragma unroll
-            for (int w = 0; w < WARPS; w++) s += red[w][tid & 15][m];
+            for (int w = 0; w < kAlong; w++) s += red[w][tid & 15][m];
             z[m * L + o] = s + p.router_bias[o];
             if (p.scores != MOE_CHOSEN) z[(kRouteRows + m) * L + o] = s + p.router_bias[o];
         }
