@@ -5,8 +5,8 @@
 // values come by TMA, a page's rows are the rows of a tensor map; two of either are on their way.
 //
 // What bounds it is the chain of a step, about 1.3 µs in a CTA alone on its SM (256 dimensions: shared memory), of which the products are 0.7, and the sums' way through registers
-// in steps that bring a new maximum; a short prompt's longest tiles are as long as the launch. The `mma.sync` kernel, which remains for pages of less than 64 keys, had four warps per
-// SM at this size. µs, with it → here: 4096 tokens, 4 heads of 256 over one key head, capped 258 → 127; 1999 tokens, the same 133 → 70; 2048 tokens, 16 heads of 128 over 4,
+// in steps that bring a new maximum; a short prompt's longest tiles are as long as the launch. The `mma.sync` kernel, which remains for small pages and short sequences (kv_prefill_fits), has four warps per
+// SM at this size. µs, with it → here: 4096 tokens, 4 heads of 256 over one key head, capped 258 → 125; 1999 tokens, the same 133 → 69; 2048 tokens, 16 heads of 128 over 4,
 // 130 → 60, the softmax's sums alone 92 → 41; keys that are the values, 32 heads of 128 over 16, four portions of 2048 tokens 2830 → 1083. Errors against 64-bit results are the same to
 // four digits (scores of either spread, capped or not; 700 and 1999 tokens).
 #include "paged_kv.cuh"
@@ -47,6 +47,9 @@ __device__ __forceinline__ void tmem_ld32(unsigned (&v)[32], unsigned from) {
           "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]),
           "=r"(v[30]), "=r"(v[31])
         : "r"(from));
+}
+__device__ __forceinline__ void tmem_ld4(unsigned* v, unsigned from) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(from));
 }
 __device__ __forceinline__ void tmem_ld16(unsigned (&v)[16], unsigned from) {
     asm volatile(
@@ -209,10 +212,12 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
             return at[(part ^ 1) * kRows];
         };
         const float* bias = bias_s + r % rep * p.nd;
-        float m = KEYS ? -INFINITY : kNoScore, l = 0.f;  // KEYS: key 0 is there for every row
+        float m = KEYS ? -INFINITY : kNoScore, l = 0.f, l2 = 0.f;  // KEYS: key 0 is there for every row
         RingAt at, tile;
         for (int i = 0; i < n; i++) {
             const int j0 = (kt0 + i) * kKeys, mine0 = j0 + part * kHalf;
+            // Key e of this thread's half. LSE: four of every eight, so that the sums have the order of paged_kv_prefill's: of each two neighbouring keys of eight one after the other, the four sums in the end.
+            auto key = [&](int e) { return LSE ? j0 + e / 4 * 8 + part * 4 + e % 4 : mine0 + e; };
             if (ok && !mbar_wait(s_full + at.s * 8, at.parity)) ok = false;
             if constexpr (KEYS)  // the factors
                 if (ok && !mbar_wait(k_full + tile.s * 8, tile.parity)) ok = false;
@@ -220,7 +225,12 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
             float s[kHalf];
             {
                 unsigned v[32];
-                tmem_ld32(v, tmem + lanes + at.s * kKeys + part * kHalf);
+                if constexpr (LSE) {
+#pragma unroll
+                    for (int n = 0; n < kHalf; n += 4) tmem_ld4(v + n, tmem + lanes + at.s * kKeys + n * 2 + part * 4);
+                } else {
+                    tmem_ld32(v, tmem + lanes + at.s * kKeys + part * kHalf);
+                }
                 tmem_ld_wait();
                 if constexpr (KEYS) {
                     const float* f = scale_s + tile.s * kKeys + part * kHalf;
@@ -245,7 +255,7 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
             if (j0 + kKeys - 1 > pos0 || j0 < last_low) {
 #pragma unroll
                 for (int e = 0; e < kHalf; e++)
-                    if (mine0 + e > pos || mine0 + e < low) s[e] = -INFINITY;
+                    if (key(e) > pos || key(e) < low) s[e] = -INFINITY;
             }
             float top = m;
 #pragma unroll
@@ -258,6 +268,7 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
                 const float keep = exp2f(m - top);
                 m = top;
                 l *= keep;
+                l2 *= keep;
                 if (!LSE && i > 0) {
                     if (ok && !added(i - 1)) ok = false;
                     after_sync();
@@ -276,7 +287,8 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
 #pragma unroll
             for (int e = 0; e < kHalf / 2; e++) {
                 const float a = exp2f(s[2 * e] - m), b = exp2f(s[2 * e + 1] - m);
-                l += a + b;
+                if constexpr (LSE) (e & 1 ? l2 : l) = (e & 1 ? l2 : l) + a + b;
+                else l += a + b;
                 w[e] = pack_bf16(a, b);
             }
             if constexpr (!LSE) {
@@ -300,6 +312,7 @@ template <int FORM, bool LSE> __global__ void __launch_bounds__(kThreads, 2) pag
             tile.next(NS);
             at.next(2);
         }
+        if (LSE) l += l2;
         l += both(n & 1, l);
         const long long token = sq.start + first + tok;
         if constexpr (LSE) {
