@@ -5,9 +5,9 @@
 // products take. Persistent pairs, one per two SMs; a warp copies weights, one activations, one issues the products of both CTAs, eight empty one
 // of two accumulators under the products of the next tile. A tile may have any multiple of 16 rows, so that rounds of tiles are even (emit_linear chooses).
 //
-// linear_tc before its loops lost their divisions → pairs, back to back, µs (TFLOP/s): 2048 × 5376 × 16 896 327 → 248 (1500), 2048 × 5376 × 43 008 gated 868 → 608 (1557),
-// 2048 × 21 504 × 5376 468 → 344 (1376), 2048 × 2560 × 20 480 gated 194 → 148, 2048 × 2560 × 2560 41.7 → 25.9, 4096 × 1152 × 4608 45 → 33, 1999 × 1152 × 13 824 gated
-// 70 → 52, 1046 × 2560 × 4160 40.6 → 26.5; 16 groups of 1024 rows, 2560 → 4096 gated: 361 → 240 behind a linear_tc with the new loops. A large tile's steps take 700
+// linear_tc at its best tile, k uncut → pairs, back to back with weights from memory, µs (TFLOP/s): 2048 × 5376 × 16 896 272 → 251 (1482), 2048 × 5376 × 43 008 gated 651 → 617
+// (1536), 2048 × 21 504 × 5376 394 → 334 (1419), 2048 × 2560 × 20 480 gated 178 → 148 (1455), 2048 × 2560 × 2560 39 → 29 (929), 4096 × 1152 × 4608 44 → 34, 1999 × 1152 × 13 824
+// gated 68 → 51, 1046 × 2560 × 4160 33 → 28; 16 groups of 1024 rows, 2560 → 4096 gated: 361 → 240. A large tile's steps take 700
 // cycles of which products are 512 (the power limit at these rates); steps of 128 rows take 450, of 64 430: small tiles are bound by their weights' bytes.
 #include <type_traits>
 

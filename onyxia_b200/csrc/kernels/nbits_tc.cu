@@ -659,12 +659,13 @@ bool pieces_apart(const TcP& t, long long m, int count) {
     return t.splits > 1 && t.n_full == 0 && apart < joined;
 }
 
-// Whether the weights are widened once, for m rows whose launches of nbits_gemm_tc are `t`. Both sides as sums of what they do, fitted to 459 times of
-// either (51 sizes, k 512 … 21 504, 512 … 61 440 weight rows, 257 … 4096 activation rows: residuals 4 % and 6 %; two other sweeps, of grouped
-// products, 5 … 8 %; by the kernels of that time, of which both have lost 5 … 20 % since). With a tenth of margin nothing measured is slower than nbits_gemm_tc alone; 0.631 of its time in the geometric mean, 0.627 with
-// the better of the two at each size. nbits_gemm_tc → widened once, µs, at 257, 1024 and 4096 rows, in brackets what is not taken: k 1152, 13 824 weight
-// rows 48 → 39, 109 → 63, 431 → 194; k 2560, 20 480: 99 → (119), 217 → (196), 858 → 574; k 5376, 5376: 58 → (55), 126 → (114), 499 → 322; k 5376,
-// 43 008: 289 → (389), 620 → (795), 2469 → (2388); k 6912, 1152: 39 → 33, 82 → 58, 332 → 99; k 21 504, 5376: 148 → (270), 308 → (430), 1219 → (1282).
+// Whether the weights are widened once, for m rows whose launches of nbits_gemm_tc are `t`. Both sides as sums of what they do, fitted to 459 times of either by kernels that took 5 … 20 %
+// longer than these. Against 267 times of either by these (30 sizes, k 512 … 21 504, 1024 … 43 008 weight rows, 257 … 4096 activation rows), with a tenth of margin: what is taken is at
+// most 0.89 of nbits_gemm_tc; over all 0.600 of its time in the geometric mean, 0.588 with the better of the two at each size. What is not taken would be up to 28 % shorter, of large
+// products above all (k 4096, 22 016 weight rows, 3000 rows: 837 and 604 µs), the wide kernel having gained more. nbits_gemm_tc → widened once, µs, at 257, 1024 and 4096 rows, in
+// brackets what is not taken: k 1152, 13 824 weight rows 53 → 40, 112 → 62, 420 → 163; k 2560, 20 480: 99 → (111), 220 → (173), 836 → 468; k 5376, 5376: 61 → (61), 136 → (104),
+// 485 → 271; k 5376, 43 008 (2047 rows for 4096): 281 → (346), 591 → (643), 1170 → (1109); k 6912, 1152: 49 → 37, 86 → 52, 314 → 90; k 21 504, 5376: 146 → (241), 296 → (383),
+// 1147 → (1137).
 bool wide_pays(const TcP& t, long long m) {
     const long long slots = sm_count(), grid = (t.row_tiles + 7) / 8, tail = grid - t.n_full;
     const double out_mb = (double)m * t.row_tiles * 32.0 / 1e6;

@@ -6,8 +6,8 @@
 // and both products read the same tile: half the bytes of separate keys and values.
 //
 //   paged_prepare         query norm, temperature and scale → q'; the new keys and r go to the pool
-//   paged_attn_prefill    sequences with several new tokens: on tcgen05 (paged_kv_prefill.cu) where a page holds 64 keys and more; here for
-//                         smaller pages: 64 (token, head) rows per CTA share each key tile; `mma.sync`, online softmax
+//   paged_attn_prefill    sequences with several new tokens: on tcgen05 (paged_kv_prefill.cu) where a page holds 64 keys and more and a
+//                         sequence several pages; here otherwise: 64 (token, head) rows per CTA share each key tile; `mma.sync`, online softmax
 //   paged_attn_decode     sequences with one new token, keys split over CTAs and warps, all of the above in one launch
 //   paged_attn_simt       f32, and shapes the tensor-core kernels do not take
 //

@@ -8,8 +8,8 @@
 // keeps the length of a vector: the mean square is taken in front of it. Angles are reduced in 64-bit turns.
 //
 //   paged_kv_prepare, paged_kv_turn   rotated, normed queries; the new keys and values go to the pools
-//   paged_kv_prefill   sequences with several new tokens: on tcgen05 (paged_kv_prefill.cu) where a page holds 64 keys and more; here for smaller
-//                      pages: 64 (token, head) rows per CTA share each tile of 64 keys, `mma.sync`. Online softmax, only the tiles that the window reaches
+//   paged_kv_prefill   sequences with several new tokens: on tcgen05 (paged_kv_prefill.cu) where a page holds 64 keys and more and a sequence several
+//                      pages; here otherwise: 64 (token, head) rows per CTA share each tile of 64 keys, `mma.sync`. Online softmax, only the tiles that the window reaches
 //   paged_kv_decode    sequences with one new token, the window's keys split over CTAs and warps, all of the above in one launch
 //   paged_kv_simt      f32, and shapes the tensor-core kernels do not take
 //
